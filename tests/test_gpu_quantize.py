@@ -43,6 +43,41 @@ def test_ragged_and_small(shape, gs, bits):
     _check(w, gs, bits)
 
 
+@pytest.mark.parametrize("shape,gs", [((1, 8), 8), ((5, 200), 128), ((4, 136), 64), ((9, 512), 256), ((3, 1040), 128), ((6, 48), 16), ((2, 24), 512)])
+@pytest.mark.parametrize("bits", [4, 8])
+def test_octets_of_columns(shape, gs, bits):
+    # rows that are a multiple of eight columns: row counts around the four rows of a thread, short last groups, values at the
+    # halves between two codes, zeros of both signs as extrema, a group without a finite value, values far from zero
+    w = H.make_weight(*shape, seed=4, std=1.0)
+    w[0, :8] = np.arange(8) / np.float16(2)
+    if shape[0] > 1:
+        w[1] = np.float16(-0.0)
+        w[1, 3] = 0.0
+        w[1, 5:8] = (0.5, 7.5, 1.5)
+    if shape[0] > 2:
+        w[2, :gs] = np.nan
+        w[2, -4] = np.inf
+    if shape[0] > 3:
+        w[3] = np.float16(1000.0) + np.arange(shape[1]) % 7
+    _check(w, gs, bits)
+    awq = H.make_awq(shape[1], 3)
+    _check(w, gs, bits, awq)
+    awq[2] = np.inf
+    _check(w, gs, bits, awq)
+
+
+def test_unaligned_rows_take_the_general_kernels():
+    # a view that starts inside a vector
+    from ironmill_b200 import ops
+    w = H.make_weight(6, 128, seed=8)
+    buf = torch.zeros(6 * 128 + 3, dtype=torch.float16, device="cuda")
+    view = buf[3:].view(6, 128)
+    view.copy_(torch.from_numpy(w))
+    packed, s, z = ops.quantize_affine(view, 128, 4)
+    codes, scales, zps = orc.quantize_groups(w, 128, 4)
+    assert (packed.cpu().numpy() == orc.pack_int4(codes)).all() and (s.cpu().numpy() == scales).all() and (z.cpu().numpy() == zps).all()
+
+
 def test_known_answer_on_gpu():
     # affine_quantize.rs:585-598 replayed through the CUDA path
     w = np.array([[-3, 0, 3, 6, 12]], dtype=np.float16)
