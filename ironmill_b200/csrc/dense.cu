@@ -11,6 +11,7 @@
 #include <algorithm>
 
 #include "stack.cuh"
+#include "tmap.cuh"
 #include "v2_device.cuh"
 
 namespace im {
@@ -541,25 +542,12 @@ TmapEncodeFn tmap_encode() {
     }();
     return fn;
 }
-// bf16 [rows, cols] with row stride ld (a multiple of 8): boxes of 64 columns x box_rows, zeros outside
-int bf16_tmap(const void *base, int rows, int cols, int ld, int box_rows, CUtensorMap *out) {
-    TmapEncodeFn enc = tmap_encode();
-    if (!enc) return fail(IM_ERR_CUDA, "cuTensorMapEncodeTiled is not available from this driver");
-    const cuuint64_t gdim[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
-    const cuuint64_t gstride[1] = {(cuuint64_t)ld * 2};
-    const cuuint32_t box[2] = {64u, (cuuint32_t)box_rows}, es[2] = {1u, 1u};
-    const CUresult r = enc(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void *>(base), gdim, gstride, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                           CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) return fail(IM_ERR_CUDA, "cuTensorMapEncodeTiled failed (%d) for bf16 [%d, %d] stride %d", (int)r, rows, cols, ld);
-    return IM_OK;
-}
-
 template <int TN>
 int gemm_launch(const Device *dev, DenseGemm p, const DenseWeight &w, const void *x, int ldx, int slices, cudaStream_t st) {
     alignas(64) CUtensorMap ta, tb;
-    int rc = bf16_tmap(w.w, w.N, w.K, w.ld, kDM, &ta);
+    int rc = tmap_2d(w.w, true, w.N, w.K, w.ld, kDM, &ta);
     if (rc != IM_OK) return rc;
-    rc = bf16_tmap(x, p.M, w.K, ldx, TN, &tb);
+    rc = tmap_2d(x, true, p.M, w.K, ldx, TN, &tb);
     if (rc != IM_OK) return rc;
     p.mtiles = (p.M + TN - 1) / TN;
     p.ntiles = (p.N + kDM - 1) / kDM;
@@ -605,6 +593,18 @@ int matvec_any(const Device *dev, const DenseWeight &w, const DenseSrc &src, con
 }
 
 }  // namespace
+
+int tmap_2d(const void *base, bool bf16, long long rows, long long cols, long long ld, int box_rows, CUtensorMap *out) {
+    TmapEncodeFn enc = tmap_encode();
+    if (!enc) return fail(IM_ERR_CUDA, "cuTensorMapEncodeTiled is not available from this driver");
+    const cuuint64_t gdim[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
+    const cuuint64_t gstride[1] = {(cuuint64_t)ld * 2};
+    const cuuint32_t box[2] = {64u, (cuuint32_t)box_rows}, es[2] = {1u, 1u};
+    const CUresult r = enc(out, bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void *>(base), gdim, gstride, box, es,
+                           CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) return fail(IM_ERR_CUDA, "cuTensorMapEncodeTiled failed (%d) for [%lld, %lld] stride %lld", (int)r, rows, cols, ld);
+    return IM_OK;
+}
 
 int dense_prepare(const Device *dev) {
     static DeviceOnce once;

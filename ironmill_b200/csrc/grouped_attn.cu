@@ -13,6 +13,7 @@
 
 #include <algorithm>
 
+#include "flash_tc.cuh"
 #include "stack.cuh"
 
 namespace im {
@@ -698,6 +699,8 @@ bool grouped_prefills(const GroupedShape &s) { return prefill_dv(s) > 0 && group
 int grouped_prepare(const Device *dev) {
     static DeviceOnce once;
     if (!once.first(dev->ordinal)) return IM_OK;
+    const int frc = flash_prepare(dev);
+    if (frc != IM_OK) return frc;
     const int mx = (int)kGroupedSmemMax;
 #define IM_SMEM(k) IM_CUDA_CHECK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, mx))
     IM_SMEM((grouped_decode_kernel<4, 1, true>)); IM_SMEM((grouped_decode_kernel<8, 1, true>)); IM_SMEM((grouped_decode_kernel<16, 1, true>));
@@ -715,6 +718,24 @@ size_t grouped_part_bytes(const Device *dev, const GroupedShape &s, int f32, int
 }
 int grouped_counters(const GroupedShape &s, int tokens) { return tokens * s.kv_heads * head_groups(s); }
 
+// The tcgen05 pass over the cached rows: keys of 128 or 192 columns and values of 128 (flash_takes); other sizes keep
+// grouped_prefill_kernel, whose rows are padded in shared memory.
+static FlashArgs grouped_flash_args(const Device *dev, const GroupedArgs &a) {
+    const GroupedShape &s = a.s;
+    FlashArgs f;
+    f.bf16 = true; f.two_terms = 1;
+    f.T = a.T; f.heads = s.heads; f.group = s.heads / s.kv_heads;
+    f.q.base = a.y; f.q.rows = a.T; f.q.ld = a.ldy; f.q.col0 = s.q_off; f.q.head_cols = s.dimP; f.q.blocks = s.dimP % 64 == 0 && s.vP == 128 ? s.dimP / 64 : 0;
+    f.k.base = a.kcache; f.k.rows = (long long)(a.host_slot + 1) * s.kv_heads * a.max_seq; f.k.ld = s.dimP; f.k.row0 = (long long)a.host_slot * s.kv_heads * a.max_seq;
+    f.k.head_rows = a.max_seq; f.k.blocks = s.dimP / 64;
+    f.v = f.k;
+    f.v.base = a.vcache; f.v.ld = s.vP; f.v.blocks = 2;
+    f.base_pos = a.host_pos; f.n_max = a.max_seq; f.chunk = s.chunk; f.scale = s.scale; f.sink = a.sink;
+    f.gate = static_cast<const __nv_bfloat16 *>(a.y) + s.g_off; f.ldg = a.ldy; f.gate_head = s.vP;
+    f.out = a.out; f.ldo = a.ldo; f.out_head = s.vP; f.err = dev->err_flag;
+    return f;
+}
+
 int grouped_attention_run(const Device *dev, const GroupedArgs &a, cudaStream_t st, int *launches) {
     const GroupedShape &s = a.s;
     const int M = a.nseq * a.T;
@@ -723,6 +744,8 @@ int grouped_attention_run(const Device *dev, const GroupedArgs &a, cudaStream_t 
         rc = rows_launch<__nv_bfloat16>(a, st);
         if (rc != IM_OK) return rc;
         *launches += 2;
+        rc = flash_run(grouped_flash_args(dev, a), st);
+        if (rc != IM_ERR_BOUNDS) return rc;
         const int dv = prefill_dv(s);
         return dv == 64 ? prefill_launch<64>(a, st) : dv == 128 ? prefill_launch<128>(a, st) : prefill_launch<256>(a, st);
     }

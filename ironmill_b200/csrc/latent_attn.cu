@@ -15,6 +15,7 @@
 
 #include <algorithm>
 
+#include "flash_tc.cuh"
 #include "stack.cuh"
 
 namespace im {
@@ -792,6 +793,8 @@ bool latent_expands(const LatentShape &s) { return prefill_dv(s) > 0 && latent_p
 int latent_prepare(const Device *dev) {
     static DeviceOnce once;
     if (!once.first(dev->ordinal)) return IM_OK;
+    const int rc = flash_prepare(dev);
+    if (rc != IM_OK) return rc;
     const int mx = (int)kLatentSmemMax;
 #define IM_SMEM(k) IM_CUDA_CHECK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, mx))
     IM_SMEM((latent_attn_kernel<2, 1>)); IM_SMEM((latent_attn_kernel<4, 1>)); IM_SMEM((latent_attn_kernel<8, 1>)); IM_SMEM((latent_attn_kernel<16, 1>));
@@ -811,6 +814,26 @@ size_t latent_part_bytes(const Device *dev, const LatentShape &s, int tokens, in
     size_t b = 0;
     for (int f32 = 0; f32 < 2; f32++) b = std::max(b, part_bytes_for(s, (size_t)tokens * s.heads, auto_splits(dev, s, f32, T, nseq, 1 << 30)));
     return b;
+}
+
+// The tcgen05 pass over expanded keys and values: head parts of whole 64-column blocks and values of 128 columns (flash_takes);
+// other sizes keep latent_prefill_kernel, whose rows are padded in shared memory. IM_ERR_BOUNDS from flash_run says which.
+static FlashArgs expanded_flash_args(const Device *dev, const LatentArgs &a, const __nv_bfloat16 *kv, int ldkv, int h0, int nh, int ctx) {
+    const LatentShape &s = a.s;
+    const bool whole = s.dimP % 64 == 0 && s.rotP % 64 == 0 && s.vP == 128;
+    FlashArgs f;
+    f.bf16 = true; f.two_terms = 1;
+    f.T = a.T; f.heads = nh; f.group = 1;
+    f.q.base = a.y; f.q.rows = a.T; f.q.ld = a.ldy; f.q.col0 = s.q_off + h0 * (s.dimP + s.rotP); f.q.head_cols = s.dimP + s.rotP;
+    f.q.blocks = whole ? (s.dimP + s.rotP) / 64 : 0;
+    f.k.base = kv; f.k.rows = ctx; f.k.ld = ldkv; f.k.head_cols = s.dimP + s.vP; f.k.blocks = s.dimP / 64;
+    f.k2.base = a.cache; f.k2.rows = (long long)(a.host_slot + 1) * a.max_seq; f.k2.ld = s.rowP; f.k2.row0 = (long long)a.host_slot * a.max_seq; f.k2.col0 = s.latP;
+    f.k2.blocks = s.rotP / 64;
+    f.v = f.k;
+    f.v.col0 = s.dimP; f.v.blocks = 2;
+    f.base_pos = a.host_pos; f.n_max = ctx; f.scale = s.scale; f.sink = a.sink ? a.sink + h0 : nullptr;
+    f.out = static_cast<__nv_bfloat16 *>(a.out) + (size_t)h0 * s.vP; f.ldo = a.ldo; f.out_head = s.vP; f.err = dev->err_flag;
+    return f;
 }
 
 int latent_attention_run(const Device *dev, const LatentArgs &a, cudaStream_t st, int *launches) {
@@ -837,6 +860,12 @@ int latent_attention_run(const Device *dev, const LatentArgs &a, cudaStream_t st
                 int rc = dense_project(dev, w, src, e, ctx, nullptr, st);
                 if (rc != IM_OK) return rc;
                 const __nv_bfloat16 *kv = static_cast<const __nv_bfloat16 *>(a.kv);
+                rc = flash_run(expanded_flash_args(dev, a, kv, ldkv, h0, nh, ctx), st);
+                if (rc != IM_ERR_BOUNDS) {
+                    if (rc != IM_OK) return rc;
+                    *launches += 2;
+                    continue;
+                }
                 rc = dv == 32 ? prefill_launch<32>(a, kv, ldkv, h0, nh, st) : dv == 64 ? prefill_launch<64>(a, kv, ldkv, h0, nh, st)
                      : dv == 128 ? prefill_launch<128>(a, kv, ldkv, h0, nh, st) : prefill_launch<256>(a, kv, ldkv, h0, nh, st);
                 if (rc != IM_OK) return rc;

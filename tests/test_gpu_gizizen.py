@@ -372,3 +372,15 @@ def test_trace_replay(tmp_path, dtype):
         if r:
             got = np.fromfile(f, dtype="<f4").reshape(len(r), -1)
             assert G.error(got, np.stack([want[k][p] for k, p in r])) < G.TOL[dtype]
+
+
+def test_long_wide_prompts():
+    """Head sizes of the tcgen05 prompt kernel over more than one block of 256 tokens."""
+    cfg = G.config([G.latent(heads=3, dim=128, rot_dim=64, vdim=128, kv_rank=96, ff=0)], width=136, vocab=90)
+    w = G.weights(cfg, 14)
+    toks = tokens(700, 90)
+    want = OracleGizizen(cfg, w).forward(toks)
+    e = engine(cfg, w, "bfloat16", max_seq_len=720)
+    assert G.error(e.prefill(toks)[None], want[-1:]) < G.TOL["bfloat16"]
+    e.reset()
+    assert G.error(e.prefill_all_logits(toks), want) < G.TOL["bfloat16"]

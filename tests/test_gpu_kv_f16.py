@@ -65,7 +65,7 @@ def test_prefill_is_causal_and_batched_sequences_use_their_own_positions(dev):
 @pytest.mark.parametrize("nh,nkv", [(4, 4), (4, 2), (8, 2), (8, 1)])
 @pytest.mark.parametrize("base,T", [(0, 16), (0, 130), (77, 50), (500, 300)])
 def test_prefill_tensor_core_pass_matches_the_oracle(dev, nh, nkv, base, T):
-    # chunks of 16 tokens and more of one sequence: the causal tensor-core pass (sdpa16_prefill_kernel); 1, 2, 4 and 8
+    # chunks of 16 tokens and more of one sequence: the causal tensor-core pass (flash_tc.cu); 1, 2, 4 and 8
     # query heads per KV head; cached prefixes of 0, 77 and 500 positions
     from ironmill_b200 import ops
     max_seq = base + T + 7
@@ -74,6 +74,46 @@ def test_prefill_tensor_core_pass_matches_the_oracle(dev, nh, nkv, base, T):
     out = ops.sdpa_f16(dev, torch.from_numpy(q).cuda(), torch.from_numpy(k).cuda(), torch.from_numpy(v).cuda(), 0.0884, nh, nkv, max_seq, base).cpu().numpy()
     ref = orc.sdpa_f16(q, k, v, 0.0884, nh, nkv, 128, max_seq, base)
     assert H.rel_err(out, ref) <= TOL, (nh, nkv, base, T)
+
+
+@pytest.mark.parametrize("base,T", [(0, 127), (0, 128), (1, 128), (0, 129), (127, 255), (128, 256), (3, 257), (0, 385), (1000, 600)])
+def test_prompt_pass_at_the_edges_of_its_tiles(dev, base, T):
+    # halves of 128 tokens, blocks of 256, tiles of 128 positions; the cache rows past the prompt and the query rows of other
+    # heads hold what nothing may read
+    from ironmill_b200 import ops
+    nh, nkv, max_seq = 4, 2, base + T + 130
+    k, v = _caches(nkv, max_seq, base + T)
+    q = H.rng_for("kv16-edge", T).standard_normal((T, nh, 128)).astype(np.float16)
+    ref = orc.sdpa_f16(q, k, v, 0.0884, nh, nkv, 128, max_seq, base)
+    k[:, base + T:] = np.nan
+    v[:, base + T:] = np.inf
+    out = ops.sdpa_f16(dev, torch.from_numpy(q).cuda(), torch.from_numpy(k).cuda(), torch.from_numpy(v).cuda(), 0.0884, nh, nkv, max_seq, base).cpu().numpy()
+    assert H.rel_err(out, ref) <= TOL, (base, T)
+
+
+def test_prompt_pass_keeps_a_poisoned_token_to_those_that_see_it(dev):
+    from ironmill_b200 import ops
+    nh, nkv, T, bad = 2, 1, 300, 200
+    k, v = _caches(nkv, T, 3)
+    q = H.rng_for("kv16-nan").standard_normal((T, nh, 128)).astype(np.float16)
+    ref = orc.sdpa_f16(q, k, v, 0.09, nh, nkv, 128, T, 0)
+    v[0, bad, 5] = np.inf
+    k[0, bad + 1] = np.nan
+    out = ops.sdpa_f16(dev, torch.from_numpy(q).cuda(), torch.from_numpy(k).cuda(), torch.from_numpy(v).cuda(), 0.09, nh, nkv, T, 0).cpu().numpy()
+    assert np.isfinite(out[:bad]).all() and H.rel_err(out[:bad], ref[:bad]) <= TOL
+    assert not np.isfinite(out[bad:, :, 5]).any()
+
+
+@pytest.mark.parametrize("scale", [-0.06, 0.0, 0.5])
+def test_prompt_pass_with_any_scale(dev, scale):
+    # large, negative and zero factors; weights that one position dominates
+    from ironmill_b200 import ops
+    nh, nkv, T = 2, 1, 200
+    k, v = _caches(nkv, T, 4)
+    q = (2 * H.rng_for("kv16-scale").standard_normal((T, nh, 128))).astype(np.float16)
+    ref = orc.sdpa_f16(q, k, v, scale, nh, nkv, 128, T, 0)
+    out = ops.sdpa_f16(dev, torch.from_numpy(q).cuda(), torch.from_numpy(k).cuda(), torch.from_numpy(v).cuda(), scale, nh, nkv, T, 0).cpu().numpy()
+    assert H.rel_err(out, ref) <= TOL
 
 
 def test_kv_scatter_writes_the_rows_of_the_new_tokens(dev):

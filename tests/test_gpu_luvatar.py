@@ -447,3 +447,16 @@ def test_trace_replay(tmp_path, dtype):
         if r:
             got = np.fromfile(f, dtype="<f4").reshape(len(r), -1)
             assert L.close(got, np.stack([want[k][p] for k, p in r]), dtype)
+
+
+@pytest.mark.parametrize("chunk", [0, 1, 100, 128, 300])
+def test_long_wide_prompts(chunk):
+    """Key and value sizes of the tcgen05 prompt kernel over more than one block of 256 tokens, chunks that end inside and at its tiles."""
+    cfg = L.config([L.attention(heads=4, kv_heads=2, dim=128, vdim=128, rot_dims=64, chunk=chunk, ff=0)], width=136, vocab=90)
+    w = L.weights(cfg, 14)
+    toks = tokens(700, 90)
+    want = OracleLuvatar(cfg, w).forward(toks)
+    e = engine(cfg, w, "bfloat16", max_seq_len=720)
+    assert L.error(e.prefill(toks)[None], want[-1:]) < L.TOL["bfloat16"]
+    e.reset()
+    assert L.error(e.prefill_all_logits(toks), want) < L.TOL["bfloat16"]
