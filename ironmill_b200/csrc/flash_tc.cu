@@ -198,7 +198,7 @@ __device__ __noinline__ void plain_row(const FlashParams &p, int h, int tok, int
     for (int i = 0; i < kFDV; i += 32) store32<BF16>(a, tok, h, i, o + i);
 }
 
-// grid (ceil(T / 256), heads). KB: 64-column blocks of a key; PN: positions of a tile; TERMS: 16-bit terms of a weight.
+// grid (heads, ceil(T / 256)). KB: 64-column blocks of a key; PN: positions of a tile; TERMS: 16-bit terms of a weight.
 template <bool BF16, int KB, int PN, int TERMS>
 __global__ void __launch_bounds__(kFThreads, 1)
     flash_tc_kernel(const __grid_constant__ FlashParams p, const __grid_constant__ CUtensorMap tq, const __grid_constant__ CUtensorMap tk, const __grid_constant__ CUtensorMap tk2,
@@ -214,7 +214,7 @@ __global__ void __launch_bounds__(kFThreads, 1)
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(ofull + 2);
     const FlashArgs &a = p.a;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int tb = gridDim.x - 1 - blockIdx.x, h = blockIdx.y, kvh = h / a.group;  // latest (longest) blocks first
+    const int tb = gridDim.y - 1 - blockIdx.y, h = blockIdx.x, kvh = h / a.group;  // every head's latest (longest) block first
     if (tid == 0) {
         for (int i = 0; i < ST; i++) {
             mbar_init(&kfull[i], 1);
@@ -463,7 +463,7 @@ int launch(const FlashArgs &a, cudaStream_t st) {
     p.a = a;
     p.scale2 = a.scale * 1.4426950408889634f;
     if (p.scale2 == 0.0f) p.scale2 = 1e-30f;  // every position alike, without 0 * inf at the hidden ones
-    IM_CUDA_CHECK(launch_k(flash_tc_kernel<BF16, KB, PN, TERMS>, dim3((a.T + 2 * kFM - 1) / (2 * kFM), a.heads), dim3(kFThreads), (size_t)FlashShape<KB, PN>::kSmem, st, p,
+    IM_CUDA_CHECK(launch_k(flash_tc_kernel<BF16, KB, PN, TERMS>, dim3(a.heads, (a.T + 2 * kFM - 1) / (2 * kFM)), dim3(kFThreads), (size_t)FlashShape<KB, PN>::kSmem, st, p,
                            tq, tk, tk2, tv));
     return IM_OK;
 }
@@ -475,7 +475,7 @@ bool flash_takes(const FlashArgs &a) {
         return reinterpret_cast<uintptr_t>(r.base) % 16 == 0 && r.ld % 8 == 0 && r.ld < (1ll << 31) && r.rows < (1ll << 31) && r.col0 % 8 == 0 && r.head_cols % 8 == 0;
     };
     const int kb = a.k.blocks + a.k2.blocks;
-    return a.T > 0 && a.heads > 0 && a.heads <= 65535 && a.group > 0 && a.heads % a.group == 0 && (kb == 2 || kb == 3) && a.q.blocks == kb && a.v.blocks == 2 && fits(a.q) &&
+    return a.T > 0 && a.T <= 65535 * 2 * kFM && a.heads > 0 && a.group > 0 && a.heads % a.group == 0 && (kb == 2 || kb == 3) && a.q.blocks == kb && a.v.blocks == 2 && fits(a.q) &&
            fits(a.k) && (!a.k2.blocks || fits(a.k2)) && fits(a.v) && reinterpret_cast<uintptr_t>(a.out) % 16 == 0 && a.ldo % 8 == 0 && a.out_head % 8 == 0 &&
            (!a.gate || (reinterpret_cast<uintptr_t>(a.gate) % 16 == 0 && a.ldg % 8 == 0 && a.gate_head % 8 == 0));
 }
