@@ -17,7 +17,7 @@ OBJ = os.path.join(HERE, "csrc", "_obj")
 LIB = os.path.join(HERE, "libironmill_cuda.so")
 # A library with one model family only: what a host that serves a single model has to compile.
 FAMILY_SOURCES = {
-    "stack": ("api.cu", "session.cu", "stack.cu", "dense.cu", "flash_tc.cu", "latent_attn.cu", "grouped_attn.cu",
+    "stack": ("api.cu", "session.cu", "stack.cu", "dense.cu", "gemm_pair.cu", "flash_tc.cu", "latent_attn.cu", "grouped_attn.cu",
               "linear_attn.cu", "linear_gated.cu"),
 }
 

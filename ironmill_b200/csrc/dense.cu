@@ -10,6 +10,8 @@
 
 #include <algorithm>
 
+#include "dense_epi.cuh"
+#include "gemm_pair.cuh"
 #include "stack.cuh"
 #include "tmap.cuh"
 #include "v2_device.cuh"
@@ -224,11 +226,10 @@ constexpr int kDM = 128, kDK = 64;  // weight rows and columns of a stage (one 1
 constexpr int kDEpi = 8;            // epilogue warps: warp w reads tensor-memory lanes 32 (w % 4) .., half w / 4 of the tokens
 constexpr int kDThreads = (kDEpi + 2) * 32;  // ... then one warp for the copies, one for tensor memory + MMA issue
 template <int TN>
-constexpr int dense_stages() { return TN >= 256 ? 4 : TN == 128 ? 3 : 4; }
+constexpr int dense_stages() { return TN == 128 ? 3 : 4; }
 template <int TN>
 constexpr int dense_gemm_smem() { return 1024 + dense_stages<TN>() * (kDM * 128 + TN * 128) + (2 * dense_stages<TN>() + 4) * 8 + 16; }
-template <int TN>
-constexpr int dense_ctas_per_sm() { return TN >= 256 ? 1 : 2; }
+constexpr int kDCtasPerSm = 2;
 
 __device__ __forceinline__ uint64_t dense_desc_sw128(uint32_t smem_addr) {
     // K-major, 128-byte swizzle: start >> 4, leading offset 1, stride offset 1024 B >> 4, version 1, layout 2 (see gemm_tc.cu)
@@ -261,15 +262,6 @@ __device__ __forceinline__ void dense_tma_2d(void *dst, const CUtensorMap *map, 
                  "r"(x), "r"(y), "r"(smem_u32(bar))
                  : "memory");
 }
-// bf16 epilogues: z sigmoid(z), and gelu_tanh(z) = z / (1 + exp(-2 u)), u = sqrt(2 / pi) (z + 0.044715 z^3); the error of the
-// fast exponential and quotient (about 1e-6) is far below the bf16 result's rounding
-__device__ __forceinline__ float silu_fast(float z) { return __fdividef(z, 1.0f + __expf(-z)); }
-__device__ __forceinline__ float pair_act_fast(float z, float up, bool silu) {
-    if (silu) return silu_fast(z) * up;
-    const float w = -1.5957691216057308f * z * fmaf(0.044715f * z, z, 1.0f);
-    return __fdividef(z * up, 1.0f + __expf(fminf(w, 80.0f)));
-}
-
 struct DenseGemm {
     int N, M, kblocks, kb_per;  // kblocks: 64-column blocks of K; kb_per: of one K slice
     int mtiles, ntiles, slices;
@@ -280,76 +272,19 @@ struct DenseGemm {
 
 // 16 tokens m .. m + 15 of row n (one per lane) of the f32 sums
 __device__ __forceinline__ void dense_store16(const DenseGemm &p, int z, int n, int n_warp, int m, const float (&v)[16]) {
-    typedef __nv_bfloat16 T;
-    const DenseEpi &e = p.epi;
-    const int lane = threadIdx.x & 31, left = p.M - m;
-    if (p.partial) {
-        if (n < p.N) {
-            float *dst = p.partial + ((size_t)z * p.M + m) * p.N + n;
-#pragma unroll
-            for (int i = 0; i < 16; i++)
-                if (i < left) dst[(size_t)i * p.N] = v[i];
-        }
-    } else if (e.kind == kEpiProj) {
-        if (n_warp + 31 >= e.pair0) {
-            // (gate, up) sit in neighbouring lanes: of two tokens, the even lane takes the first, the odd lane the second
-            // (pair0 is a multiple of eight: no pair straddles it)
-            T *act = static_cast<T *>(e.act) + (size_t)m * e.ldact + ((n - e.pair0) >> 1);
-            T *y = static_cast<T *>(e.y) + (size_t)m * e.ldy + n;
-            const bool odd = lane & 1, pair = n >= e.pair0;
-#pragma unroll
-            for (int i = 0; i < 16; i += 2) {
-                const float got = __shfl_xor_sync(0xffffffffu, odd ? v[i] : v[i + 1], 1);
-                if (pair) {
-                    const float r = odd ? pair_act_fast(got, v[i + 1], e.pair_silu) : pair_act_fast(v[i], got, e.pair_silu);
-                    if (n < p.N && i + odd < left) act[(size_t)(i + odd) * e.ldact] = from_f<T>(r);
-                } else {
-#pragma unroll
-                    for (int j = 0; j < 2; j++)
-                        if (i + j < left) {
-                            if (n >= e.f0) e.xf[(size_t)(m + i + j) * e.ldx + (n - e.f0)] = v[i + j];
-                            else y[(size_t)(i + j) * e.ldy] = from_f<T>(n < e.silu_end ? silu_fast(v[i + j]) : v[i + j]);
-                        }
-                }
-            }
-        } else {
-            T *y = static_cast<T *>(e.y) + (size_t)m * e.ldy + n;
-            const bool act = n < e.silu_end;
-            if (n < p.N && n >= e.f0) {
-                float *f = e.xf + (size_t)m * e.ldx + (n - e.f0);
-#pragma unroll
-                for (int i = 0; i < 16; i++)
-                    if (i < left) f[(size_t)i * e.ldx] = v[i];
-            } else if (n < p.N) {
-#pragma unroll
-                for (int i = 0; i < 16; i++)
-                    if (i < left) y[(size_t)i * e.ldy] = from_f<T>(act ? silu_fast(v[i]) : v[i]);
-            }
-        }
+    if (!p.partial) {
+        epi_store16<__nv_bfloat16>(p.epi, p.N, p.M, n, n_warp, m, v);
     } else if (n < p.N) {
-        float *x = e.xf + (size_t)m * e.ldx + n;
-        if (e.kind == kEpiResidual) {
-            float old[16];
+        float *dst = p.partial + ((size_t)z * p.M + m) * p.N + n;
 #pragma unroll
-            for (int i = 0; i < 16; i++) old[i] = i < left ? x[(size_t)i * e.ldx] : 0.0f;
-#pragma unroll
-            for (int i = 0; i < 16; i++)
-                if (i < left) x[(size_t)i * e.ldx] = old[i] + v[i];
-        } else {
-            const float b = e.bias ? e.bias[n] : 0.0f;
-#pragma unroll
-            for (int i = 0; i < 16; i++) {
-                float r = v[i] + b;
-                if (e.cap > 0.0f) r = e.cap * tanhf(r / e.cap);
-                if (i < left) x[(size_t)i * e.ldx] = r;
-            }
-        }
+        for (int i = 0; i < 16; i++)
+            if (i < p.M - m) dst[(size_t)i * p.N] = v[i];
     }
 }
 
 // D[128 weight rows x TN tokens] += W[128 x 64] X[TN x 64]^T per stage.
 template <int TN>
-__global__ void __launch_bounds__(kDThreads, dense_ctas_per_sm<TN>()) dense_gemm_tc_kernel(const DenseGemm p, const __grid_constant__ CUtensorMap ta,
+__global__ void __launch_bounds__(kDThreads, kDCtasPerSm) dense_gemm_tc_kernel(const DenseGemm p, const __grid_constant__ CUtensorMap ta,
                                                                                          const __grid_constant__ CUtensorMap tb) {
     constexpr int S = dense_stages<TN>();
     constexpr int kA = kDM * 128, kB = TN * 128, kCols = 2 * TN;
@@ -552,7 +487,7 @@ int gemm_launch(const Device *dev, DenseGemm p, const DenseWeight &w, const void
     p.mtiles = (p.M + TN - 1) / TN;
     p.ntiles = (p.N + kDM - 1) / kDM;
     p.slices = slices;
-    const int ctas = std::min(p.mtiles * p.ntiles * slices, dev->sm_count * dense_ctas_per_sm<TN>());
+    const int ctas = std::min(p.mtiles * p.ntiles * slices, dev->sm_count * kDCtasPerSm);
     IM_CUDA_CHECK(launch_k(dense_gemm_tc_kernel<TN>, dim3(ctas), dim3(kDThreads), (size_t)dense_gemm_smem<TN>(), st, p, ta, tb));
     if (p.partial) {
         const size_t n = (size_t)p.M * ((p.N + 1) / 2);
@@ -615,7 +550,7 @@ int dense_prepare(const Device *dev) {
     IM_SMEM((dense_matvec_kernel<__nv_bfloat16, 4>), mv); IM_SMEM((dense_matvec_kernel<__nv_bfloat16, 8>), mv);
     IM_SMEM((dense_matvec_kernel<float, 1>), mv); IM_SMEM((dense_matvec_kernel<float, 2>), mv);
     IM_SMEM((dense_matvec_kernel<float, 4>), mv); IM_SMEM((dense_matvec_kernel<float, 8>), mv);
-    IM_SMEM(dense_gemm_tc_kernel<256>, dense_gemm_smem<256>()); IM_SMEM(dense_gemm_tc_kernel<128>, dense_gemm_smem<128>());
+    IM_SMEM(dense_gemm_tc_kernel<128>, dense_gemm_smem<128>());
     IM_SMEM(dense_gemm_tc_kernel<64>, dense_gemm_smem<64>()); IM_SMEM(dense_gemm_tc_kernel<32>, dense_gemm_smem<32>());
 #undef IM_SMEM
     return IM_OK;
@@ -643,6 +578,7 @@ int dense_project(const Device *dev, const DenseWeight &w, const DenseSrc &src, 
         IM_CUDA_CHECK(launch_k(dense_gemm_f32_kernel, dim3((w.N + 63) / 64, (M + 63) / 64), dim3(256), 0, st, w, static_cast<const float *>(x), ldx, epi, M));
         return IM_OK;
     }
+    if (pair_gemm_takes(dev, w.N, M)) return pair_gemm_bf16(dev, w.w, w.ld, w.N, w.K, x, ldx, M, epi, st);
     DenseGemm p{};
     p.N = w.N; p.M = M; p.kblocks = (w.K + kDK - 1) / kDK; p.kb_per = p.kblocks; p.err = dev->err_flag; p.epi = epi;
     const int tiles = (w.N + kDM - 1) / kDM;
@@ -657,8 +593,6 @@ int dense_project(const Device *dev, const DenseWeight &w, const DenseSrc &src, 
             p.partial = dev->gemm_partial;
         }
     }
-    const long long ctas256 = (long long)tiles * ((M + 255) / 256);
-    if (M > 128 && ctas256 >= dev->sm_count) return gemm_launch<256>(dev, p, w, x, ldx, slices, st);
     if (M > 64) return gemm_launch<128>(dev, p, w, x, ldx, slices, st);
     if (M > 32) return gemm_launch<64>(dev, p, w, x, ldx, slices, st);
     return gemm_launch<32>(dev, p, w, x, ldx, slices, st);

@@ -24,6 +24,8 @@
 #include <algorithm>
 
 #include "common.cuh"
+#include "dequant.cuh"
+#include "gemm_pair.cuh"
 #include "v2_device.cuh"
 
 namespace im {
@@ -92,69 +94,17 @@ struct GemmParams {
     int gps;
 };
 
-// 8 nibbles of a word -> 8 fp16 values (q - z) * s in memory order.  c = 1024 + z, exact for integer z in
-// [-1024, 1023]: 0x6400 | q is the fp16 number 1024 + q, the subtraction is exact, the product is rounded once.
-__device__ __forceinline__ uint4 dequant8_fast(uint32_t w, __half2 c, __half2 s) {
-    constexpr uint32_t M = 0x000F000Fu, E = 0x64006400u;
-    uint32_t h04 = (w & M) | E, h15 = ((w >> 4) & M) | E, h26 = ((w >> 8) & M) | E, h37 = ((w >> 12) & M) | E;
-    __half2 v04 = __hmul2(__hsub2(*reinterpret_cast<__half2 *>(&h04), c), s);
-    __half2 v15 = __hmul2(__hsub2(*reinterpret_cast<__half2 *>(&h15), c), s);
-    __half2 v26 = __hmul2(__hsub2(*reinterpret_cast<__half2 *>(&h26), c), s);
-    __half2 v37 = __hmul2(__hsub2(*reinterpret_cast<__half2 *>(&h37), c), s);
-    const uint32_t a = *reinterpret_cast<uint32_t *>(&v04), b = *reinterpret_cast<uint32_t *>(&v15);
-    const uint32_t cc = *reinterpret_cast<uint32_t *>(&v26), d = *reinterpret_cast<uint32_t *>(&v37);
-    return make_uint4(__byte_perm(a, b, 0x5410), __byte_perm(cc, d, 0x5410), __byte_perm(a, b, 0x7632), __byte_perm(cc, d, 0x7632));
-}
-// 8-bit codes: the 8 bytes of two words -> 8 fp16 values (q - z) * s in memory order.  0x6400 | q is 1024 + q for q < 1024.
-__device__ __forceinline__ uint4 dequant8b_fast(uint32_t w0, uint32_t w1, __half2 c, __half2 s) {
-    uint32_t h[4] = {__byte_perm(w0, 0x64u, 0x4140), __byte_perm(w0, 0x64u, 0x4342), __byte_perm(w1, 0x64u, 0x4140), __byte_perm(w1, 0x64u, 0x4342)};
-    uint32_t o[4];
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-        const __half2 v = __hmul2(__hsub2(*reinterpret_cast<__half2 *>(&h[i]), c), s);
-        o[i] = *reinterpret_cast<const uint32_t *>(&v);
-    }
-    return make_uint4(o[0], o[1], o[2], o[3]);
-}
-__device__ __forceinline__ uint4 dequant8b_slow(uint32_t w0, uint32_t w1, float z, float s) {
-    uint32_t o[4];
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-        const uint32_t w = i < 2 ? w0 : w1;
-        const float lo = ((float)((w >> (16 * (i & 1))) & 255u) - z) * s, hi = ((float)((w >> (16 * (i & 1) + 8)) & 255u) - z) * s;
-        o[i] = (uint32_t)__half_as_ushort(__float2half_rn(lo)) | ((uint32_t)__half_as_ushort(__float2half_rn(hi)) << 16);
-    }
-    return make_uint4(o[0], o[1], o[2], o[3]);
-}
-__device__ __forceinline__ uint4 dequant8_slow(uint32_t w, float z, float s) {  // any zero point: f32, one rounding
-    uint32_t o[4];
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-        const float lo = ((float)((w >> (8 * i)) & 15u) - z) * s, hi = ((float)((w >> (8 * i + 4)) & 15u) - z) * s;
-        o[i] = (uint32_t)__half_as_ushort(__float2half_rn(lo)) | ((uint32_t)__half_as_ushort(__float2half_rn(hi)) << 16);
-    }
-    return make_uint4(o[0], o[1], o[2], o[3]);
-}
-
-// ring depth by token tile: 96 KB per stage at TN = 256 leaves room for two, 64 KB at TN = 128 for three (deeper rings
-// measured no faster: the weight warps, not the pipeline depth, set the pace)
-// (also for the small token tiles: five stages with four activation copies in flight at 32 tokens, four with three at
-// 64, measured 20-60 % slower than three stages with two in flight on 16-64 tokens)
-// Two 256-token tiles per dequantised weight stage (512 tokens per CTA, all of tensor memory) were built and measured at
-// 2048 tokens: 2.5 us per pair of products = the 136 KB of operands a CTA then pulls per group at ~54 GB/s per SM, i.e.
-// the L2 -> SM bandwidth bounds the activation supply, not the weight warps: +5-11 % where the CTAs formed one wave
-// (o, down), -17 % where they did not (qkv); not kept.  Halving the activation bytes per product needs CTA pairs
-// (cta_group::2) that share one activation tile.
-template <int TN>
-constexpr int gemm_stages() { return TN >= 256 ? 2 : 3; }
+// 64 KB per stage at TN = 128: three (deeper rings measured no faster: the weight warps, not the pipeline depth, set the pace; also
+// for the small token tiles: five stages with four activation copies in flight at 32 tokens, four with three at 64, measured 20-60 %
+// slower than three stages with two in flight on 16-64 tokens)
+constexpr int kGStages = 3;
 
 // The weight warps' work for one CTA: dequantise the groups [g_begin, g_begin + G) of rows n0 .. n0 + 127 into the A ring
-// (STAGES slots of 32 KB), one stage per group; full barriers are arrived at once per warp and stage, empty barriers
+// (kGStages slots of 32 KB), one stage per group; full barriers are arrived at once per warp and stage, empty barriers
 // are waited on before a slot is reused.
-template <int BITS, int STAGES>
+template <int BITS>
 __device__ __forceinline__ void gemm_weight_warps(const GemmParams &p, unsigned char *As, uint64_t *full, uint64_t *empty, int g_begin, int G, int n0,
                                                   bool &ok) {
-    constexpr int kGStages = STAGES;
     constexpr int kABytes = kGM * kGK * 2;
     constexpr int kCodeVec = BITS == 4 ? 1 : 2;      // 16-byte vectors of codes per thread and stage (32 columns)
     constexpr int kAheadA = BITS == 4 ? kGAhead : 2;  // stages of codes in flight in registers (16 registers either way)
@@ -239,7 +189,6 @@ __device__ __forceinline__ void gemm_weight_warps(const GemmParams &p, unsigned 
 
 template <int TN, int BITS>
 __global__ void __launch_bounds__(kGThreads, 1) gemm_int4_tc_kernel(const GemmParams p, const __grid_constant__ CUtensorMap tmap_b) {
-    constexpr int kGStages = gemm_stages<TN>();
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     // 1024-byte alignment of every operand buffer: the swizzle is a function of the address bits
     unsigned char *smem = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -276,7 +225,7 @@ __global__ void __launch_bounds__(kGThreads, 1) gemm_int4_tc_kernel(const GemmPa
     const int G = min(p.G, g_begin + p.gps) - g_begin;  // this CTA's groups (stages), >= 1 by construction of the grid
     bool ok = true;
     if (warp < kGWarpsA) {
-        gemm_weight_warps<BITS, kGStages>(p, As, full, empty, g_begin, G, n0, ok);
+        gemm_weight_warps<BITS>(p, As, full, empty, g_begin, G, n0, ok);
     } else if (warp == kGWarpsA) {
         // ---------------------------------------------------------------- activations: TMA into operand B
         // One thread per stage: wait for the slot, announce the bytes on the stage's full barrier and issue the two
@@ -419,7 +368,6 @@ static int make_act_tmap(const GemmParams &p, int rows, CUtensorMap *tmap) {
 
 template <int TN, int BITS>
 int gemm_launch(const GemmParams &p, const Device *dev, cudaStream_t st) {
-    constexpr int kGStages = gemm_stages<TN>();
     const size_t smem = 1024 + (size_t)kGStages * (kGM * kGK * 2 + TN * kGK * 2) + (2 * kGStages + 1) * 8 + 16;
     if (smem > dev->smem_optin) return IM_ERR_BOUNDS;
     auto kern = gemm_int4_tc_kernel<TN, BITS>;
@@ -439,13 +387,34 @@ int gemm_launch(const GemmParams &p, const Device *dev, cudaStream_t st) {
 
 }  // namespace
 
+static bool gemm_takes(const AffineWeight *w) { return (w->bits == 4 || w->bits == 8) && w->group_size == 128 && w->K % 128 == 0; }
+
+// The tokens as the projection reads them: x itself, or f16(x / awq) in the scratch.
+static int scaled_tokens(const AffineWeight *w, const __half *x, int M, __half *xs_scratch, cudaStream_t st, const __half **out) {
+    *out = x;
+    if (!w->awq && reinterpret_cast<uintptr_t>(x) % 16 == 0) return IM_OK;
+    const size_t n = (size_t)M * w->K;
+    IM_CUDA_CHECK(launch_k(act_scale_kernel, dim3((unsigned)((n / 8 + 255) / 256)), dim3(256), 0, st, x, (const __half *)w->awq, xs_scratch, n, w->K));
+    *out = xs_scratch;
+    return IM_OK;
+}
+
+bool gemm_affine_joins(const AffineWeight *gate, int M) { return gemm_takes(gate) && pair_gemm_takes(gate->dev, 2 * gate->N, M); }
+
+int gemm_affine_gate_up(const AffineWeight *gate, const AffineWeight *up, const __half *x, __half *y, int M, __half *xs_scratch, cudaStream_t st) {
+    const __half *xs;
+    const int rc = scaled_tokens(gate, x, M, xs_scratch, st, &xs);
+    return rc != IM_OK ? rc : pair_gemm_affine(gate, up, xs, y, M, st);
+}
+
 // Y[M, N] = f16(X / awq) * dequant(W)^T for M tokens.  xs_scratch: M * K halves.  IM_ERR_BOUNDS when the weight is not
 // INT4 group-128 with K a multiple of 128 (the caller falls back to the matvec kernels).
 int gemm_affine_tc(const AffineWeight *w, const __half *x, __half *y, int M, __half *xs_scratch, cudaStream_t st) {
-    if ((w->bits != 4 && w->bits != 8) || w->group_size != 128 || w->K % 128 != 0 || M < 1) return IM_ERR_BOUNDS;
-    const size_t n = (size_t)M * w->K;
-    IM_CUDA_CHECK(launch_k(act_scale_kernel, dim3((unsigned)((n / 8 + 255) / 256)), dim3(256), 0, st, x, (const __half *)w->awq, xs_scratch, n, w->K));
-    GemmParams p{w->codes, w->sz, xs_scratch, y, w->N, w->K, w->G, M, w->dev->err_flag, nullptr, w->G};
+    if (!gemm_takes(w) || M < 1) return IM_ERR_BOUNDS;
+    const __half *xs;
+    if (const int rc = scaled_tokens(w, x, M, xs_scratch, st, &xs); rc != IM_OK) return rc;
+    if (pair_gemm_takes(w->dev, w->N, M)) return pair_gemm_affine(w, nullptr, xs, y, M, st);
+    GemmParams p{w->codes, w->sz, xs, y, w->N, w->K, w->G, M, w->dev->err_flag, nullptr, w->G};
     // Few tokens and few row tiles (decode batches of 16-64 against 4096-6144 rows: 32-48 CTAs of 32-112 sequential
     // stages): split K so that the grid covers the GPU.  At least four groups per slice; the slices' f32 sums go through
     // the device handle's scratch (one GEMM in flight per handle, like the tiled matvec).
@@ -458,16 +427,11 @@ int gemm_affine_tc(const AffineWeight *w, const __half *x, __half *y, int M, __h
             p.partial = w->dev->gemm_partial;
         }
     }
-    // a 256-token tile shares every dequantised weight tile between twice as many tokens, but halves the CTA count:
-    // worth it only once the grid still covers the GPU
-    const long long ctas256 = (long long)((w->N + kGM - 1) / kGM) * ((M + 255) / 256);
     if (w->bits == 8) {  // superblock_matmul_int8 (affine_matmul.metal:155-290): the same kernel, byte codes
-        if (M > 128 && ctas256 >= w->dev->sm_count) return gemm_launch<256, 8>(p, w->dev, st);
         if (M > 64) return gemm_launch<128, 8>(p, w->dev, st);
         if (M > 32) return gemm_launch<64, 8>(p, w->dev, st);
         return gemm_launch<32, 8>(p, w->dev, st);
     }
-    if (M > 128 && ctas256 >= w->dev->sm_count) return gemm_launch<256, 4>(p, w->dev, st);
     if (M > 64) return gemm_launch<128, 4>(p, w->dev, st);
     if (M > 32) return gemm_launch<64, 4>(p, w->dev, st);
     return gemm_launch<32, 4>(p, w->dev, st);

@@ -191,6 +191,7 @@ struct Layer {
     AffineWeight *qkv = nullptr;     // rows [q | k | v] of this rank
     AffineWeight q_rows{}, kv_rows{};  // non-owning views of qkv's Q rows and K | V rows (same device arrays)
     AffineWeight *o = nullptr, *gate = nullptr, *up = nullptr, *down = nullptr;
+    bool ffn_joint = false;          // gate and up have the same form and activation scales: one projection serves both
     __half *input_ln = nullptr, *post_ln = nullptr, *q_norm = nullptr, *k_norm = nullptr;
     uint8_t *kc = nullptr, *vc = nullptr;
     float *ks = nullptr, *vs = nullptr, *krn = nullptr;
@@ -334,6 +335,16 @@ static int slice_affine(HostAffine *out, const void *qdata, const void *scales, 
     }
     out->awq.clear();
     if (awq) out->awq.assign(static_cast<const uint16_t *>(awq) + c0, static_cast<const uint16_t *>(awq) + c0 + nc);
+    return IM_OK;
+}
+
+static int same_scales(const AffineWeight *a, const AffineWeight *b, bool *same) {
+    *same = a->awq == nullptr && b->awq == nullptr;
+    if (!a->awq || !b->awq || a->K != b->K) return IM_OK;
+    std::vector<uint16_t> x(a->K), y(a->K);
+    IM_CUDA_CHECK(cudaMemcpy(x.data(), a->awq, x.size() * 2, cudaMemcpyDeviceToHost));
+    IM_CUDA_CHECK(cudaMemcpy(y.data(), b->awq, y.size() * 2, cudaMemcpyDeviceToHost));
+    *same = x == y;
     return IM_OK;
 }
 
@@ -483,20 +494,25 @@ int Model::forward(int nseq, int T, cudaStream_t st, int *launches, Prof *prof, 
         if (m->world > 1) IM_MARK(kCatComm);
         IM_TRY(im_cuda_fused_residual_rms_norm(m->hidden, m->ffn_down, L.post_ln, m->norm_out, m->residual, H, MT, eps, st));
         IM_MARK(kCatResNorm);
-        IM_TRY(gemm_affine_tc(L.gate, m->norm_out, m->ffn_gate, MT, m->xs_scratch, st));
-        IM_TRY(gemm_affine_tc(L.up, m->norm_out, m->ffn_up, MT, m->xs_scratch, st));
-        {
-            const size_t n = (size_t)MT * m->I_l;
-            cudaError_t le = launch_k(silu_mul_kernel, dim3((unsigned)((n / 2 + 255) / 256)), dim3(256), 0, st, (const __half *)m->ffn_gate,
-                                      (const __half *)m->ffn_up, m->ffn_gate, n);
-            if (le != cudaSuccess) return fail(IM_ERR_CUDA, "launch failed: %s", cudaGetErrorString(le));
+        const bool joint = L.ffn_joint && gemm_affine_joins(L.gate, MT);
+        if (joint) {
+            IM_TRY(gemm_affine_gate_up(L.gate, L.up, m->norm_out, m->ffn_gate, MT, m->xs_scratch, st));
+        } else {
+            IM_TRY(gemm_affine_tc(L.gate, m->norm_out, m->ffn_gate, MT, m->xs_scratch, st));
+            IM_TRY(gemm_affine_tc(L.up, m->norm_out, m->ffn_up, MT, m->xs_scratch, st));
+            {
+                const size_t n = (size_t)MT * m->I_l;
+                cudaError_t le = launch_k(silu_mul_kernel, dim3((unsigned)((n / 2 + 255) / 256)), dim3(256), 0, st, (const __half *)m->ffn_gate,
+                                          (const __half *)m->ffn_up, m->ffn_gate, n);
+                if (le != cudaSuccess) return fail(IM_ERR_CUDA, "launch failed: %s", cudaGetErrorString(le));
+            }
         }
         IM_MARK(kCatFfn);
         IM_TRY(gemm_affine_tc(L.down, m->ffn_gate, m->ffn_down, MT, m->xs_scratch, st));
         IM_MARK(kCatDown);
         IM_TRY(tp_allreduce(m, m->ffn_down, (size_t)MT * H, st));  // tensor parallel: down is row-split
         if (m->world > 1) IM_MARK(kCatComm);
-        nl += 11 + (m->world > 1 ? 2 : 0);
+        nl += (joint ? 7 : 11) + (m->world > 1 ? 2 : 0);
         if (l + 1 < c.num_layers) {
             Layer &Nx = m->layers[l + 1];
             IM_TRY(im_cuda_fused_residual_rms_norm(m->residual, m->ffn_down, Nx.input_ln, m->norm_out, m->hidden, H, MT, eps, st));
@@ -1131,6 +1147,8 @@ int Model::finalize() {
         IM_TRY(make_weight(m, f, &L.qkv));
         L.q_rows = row_view(L.qkv, 0, m->q_dim);
         L.kv_rows = row_view(L.qkv, m->q_dim, 2 * m->kv_dim);
+        IM_TRY(same_scales(L.gate, L.up, &L.ffn_joint));
+        L.ffn_joint = L.ffn_joint && L.gate->bits == L.up->bits && L.gate->N == L.up->N && L.gate->K == L.up->K;
         L.hq = HostAffine(); L.hk = HostAffine(); L.hv = HostAffine();
         // KV cache of this rank's heads (MetalKvCache, crates/ironmill-inference/src/metal/turboquant/cache.rs:104-354)
         const size_t rows = (size_t)c.max_batch * m->nkv_l * c.max_seq_len;

@@ -22,7 +22,7 @@ __device__ __forceinline__ float load_weight(const __half *w, const __half *awq,
 // Bound: HBM (2 bytes in, 0.5 or 1 byte and 8 bytes per group out).  A thread owns the same eight columns of kQRows
 // consecutive rows, so that its loads are in flight together and one index division and one load of the AWQ vector serve
 // them all; the L = group / 8 lanes of a group find its extrema by shuffles and the codes are formed from the values still in
-// registers.  14336 x 4096, 4-bit with AWQ: QUANT_FIGURES.
+// registers.  14336 x 4096, 4-bit with AWQ: 406 -> 90 us (1.7 TB/s; issue bounds it: about eight instructions per element).
 //
 // Codes without a division per element: t = x * (1 / scale) + zp differs from the defining fl(fl(x / scale) + zp) by less
 // than 2^-20 (|x / scale| + |zp| + 1), so the two round to the same integer unless t lies that close to a half; a thread

@@ -57,6 +57,22 @@ def test_many_token_tiles_of_256(dev):
     _check(dev, H.QWeight(1024, 512, awq=True, seed=77, name="gt"), 4700)
 
 
+@pytest.mark.parametrize("bits", [4, 8])
+@pytest.mark.parametrize("N,K,M,awq", [(9480, 128, 129, False), (9472, 384, 257, True), (2376, 640, 1025, True), (2504, 1792, 2047, False), (20000, 256, 300, True)])
+def test_cta_pairs(dev, N, K, M, awq, bits):
+    # tiles of 256 rows x 128 or 256 tokens: ragged last row tile (N % 256 from 0 to 248), one token more and less than a tile,
+    # one to fourteen groups against rings of three and four stages, more tiles than pairs
+    from ironmill_b200 import ops
+    qw = H.QWeight(N, K, bits=bits, awq=awq, seed=N + M + bits, name="gp")
+    qw.zps = qw.zps.copy()
+    qw.zps[5::977] += 0.5  # a zero point that is no integer: the f32 path
+    qw.zps_f16 = orc.f32_to_f16(qw.zps)
+    x = (H.rng_for("gemm-xp", M).standard_normal((M, K))).astype(np.float16)
+    y = ops.matmul_affine(qw.gpu(dev), torch.from_numpy(x).cuda()).cpu().numpy()
+    ref = orc.matmul_affine(qw.packed, qw.scales_f16, qw.zps_f16, x, N, K, 128, bits, awq=qw.awq, threads=8)
+    assert H.rel_err(y, ref) <= TOL, (N, K, M)
+
+
 def test_awq_and_ragged_rows(dev):
     # N not a multiple of the 128-row CTA tile: the last CTA's spare rows are masked
     _check(dev, H.QWeight(200, 512, awq=True, seed=3, name="ga"), 48)

@@ -384,3 +384,14 @@ def test_long_wide_prompts():
     assert G.error(e.prefill(toks)[None], want[-1:]) < G.TOL["bfloat16"]
     e.reset()
     assert G.error(e.prefill_all_logits(toks), want) < G.TOL["bfloat16"]
+
+
+@pytest.mark.parametrize("width,ff,n", [(136, 4900, 300), (1032, 64, 1100)])
+def test_prompts_on_cta_pairs(width, ff, n):
+    """Projections of enough rows and tokens for CTA pairs: (gate, up) pairs and mixer rows, and the residual's."""
+    cfg = G.config([G.latent(ff=ff), G.lightning(ff=ff)], width=width, vocab=90)
+    w = G.weights(cfg, 15)
+    toks = tokens(n, 90)
+    want = OracleGizizen(cfg, w).forward(toks)
+    e = engine(cfg, w, "bfloat16", max_seq_len=n + 8)
+    assert G.error(e.prefill(toks)[None], want[-1:]) < G.TOL["bfloat16"]

@@ -176,3 +176,20 @@ def test_model_with_turboquant_off_matches_the_oracle(arch):
     assert sorted(out) == sorted([s0, s1])
     w0, w1 = r0.forward(np.array([orc.argmax(l0)], dtype=np.uint32)), r1.forward(np.array([orc.argmax(l1)], dtype=np.uint32))
     assert np.abs(out[s0] - w0).max() <= 5e-2 and np.abs(out[s1] - w1).max() <= 5e-2
+
+
+@pytest.mark.parametrize("awq,bits", [(False, 4), (True, 4), (True, 8)])
+def test_prompt_with_gate_and_up_in_one_projection(awq, bits):
+    # wide enough for CTA pairs: even weight rows from gate, odd rows from up, both rounded before the activation; a second layer reads
+    # what the first left
+    from ironmill_b200.bundle import ModelConfig
+    from ironmill_b200.engine import CudaConfig, CudaInference
+    from tests.oracle_model import DictProvider, OracleModel, synth_model
+    cfg = ModelConfig(architecture="llama", hidden_size=256, intermediate_size=2688, num_hidden_layers=2, num_attention_heads=2,
+                      num_key_value_heads=1, head_dim=128, vocab_size=400, max_position_embeddings=512, rms_norm_eps=1e-5, rope_theta=5e5,
+                      tie_word_embeddings=True)
+    tensors = synth_model(cfg, seed=6, awq=awq, bits=bits)
+    eng = CudaInference(CudaConfig(max_seq_len=256).without_turboquant())
+    eng.load_weights(DictProvider(cfg, tensors))
+    prompt = H.rng_for("kv16-joint").integers(0, 400, 203).astype(np.uint32)
+    assert np.abs(eng.prefill(prompt) - OracleModel(cfg, tensors, None, 256, kv_f16=True).forward(prompt)).max() <= 5e-2
