@@ -212,12 +212,21 @@ struct Tq {
 };
 
 int tq_auto_splits(const Device *dev, int nseq, int T, int nkv, int seq_len);
-int tq_reduce_launch(const Tq *tq, const float *po, const float *pm, const float *pl, __half *out, int tokens, int nh, int splits, cudaStream_t st);
 // Prefill chunks of one sequence: dequantise the cached rows once, causal flash attention on the tensor cores (tq_prefill.cu).
 size_t tq_prefill_scratch_bytes(int nkv, int max_seq);
-int tq_prefill_attention_launch(const Tq *tq, float *partials, void *dq, const float *qrot, const uint8_t *kc, const uint8_t *vc, const float *ks,
+struct TqPromptQuery {       // query rows as projected: head h at column 128 h
+    const __half *q;
+    int stride;
+    const __half *qw = nullptr;  // norm weights, or none
+    float eps = 0.0f;
+    const __half *cosc = nullptr, *sinc = nullptr;
+    int rotary_dim = 0;
+};
+int tq_prefill_attention_launch(const Tq *tq, void *q_rows, void *dq, const TqPromptQuery &q, const uint8_t *kc, const uint8_t *vc, const float *ks,
                                 const float *vs, const float *krn, float attn_scale, __half *out, int slot, int nh, int nkv, int max_seq,
-                                const int *pos_dev, int T, int ctx_end, cudaStream_t st, int base_pos = 0, bool project_queries = true);
+                                const int *pos_dev, int T, int ctx_end, cudaStream_t st, int base_pos = 0);
+struct TqPrep;
+int tq_prompt_encode_launch(const Tq *tq, const TqPrep &a, int slot, cudaStream_t st);
 bool tq_prefill_takes(int nh, int nkv);  // head groupings the prefill pass is built for
 // Inputs of the fused RoPE + cache write + query rotation launch (turboquant.cu).
 struct TqPrep {
@@ -234,7 +243,6 @@ struct TqPrep {
     __half *q_out;  // optional out [nseq*T, nh, hd]
     uint8_t *kc, *vc;
     float *ks, *vs, *krn;
-    int no_q_proj = 0;  // query heads: leave S * (rotated query) to the consumer (the prefill attention pass projects it itself)
 };
 int tq_prep_launch(const Tq *tq, const TqPrep &a, cudaStream_t st);
 int tq_attention_launch(const Tq *tq, float *scratch, const __half *q, const uint8_t *kc, const uint8_t *vc, const float *ks,

@@ -8,7 +8,7 @@
 //                  pairs over the scores' own columns (two terms: the rounded weight and what the rounding left, side by side)
 //     O += P V     A operand P from tensor memory, B operand V with the head dimension contiguous (MN-major), f32 accumulator
 // The two halves take turns: while one half's four warps exponentiate, the other half's products run. Tensor memory is full:
-// 2 x PN columns of scores / weights and 2 x 128 of outputs. An accumulator is rescaled only when a row's maximum has grown by
+// scores / weights of two halves in 256 columns, outputs in 256 more. An accumulator is rescaled only when a row's maximum has grown by
 // more than 2^8 since the last time (weights up to 2^8 are representable and the normalisation uses the same maximum).
 //
 // Order: every product is issued by one thread, so S of the next tile cannot overtake the P V product that still reads the same
@@ -39,12 +39,16 @@ struct FlashParams {
     float scale2;                        // scale / ln 2: scores in powers of two
 };
 
+// TQ: rows of a quantized cache (KB = 4): two score accumulators, factors per position, outputs rotated back
 template <int KB, int PN>
 struct FlashShape {
+    static constexpr bool kTq = KB == 4;
+    static constexpr int kScore = kTq ? 2 * PN : PN;    // tensor-memory columns of a half's scores
+    static constexpr int kFactors = kTq ? 3 * PN * 4 : 0;
     static constexpr int kQ = 2 * KB * kFM * 128;       // both halves' queries
     static constexpr int kK = KB * PN * 128, kV = 2 * PN * 128;
-    static constexpr int kStages = KB == 2 ? 2 : 3;
-    static constexpr int kSmem = 1024 + kQ + kStages * (kK + kV) + (4 * kStages + 7) * 8 + 16;
+    static constexpr int kStages = KB == 3 ? 3 : 2;
+    static constexpr int kSmem = 1024 + kQ + kStages * (kK + kV + kFactors) + (4 * kStages + 7) * 8 + 16;
 };
 
 __device__ __forceinline__ uint64_t desc_sw128(uint32_t addr, uint32_t lbo_bytes) {
@@ -68,6 +72,11 @@ __device__ __forceinline__ void commit(uint64_t *bar) {
 __device__ __forceinline__ void tma_2d(void *dst, const CUtensorMap *map, int x, int y, uint64_t *bar) {  // x: a multiple of eight elements (flash_takes)
     asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(smem_u32(dst)), "l"(map),
                  "r"(x), "r"(y), "r"(smem_u32(bar))
+                 : "memory");
+}
+__device__ __forceinline__ void bulk_copy(void *dst, const void *src, uint32_t bytes, uint64_t *bar) {  // 16-byte aligned
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(dst)), "l"(src), "r"(bytes),
+                 "r"(smem_u32(bar))
                  : "memory");
 }
 __device__ __forceinline__ void ld32(uint32_t taddr, uint32_t *r) {  // no wait: tmem_wait_ld
@@ -204,12 +213,15 @@ __global__ void __launch_bounds__(kFThreads, 1)
     flash_tc_kernel(const __grid_constant__ FlashParams p, const __grid_constant__ CUtensorMap tq, const __grid_constant__ CUtensorMap tk, const __grid_constant__ CUtensorMap tk2,
                     const __grid_constant__ CUtensorMap tv) {
     using Shape = FlashShape<KB, PN>;
-    constexpr int ST = Shape::kStages;
+    constexpr int ST = Shape::kStages, kScore = Shape::kScore;
+    constexpr bool TQ = Shape::kTq;
     static_assert(TERMS * PN / 2 <= PN, "the weights lie over the scores");
+    static_assert(2 * kScore <= 256, "scores and outputs fill tensor memory");
     extern __shared__ __align__(1024) unsigned char flash_smem[];
     unsigned char *smem = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(flash_smem) + 1023) & ~(uintptr_t)1023);
     unsigned char *Qs = smem, *Ks = smem + Shape::kQ, *Vs = Ks + ST * Shape::kK;
-    uint64_t *kfull = reinterpret_cast<uint64_t *>(Vs + ST * Shape::kV), *kempty = kfull + ST, *vfull = kempty + ST, *vempty = vfull + ST;
+    float *Fs = reinterpret_cast<float *>(Vs + ST * Shape::kV);
+    uint64_t *kfull = reinterpret_cast<uint64_t *>(Vs + ST * (Shape::kV + Shape::kFactors)), *kempty = kfull + ST, *vfull = kempty + ST, *vempty = vfull + ST;
     uint64_t *qfull = vempty + ST, *sfull = qfull + 1, *pfull = sfull + 2, *ofull = pfull + 2;
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(ofull + 2);
     const FlashArgs &a = p.a;
@@ -278,7 +290,8 @@ __global__ void __launch_bounds__(kFThreads, 1)
             __syncwarp();
             if (ok && use > 0 && !wait_for(&vempty[s], (use - 1) & 1, a.err)) ok = false;
             if (lane == 0 && ok) {
-                mbar_expect_tx(&vfull[s], (uint32_t)Shape::kV);
+                mbar_expect_tx(&vfull[s], (uint32_t)(Shape::kV + Shape::kFactors));
+                if constexpr (TQ) bulk_copy(Fs + s * 3 * PN, a.scales + ((size_t)kvh * a.scale_tiles + it) * (3 * PN), Shape::kFactors, &vfull[s]);
                 for (int b = 0; b < 2; b++) tma_2d(Vs + (size_t)s * Shape::kV + (size_t)b * PN * 128, &tv, vx + b * 64, vy + it * PN, &vfull[s]);
             }
             __syncwarp();
@@ -310,7 +323,7 @@ __global__ void __launch_bounds__(kFThreads, 1)
                     }
                     fence_after();
                     if (lane == 0 && ok) {
-                        const uint32_t v0 = smem_u32(Vs + (size_t)sp * Shape::kV), pw = tmem + (uint32_t)(i * PN), o = tmem + 256u + (uint32_t)(i * kFDV);
+                        const uint32_t v0 = smem_u32(Vs + (size_t)sp * Shape::kV), pw = tmem + (uint32_t)(i * kScore), o = tmem + 256u + (uint32_t)(i * kFDV);
 #pragma unroll
                         for (int t = 0; t < TERMS; t++)
 #pragma unroll
@@ -327,8 +340,8 @@ __global__ void __launch_bounds__(kFThreads, 1)
                         const uint32_t q0 = smem_u32(Qs + (size_t)i * KB * kFM * 128), k0 = smem_u32(Ks + (size_t)s * Shape::kK);
 #pragma unroll
                         for (int j = 0; j < KB * 4; j++)
-                            mma_ss(tmem + (uint32_t)(i * PN), desc_sw128(q0 + (j >> 2) * (kFM * 128) + (j & 3) * 32, 16), desc_sw128(k0 + (j >> 2) * (PN * 128) + (j & 3) * 32, 16),
-                                   kS, j > 0 ? 1u : 0u);
+                            mma_ss(tmem + (uint32_t)(i * kScore + (TQ && j >= 8 ? PN : 0)), desc_sw128(q0 + (j >> 2) * (kFM * 128) + (j & 3) * 32, 16),
+                                   desc_sw128(k0 + (j >> 2) * (PN * 128) + (j & 3) * 32, 16), kS, (TQ ? j & 7 : j) > 0 ? 1u : 0u);
                         commit(&sfull[i]);
                     }
                     __syncwarp();
@@ -343,7 +356,7 @@ __global__ void __launch_bounds__(kFThreads, 1)
     } else {
         const int i = warp >> 2, row = (warp & 3) * 32 + lane, tok = t0 + i * kFM + row;
         const uint32_t lanes = (uint32_t)((warp & 3) * 32) << 16;
-        const uint32_t ts = tmem + lanes + (uint32_t)(i * PN), to = tmem + lanes + 256u + (uint32_t)(i * kFDV);
+        const uint32_t ts = tmem + lanes + (uint32_t)(i * kScore), to = tmem + lanes + 256u + (uint32_t)(i * kFDV);
         const float sink = a.sink ? a.sink[h] * 1.4426950408889634f : -INFINITY;
         if (i < halves) {
             const int first = P + t0 + i * kFM, last = P + min(t0 + i * kFM + kFM, a.T) - 1;
@@ -354,10 +367,33 @@ __global__ void __launch_bounds__(kFThreads, 1)
                 if (ok && !wait_for(&sfull[i], (it - lo[i]) & 1, a.err)) ok = false;
                 fence_after();
                 const int p0 = n_begin + it * PN;
-                float s[PN];
+                float s[PN], lazy = kLazy;
+                const float *ks = Fs + (it % ST) * 3 * PN, *kr = ks + PN, *vs = kr + PN;
+                if constexpr (TQ) {
+                    if (ok && !wait_for(&vfull[it % ST], (it / ST) & 1, a.err)) ok = false;
+                    // a weight times vs has to stay in fp16's range: where vs is large the maximum follows at once
+                    const unsigned vm = __reduce_max_sync(0xffffffffu, max(__float_as_uint(fabsf(vs[lane])), __float_as_uint(fabsf(vs[lane + 32]))));
+                    if (vm > __float_as_uint(128.0f)) lazy = 0.0f;
 #pragma unroll
-                for (int c = 0; c < PN; c += 32) ld32(ts + (uint32_t)c, reinterpret_cast<uint32_t *>(s) + c);
-                tmem_wait_ld();
+                    for (int c = 0; c < PN; c += 32) {
+                        float t[32];
+                        ld32(ts + (uint32_t)c, reinterpret_cast<uint32_t *>(s) + c);
+                        ld32(ts + (uint32_t)(PN + c), reinterpret_cast<uint32_t *>(t));
+                        tmem_wait_ld();
+#pragma unroll
+                        for (int j = 0; j < 32; j += 4) {
+                            const float4 a4 = *reinterpret_cast<const float4 *>(ks + c + j), b4 = *reinterpret_cast<const float4 *>(kr + c + j);
+                            s[c + j] = a4.x * fmaf(b4.x, t[j], s[c + j]);
+                            s[c + j + 1] = a4.y * fmaf(b4.y, t[j + 1], s[c + j + 1]);
+                            s[c + j + 2] = a4.z * fmaf(b4.z, t[j + 2], s[c + j + 2]);
+                            s[c + j + 3] = a4.w * fmaf(b4.w, t[j + 3], s[c + j + 3]);
+                        }
+                    }
+                } else {
+#pragma unroll
+                    for (int c = 0; c < PN; c += 32) ld32(ts + (uint32_t)c, reinterpret_cast<uint32_t *>(s) + c);
+                    tmem_wait_ld();
+                }
                 if (p0 + PN - 1 > first || p0 < from_last || p0 + PN > a.n_max) {  // some row does not see all of the tile
                     const float hide = p.scale2 > 0.0f ? -INFINITY : INFINITY;
 #pragma unroll
@@ -378,7 +414,7 @@ __global__ void __launch_bounds__(kFThreads, 1)
                     mx[0] = fminf(fminf(mx[0], mx[1]), fminf(mx[2], mx[3]));
                 }
                 const float top = mx[0] * p.scale2;
-                if (__any_sync(0xffffffffu, top > m + kLazy)) {  // (-inf + anything is -inf: a row's first visible position is one)
+                if (__any_sync(0xffffffffu, top > m + lazy)) {  // (-inf + anything is -inf: a row's first visible position is one)
                     const float m_new = fmaxf(m, top), corr = m_new == -INFINITY ? 1.0f : ex2(m - m_new);
                     m = m_new;
                     l *= corr;
@@ -405,7 +441,12 @@ __global__ void __launch_bounds__(kFThreads, 1)
                         const float x0 = ex2(fmaf(s[c + 2 * j], p.scale2, -base)), x1 = ex2(fmaf(s[c + 2 * j + 1], p.scale2, -base));
                         sum[(2 * j) & 3] += x0;
                         sum[(2 * j + 1) & 3] += x1;
-                        w[j] = pack2<BF16>(x0, x1);
+                        if constexpr (TQ) {
+                            const float2 v2 = *reinterpret_cast<const float2 *>(vs + c + 2 * j);
+                            w[j] = pack2<BF16>(x0 * v2.x, x1 * v2.y);
+                        } else {
+                            w[j] = pack2<BF16>(x0, x1);
+                        }
                         if (TERMS > 1) {
                             const float2 r = unpack2<BF16>(w[j]);
                             w2[j] = pack2<BF16>(x0 - r.x, x1 - r.y);
@@ -424,9 +465,56 @@ __global__ void __launch_bounds__(kFThreads, 1)
             fence_after();
             const float gm = fmaxf(m, sink), c0 = m == -INFINITY ? 0.0f : ex2(m - gm);
             const float inv = c0 / fmaxf(l * c0 + (sink == -INFINITY ? 0.0f : ex2(sink - gm)), 1e-10f);
+            if constexpr (TQ) {
+                // back from the rotated space: signs, butterflies over the row's 128 values, signs / sqrt(128); the widest butterfly first, so
+                // that the rest works on 64 registers at a time
+                const float4 *sg = reinterpret_cast<const float4 *>(a.signs);
+#pragma unroll 1
+                for (int c = 0; c < 64; c += 32) {
+                    uint32_t x[32], y[32];
+                    ld32(to + (uint32_t)c, x);
+                    ld32(to + (uint32_t)c + 64u, y);
+                    tmem_wait_ld();
+#pragma unroll
+                    for (int j = 0; j < 32; j++) {
+                        const float u = __uint_as_float(x[j]) * (inv * __ldg(a.signs + c + j)), v = __uint_as_float(y[j]) * (inv * __ldg(a.signs + c + 64 + j));
+                        x[j] = __float_as_uint(u + v);
+                        y[j] = __float_as_uint(u - v);
+                    }
+                    st32(to + (uint32_t)c, x);
+                    st32(to + (uint32_t)c + 64u, y);
+                }
+                tmem_wait_st();
+                constexpr float kRoot = 0.08838834764831845f;  // 1 / sqrt(128)
+#pragma unroll 1
+                for (int c = 0; c < kFDV; c += 64) {
+                    float o[64];
+                    ld32(to + (uint32_t)c, reinterpret_cast<uint32_t *>(o));
+                    ld32(to + (uint32_t)c + 32u, reinterpret_cast<uint32_t *>(o) + 32);
+                    tmem_wait_ld();
+#pragma unroll
+                    for (int step = 1; step < 64; step *= 2)
+#pragma unroll
+                        for (int j = 0; j < 64; j++)
+                            if (!(j & step)) {
+                                const float x = o[j], y = o[j + step];
+                                o[j] = x + y;
+                                o[j + step] = x - y;
+                            }
+#pragma unroll
+                    for (int j = 0; j < 64; j += 4) {
+                        const float4 g = __ldg(sg + (c + j) / 4);
+                        o[j] *= kRoot * g.x; o[j + 1] *= kRoot * g.y; o[j + 2] *= kRoot * g.z; o[j + 3] *= kRoot * g.w;
+                    }
+                    if (tok < a.T && ok) {
+                        store32<BF16>(a, tok, h, c, o);
+                        store32<BF16>(a, tok, h, c + 32, o + 32);
+                    }
+                }
+            }
             bool finite = true;
 #pragma unroll 1
-            for (int c = 0; c < kFDV; c += 32) {
+            for (int c = 0; c < kFDV && !TQ; c += 32) {
                 uint32_t o[32];
                 ld32(to + (uint32_t)c, o);
                 tmem_wait_ld();
@@ -475,7 +563,8 @@ bool flash_takes(const FlashArgs &a) {
         return reinterpret_cast<uintptr_t>(r.base) % 16 == 0 && r.ld % 8 == 0 && r.ld < (1ll << 31) && r.rows < (1ll << 31) && r.col0 % 8 == 0 && r.head_cols % 8 == 0;
     };
     const int kb = a.k.blocks + a.k2.blocks;
-    return a.T > 0 && a.T <= 65535 * 2 * kFM && a.heads > 0 && a.group > 0 && a.heads % a.group == 0 && (kb == 2 || kb == 3) && a.q.blocks == kb && a.v.blocks == 2 && fits(a.q) &&
+    const bool tq = a.scales != nullptr;
+    return a.T > 0 && a.T <= 65535 * 2 * kFM && a.heads > 0 && a.group > 0 && a.heads % a.group == 0 && (tq ? kb == 4 && a.chunk == 0 && a.signs : kb == 2 || kb == 3) && a.q.blocks == kb && a.v.blocks == 2 && fits(a.q) &&
            fits(a.k) && (!a.k2.blocks || fits(a.k2)) && fits(a.v) && reinterpret_cast<uintptr_t>(a.out) % 16 == 0 && a.ldo % 8 == 0 && a.out_head % 8 == 0 &&
            (!a.gate || (reinterpret_cast<uintptr_t>(a.gate) % 16 == 0 && a.ldg % 8 == 0 && a.gate_head % 8 == 0));
 }
@@ -488,6 +577,7 @@ int flash_prepare(const Device *dev) {
     IM_SMEM(false, 2, 128, 1);
     IM_SMEM(true, 2, 128, 2);
     IM_SMEM(true, 3, 64, 2);
+    IM_SMEM(false, 4, 64, 1);
 #undef IM_SMEM
     return IM_OK;
 }
@@ -498,6 +588,7 @@ int flash_run(const FlashArgs &a, cudaStream_t st) {
     if (!a.bf16 && !a.two_terms && kb == 2) return launch<false, 2, 128, 1>(a, st);
     if (a.bf16 && a.two_terms && kb == 2) return launch<true, 2, 128, 2>(a, st);
     if (a.bf16 && a.two_terms && kb == 3) return launch<true, 3, 64, 2>(a, st);
+    if (!a.bf16 && !a.two_terms && kb == 4) return launch<false, 4, 64, 1>(a, st);
     return IM_ERR_BOUNDS;
 }
 

@@ -25,6 +25,11 @@ struct FlashArgs {
     int chunk = 0;               // a position sees its own chunk of so many positions (0: everything before it)
     float scale = 1.0f;
     const float *sink = nullptr; // a keyless logit per head
+    // Quantized caches in the rotated space (fp16, keys of 256 columns): q rows [R q | S R q], k rows [centroids | signs], v rows centroids.
+    // A score is ks (q . k over the first 128 columns + kr (q . k over the last 128)), a weight enters the outputs times vs, and the
+    // outputs are rotated back with `signs`. scales: per key / value head and tile of 64 positions 64 of ks, 64 of kr, 64 of vs.
+    const float *scales = nullptr, *signs = nullptr;
+    int scale_tiles = 0;         // tiles per head
     const void *gate = nullptr;  // outputs times sigmoid(gate): [T, ldg], head h at column h * gate_head
     int ldg = 0, gate_head = 0;
     void *out = nullptr;         // [T, ldo], head h at column h * out_head
@@ -32,7 +37,7 @@ struct FlashArgs {
     int *err = nullptr;
 };
 
-// Shapes it is built for: keys of 128 or 192 columns, values of 128, everything 16-byte aligned.
+// Shapes it is built for: keys of 128, 192 or (with scales) 256 columns, values of 128, everything 16-byte aligned.
 bool flash_takes(const FlashArgs &a);
 int flash_prepare(const Device *dev);  // launch attributes, on the current device
 int flash_run(const FlashArgs &a, cudaStream_t st);

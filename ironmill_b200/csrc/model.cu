@@ -428,17 +428,12 @@ static int attention_block(Model *m, int part, const TqPrep &a, __half *q_buf, L
     }
     // a prefill chunk of one sequence: dequantise the cached rows once, causal tensor-core pass (which also projects the queries)
     const bool flash = nseq == 1 && T >= 16 && m->pf_dq && m->prefill_slot_id >= 0 && tq_prefill_takes(a.nh, a.nkv);
-    if (part == 0) {
-        TqPrep b = a;
-        b.no_q_proj = flash ? 1 : 0;
-        return tq_prep_launch(reinterpret_cast<const Tq *>(m->tq), b, st);
-    }
-    if (flash) {
-        const int rc = tq_prefill_attention_launch(reinterpret_cast<const Tq *>(m->tq), m->scratch_ref, m->pf_dq, m->qrot, L.kc, L.vc, L.ks, L.vs, L.krn,
-                                                   attn_scale, m->attn_out, m->prefill_slot_id, a.nh, a.nkv, c.max_seq_len, m->pos_dev, T,
-                                                   m->prefill_ctx_end, st);
-        if (rc != IM_ERR_BOUNDS) return rc;  // head groupings it does not take: the per-token kernel below
-    }
+    if (part == 0)
+        return flash ? tq_prompt_encode_launch(reinterpret_cast<const Tq *>(m->tq), a, m->prefill_slot_id, st) : tq_prep_launch(reinterpret_cast<const Tq *>(m->tq), a, st);
+    if (flash)
+        return tq_prefill_attention_launch(reinterpret_cast<const Tq *>(m->tq), m->qrot, m->pf_dq,
+                                           TqPromptQuery{a.qkv, a.stride, a.with_norm ? a.qw : nullptr, a.eps, a.cosc, a.sinc, a.rotary_dim}, L.kc, L.vc, L.ks, L.vs, L.krn,
+                                           attn_scale, m->attn_out, m->prefill_slot_id, a.nh, a.nkv, c.max_seq_len, m->pos_dev, T, m->prefill_ctx_end, st);
     return tq_attention_launch(reinterpret_cast<const Tq *>(m->tq), m->scratch_ref, nullptr, L.kc, L.vc, L.ks, L.vs, L.krn, attn_scale, m->attn_out,
                                nseq, a.nh, a.nkv, c.max_seq_len, 0, m->pos_dev, T, attn_splits, st, m->qrot, slots);
 }

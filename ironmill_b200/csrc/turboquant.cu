@@ -633,19 +633,13 @@ int tq_prep_launch(const Tq *tq, const TqPrep &a, cudaStream_t st) {
     k.qw = a.qw; k.kw = a.kw; k.cosc = a.cosc; k.sinc = a.sinc;
     k.nh = a.nh; k.nkv = a.nkv; k.rotary_dim = a.rotary_dim ? a.rotary_dim : kHd; k.with_norm = a.with_norm;
     k.T = a.T; k.max_seq = a.max_seq; k.base_pos = a.base_pos; k.eps = a.eps; k.pos_dev = a.pos_dev; k.slot_map = a.slot_map;
-    k.qrot = a.qrot; k.q_out = a.q_out; k.no_q_proj = a.no_q_proj;
+    k.qrot = a.qrot; k.q_out = a.q_out;
     k.ktab = EncodeTables{tq->signs, tq->k_cb, tq->k_bd, tq->qjl_t, tq->k_levels, 1, tq->n_bits};
     k.vtab = EncodeTables{tq->signs, tq->v_cb, tq->v_bd, tq->qjl_t, tq->v_levels, 0, tq->n_bits};
     k.kc = a.kc; k.vc = a.vc; k.ks = a.ks; k.vs = a.vs; k.krn = a.krn;
     const int tokens = a.nseq * a.T;
     dim3 grid(tokens, a.nh + 2 * a.nkv);
     IM_CUDA_CHECK(launch_k(tq->n_bits == 4 ? tq_qkv_prep_kernel<4> : tq_qkv_prep_kernel<8>, grid, dim3(kHd), 0, st, k));
-    return IM_OK;
-}
-
-// Combination of split partials (normalise, rotate back, fp16) for `tokens` x nh heads: shared with tq_prefill.cu.
-int tq_reduce_launch(const Tq *tq, const float *po, const float *pm, const float *pl, __half *out, int tokens, int nh, int splits, cudaStream_t st) {
-    IM_CUDA_CHECK(launch_k(tq_reduce_kernel, dim3(tokens, nh), dim3(kHd), 0, st, po, pm, pl, (const float *)tq->signs, out, nh, splits));
     return IM_OK;
 }
 
@@ -730,12 +724,9 @@ IM_EXPORT int im_cuda_tq_prefill_attention(im_tq *tq, const void *q_dev, const v
         int rc = im_cuda_tq_reserve_scratch(tq, need);
         if (rc != IM_OK) return rc;
     }
-    float *qrot = tq->scratch + tq_partial_bytes(1, T, nh, kHd, 1) / sizeof(float);
-    IM_CUDA_CHECK(launch_k(tq_qrot_kernel, dim3(T, nh), dim3(kHd), 0, as_stream(stream), static_cast<const __half *>(q_dev), (const float *)tq->signs,
-                           (const float *)tq->qjl_t, qrot, nh));
-    const int rc = tq_prefill_attention_launch(tq, tq->scratch, dq_dev, qrot, static_cast<const uint8_t *>(k_cache_dev), static_cast<const uint8_t *>(v_cache_dev),
-                                               k_scale_dev, v_scale_dev, k_rnorm_dev, attn_scale, static_cast<__half *>(out_dev), 0, nh, nkv, max_seq, nullptr, T,
-                                               base_pos + T, as_stream(stream), base_pos);
+    const int rc = tq_prefill_attention_launch(tq, tq->scratch, dq_dev, TqPromptQuery{static_cast<const __half *>(q_dev), nh * kHd}, static_cast<const uint8_t *>(k_cache_dev),
+                                               static_cast<const uint8_t *>(v_cache_dev), k_scale_dev, v_scale_dev, k_rnorm_dev, attn_scale, static_cast<__half *>(out_dev), 0, nh,
+                                               nkv, max_seq, nullptr, T, base_pos + T, as_stream(stream), base_pos);
     if (rc == IM_ERR_BOUNDS) return fail(IM_ERR_INVALID, "query heads per KV head must be 1, 2, 4 or 8 (got %d/%d)", nh, nkv);
     return rc;
     IM_GUARD_END

@@ -63,6 +63,17 @@ def test_int4_kv_cache_parity(schedule):
     assert err <= 5e-2 and agree >= 0.99, (err, agree)
 
 
+@pytest.mark.parametrize("n_bits,nh,nkv,prompt_len", [(8, 4, 2, 16), (8, 4, 2, 131), (4, 8, 2, 70), (8, 2, 2, 300)])
+def test_prompt_chunks_with_qk_norm(n_bits, nh, nkv, prompt_len):
+    # the prompt's own kernels (chunks of 16 tokens and more): norms and rotation of queries and keys, cache rows that later steps read,
+    # token counts around the four rows of an encoding warp and the 64 positions of an attention tile
+    cfg = _cfg("qwen3", 2, 256, 512, nh, nkv, 500, 1e6, 1e-6)
+    # the stated gate: a last bit of a key or value can become a whole step of its codebook, which few positions average out (0.010 seen at
+    # 16 tokens, 0.004 at 300); no top-1 gate over nine steps, which one pair of close logits decides
+    err, _, _ = _run_parity(cfg, synth_model(cfg, seed=21, gamma_jitter=0.2), prompt_len=prompt_len, steps=8, max_seq=prompt_len + 13, n_bits=n_bits)
+    assert err <= 5e-2, err
+
+
 def test_tiny_llama_shape_awq_int8_parity():
     # no QK-norm (plain RoPE), AWQ scales, GQA 4, tied embeddings, INT8 weights
     cfg = _cfg("llama", 2, 512, 1024, 8, 2, 777, 5e5, 1e-5, tie=True)
