@@ -9,6 +9,7 @@
 #include <cuda.h>
 
 #include <algorithm>
+#include <type_traits>
 
 #include "dense_epi.cuh"
 #include "gemm_pair.cuh"
@@ -271,9 +272,10 @@ struct DenseGemm {
 };
 
 // 16 tokens m .. m + 15 of row n (one per lane) of the f32 sums
+template <typename T>
 __device__ __forceinline__ void dense_store16(const DenseGemm &p, int z, int n, int n_warp, int m, const float (&v)[16]) {
     if (!p.partial) {
-        epi_store16<__nv_bfloat16>(p.epi, p.N, p.M, n, n_warp, m, v);
+        epi_store16<T>(p.epi, p.N, p.M, n, n_warp, m, v);
     } else if (n < p.N) {
         float *dst = p.partial + ((size_t)z * p.M + m) * p.N + n;
 #pragma unroll
@@ -283,7 +285,7 @@ __device__ __forceinline__ void dense_store16(const DenseGemm &p, int z, int n, 
 }
 
 // D[128 weight rows x TN tokens] += W[128 x 64] X[TN x 64]^T per stage.
-template <int TN>
+template <int TN, typename T>
 __global__ void __launch_bounds__(kDThreads, kDCtasPerSm) dense_gemm_tc_kernel(const DenseGemm p, const __grid_constant__ CUtensorMap ta,
                                                                                          const __grid_constant__ CUtensorMap tb) {
     constexpr int S = dense_stages<TN>();
@@ -334,8 +336,9 @@ __global__ void __launch_bounds__(kDThreads, kDCtasPerSm) dense_gemm_tc_kernel(c
             }
         }
     } else if (warp == kDEpi + 1) {
-        // f32 accumulator, bf16 operands, both K-major, N >> 3 in bits 17-22, M >> 4 in bits 24-28
-        constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(TN >> 3) << 17) | ((uint32_t)(kDM >> 4) << 24);
+        // f32 accumulator, bf16 (1) or fp16 (0) operands, both K-major, N >> 3 in bits 17-22, M >> 4 in bits 24-28
+        constexpr uint32_t fmt = std::is_same<T, __half>::value ? 0u : 1u;
+        constexpr uint32_t idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)(TN >> 3) << 17) | ((uint32_t)(kDM >> 4) << 24);
         int it = 0, cnt = 0;
         for (int w = blockIdx.x; w < items; w += gridDim.x, cnt++) {
             const int kb0 = w / (p.mtiles * p.ntiles) * p.kb_per, kb1 = min(p.kblocks, kb0 + p.kb_per);
@@ -370,7 +373,7 @@ __global__ void __launch_bounds__(kDThreads, kDCtasPerSm) dense_gemm_tc_kernel(c
                 for (int c = c_begin; c < c_begin + TN / 2 && m0 + c < p.M; c += 16) {
                     float v[16];
                     dense_tmem_ld16(tmem_d + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(acc * TN + c), v);
-                    dense_store16(p, z, n_warp + lane, n_warp, m0 + c, v);
+                    dense_store16<T>(p, z, n_warp + lane, n_warp, m0 + c, v);
                 }
             }
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -477,18 +480,19 @@ TmapEncodeFn tmap_encode() {
     }();
     return fn;
 }
-template <int TN>
+template <int TN, typename T = __nv_bfloat16>
 int gemm_launch(const Device *dev, DenseGemm p, const DenseWeight &w, const void *x, int ldx, int slices, cudaStream_t st) {
     alignas(64) CUtensorMap ta, tb;
-    int rc = tmap_2d(w.w, true, w.N, w.K, w.ld, kDM, &ta);
+    constexpr bool bf = std::is_same<T, __nv_bfloat16>::value;
+    int rc = tmap_2d(w.w, bf, w.N, w.K, w.ld, kDM, &ta);
     if (rc != IM_OK) return rc;
-    rc = tmap_2d(x, true, p.M, w.K, ldx, TN, &tb);
+    rc = tmap_2d(x, bf, p.M, w.K, ldx, TN, &tb);
     if (rc != IM_OK) return rc;
     p.mtiles = (p.M + TN - 1) / TN;
     p.ntiles = (p.N + kDM - 1) / kDM;
     p.slices = slices;
     const int ctas = std::min(p.mtiles * p.ntiles * slices, dev->sm_count * kDCtasPerSm);
-    IM_CUDA_CHECK(launch_k(dense_gemm_tc_kernel<TN>, dim3(ctas), dim3(kDThreads), (size_t)dense_gemm_smem<TN>(), st, p, ta, tb));
+    IM_CUDA_CHECK(launch_k(dense_gemm_tc_kernel<TN, T>, dim3(ctas), dim3(kDThreads), (size_t)dense_gemm_smem<TN>(), st, p, ta, tb));
     if (p.partial) {
         const size_t n = (size_t)p.M * ((p.N + 1) / 2);
         IM_CUDA_CHECK(launch_k(dense_splitk_reduce_kernel<__nv_bfloat16>, dim3((unsigned)((n + 255) / 256)), dim3(256), 0, st, (const float *)p.partial, p.epi, p.M, p.N,
@@ -550,8 +554,10 @@ int dense_prepare(const Device *dev) {
     IM_SMEM((dense_matvec_kernel<__nv_bfloat16, 4>), mv); IM_SMEM((dense_matvec_kernel<__nv_bfloat16, 8>), mv);
     IM_SMEM((dense_matvec_kernel<float, 1>), mv); IM_SMEM((dense_matvec_kernel<float, 2>), mv);
     IM_SMEM((dense_matvec_kernel<float, 4>), mv); IM_SMEM((dense_matvec_kernel<float, 8>), mv);
-    IM_SMEM(dense_gemm_tc_kernel<128>, dense_gemm_smem<128>());
-    IM_SMEM(dense_gemm_tc_kernel<64>, dense_gemm_smem<64>()); IM_SMEM(dense_gemm_tc_kernel<32>, dense_gemm_smem<32>());
+    IM_SMEM((dense_gemm_tc_kernel<128, __nv_bfloat16>), dense_gemm_smem<128>());
+    IM_SMEM((dense_gemm_tc_kernel<64, __nv_bfloat16>), dense_gemm_smem<64>()); IM_SMEM((dense_gemm_tc_kernel<32, __nv_bfloat16>), dense_gemm_smem<32>());
+    IM_SMEM((dense_gemm_tc_kernel<128, __half>), dense_gemm_smem<128>());
+    IM_SMEM((dense_gemm_tc_kernel<64, __half>), dense_gemm_smem<64>()); IM_SMEM((dense_gemm_tc_kernel<32, __half>), dense_gemm_smem<32>());
 #undef IM_SMEM
     return IM_OK;
 }
@@ -596,6 +602,19 @@ int dense_project(const Device *dev, const DenseWeight &w, const DenseSrc &src, 
     if (M > 64) return gemm_launch<128>(dev, p, w, x, ldx, slices, st);
     if (M > 32) return gemm_launch<64>(dev, p, w, x, ldx, slices, st);
     return gemm_launch<32>(dev, p, w, x, ldx, slices, st);
+}
+
+int dense_rows_f16(const Device *dev, const __half *w, int N, int K, const __half *x, __half *y, int M, cudaStream_t st) {
+    if (K % 8 != 0 || (reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(x)) % 16 != 0) return IM_ERR_BOUNDS;
+    if (const int rc = dense_prepare(dev); rc != IM_OK) return rc;
+    DenseWeight dw;
+    dw.N = N; dw.K = K; dw.ld = K; dw.w = const_cast<__half *>(w);
+    DenseGemm p{};
+    p.N = N; p.M = M; p.kblocks = (K + kDK - 1) / kDK; p.kb_per = p.kblocks; p.err = dev->err_flag;
+    p.epi.kind = kEpiProj; p.epi.pair0 = 1 << 30; p.epi.y = y; p.epi.ldy = N;
+    if (M > 64) return gemm_launch<128, __half>(dev, p, dw, x, K, 1, st);
+    if (M > 32) return gemm_launch<64, __half>(dev, p, dw, x, K, 1, st);
+    return gemm_launch<32, __half>(dev, p, dw, x, K, 1, st);
 }
 
 int stack_embed(const uint32_t *tokens, const void *table, int f32, int ld, const float *gamma, float scale, float *x, float *x0, int width, uint32_t vocab, float eps,

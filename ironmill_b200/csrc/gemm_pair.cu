@@ -160,8 +160,13 @@ __device__ __forceinline__ void weight_warps(const PairGemm &p, unsigned char *A
 #pragma unroll
     for (int u = 0; u < kAhead; u++) request(u);
     const uint32_t full0 = leader_addr(full);
+    auto hand_over = [&](int stage) {
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // generic-proxy writes -> visible to the tensor cores
+        __syncwarp();
+        if (lane == 0) arrive_at(full0 + stage * 8);
+    };
     bool ok = true;
-    int s = 0, use = 0;
+    int s = 0, use = 0, prev = 0;
     for (int base = 0; base < total; base += kAhead) {
 #pragma unroll
         for (int u = 0; u < kAhead; u++) {
@@ -190,17 +195,18 @@ __device__ __forceinline__ void weight_warps(const PairGemm &p, unsigned char *A
 #pragma unroll
                     for (int i = 0; i < 4; i++) v[i] = BITS == 4 ? dequant8_slow(in[i].x, zf, sf) : dequant8b_slow(in[i].x, in[i].y, zf, sf);
                 }
+                // the previous stage is handed over only now: its stores have landed while this one was converted, and the fence does not wait
+                if (base + u > 0) hand_over(prev);
                 if (ok && use > 0 && !pair_wait_warp(&empty[s], (use - 1) & 1, p.err)) ok = false;
                 unsigned char *dst = As + (size_t)s * S::kA + row_off;
 #pragma unroll
                 for (int i = 0; i < 4; i++) *reinterpret_cast<uint4 *>(dst + (((c0 + (i ^ swap)) ^ x) << 4)) = v[i];
-                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // generic-proxy writes -> visible to the tensor cores
-                __syncwarp();
-                if (lane == 0) arrive_at(full0 + s * 8);
+                prev = s;
                 if (++s == S::kStages) s = 0, use++;
             }
         }
     }
+    if (total > 0) hand_over(prev);
 }
 
 template <typename T, int TN, int BITS>

@@ -136,6 +136,11 @@ __device__ __forceinline__ void gemm_weight_warps(const GemmParams &p, unsigned 
             szb[u] = szrow[u];
         }
     }
+    auto hand_over = [&](int stage) {
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // generic-proxy writes -> visible to the tensor core
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&full[stage]);
+    };
     for (int kt0 = 0; kt0 < G; kt0 += kAheadA) {
 #pragma unroll
         for (int u = 0; u < kAheadA; u++) {
@@ -172,6 +177,8 @@ __device__ __forceinline__ void gemm_weight_warps(const GemmParams &p, unsigned 
                     v0 = dequant8b_slow(cw[0].x, cw[0].y, zf, sf); v1 = dequant8b_slow(cw[0].z, cw[0].w, zf, sf);
                     v2 = dequant8b_slow(cw[kCodeVec - 1].x, cw[kCodeVec - 1].y, zf, sf); v3 = dequant8b_slow(cw[kCodeVec - 1].z, cw[kCodeVec - 1].w, zf, sf);
                 }
+                // the previous stage is handed over only now: its stores have landed while this one was converted, and the fence does not wait
+                if (kt > 0) hand_over((kt - 1) % kGStages);
                 if (ok && use > 0 && !mbar_wait_warp(&empty[s], (use - 1) & 1, p.err)) ok = false;
                 unsigned char *dst = As + (size_t)s * kABytes + row_off;
                 const int x = r & 7;  // chunk c = columns 8c .. 8c + 7 of the atom's 64, stored at chunk c ^ (row & 7)
@@ -179,12 +186,10 @@ __device__ __forceinline__ void gemm_weight_warps(const GemmParams &p, unsigned 
                 *reinterpret_cast<uint4 *>(dst + (((c0 + 1) ^ x) << 4)) = v1;
                 *reinterpret_cast<uint4 *>(dst + (((c0 + 2) ^ x) << 4)) = v2;
                 *reinterpret_cast<uint4 *>(dst + (((c0 + 3) ^ x) << 4)) = v3;
-                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // generic-proxy writes -> visible to the tensor core
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&full[s]);
             }
         }
     }
+    hand_over((G - 1) % kGStages);
 }
 
 template <int TN, int BITS>
@@ -390,29 +395,29 @@ int gemm_launch(const GemmParams &p, const Device *dev, cudaStream_t st) {
 static bool gemm_takes(const AffineWeight *w) { return (w->bits == 4 || w->bits == 8) && w->group_size == 128 && w->K % 128 == 0; }
 
 // The tokens as the projection reads them: x itself, or f16(x / awq) in the scratch.
-static int scaled_tokens(const AffineWeight *w, const __half *x, int M, __half *xs_scratch, cudaStream_t st, const __half **out) {
+static int scaled_tokens(const AffineWeight *w, const __half *x, int M, __half *xs_scratch, bool scaled, cudaStream_t st, const __half **out) {
     *out = x;
-    if (!w->awq && reinterpret_cast<uintptr_t>(x) % 16 == 0) return IM_OK;
+    if ((scaled || !w->awq) && reinterpret_cast<uintptr_t>(x) % 16 == 0) return IM_OK;
     const size_t n = (size_t)M * w->K;
-    IM_CUDA_CHECK(launch_k(act_scale_kernel, dim3((unsigned)((n / 8 + 255) / 256)), dim3(256), 0, st, x, (const __half *)w->awq, xs_scratch, n, w->K));
+    IM_CUDA_CHECK(launch_k(act_scale_kernel, dim3((unsigned)((n / 8 + 255) / 256)), dim3(256), 0, st, x, (const __half *)(scaled ? nullptr : w->awq), xs_scratch, n, w->K));
     *out = xs_scratch;
     return IM_OK;
 }
 
 bool gemm_affine_joins(const AffineWeight *gate, int M) { return gemm_takes(gate) && pair_gemm_takes(gate->dev, 2 * gate->N, M); }
 
-int gemm_affine_gate_up(const AffineWeight *gate, const AffineWeight *up, const __half *x, __half *y, int M, __half *xs_scratch, cudaStream_t st) {
+int gemm_affine_gate_up(const AffineWeight *gate, const AffineWeight *up, const __half *x, __half *y, int M, __half *xs_scratch, cudaStream_t st, bool scaled) {
     const __half *xs;
-    const int rc = scaled_tokens(gate, x, M, xs_scratch, st, &xs);
+    const int rc = scaled_tokens(gate, x, M, xs_scratch, scaled, st, &xs);
     return rc != IM_OK ? rc : pair_gemm_affine(gate, up, xs, y, M, st);
 }
 
 // Y[M, N] = f16(X / awq) * dequant(W)^T for M tokens.  xs_scratch: M * K halves.  IM_ERR_BOUNDS when the weight is not
 // INT4 group-128 with K a multiple of 128 (the caller falls back to the matvec kernels).
-int gemm_affine_tc(const AffineWeight *w, const __half *x, __half *y, int M, __half *xs_scratch, cudaStream_t st) {
+int gemm_affine_tc(const AffineWeight *w, const __half *x, __half *y, int M, __half *xs_scratch, cudaStream_t st, bool scaled) {
     if (!gemm_takes(w) || M < 1) return IM_ERR_BOUNDS;
     const __half *xs;
-    if (const int rc = scaled_tokens(w, x, M, xs_scratch, st, &xs); rc != IM_OK) return rc;
+    if (const int rc = scaled_tokens(w, x, M, xs_scratch, scaled, st, &xs); rc != IM_OK) return rc;
     if (pair_gemm_takes(w->dev, w->N, M)) return pair_gemm_affine(w, nullptr, xs, y, M, st);
     GemmParams p{w->codes, w->sz, xs, y, w->N, w->K, w->G, M, w->dev->err_flag, nullptr, w->G};
     // Few tokens and few row tiles (decode batches of 16-64 against 4096-6144 rows: 32-48 CTAs of 32-112 sequential

@@ -257,6 +257,37 @@ __global__ void silu_mul_kernel(const __half *__restrict__ gate, const __half *_
     *reinterpret_cast<__half2 *>(out + i) = __floats2half2_rn((g.x / (1.0f + expf(-g.x))) * u.x, (g.y / (1.0f + expf(-g.y))) * u.y);
 }
 
+// The same for rows of I values, eight at a time, 16-byte aligned; div: the result, rounded, divided by div[column]
+__global__ void __launch_bounds__(256) silu_mul_rows_kernel(const uint4 *__restrict__ gate, const uint4 *__restrict__ up, const uint4 *__restrict__ div,
+                                                            uint4 *__restrict__ out, size_t n8, int row8) {
+    pdl_trigger();
+    pdl_wait();
+    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n8) return;
+    const uint4 gv = gate[i], uv = up[i];
+    uint4 dv = make_uint4(0, 0, 0, 0), r;
+    if (div) dv = div[i % (size_t)row8];
+    const __half2 *hg = reinterpret_cast<const __half2 *>(&gv), *hu = reinterpret_cast<const __half2 *>(&uv), *hd = reinterpret_cast<const __half2 *>(&dv);
+    __half2 *hr = reinterpret_cast<__half2 *>(&r);
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+        const float2 g = __half22float2(hg[j]), u = __half22float2(hu[j]);
+        hr[j] = __floats2half2_rn((g.x / (1.0f + expf(-g.x))) * u.x, (g.y / (1.0f + expf(-g.y))) * u.y);
+        if (div) {
+            const float2 q = __half22float2(hr[j]), d = __half22float2(hd[j]);
+            hr[j] = __floats2half2_rn(q.x / d.x, q.y / d.y);
+        }
+    }
+    out[i] = r;
+}
+// I: a multiple of 128 (the projections that call for it)
+static int silu_mul_rows(const __half *gate, const __half *up, const __half *div, __half *out, int M, int I, cudaStream_t st) {
+    const size_t n8 = (size_t)M * I / 8;
+    IM_CUDA_CHECK(launch_k(silu_mul_rows_kernel, dim3((unsigned)((n8 + 255) / 256)), dim3(256), 0, st, reinterpret_cast<const uint4 *>(gate),
+                           reinterpret_cast<const uint4 *>(up), reinterpret_cast<const uint4 *>(div), reinterpret_cast<uint4 *>(out), n8, I / 8));
+    return IM_OK;
+}
+
 }  // namespace im
 // silu_gate as an entry point of its own (the prefill form of the FFN: gate and up are rounded to fp16 first).
 // out may alias gate.  n even.
@@ -438,6 +469,25 @@ static int attention_block(Model *m, int part, const TqPrep &a, __half *q_buf, L
                                nseq, a.nh, a.nkv, c.max_seq_len, 0, m->pos_dev, T, attn_splits, st, m->qrot, slots);
 }
 
+// Logits of `rows` normed rows. The matvec reads the whole table for every four rows (up to 64 rows per call); from five rows on one pass on the
+// tensor cores reads it once (24 rows, 32768 x 4096: six passes of 65 us, one of 50).
+static int head_rows(Model *m, const __half *x, __half *out, int rows, cudaStream_t st, int *nl) {
+    const int H = m->cfg.hidden_size;
+    if (rows > 4) {
+        const int rc = dense_rows_f16(m->dev, m->lm_head, m->vocab_l, H, x, out, rows, st);
+        if (rc != IM_ERR_BOUNDS) {
+            ++*nl;
+            return rc;
+        }
+    }
+    for (int r = 0; r < rows; r += 64) {
+        const int nb = rows - r < 64 ? rows - r : 64;
+        IM_TRY(im_cuda_matvec_f16(m->lm_head, x + (size_t)r * H, out + (size_t)r * m->vocab_l, m->vocab_l, H, nb, st));
+        *nl += (nb + 3) / 4;
+    }
+    return IM_OK;
+}
+
 int Model::forward(int nseq, int T, cudaStream_t st, int *launches, Prof *prof, bool all_logits, const int *slots) {
     Model *const m = this;
     const im_model_config &c = m->cfg;
@@ -487,32 +537,35 @@ int Model::forward(int nseq, int T, cudaStream_t st, int *launches, Prof *prof, 
         IM_MARK(kCatOProj);
         IM_TRY(tp_allreduce(m, m->ffn_down, (size_t)MT * H, st));  // tensor parallel: o is row-split
         if (m->world > 1) IM_MARK(kCatComm);
-        IM_TRY(im_cuda_fused_residual_rms_norm(m->hidden, m->ffn_down, L.post_ln, m->norm_out, m->residual, H, MT, eps, st));
+        // what a projection with activation scales reads, f16(x / awq), is written by the norm and by the activation's own kernel; in the epilogues of
+        // attention and of the joint projection the divisions took more time than the pass that they would save
+        int rc = L.ffn_joint ? residual_norm_scaled(m->hidden, m->ffn_down, L.post_ln, L.gate->awq, m->norm_out, m->residual, H, MT, eps, st) : IM_ERR_BOUNDS;
+        const bool scaled = rc == IM_OK;
+        if (rc == IM_ERR_BOUNDS) rc = im_cuda_fused_residual_rms_norm(m->hidden, m->ffn_down, L.post_ln, m->norm_out, m->residual, H, MT, eps, st);
+        IM_TRY(rc);
         IM_MARK(kCatResNorm);
         const bool joint = L.ffn_joint && gemm_affine_joins(L.gate, MT);
         if (joint) {
-            IM_TRY(gemm_affine_gate_up(L.gate, L.up, m->norm_out, m->ffn_gate, MT, m->xs_scratch, st));
+            IM_TRY(gemm_affine_gate_up(L.gate, L.up, m->norm_out, m->ffn_gate, MT, m->xs_scratch, st, scaled));
         } else {
-            IM_TRY(gemm_affine_tc(L.gate, m->norm_out, m->ffn_gate, MT, m->xs_scratch, st));
-            IM_TRY(gemm_affine_tc(L.up, m->norm_out, m->ffn_up, MT, m->xs_scratch, st));
-            {
-                const size_t n = (size_t)MT * m->I_l;
-                cudaError_t le = launch_k(silu_mul_kernel, dim3((unsigned)((n / 2 + 255) / 256)), dim3(256), 0, st, (const __half *)m->ffn_gate,
-                                          (const __half *)m->ffn_up, m->ffn_gate, n);
-                if (le != cudaSuccess) return fail(IM_ERR_CUDA, "launch failed: %s", cudaGetErrorString(le));
-            }
+            IM_TRY(gemm_affine_tc(L.gate, m->norm_out, m->ffn_gate, MT, m->xs_scratch, st, scaled));
+            IM_TRY(gemm_affine_tc(L.up, m->norm_out, m->ffn_up, MT, m->xs_scratch, st, scaled));
+            IM_TRY(silu_mul_rows(m->ffn_gate, m->ffn_up, L.down->awq, m->ffn_gate, MT, m->I_l, st));
         }
         IM_MARK(kCatFfn);
-        IM_TRY(gemm_affine_tc(L.down, m->ffn_gate, m->ffn_down, MT, m->xs_scratch, st));
+        IM_TRY(gemm_affine_tc(L.down, m->ffn_gate, m->ffn_down, MT, m->xs_scratch, st, !joint));
         IM_MARK(kCatDown);
         IM_TRY(tp_allreduce(m, m->ffn_down, (size_t)MT * H, st));  // tensor parallel: down is row-split
         if (m->world > 1) IM_MARK(kCatComm);
-        nl += (joint ? 7 : 11) + (m->world > 1 ? 2 : 0);
+        nl += 7 + (m->world > 1 ? 2 : 0);
         if (l + 1 < c.num_layers) {
             Layer &Nx = m->layers[l + 1];
-            IM_TRY(im_cuda_fused_residual_rms_norm(m->residual, m->ffn_down, Nx.input_ln, m->norm_out, m->hidden, H, MT, eps, st));
-            IM_TRY(gemm_affine_tc(Nx.qkv, m->norm_out, m->qkv, MT, m->xs_scratch, st));
-            nl += 3;
+            rc = residual_norm_scaled(m->residual, m->ffn_down, Nx.input_ln, Nx.qkv->awq, m->norm_out, m->hidden, H, MT, eps, st);
+            const bool qkv_scaled = rc == IM_OK;
+            if (rc == IM_ERR_BOUNDS) rc = im_cuda_fused_residual_rms_norm(m->residual, m->ffn_down, Nx.input_ln, m->norm_out, m->hidden, H, MT, eps, st);
+            IM_TRY(rc);
+            IM_TRY(gemm_affine_tc(Nx.qkv, m->norm_out, m->qkv, MT, m->xs_scratch, st, qkv_scaled));
+            nl += 2;
             IM_MARK(kCatQkv);
         } else {
             IM_TRY(im_cuda_residual_add(m->residual, m->ffn_down, m->hidden, (size_t)MT * H, st));
@@ -594,11 +647,8 @@ int Model::forward(int nseq, int T, cudaStream_t st, int *launches, Prof *prof, 
     }
     if (all_logits) {  // final norm + lm_head on every token of the (single) sequence: prefill_all_logits
         IM_TRY(im_cuda_rms_norm(m->hidden, m->final_norm, m->norm_out, H, MT, eps, st));
-        for (int r = 0; r < MT; r += 64) {  // the fp16 matvec takes up to 64 rows per call
-            const int nb = MT - r < 64 ? MT - r : 64;
-            IM_TRY(im_cuda_matvec_f16(m->lm_head, m->norm_out + (size_t)r * H, m->logits_seq + (size_t)r * m->vocab_l, m->vocab_l, H, nb, st));
-        }
-        nl += 1 + (MT + 3) / 4;
+        IM_TRY(head_rows(m, m->norm_out, m->logits_seq, MT, st, &nl));
+        nl++;
         if (m->world > 1) {
 #if IM_HAVE_NCCL_H
             IM_NCCL_CHECK(nccl()->AllGather(m->logits_seq, m->logits_seq_all, (size_t)MT * m->vocab_l, ncclHalf, m->comm, st));
@@ -609,13 +659,16 @@ int Model::forward(int nseq, int T, cudaStream_t st, int *launches, Prof *prof, 
         return IM_OK;
     }
     // final norm + lm_head on the last token of each sequence
-    for (int s = 0; s < nseq; s++) {
+    if (T == 1) {  // one row per sequence: one launch
+        IM_TRY(im_cuda_rms_norm(m->hidden, m->final_norm, m->norm_out, H, nseq, eps, st));
+        nl++;
+    }
+    for (int s = 0; s < nseq && T > 1; s++) {
         const __half *last = m->hidden + ((size_t)s * T + (T - 1)) * H;
         IM_TRY(im_cuda_rms_norm(last, m->final_norm, m->norm_out + (size_t)s * H, H, 1, eps, st));
         nl++;
     }
-    IM_TRY(im_cuda_matvec_f16(m->lm_head, m->norm_out, m->logits, m->vocab_l, H, nseq, st));
-    nl += (nseq + 3) / 4;
+    IM_TRY(head_rows(m, m->norm_out, m->logits, nseq, st, &nl));
     if (m->world > 1) {
 #if IM_HAVE_NCCL_H
         IM_NCCL_CHECK(nccl()->AllGather(m->logits, m->logits_all, (size_t)nseq * m->vocab_l, ncclHalf, m->comm, st));

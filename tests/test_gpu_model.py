@@ -393,3 +393,17 @@ def test_gpu_quantizer_produces_a_loadable_bundle(tmp_path):
     prompt = np.array([3, 250, 17, 99, 4], np.uint32)
     assert np.abs(eng.prefill(prompt) - ref.forward(prompt)).max() <= 5e-2
     assert np.abs(eng.decode_step(8) - ref.forward([8])).max() <= 5e-2
+
+
+def test_head_of_many_rows_and_ragged_rows():
+    # from five rows on the head is one pass on the tensor cores; a vocabulary of no multiple of eight
+    cfg = _cfg("llama", 2, 256, 384, 2, 1, 333, 5e5, 1e-5, tie=True)
+    tensors = synth_model(cfg, seed=31, awq=True)
+    eng, ref = _engines(cfg, tensors, 64)
+    toks = H.rng_for("rows").integers(0, 333, 37).astype(np.uint32)
+    rows = eng.prefill_all_logits(toks)
+    assert np.abs(rows[-1] - ref.forward(toks)).max() <= 5e-2
+    eng.reset()
+    for n in (5, 16, 36):
+        eng.reset()
+        assert np.abs(eng.prefill(toks[:n]) - rows[n - 1]).max() <= 5e-2
