@@ -19,6 +19,7 @@
 #include <math.h>
 
 #include <new>
+#include <algorithm>
 #include <vector>
 
 #include "common.cuh"
@@ -172,30 +173,32 @@ __global__ void __launch_bounds__(kHd) tq_reduce_kernel(const float *__restrict_
 // The split attention above spends its time in shared-memory gathers (one codebook lookup per cached byte, bank
 // conflicts included) and f32 FMAs; at long context it reaches a few per cent of HBM bandwidth.  This kernel keeps
 // the same arithmetic contract and partial format but
-//   * every warp walks its own run of 32-position tiles: the K and V rows go from global memory straight into
-//     registers (a lane owns 32-byte / 16-byte pieces of whole rows, all coalesced), no block barrier in the loop;
-//   * the codebooks are shared-memory tables replicated once per lane (entry b of lane l at word 32 b + l): a
-//     gather never meets a bank conflict.  K entries carry (centroid, QJL sign) as an fp16 pair, V entries the centroid;
-//   * the dot products run on mma.sync m16n8k16 (fp16 operands, f32 accumulation): scores as
-//     [16 positions x 16 dims] x [16 dims x 8] with columns 0-3 = the GQ rotated queries against the centroid
-//     fragment and columns 4-7 = S q against the sign fragment; outputs as [16 dims x 16 positions] x
+//   * every warp walks its own 32-position tiles: the K and V rows go from global memory straight into
+//     registers (a lane owns 32-byte / 16-byte pieces of whole rows, all coalesced), V rows requested before the scores, the next
+//     tile's K rows after them; no block barrier in the loop;
+//   * the codebooks are shared-memory tables replicated once per lane: a gather never meets a bank conflict, and its address is one byte
+//     permute of the cache word (lut_at).  K entries carry (centroid, QJL sign) as an fp16 pair, V entries the centroid;
+//   * the dot products run on mma.sync m16n8k16 (fp16 operands, f32 accumulation): scores with (centroid, sign) as neighbouring
+//     elements of the inner dimension, so that a table entry is an operand register as it is: columns 0-3 = the GQ rotated queries with zeros
+//     against the signs, columns 4-7 = S q with zeros against the centroids; outputs as [16 dims x 16 positions] x
 //     [16 positions x 8 heads].  The fragment <-> (dimension, position) assignment is chosen so that a fragment
 //     register is built from bytes the lane already holds.
-// The eight warps of a CTA take consecutive runs of one (KV head, token, split) and merge their results in shared
-// memory, so the number of partials per head is the same as with the kernel above.
-constexpr int kTcWarps = 8;
+// The warps of a CTA take the tiles of one (KV head, token, split) in turn and merge their results in shared
+// memory, so the number of partials per head is the same as with the kernel above.  Two CTAs per SM walk all (KV head, token, split) items
+// with one table.  mma.sync issue bounds it (48 products per tile, one per 32 clocks and SM quarter).  16 sequences of 1024 .. 8192
+// positions, 32 / 8 heads: 166 us with eight warps, rows loaded where they were used and a CTA per item.
+constexpr int kTcWarps = 6;  // two CTAs per SM: 168 registers a thread, for a tile's V rows and the next tile's K rows in flight
 __device__ __forceinline__ void mma_f16(float (&c)[4], unsigned a0, unsigned a1, unsigned a2, unsigned a3, unsigned b0, unsigned b1) {
     asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
                  : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
                  : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
-// table word of element `idx` of cache word w for this lane: bytes (BITS = 8, idx 0-3) or nibbles (BITS = 4, idx 0-7)
+// Table words of the lane: entry b of lane l at byte 256 b + 4 l (K: centroid | sign) and 256 b + 128 + 4 l (V: centroid), so that one byte permute
+// of the cache word forms the address.  idx: byte (BITS = 8, 0-3) or nibble (BITS = 4, 0-7) of w.
 template <int BITS>
-__device__ __forceinline__ unsigned lut_at(unsigned lane_base, unsigned w, int idx) {
-    const unsigned b = BITS == 8 ? __byte_perm(w, 0, 0x4440 + idx) : ((w >> (4 * idx)) & 15u);
-    unsigned v;
-    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(b * 128u + lane_base));
-    return v;
+__device__ __forceinline__ unsigned lut_at(const unsigned char *lut, unsigned lane_off, unsigned w, int idx) {
+    const unsigned at = BITS == 8 ? __byte_perm(w, lane_off, 0x5504 + (idx << 4)) : (((idx >= 2 ? w >> (4 * idx - 8) : w << (8 - 4 * idx)) & 0xF00u) | lane_off);
+    return *reinterpret_cast<const unsigned *>(lut + at);
 }
 __device__ __forceinline__ unsigned pack_h2(float a, float b) {
     const __half2 h = __floats2half2_rn(a, b);
@@ -203,241 +206,242 @@ __device__ __forceinline__ unsigned pack_h2(float a, float b) {
 }
 
 template <int GQ, int BITS>
-__global__ void __launch_bounds__(kTcWarps * 32, 2) tq_attention_tc_kernel(const AttnParams p) {
+__global__ void __launch_bounds__(kTcWarps * 32, 2) tq_attention_tc_kernel(const AttnParams p, int items) {
     constexpr int kRowB = BITS == 4 ? kHd / 2 : kHd;  // bytes of a cached row
-    extern __shared__ __align__(16) unsigned char tc_smem[];
-    unsigned *lutk = reinterpret_cast<unsigned *>(tc_smem);        // [256][32]: (centroid, sign) fp16 pair
-    unsigned *lutv = lutk + 256 * 32;                               // [256][32]: (centroid, 0)
-    __half *pw = reinterpret_cast<__half *>(lutv + 256 * 32);       // [warps][4 heads][32 positions] softmax weights x v scale
+    constexpr int kKV = BITS == 8 ? 2 : 1;            // 16-byte vectors of a lane's piece of a K row
+    extern __shared__ __align__(256) unsigned char tc_smem[];
+    unsigned char *lut = tc_smem;                                  // [256][K of 32 lanes | V of 32 lanes] (16 entries for 4-bit caches)
+    __half *pw = reinterpret_cast<__half *>(lut + 256 * 256);      // [warps][4 heads][32 positions] softmax weights x v scale
     float *comb = reinterpret_cast<float *>(pw + kTcWarps * 4 * 32);  // [warps][4 heads][130]: o, m, l of each warp
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
-    const int kvh = blockIdx.x, st = blockIdx.y, split = blockIdx.z;
     pdl_trigger();
     {   // tables (constants): before the dependency wait
-        const int b = tid;  // 256 threads, one stored value each (4-bit caches use the first 16 entries)
         constexpr int kSign = 1 << (BITS - 1), kVals = 1 << BITS;
-        const __half2 ke = __floats2half2_rn(p.k_cb[b & (kSign - 1)], (b & kSign) ? 1.0f : -1.0f);
-        const __half2 ve = __floats2half2_rn(p.v_cb[b & (kVals - 1)], 0.0f);
-        const unsigned ku = *reinterpret_cast<const unsigned *>(&ke), vu = *reinterpret_cast<const unsigned *>(&ve);
-        uint4 *dk = reinterpret_cast<uint4 *>(lutk + b * 32), *dv = reinterpret_cast<uint4 *>(lutv + b * 32);
-#pragma unroll
-        for (int i = 0; i < 8; i++) {
-            dk[i] = make_uint4(ku, ku, ku, ku);
-            dv[i] = make_uint4(vu, vu, vu, vu);
+        for (int i = tid; i < kVals * 16; i += kTcWarps * 32) {  // sixteen 16-byte stores per entry
+            const int b = i >> 4;
+            const __half2 ke = __floats2half2_rn(p.k_cb[b & (kSign - 1)], (b & kSign) ? 1.0f : -1.0f);
+            const __half2 ve = __floats2half2_rn(p.v_cb[b], 0.0f);
+            const unsigned u = (i & 8) ? *reinterpret_cast<const unsigned *>(&ve) : *reinterpret_cast<const unsigned *>(&ke);
+            reinterpret_cast<uint4 *>(lut)[i] = make_uint4(u, u, u, u);
         }
     }
     pdl_wait();
     __syncthreads();
-
-    const int seq = st / p.T, tt = st % p.T;
-    const int slot = cache_slot(p.slot_map, seq);
-    const int seq_len = min(p.base_pos + (p.pos_dev ? p.pos_dev[slot] : 0) + tt + 1, p.max_seq);  // see tq_attention_kernel
-    const int chunk = (seq_len + p.splits - 1) / p.splits;
-    const int c0 = split * chunk, c1 = min(c0 + chunk, seq_len);
-    // this warp's run: whole tiles of the split's range
-    const int tiles = (max(c1 - c0, 0) + kTile - 1) / kTile, per = (tiles + kTcWarps - 1) / kTcWarps;
-    const int r0 = c0 + warp * per * kTile, r1 = min(c1, r0 + per * kTile);
-    const int h0 = kvh * GQ;
-    const size_t head_base = ((size_t)slot * p.nkv + kvh) * p.max_seq;
-    const unsigned lk = (unsigned)__cvta_generic_to_shared(lutk) + lane * 4u, lv = (unsigned)__cvta_generic_to_shared(lutv) + lane * 4u;
-
-    // B fragments of the score products: lane (n = g, t) holds dims 32 t + 4 j + {0..3} of column n: the rotated query
-    // of head n (n < GQ, against centroids) or S q of head n - 4 (4 <= n < 4 + GQ, against signs); zero otherwise
-    // (one register set: a lane has either query or S q values; the other product of the pair gets zeros)
-    unsigned bx[16];
-#pragma unroll
-    for (int i = 0; i < 16; i++) bx[i] = 0u;
-    const bool is_c = g < 4;  // this lane's column belongs to the centroid product
-    if (g < GQ || (g >= 4 && g < 4 + GQ)) {
-        const float *src = p.qrot + ((size_t)st * p.nh + h0 + (g < 4 ? g : g - 4)) * 2 * kHd + (g < 4 ? 0 : kHd) + 32 * t;
-#pragma unroll
-        for (int j = 0; j < 8; j++) {
-            const float4 v = *reinterpret_cast<const float4 *>(src + 4 * j);
-            bx[2 * j] = pack_h2(v.x, v.y);
-            bx[2 * j + 1] = pack_h2(v.z, v.w);
-        }
-    }
-
-    float m_run[2] = {-INFINITY, -INFINITY}, l_run[2] = {0.0f, 0.0f};  // lanes t < 2: heads 2t, 2t + 1
-    float o[8][4];                                                       // o[mb]: dims 16g + 2mb, +1 (rows) x heads 2t, 2t+1
-#pragma unroll
-    for (int i = 0; i < 8; i++) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.0f;
+    const unsigned lane_k = lane * 4u, lane_v = 128u + lane * 4u;
+    // halves of a packed query pair as B operand words against (centroid, sign) pairs: (q, 0) for the columns of centroid sums (g < 4),
+    // (0, S q) for the columns of sign sums
+    const unsigned sel0 = g < 4 ? 0x4410u : 0x1044u, sel1 = g < 4 ? 0x4432u : 0x3244u;
     __half *pwarp = pw + warp * 4 * 32;
 
-    for (int ts = r0; ts < r1; ts += kTile) {
-        const int nt = min(kTile, r1 - ts);
-        // ---- K rows g, g+8, g+16, g+24 of the tile: dims 32t .. 32t+31 each (32 bytes, or 16 bytes of nibbles) ----
-        uint4 kq[4][BITS == 8 ? 2 : 1];
-        float ksv[4], rwv[4], vsv[4];
+    for (int item = blockIdx.x; item < items; item += gridDim.x) {
+        const int kvh = item % p.nkv, rest = item / p.nkv, split = rest % p.splits, st = rest / p.splits;
+        const int seq = st / p.T, tt = st % p.T;
+        const int slot = cache_slot(p.slot_map, seq);
+        const int seq_len = min(p.base_pos + (p.pos_dev ? p.pos_dev[slot] : 0) + tt + 1, p.max_seq);  // see tq_attention_kernel
+        const int chunk = ((seq_len + p.splits - 1) / p.splits + kTile - 1) / kTile * kTile;
+        const int c0 = split * chunk, c1 = min(c0 + chunk, seq_len);
+        // this warp's tiles of the split's range: every kTcWarps-th
+        const int tiles = (max(c1 - c0, 0) + kTile - 1) / kTile;
+        const int h0 = kvh * GQ;
+        const size_t head_base = ((size_t)slot * p.nkv + kvh) * p.max_seq;
+        const uint8_t *krow = p.kc + head_base * kRowB, *vrow = p.vc + head_base * kRowB;
+
+        // B fragments of the score products: lane (n = g, t) holds dims 32 t + 2 i, + 1 of column n: the rotated query
+        // of head n (n < GQ) or S q of head n - 4 (4 <= n < 4 + GQ); zero otherwise
+        unsigned bx[16];
 #pragma unroll
-        for (int r = 0; r < 4; r++) {
-            const int pos = g + 8 * r;
-            kq[r][0] = make_uint4(0, 0, 0, 0);
-            if (BITS == 8) kq[r][BITS == 8 ? 1 : 0] = make_uint4(0, 0, 0, 0);
-            ksv[r] = rwv[r] = vsv[r] = 0.0f;
-            if (pos < nt) {
-                const uint4 *src = reinterpret_cast<const uint4 *>(p.kc + (head_base + ts + pos) * kRowB + (kRowB / 4) * t);
-                kq[r][0] = ldg_stream_v4(src);
-                if (BITS == 8) kq[r][BITS == 8 ? 1 : 0] = ldg_stream_v4(src + 1);
-                ksv[r] = p.ks[head_base + ts + pos];
-                rwv[r] = p.krn[head_base + ts + pos] * p.qjl_factor;
-                vsv[r] = p.vs[head_base + ts + pos];
-            }
-        }
-        // ---- scores: two 16-position row blocks ----
-        float sc[2][4];  // [row block][c0..c3]
+        for (int i = 0; i < 16; i++) bx[i] = 0u;
+        if (g < GQ || (g >= 4 && g < 4 + GQ)) {
+            const float *src = p.qrot + ((size_t)st * p.nh + h0 + (g < 4 ? g : g - 4)) * 2 * kHd + (g < 4 ? 0 : kHd) + 32 * t;
 #pragma unroll
-        for (int rb = 0; rb < 2; rb++) {
-            float c[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-            const unsigned *wa = reinterpret_cast<const unsigned *>(&kq[2 * rb][0]);      // row g + 16 rb
-            const unsigned *wb = reinterpret_cast<const unsigned *>(&kq[2 * rb + 1][0]);  // row g + 8 + 16 rb
-#pragma unroll
-            for (int j = 0; j < 8; j++) {  // dims 32 t + 4 j + {0..3}: word j (bytes), or half of word j / 2 (nibbles)
-                const unsigned a = BITS == 8 ? wa[j] : wa[j >> 1], b = BITS == 8 ? wb[j] : wb[j >> 1];
-                constexpr int e1 = 1, e2 = 2, e3 = 3;
-                const int e0 = BITS == 8 ? 0 : (j & 1) * 4;
-                const unsigned la0 = lut_at<BITS>(lk, a, e0), la1 = lut_at<BITS>(lk, a, e0 + e1), la2 = lut_at<BITS>(lk, a, e0 + e2), la3 = lut_at<BITS>(lk, a, e0 + e3);
-                const unsigned lb0 = lut_at<BITS>(lk, b, e0), lb1 = lut_at<BITS>(lk, b, e0 + e1), lb2 = lut_at<BITS>(lk, b, e0 + e2), lb3 = lut_at<BITS>(lk, b, e0 + e3);
-                // centroids in the low halves, signs in the high halves
-                mma_f16(c, __byte_perm(la0, la1, 0x5410), __byte_perm(lb0, lb1, 0x5410), __byte_perm(la2, la3, 0x5410),
-                        __byte_perm(lb2, lb3, 0x5410), is_c ? bx[2 * j] : 0u, is_c ? bx[2 * j + 1] : 0u);
-                mma_f16(c, __byte_perm(la0, la1, 0x7632), __byte_perm(lb0, lb1, 0x7632), __byte_perm(la2, la3, 0x7632),
-                        __byte_perm(lb2, lb3, 0x7632), is_c ? 0u : bx[2 * j], is_c ? 0u : bx[2 * j + 1]);
-            }
-            sc[rb][0] = c[0]; sc[rb][1] = c[1]; sc[rb][2] = c[2]; sc[rb][3] = c[3];
-        }
-        // ---- V rows 2t, 2t+1, 2t+8, 2t+9 (+16): dims 16g .. 16g+15 each (16 bytes, or 8 bytes of nibbles in .x/.y) ----
-        uint4 vq[8];
-#pragma unroll
-        for (int r = 0; r < 8; r++) {
-            const int pos = 2 * t + (r & 1) + 8 * ((r >> 1) & 1) + 16 * (r >> 2);
-            vq[r] = make_uint4(0, 0, 0, 0);
-            if (pos < nt) {
-                if (BITS == 8) {
-                    vq[r] = ldg_stream_v4(reinterpret_cast<const uint4 *>(p.vc + (head_base + ts + pos) * kRowB + 16 * g));
-                } else {
-                    const uint2 v2 = __ldcs(reinterpret_cast<const uint2 *>(p.vc + (head_base + ts + pos) * kRowB + 8 * g));
-                    vq[r].x = v2.x;
-                    vq[r].y = v2.y;
-                }
+            for (int j = 0; j < 8; j++) {
+                const float4 v = *reinterpret_cast<const float4 *>(src + 4 * j);
+                bx[2 * j] = pack_h2(v.x, v.y);
+                bx[2 * j + 1] = pack_h2(v.z, v.w);
             }
         }
 
-        // lanes t < 2 hold the centroid sums of heads 2t, 2t+1; lanes t + 2 the sign sums of the same heads
-        float s[4][2];  // [position g + 8 r][head 2t + i]
+        float m_run[2] = {-INFINITY, -INFINITY}, l_run[2] = {0.0f, 0.0f};  // lanes t < 2: heads 2t, 2t + 1
+        float o[8][4];                                                       // o[mb]: dims 16g + 2mb, +1 (rows) x heads 2t, 2t+1
 #pragma unroll
-        for (int rb = 0; rb < 2; rb++)
-#pragma unroll
-            for (int q = 0; q < 4; q++) {
-                const float other = __shfl_xor_sync(0xffffffffu, sc[rb][q], 2);
-                const int r = 2 * rb + (q >> 1), i = q & 1;  // c0,c1: row g ; c2,c3: row g + 8
-                const bool live = t < 2 && g + 8 * r < nt;  // lanes t >= 2 only feed the shuffle above
-                s[r][i] = live ? p.attn_scale * (ksv[r] * (sc[rb][q] + rwv[r] * other)) : -INFINITY;
-            }
-        // ---- online softmax over the tile (meaningful on lanes t < 2; the others carry copies of no use) ----
-        float wgt[4][2];
-#pragma unroll
-        for (int i = 0; i < 2; i++) {
-            float mx = fmaxf(fmaxf(s[0][i], s[1][i]), fmaxf(s[2][i], s[3][i]));
-            mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 4));
-            mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 8));
-            mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 16));
-            const float m_new = fmaxf(m_run[i], mx);
-            const float corr = m_new == -INFINITY ? 1.0f : __expf(m_run[i] - m_new);
-            float sum = 0.0f;
+        for (int i = 0; i < 8; i++) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.0f;
+
+        // K rows g, g+8, g+16, g+24 of a tile: dims 32t .. 32t+31 each (32 bytes, or 16 bytes of nibbles), and the rows' factors
+        uint4 kq[4][kKV];
+        float ksv[4], rwv[4], vsv[4];
+        auto request = [&](int ts) {
 #pragma unroll
             for (int r = 0; r < 4; r++) {
-                wgt[r][i] = s[r][i] == -INFINITY ? 0.0f : __expf(s[r][i] - m_new);
-                sum += wgt[r][i];
-            }
-            sum += __shfl_xor_sync(0xffffffffu, sum, 4);
-            sum += __shfl_xor_sync(0xffffffffu, sum, 8);
-            sum += __shfl_xor_sync(0xffffffffu, sum, 16);
-            l_run[i] = l_run[i] * corr + sum;
-            m_run[i] = m_new;
+                const int pos = ts + g + 8 * r;
+                ksv[r] = rwv[r] = vsv[r] = 0.0f;
 #pragma unroll
-            for (int mb = 0; mb < 8; mb++) {  // heads 2t + i live in accumulator columns i (rows d0) and i + 2 (rows d1)
-                o[mb][i] *= corr;
-                o[mb][i + 2] *= corr;
+                for (int v = 0; v < kKV; v++) kq[r][v] = make_uint4(0, 0, 0, 0);
+                if (pos < c1) {
+                    const uint4 *src = reinterpret_cast<const uint4 *>(krow + (size_t)pos * kRowB + (kRowB / 4) * t);
+#pragma unroll
+                    for (int v = 0; v < kKV; v++) kq[r][v] = __ldcs(src + v);
+                    ksv[r] = p.ks[head_base + pos];
+                    rwv[r] = p.krn[head_base + pos];
+                    vsv[r] = p.vs[head_base + pos];
+                }
+            }
+        };
+        request(c0 + warp * kTile);
+        for (int tile = warp; tile < tiles; tile += kTcWarps) {
+            const int ts = c0 + tile * kTile, nt = min(kTile, c1 - ts);
+            // ---- V rows 2t, 2t+1, 2t+8, 2t+9 (+16): dims 16g .. 16g+15 each (16 bytes, or 8 bytes of nibbles in .x/.y), in flight during the scores ----
+            uint4 vq[8];
+#pragma unroll
+            for (int r = 0; r < 8; r++) {
+                const int pos = 2 * t + (r & 1) + 8 * ((r >> 1) & 1) + 16 * (r >> 2);
+                vq[r] = make_uint4(0, 0, 0, 0);
+                if (pos < nt) {
+                    if (BITS == 8) {
+                        vq[r] = __ldcs(reinterpret_cast<const uint4 *>(vrow + (size_t)(ts + pos) * kRowB + 16 * g));
+                    } else {
+                        const uint2 v2 = __ldcs(reinterpret_cast<const uint2 *>(vrow + (size_t)(ts + pos) * kRowB + 8 * g));
+                        vq[r].x = v2.x;
+                        vq[r].y = v2.y;
+                    }
+                }
+            }
+            // ---- scores: a product of 16 positions x (centroid, sign) of eight dimensions per step, two row blocks ----
+            float sc[2][4];  // [row block][c0..c3]
+#pragma unroll
+            for (int rb = 0; rb < 2; rb++) sc[rb][0] = sc[rb][1] = sc[rb][2] = sc[rb][3] = 0.0f;
+#pragma unroll
+            for (int i = 0; i < 16; i++) {  // dims 32 t + 2 i, + 1
+                const unsigned b0 = __byte_perm(bx[i], 0, sel0), b1 = __byte_perm(bx[i], 0, sel1);
+                const int w = BITS == 8 ? i >> 1 : i >> 2, e = BITS == 8 ? 2 * (i & 1) : 2 * (i & 3);
+#pragma unroll
+                for (int rb = 0; rb < 2; rb++) {
+                    const unsigned a = reinterpret_cast<const unsigned *>(&kq[2 * rb][0])[w], b = reinterpret_cast<const unsigned *>(&kq[2 * rb + 1][0])[w];  // rows g, g + 8 (+ 16 rb)
+                    mma_f16(sc[rb], lut_at<BITS>(lut, lane_k, a, e), lut_at<BITS>(lut, lane_k, b, e), lut_at<BITS>(lut, lane_k, a, e + 1), lut_at<BITS>(lut, lane_k, b, e + 1),
+                            b0, b1);
+                }
+            }
+            // lanes t < 2 hold the centroid sums of heads 2t, 2t+1; lanes t + 2 the sign sums of the same heads
+            float s[4][2], vw[4];  // [position g + 8 r][head 2t + i]
+#pragma unroll
+            for (int rb = 0; rb < 2; rb++)
+#pragma unroll
+                for (int q = 0; q < 4; q++) {
+                    const float other = __shfl_xor_sync(0xffffffffu, sc[rb][q], 2);
+                    const int r = 2 * rb + (q >> 1), i = q & 1;  // c0,c1: row g ; c2,c3: row g + 8
+                    const bool live = t < 2 && g + 8 * r < nt;  // lanes t >= 2 only feed the shuffle above
+                    s[r][i] = live ? p.attn_scale * (ksv[r] * (sc[rb][q] + rwv[r] * p.qjl_factor * other)) : -INFINITY;
+                }
+#pragma unroll
+            for (int r = 0; r < 4; r++) vw[r] = vsv[r];
+            request(tile + kTcWarps < tiles ? ts + kTcWarps * kTile : c1);  // the next tile's K rows travel during the rest of this one
+            // ---- online softmax over the tile (meaningful on lanes t < 2; the others carry copies of no use) ----
+            float wgt[4][2];
+#pragma unroll
+            for (int i = 0; i < 2; i++) {
+                float mx = fmaxf(fmaxf(s[0][i], s[1][i]), fmaxf(s[2][i], s[3][i]));
+                mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 4));
+                mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 8));
+                mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 16));
+                const float m_new = fmaxf(m_run[i], mx);
+                const float corr = m_new == -INFINITY ? 1.0f : __expf(m_run[i] - m_new);
+                float sum = 0.0f;
+#pragma unroll
+                for (int r = 0; r < 4; r++) {
+                    wgt[r][i] = s[r][i] == -INFINITY ? 0.0f : __expf(s[r][i] - m_new);
+                    sum += wgt[r][i];
+                }
+                l_run[i] = l_run[i] * corr + sum;  // this lane's own positions; added up over the lanes at the end
+                m_run[i] = m_new;
+                if (__any_sync(0xffffffffu, corr != 1.0f)) {
+#pragma unroll
+                    for (int mb = 0; mb < 8; mb++) {  // heads 2t + i live in accumulator columns i (rows d0) and i + 2 (rows d1)
+                        o[mb][i] *= corr;
+                        o[mb][i + 2] *= corr;
+                    }
+                }
+            }
+            // weights x V scale, as fp16, to this warp's P[head][position] for the output products
+            __syncwarp();
+            if (t < 2) {
+#pragma unroll
+                for (int r = 0; r < 4; r++)
+#pragma unroll
+                    for (int i = 0; i < 2; i++)
+                        if (2 * t + i < 4) pwarp[(2 * t + i) * 32 + g + 8 * r] = __float2half_rn(wgt[r][i] * vw[r]);
+            }
+            __syncwarp();
+            // ---- outputs: O^T[dims][heads] += V^T[dims][positions] P^T[positions][heads] ----
+#pragma unroll
+            for (int kb = 0; kb < 2; kb++) {
+                unsigned b0 = 0u, b1 = 0u;  // lane (n = g): P[head g][16 kb + 2t, +1] and [.. + 8, + 9]
+                if (g < GQ) {
+                    b0 = *reinterpret_cast<const unsigned *>(pwarp + g * 32 + 16 * kb + 2 * t);
+                    b1 = *reinterpret_cast<const unsigned *>(pwarp + g * 32 + 16 * kb + 2 * t + 8);
+                }
+                const unsigned *v0 = reinterpret_cast<const unsigned *>(&vq[4 * kb + 0]);  // position 16 kb + 2t
+                const unsigned *v1 = reinterpret_cast<const unsigned *>(&vq[4 * kb + 1]);  // + 1
+                const unsigned *v2 = reinterpret_cast<const unsigned *>(&vq[4 * kb + 2]);  // + 8
+                const unsigned *v3 = reinterpret_cast<const unsigned *>(&vq[4 * kb + 3]);  // + 9
+#pragma unroll
+                for (int mb = 0; mb < 8; mb++) {  // rows g, g + 8 of the block: dims 16 g + 2 mb, + 1
+                    const int w = BITS == 8 ? mb >> 1 : mb >> 2, by = BITS == 8 ? 2 * (mb & 1) : 2 * (mb & 3);
+                    auto pair = [&](unsigned x, unsigned y, int e) {
+                        return __byte_perm(lut_at<BITS>(lut, lane_v, x, e), lut_at<BITS>(lut, lane_v, y, e), 0x5410);
+                    };
+                    mma_f16(o[mb], pair(v0[w], v1[w], by), pair(v0[w], v1[w], by + 1), pair(v2[w], v3[w], by), pair(v2[w], v3[w], by + 1), b0, b1);
+                }
             }
         }
-        // weights x V scale, as fp16, to this warp's P[head][position] for the output products
-        __syncwarp();
+#pragma unroll
+        for (int i = 0; i < 2; i++)
+#pragma unroll
+            for (int d = 4; d < 32; d <<= 1) l_run[i] += __shfl_xor_sync(0xffffffffu, l_run[i], d);
+
+        // ---- merge the warps: comb[warp][head][130] = o (dims 0..127), m, l ----
+        __syncthreads();  // the previous item's sums have been read
         if (t < 2) {
 #pragma unroll
-            for (int r = 0; r < 4; r++)
+            for (int i = 0; i < 2; i++) {
+                const int h = 2 * t + i;
+                if (h < 4) {
+                    float *dst = comb + (warp * 4 + h) * 130;
 #pragma unroll
-                for (int i = 0; i < 2; i++)
-                    if (2 * t + i < 4) pwarp[(2 * t + i) * 32 + g + 8 * r] = __float2half_rn(wgt[r][i] * vsv[r]);
-        }
-        __syncwarp();
-        // ---- outputs: O^T[dims][heads] += V^T[dims][positions] P^T[positions][heads] ----
-#pragma unroll
-        for (int kb = 0; kb < 2; kb++) {
-            unsigned b0 = 0u, b1 = 0u;  // lane (n = g): P[head g][16 kb + 2t, +1] and [.. + 8, + 9]
-            if (g < GQ) {
-                b0 = *reinterpret_cast<const unsigned *>(pwarp + g * 32 + 16 * kb + 2 * t);
-                b1 = *reinterpret_cast<const unsigned *>(pwarp + g * 32 + 16 * kb + 2 * t + 8);
-            }
-            const unsigned *v0 = reinterpret_cast<const unsigned *>(&vq[4 * kb + 0]);  // position 16 kb + 2t
-            const unsigned *v1 = reinterpret_cast<const unsigned *>(&vq[4 * kb + 1]);  // + 1
-            const unsigned *v2 = reinterpret_cast<const unsigned *>(&vq[4 * kb + 2]);  // + 8
-            const unsigned *v3 = reinterpret_cast<const unsigned *>(&vq[4 * kb + 3]);  // + 9
-#pragma unroll
-            for (int mb = 0; mb < 8; mb++) {  // rows g, g + 8 of the block: dims 16 g + 2 mb, + 1
-                const int w = BITS == 8 ? mb >> 1 : mb >> 2, by = BITS == 8 ? 2 * (mb & 1) : 2 * (mb & 3);
-                const unsigned e00 = lut_at<BITS>(lv, v0[w], by), e01 = lut_at<BITS>(lv, v1[w], by), e10 = lut_at<BITS>(lv, v0[w], by + 1), e11 = lut_at<BITS>(lv, v1[w], by + 1);
-                const unsigned f00 = lut_at<BITS>(lv, v2[w], by), f01 = lut_at<BITS>(lv, v3[w], by), f10 = lut_at<BITS>(lv, v2[w], by + 1), f11 = lut_at<BITS>(lv, v3[w], by + 1);
-                mma_f16(o[mb], __byte_perm(e00, e01, 0x5410), __byte_perm(e10, e11, 0x5410), __byte_perm(f00, f01, 0x5410),
-                        __byte_perm(f10, f11, 0x5410), b0, b1);
-            }
-        }
-        __syncwarp();
-    }
-
-    // ---- merge the warps: comb[warp][head][130] = o (dims 0..127), m, l ----
-    if (t < 2) {
-#pragma unroll
-        for (int i = 0; i < 2; i++) {
-            const int h = 2 * t + i;
-            if (h < 4) {
-                float *dst = comb + (warp * 4 + h) * 130;
-#pragma unroll
-                for (int mb = 0; mb < 8; mb++) {
-                    dst[16 * g + 2 * mb] = o[mb][i];
-                    dst[16 * g + 2 * mb + 1] = o[mb][i + 2];
-                }
-                if (g == 0) {
-                    dst[128] = m_run[i];
-                    dst[129] = l_run[i];
+                    for (int mb = 0; mb < 8; mb++) {
+                        dst[16 * g + 2 * mb] = o[mb][i];
+                        dst[16 * g + 2 * mb + 1] = o[mb][i + 2];
+                    }
+                    if (g == 0) {
+                        dst[128] = m_run[i];
+                        dst[129] = l_run[i];
+                    }
                 }
             }
         }
-    }
-    __syncthreads();
-    for (int idx = tid; idx < GQ * kHd; idx += kTcWarps * 32) {
-        const int h = idx >> 7, d = idx & 127;
-        float gm = -INFINITY;
+        __syncthreads();
+        for (int idx = tid; idx < GQ * kHd; idx += kTcWarps * 32) {
+            const int h = idx >> 7, d = idx & 127;
+            float gm = -INFINITY;
 #pragma unroll
-        for (int w = 0; w < kTcWarps; w++) gm = fmaxf(gm, comb[(w * 4 + h) * 130 + 128]);
-        float acc = 0.0f, lsum = 0.0f;
+            for (int w = 0; w < kTcWarps; w++) gm = fmaxf(gm, comb[(w * 4 + h) * 130 + 128]);
+            float acc = 0.0f, lsum = 0.0f;
 #pragma unroll
-        for (int w = 0; w < kTcWarps; w++) {
-            const float m = comb[(w * 4 + h) * 130 + 128];
-            const float corr = m == -INFINITY ? 0.0f : __expf(m - gm);
-            acc += comb[(w * 4 + h) * 130 + d] * corr;
-            lsum += comb[(w * 4 + h) * 130 + 129] * corr;
-        }
-        const size_t pi = ((size_t)st * p.nh + h0 + h) * p.splits + split;
-        p.po[pi * kHd + d] = acc;
-        if (d == 0) {
-            p.pm[pi] = gm;
-            p.pl[pi] = lsum;
+            for (int w = 0; w < kTcWarps; w++) {
+                const float m = comb[(w * 4 + h) * 130 + 128];
+                const float corr = m == -INFINITY ? 0.0f : __expf(m - gm);
+                acc += comb[(w * 4 + h) * 130 + d] * corr;
+                lsum += comb[(w * 4 + h) * 130 + 129] * corr;
+            }
+            const size_t pi = ((size_t)st * p.nh + h0 + h) * p.splits + split;
+            p.po[pi * kHd + d] = acc;
+            if (d == 0) {
+                p.pm[pi] = gm;
+                p.pl[pi] = lsum;
+            }
         }
     }
 }
-constexpr size_t kTcSmem = 2 * 256 * 32 * 4 + kTcWarps * 4 * 32 * 2 + kTcWarps * 4 * 130 * 4;
+constexpr size_t kTcSmem = 256 * 256 + kTcWarps * 4 * 32 * 2 + kTcWarps * 4 * 130 * 4;
 
 // Rotated query and S * rotated query for every (token, head), computed once instead of once per split:
 // grid (nseq*T, nh), 128 threads.  q fp16 [nseq*T, nh, 128] -> qrot f32 [nseq*T, nh, 2, 128].
@@ -608,6 +612,12 @@ IM_EXPORT size_t im_cuda_tq_scratch_bytes(int nseq, int T, int nh, int head_dim,
     return tq_partial_bytes(nseq, T, nh, head_dim, splits) + (size_t)nseq * T * nh * 2 * head_dim * sizeof(float);
 }
 
+namespace im {
+// Automatic split count of a call: from the longest context that it can meet (positions on the device: the cache's length), and scratch for it.  Inside a
+// capture the scratch cannot grow: fewer splits then, if those fit.
+static int tq_call_scratch(im_tq *tq, int num_splits, int nseq, int T, int nh, int nkv, int max_seq, int base_pos, const int *pos_dev, cudaStream_t st, int *out);
+}  // namespace im
+
 IM_EXPORT int im_cuda_tq_reserve_scratch(im_tq *tq, size_t bytes) {
     IM_GUARD_BEGIN
     IM_REQUIRE(tq, "bad argument");
@@ -643,13 +653,12 @@ int tq_prep_launch(const Tq *tq, const TqPrep &a, cudaStream_t st) {
     return IM_OK;
 }
 
+// Parts that the positions of a (sequence, token, KV head) are cut into: enough for two CTAs per SM with one tile per warp of a part; and where parts
+// can hold three tiles per warp, four times as many as CTAs, so that sequences of different lengths share the GPU evenly.
 int tq_auto_splits(const Device *dev, int nseq, int T, int nkv, int seq_len) {
-    const int ctas = nseq * T * nkv;
-    int s = (2 * dev->sm_count + ctas - 1) / ctas;                // two 8-warp CTAs per SM
-    const int by_len = (seq_len + 8 * kTile - 1) / (8 * kTile);  // at least one tile per warp of a split
-    if (s > by_len) s = by_len;
-    if (s > 128) s = 128;
-    return s < 1 ? 1 : s;
+    const long long ctas = (long long)nseq * T * nkv, fill = 2 * dev->sm_count, run = kTcWarps * kTile;
+    const long long a = std::min((fill + ctas - 1) / ctas, (seq_len + run - 1) / run), b = std::min((4 * fill + ctas - 1) / ctas, seq_len / (3 * run));
+    return (int)std::max(1ll, std::min(128ll, std::max(a, b)));
 }
 
 int tq_attention_launch(const Tq *tq, float *scratch, const __half *q, const uint8_t *kc, const uint8_t *vc, const float *ks,
@@ -683,9 +692,9 @@ int tq_attention_launch(const Tq *tq, float *scratch, const __half *q, const uin
         }
         auto kern = tq->n_bits == 4 ? (gq == 1 ? tq_attention_tc_kernel<1, 4> : (gq == 2 ? tq_attention_tc_kernel<2, 4> : tq_attention_tc_kernel<4, 4>))
                                     : (gq == 1 ? tq_attention_tc_kernel<1, 8> : (gq == 2 ? tq_attention_tc_kernel<2, 8> : tq_attention_tc_kernel<4, 8>));
-        int rc = IM_OK;
-        IM_CUDA_CHECK(launch_k(kern, grid, dim3(kTcWarps * 32), kTcSmem, st, p));
-        if (rc != IM_OK) return rc;
+        const long long items = (long long)nkv * nseq * T * splits;
+        if (items > 0x7fffffffll) return fail(IM_ERR_BOUNDS, "attention over %lld parts", items);
+        IM_CUDA_CHECK(launch_k(kern, dim3((unsigned)std::min(items, 2ll * tq->dev->sm_count)), dim3(kTcWarps * 32), kTcSmem, st, p, (int)items));
     } else
     {
         const bool b4 = tq->n_bits == 4;
@@ -732,6 +741,20 @@ IM_EXPORT int im_cuda_tq_prefill_attention(im_tq *tq, const void *q_dev, const v
     IM_GUARD_END
 }
 
+int im::tq_call_scratch(im_tq *tq, int num_splits, int nseq, int T, int nh, int nkv, int max_seq, int base_pos, const int *pos_dev, cudaStream_t st, int *out) {
+    int splits = num_splits > 0 ? num_splits : tq_auto_splits(tq->dev, nseq, T, nkv, pos_dev ? max_seq : base_pos + T);
+    if (im_cuda_tq_scratch_bytes(nseq, T, nh, kHd, splits) > tq->scratch_bytes) {
+        cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+        if (num_splits <= 0 && cudaStreamIsCapturing(st, &cs) == cudaSuccess && cs != cudaStreamCaptureStatusNone)
+            while (splits > 1 && im_cuda_tq_scratch_bytes(nseq, T, nh, kHd, splits) > tq->scratch_bytes) splits--;
+        const size_t need = im_cuda_tq_scratch_bytes(nseq, T, nh, kHd, splits);
+        if (need > tq->scratch_bytes)
+            if (const int rc = im_cuda_tq_reserve_scratch(tq, need); rc != IM_OK) return rc;
+    }
+    *out = splits;
+    return IM_OK;
+}
+
 IM_EXPORT int im_cuda_tq_attention(im_tq *tq, const void *q_dev, const void *k_cache_dev, const void *v_cache_dev,
                                    const float *k_scale_dev, const float *v_scale_dev, const float *k_rnorm_dev, float attn_scale,
                                    void *out_dev, int nseq, int nh, int nkv, int max_seq, int base_pos, const int *pos_dev, int T,
@@ -744,13 +767,9 @@ IM_EXPORT int im_cuda_tq_attention(im_tq *tq, const void *q_dev, const void *k_c
     if (nseq == 0 || T == 0) return IM_OK;
     if (!pos_dev && base_pos + T > max_seq)
         return fail(IM_ERR_BOUNDS, "sequence position %d + %d tokens exceeds max_seq_len %d", base_pos, T, max_seq);
-    int splits = num_splits > 0 ? num_splits : tq_auto_splits(tq->dev, nseq, T, nkv, base_pos + T);
-    IM_REQUIRE(splits <= 1024, "too many splits");
-    const size_t need = im_cuda_tq_scratch_bytes(nseq, T, nh, kHd, splits);
-    if (need > tq->scratch_bytes) {
-        int rc = im_cuda_tq_reserve_scratch(tq, need);
-        if (rc != IM_OK) return rc;
-    }
+    IM_REQUIRE(num_splits <= 1024, "too many splits");
+    int splits = 0;
+    if (const int rc = tq_call_scratch(tq, num_splits, nseq, T, nh, nkv, max_seq, base_pos, pos_dev, as_stream(stream), &splits); rc != IM_OK) return rc;
     // rotate the queries once (every split of a head would otherwise redo the rotation and the 128 x 128 projection)
     float *qrot = tq->scratch + tq_partial_bytes(nseq, T, nh, kHd, splits) / sizeof(float);
     IM_CUDA_CHECK(launch_k(tq_qrot_kernel, dim3(nseq * T, nh), dim3(kHd), 0, as_stream(stream), static_cast<const __half *>(q_dev),
@@ -778,12 +797,8 @@ IM_EXPORT int im_cuda_tq_fused_attention(im_tq *tq, const void *qkv_dev, int qkv
     if (nseq == 0 || T == 0) return IM_OK;
     if (!pos_dev && base_pos + T > max_seq)
         return fail(IM_ERR_BOUNDS, "sequence position %d + %d tokens exceeds max_seq_len %d", base_pos, T, max_seq);
-    const int splits = num_splits > 0 ? num_splits : tq_auto_splits(tq->dev, nseq, T, nkv, base_pos + T);
-    const size_t need = im_cuda_tq_scratch_bytes(nseq, T, nh, kHd, splits);
-    if (need > tq->scratch_bytes) {
-        int rc = im_cuda_tq_reserve_scratch(tq, need);
-        if (rc != IM_OK) return rc;
-    }
+    int splits = 0;
+    if (const int src = tq_call_scratch(tq, num_splits, nseq, T, nh, nkv, max_seq, base_pos, pos_dev, as_stream(stream), &splits); src != IM_OK) return src;
     TqPrep a{};
     a.qkv = static_cast<const __half *>(qkv_dev); a.stride = qkv_stride; a.k_off = k_offset; a.v_off = v_offset;
     a.qw = static_cast<const __half *>(q_norm_w_dev); a.kw = static_cast<const __half *>(k_norm_w_dev);
@@ -834,7 +849,7 @@ IM_EXPORT int im_cuda_tq_attention_static(const im_tq *tq, const void *q_dev, co
     // The array holds what im_cuda_tq_attention keeps in its allocated scratch: the split partials, then the rotated
     // queries of the pre-pass (so both entry points run the same kernels).  A split count chosen here shrinks until
     // the request fits; one given by the caller is taken as it is or refused.
-    int splits = num_splits > 0 ? num_splits : tq_auto_splits(tq->dev, nseq, T, nkv, base_pos + T);
+    int splits = num_splits > 0 ? num_splits : tq_auto_splits(tq->dev, nseq, T, nkv, pos_dev ? max_seq : base_pos + T);
     while (num_splits <= 0 && splits > 1 && im_cuda_tq_scratch_bytes(nseq, T, nh, kHd, splits) > kStaticScratchFloats * sizeof(float)) splits--;
     const size_t need = im_cuda_tq_scratch_bytes(nseq, T, nh, kHd, splits);
     if (need > kStaticScratchFloats * sizeof(float))
