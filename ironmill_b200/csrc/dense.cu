@@ -80,6 +80,56 @@ __device__ __forceinline__ void stage_row(const DenseSrc &s, int m, int K, int l
         return;
     }
     float ss = 0.0f;
+    // Rows of up to 16 values per thread in registers, 16-byte accesses: one trip to memory before the sums instead of one per pass (2048
+    // values by 256 threads; STAGE_FIGURE).  Other rows: below.
+    constexpr int kVecs = 4;
+    const float *add_row = s.kind == kSrcAddNorm && s.xf2 ? s.xf2 + (size_t)m * s.ldx : nullptr;
+    float *out_row = s.kind == kSrcAddNorm && keep && s.xout ? s.xout + (size_t)m * s.ldx : nullptr;
+    const float *g2 = s.kind == kSrcAddNorm ? s.gamma2 : s.gamma;
+    if (K % 4 == 0 && K <= 4 * kVecs * nt &&
+        ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(add_row) | reinterpret_cast<uintptr_t>(out_row) | reinterpret_cast<uintptr_t>(s.gamma) |
+          reinterpret_cast<uintptr_t>(g2) | reinterpret_cast<uintptr_t>(dst)) & 15) == 0) {
+        const int nv = K / 4;
+        float4 v[kVecs], a[kVecs];
+#pragma unroll
+        for (int j = 0; j < kVecs; j++)
+            if (tid + j * nt < nv) {
+                v[j] = reinterpret_cast<const float4 *>(x)[tid + j * nt];
+                if (add_row) a[j] = reinterpret_cast<const float4 *>(add_row)[tid + j * nt];
+            }
+        auto sum_sq = [&](const float4 *r) {
+            float t = 0.0f;
+#pragma unroll
+            for (int j = 0; j < kVecs; j++)
+                if (tid + j * nt < nv) t = fmaf(r[j].x, r[j].x, fmaf(r[j].y, r[j].y, fmaf(r[j].z, r[j].z, fmaf(r[j].w, r[j].w, t))));
+            return 1.0f / sqrtf(block_sum_f(t, sh) / (float)K + s.eps);
+        };
+        if (add_row) {
+            const float inv = sum_sq(a);
+#pragma unroll
+            for (int j = 0; j < kVecs; j++)
+                if (tid + j * nt < nv) {
+                    const float4 g = reinterpret_cast<const float4 *>(s.gamma)[tid + j * nt];
+                    v[j].x += a[j].x * inv * g.x; v[j].y += a[j].y * inv * g.y; v[j].z += a[j].z * inv * g.z; v[j].w += a[j].w * inv * g.w;
+                }
+        }
+        const float inv2 = g2 ? sum_sq(v) : 1.0f;
+#pragma unroll
+        for (int j = 0; j < kVecs; j++)
+            if (tid + j * nt < nv) {
+                const int i = tid + j * nt;
+                if (out_row) reinterpret_cast<float4 *>(out_row)[i] = v[j];
+                if (g2) {
+                    const float4 g = reinterpret_cast<const float4 *>(g2)[i];
+                    v[j].x *= inv2 * g.x; v[j].y *= inv2 * g.y; v[j].z *= inv2 * g.z; v[j].w *= inv2 * g.w;
+                }
+                T q[4] = {from_f<T>(v[j].x), from_f<T>(v[j].y), from_f<T>(v[j].z), from_f<T>(v[j].w)};
+                if (sizeof(T) == 4) reinterpret_cast<uint4 *>(dst)[i] = *reinterpret_cast<const uint4 *>(q);
+                else reinterpret_cast<uint2 *>(dst)[i] = *reinterpret_cast<const uint2 *>(q);
+            }
+        for (int i = K + tid; i < ld; i += nt) dst[i] = from_f<T>(0.0f);
+        return;
+    }
     if (s.kind == kSrcAddNorm) {
         const float *add = s.xf2 ? s.xf2 + (size_t)m * s.ldx : nullptr;
         float inv = 0.0f;

@@ -114,7 +114,9 @@ __device__ __forceinline__ void gemm_weight_warps(const GemmParams &p, unsigned 
     // 16-byte chunks of one swizzle atom.  The codes of the next stages are requested before this stage is converted,
     // so the memory latency is paid once.  Sixteen such warps: four per scheduler to cover each other's dependent
     // chains (eight measured 43 % issue utilisation).
-    const int r = tid & 127, q = tid >> 7, n = n0 + r;
+    // Four neighbouring lanes own a row (whole 32-byte sectors of codes); in the upper 64 columns the words are taken in the order 2, 3, 0, 1,
+    // so that the eight lanes of a store phase hit eight different 16-byte columns of the swizzle.
+    const int r = tid >> 2, q = tid & 3, n = n0 + r, swap = q & 2;
     const bool live = n < p.N;
     const uint8_t *crow = p.codes + (size_t)(live ? n : 0) * ((size_t)p.K * BITS / 8) + (size_t)g_begin * (16 * BITS) + q * (4 * BITS);
     const __half2 *szrow = p.sz + (size_t)(live ? n : 0) * p.G + g_begin;
@@ -136,6 +138,7 @@ __device__ __forceinline__ void gemm_weight_warps(const GemmParams &p, unsigned 
             szb[u] = szrow[u];
         }
     }
+    pdl_wait();  // the codes above are constants; what follows ends in global writes
     auto hand_over = [&](int stage) {
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // generic-proxy writes -> visible to the tensor core
         __syncwarp();
@@ -149,7 +152,11 @@ __device__ __forceinline__ void gemm_weight_warps(const GemmParams &p, unsigned 
                 const int s = kt % kGStages, use = kt / kGStages;
                 uint4 cw[kCodeVec];
 #pragma unroll
-                for (int v = 0; v < kCodeVec; v++) cw[v] = wb[u][v];
+                for (int v = 0; v < kCodeVec; v++) {
+                    const uint4 t = wb[u][v], other = wb[u][kCodeVec - 1 - v];
+                    if (BITS == 4) cw[v] = swap ? make_uint4(t.z, t.w, t.x, t.y) : t;
+                    else cw[v] = swap ? other : t;
+                }
                 const __half2 szc = szb[u];
                 if (live && kt + kAheadA < G) {
                     const uint4 *src = reinterpret_cast<const uint4 *>(crow + (size_t)(kt + kAheadA) * (16 * BITS));
@@ -182,10 +189,10 @@ __device__ __forceinline__ void gemm_weight_warps(const GemmParams &p, unsigned 
                 if (ok && use > 0 && !mbar_wait_warp(&empty[s], (use - 1) & 1, p.err)) ok = false;
                 unsigned char *dst = As + (size_t)s * kABytes + row_off;
                 const int x = r & 7;  // chunk c = columns 8c .. 8c + 7 of the atom's 64, stored at chunk c ^ (row & 7)
-                *reinterpret_cast<uint4 *>(dst + (((c0 + 0) ^ x) << 4)) = v0;
-                *reinterpret_cast<uint4 *>(dst + (((c0 + 1) ^ x) << 4)) = v1;
-                *reinterpret_cast<uint4 *>(dst + (((c0 + 2) ^ x) << 4)) = v2;
-                *reinterpret_cast<uint4 *>(dst + (((c0 + 3) ^ x) << 4)) = v3;
+                *reinterpret_cast<uint4 *>(dst + (((c0 + (0 ^ swap)) ^ x) << 4)) = v0;
+                *reinterpret_cast<uint4 *>(dst + (((c0 + (1 ^ swap)) ^ x) << 4)) = v1;
+                *reinterpret_cast<uint4 *>(dst + (((c0 + (2 ^ swap)) ^ x) << 4)) = v2;
+                *reinterpret_cast<uint4 *>(dst + (((c0 + (3 ^ swap)) ^ x) << 4)) = v3;
             }
         }
     }
@@ -224,7 +231,7 @@ __global__ void __launch_bounds__(kGThreads, 1) gemm_int4_tc_kernel(const GemmPa
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem_d = *tmem_slot;
-    pdl_wait();
+    if (warp >= kGWarpsA) pdl_wait();
 
     const int g_begin = blockIdx.z * p.gps;
     const int G = min(p.G, g_begin + p.gps) - g_begin;  // this CTA's groups (stages), >= 1 by construction of the grid
