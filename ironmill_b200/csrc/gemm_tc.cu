@@ -1,12 +1,12 @@
 // INT4 group-128 GEMM on the 5th-generation tensor cores (tcgen05 + TMEM) for the dense-contraction cases of the
-// hot path: prefill chunks and decode batches of 16 tokens and more.
+// hot path: decode batches of 16 tokens and more and prefill chunks that do not fill CTA pairs (gemm_pair.cu).
 //   crates/ironmill-inference/src/metal/shaders/quantized/affine_matmul.metal:10-152 (superblock_matmul_int4):
 //   C[m, n] = sum_k f16(A[m, k] / awq[k]) * f16((q[n, k] - z) * s), f32 accumulation, fp16 result.
 //
 // Shape of the computation: D[128 weight rows x TN tokens] (f32, in tensor memory) += W[128 x 16] * X[TN x 16]^T, issued
 // by one thread with tcgen05.mma (kind::f16, UMMA M = 128, N = TN, K = 16), eight per stage of one quantisation
 // group (128 columns).  Both operands sit in shared memory, K-major with the 128-byte swizzle:
-//   * A: the weights.  Eight warps (thread = row and half of the group) read the packed 4-bit codes, 32 bytes per
+//   * A: the weights.  Sixteen warps (thread = row and quarter of the group) read the packed 4-bit codes, 16 bytes per
 //     thread and stage, and the row's (scale, zero), dequantise in packed fp16 arithmetic - (q - z) * s with one
 //     rounding, the reference's f16((q - z) s) - and store fp16 straight into the swizzled operand layout: the
 //     dequantisation is fused into the operand load, HBM carries 4 bits per weight.  The codes of the next stage
@@ -15,7 +15,7 @@
 //     the copy engine: one thread issues two cp.async.bulk.tensor copies per stage (boxes of 64 columns x TN token
 //     rows of a 2-D tensor map with the 128-byte swizzle; rows past the last token come back as zeros), completion
 //     counted in bytes on the stage's full barrier.  The map covers this GPU's own buffer; no multicast.
-// A ring of stages decouples the producers from the tensor core: full barriers count the eight weight warps and the
+// A ring of stages decouples the producers from the tensor core: full barriers count the weight warps and the
 // announcement of the activation bytes, tcgen05.commit releases a stage when its eight MMAs have read it.  After the last group warps 0-3 read their 32
 // TMEM lanes each (tcgen05.ld 32x32b), convert and write fp16 outputs.  Every wait is bounded; a wait that runs
 // out sets the device error word, the kernel still frees its tensor memory and returns.
@@ -144,12 +144,12 @@ __device__ __forceinline__ void gemm_weight_warps(const GemmParams &p, unsigned 
         __syncwarp();
         if (lane == 0) mbar_arrive(&full[stage]);
     };
+    int s = 0, use = 0, prev = 0;  // ring slot, how often it has been used, the slot before
     for (int kt0 = 0; kt0 < G; kt0 += kAheadA) {
 #pragma unroll
         for (int u = 0; u < kAheadA; u++) {
             const int kt = kt0 + u;
             if (kt < G) {  // warp-uniform
-                const int s = kt % kGStages, use = kt / kGStages;
                 uint4 cw[kCodeVec];
 #pragma unroll
                 for (int v = 0; v < kCodeVec; v++) {
@@ -185,18 +185,21 @@ __device__ __forceinline__ void gemm_weight_warps(const GemmParams &p, unsigned 
                     v2 = dequant8b_slow(cw[kCodeVec - 1].x, cw[kCodeVec - 1].y, zf, sf); v3 = dequant8b_slow(cw[kCodeVec - 1].z, cw[kCodeVec - 1].w, zf, sf);
                 }
                 // the previous stage is handed over only now: its stores have landed while this one was converted, and the fence does not wait
-                if (kt > 0) hand_over((kt - 1) % kGStages);
-                if (ok && use > 0 && !mbar_wait_warp(&empty[s], (use - 1) & 1, p.err)) ok = false;
+                if (kt > 0) hand_over(prev);
+                // usually free already: one look by the whole warp, then the bounded wait
+                if (ok && use > 0 && !__all_sync(0xffffffffu, mbar_try_wait(&empty[s], (use - 1) & 1)) && !mbar_wait_warp(&empty[s], (use - 1) & 1, p.err)) ok = false;
                 unsigned char *dst = As + (size_t)s * kABytes + row_off;
                 const int x = r & 7;  // chunk c = columns 8c .. 8c + 7 of the atom's 64, stored at chunk c ^ (row & 7)
                 *reinterpret_cast<uint4 *>(dst + (((c0 + (0 ^ swap)) ^ x) << 4)) = v0;
                 *reinterpret_cast<uint4 *>(dst + (((c0 + (1 ^ swap)) ^ x) << 4)) = v1;
                 *reinterpret_cast<uint4 *>(dst + (((c0 + (2 ^ swap)) ^ x) << 4)) = v2;
                 *reinterpret_cast<uint4 *>(dst + (((c0 + (3 ^ swap)) ^ x) << 4)) = v3;
+                prev = s;
+                if (++s == kGStages) s = 0, use++;
             }
         }
     }
-    hand_over((G - 1) % kGStages);
+    hand_over(prev);
 }
 
 template <int TN, int BITS>

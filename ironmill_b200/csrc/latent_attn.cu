@@ -543,7 +543,13 @@ __global__ void __launch_bounds__(256) latent_out_kernel(const LatentArgs a, con
 #pragma unroll
             for (int b = 0; b < MB; b++)
 #pragma unroll
-                for (int j = 0; j < V; j++) acc[b] = fmaf(w[j], os[b * s.latP + i * V + j], acc[b]);
+                for (int j = 0; j < V; j += 4) {  // 16 bytes a lane: word by word, 32 lanes would meet on four banks
+                    const float4 x = *reinterpret_cast<const float4 *>(os + b * s.latP + i * V + j);
+                    acc[b] = fmaf(w[j], x.x, acc[b]);
+                    acc[b] = fmaf(w[j + 1], x.y, acc[b]);
+                    acc[b] = fmaf(w[j + 2], x.z, acc[b]);
+                    acc[b] = fmaf(w[j + 3], x.w, acc[b]);
+                }
         }
 #pragma unroll
         for (int b = 0; b < MB; b++) {
@@ -841,7 +847,8 @@ int latent_attention_run(const Device *dev, const LatentArgs &a, cudaStream_t st
     const int M = a.nseq * a.T;
     const int dv = prefill_dv(s);
     const size_t per_head = (size_t)(s.dimP + s.vP) * 2;
-    if (!a.f32 && a.nseq == 1 && a.host_slot >= 0 && a.T >= kLatentExpandMin && latent_expands(s) && a.kv) {
+    if (!a.f32 && a.nseq == 1 && a.host_slot >= 0 && (a.T >= kLatentExpandMin || (a.T >= kLatentExpandShort && a.host_pos <= 3 * a.T)) &&
+        latent_expands(s) && a.kv) {
         const int ctx = a.host_pos + a.T;
         const int group = (int)std::min<size_t>(s.heads, a.kv_bytes / (per_head * ctx));
         if (group >= 1) {

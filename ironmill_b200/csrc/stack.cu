@@ -470,7 +470,7 @@ int StackModel::logits_of(DenseSrc src, int row, int n, float *out, cudaStream_t
     }
     DenseEpi e;
     e.kind = kEpiF32; e.xf = out; e.ldx = cfg.vocab_size; e.cap = sc.logit_softcap;
-    *nl += dense_launches(n, W, src.kind);
+    *nl += dense_launches(n, f32, src.kind);
     return dense_project(dev, sc.tied_head ? embed : head, src, e, n, h, st);
 }
 
@@ -512,7 +512,7 @@ int StackModel::forward(int nseq, int T, cudaStream_t st, int *launches, Prof *p
     res.kind = post ? kSrcAddNorm : kSrcNorm;
     auto read_residual = [&](const DenseWeight &w, const DenseEpi &e) -> int {
         IM_TRY(dense_project(dev, w, res, e, M, h, st));
-        nl += dense_launches(M, w.K, res.kind);
+        nl += dense_launches(M, f32, res.kind);
         if (res.xf2) {  // the sum has been written to `other`
             std::swap(cur, other);
             res.xf = cur; res.xf2 = nullptr; res.gamma = nullptr; res.xout = nullptr;
@@ -525,7 +525,7 @@ int StackModel::forward(int nseq, int T, cudaStream_t st, int *launches, Prof *p
         DenseEpi e;
         e.kind = post ? kEpiF32 : kEpiResidual; e.xf = post ? sub : cur; e.ldx = W;
         IM_TRY(dense_project(dev, w, s, e, M, nullptr, st));
-        nl += dense_launches(M, w.K, s.kind);
+        nl += dense_launches(M, f32, s.kind);
         if (post) {
             res.xf2 = sub; res.gamma = gamma; res.xout = other;
         }
@@ -539,7 +539,7 @@ int StackModel::forward(int nseq, int T, cudaStream_t st, int *launches, Prof *p
             DenseEpi e;
             e.kind = kEpiF32; e.xf = other; e.ldx = W; e.bias = loop_step + (size_t)r.pass * W;
             IM_TRY(dense_project(dev, loop_in, s, e, M, h, st));
-            nl += dense_launches(M, 2 * W, s.kind);
+            nl += dense_launches(M, f32, s.kind);
             std::swap(cur, other);
             res.xf = cur;
             IM_MARK(kCatResNorm);

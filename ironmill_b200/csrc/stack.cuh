@@ -54,14 +54,16 @@ struct DenseEpi {
     float cap = 0.0f;
 };
 
-constexpr int kDenseGemmMin = 16;  // tokens from which a projection is a dense contraction
+// Tokens from which a projection is a dense contraction. bf16: the matvec's multiply-adds grow with the rows (2048-wide model, 12 MB to 82 MB of weights: 15 us
+// a launch for one row, 30 for three or four, 71 for eight) while the tensor-core pass takes 19 to 21 us up to 32 rows. f32 has no tensor-core pass.
+constexpr int kDenseGemmMin = 5, kDenseGemmMinF32 = 16;
 constexpr int kDenseMaxRows = 8;   // tokens per matvec launch
 
-// y = W x for M tokens.  h_scratch: M x round_up(K, 8) elements, used when the source is not plain and M >= kDenseGemmMin.
+// y = W x for M tokens.  h_scratch: M x round_up(K, 8) elements, used when the source is not plain and M >= kDenseGemmMin (kDenseGemmMinF32).
 int dense_project(const Device *dev, const DenseWeight &w, const DenseSrc &src, const DenseEpi &epi, int M, void *h_scratch, cudaStream_t st);
 // Sets every launch attribute of this file's kernels on the current device (so that a capture can be their first use).
 int dense_prepare(const Device *dev);
-int dense_launches(int M, int K, int src_kind);
+int dense_launches(int M, int f32, int src_kind);
 
 // x[m] = x0[m] = rms(table[token]) * gamma, or without gamma table[token] * scale (f32); tokens past the vocabulary read as zeros.
 int stack_embed(const uint32_t *tokens, const void *table, int f32, int ld, const float *gamma, float scale, float *x, float *x0, int width, uint32_t vocab, float eps,
@@ -104,7 +106,9 @@ struct LatentArgs {
     int host_slot;
     int splits_ctx;          // context length the split count is chosen for
 };
-constexpr int kLatentExpandMin = 64;  // tokens of one sequence from which keys and values are expanded per head
+// Tokens of one sequence from which keys and values are expanded per head; and where the portion is at least a quarter of the context, so that
+// expanding it costs no more than a few of its own projections (a prompt of 50 tokens, 16 heads: 19 + 13 + 41 us absorbed, 20 + 12 us expanded).
+constexpr int kLatentExpandMin = 64, kLatentExpandShort = 16;
 int latent_attention_run(const Device *dev, const LatentArgs &a, cudaStream_t st, int *launches);
 size_t latent_part_bytes(const Device *dev, const LatentShape &s, int tokens, int nseq);
 bool latent_expands(const LatentShape &s);  // prompt chunks of this shape can take the expanded form
