@@ -1270,7 +1270,7 @@ int Model::finalize() {
         IM_TRY(m->alloc((void **)&m->kv16_scratch, n16));
         m->kv16_scratch_bytes = n16;
     }
-    if (c.tq_bits != 16 && tq_prefill_scratch_bytes(m->nkv_l, c.max_seq_len) <= ((size_t)2 << 30))  // (longer caches: the per-token kernel)
+    if (c.tq_bits != 16 && (size_t)m->nkv_l * c.max_seq_len * 768 <= ((size_t)2 << 30))  // rows of K' and V' (longer caches: the per-token kernel)
         IM_TRY(m->alloc(&m->pf_dq, tq_prefill_scratch_bytes(m->nkv_l, c.max_seq_len)));
     IM_TRY(im_cuda_tq_reserve_scratch(m->tq, need));
     m->scratch_ref = reinterpret_cast<Tq *>(m->tq)->scratch;

@@ -450,6 +450,7 @@ size_t tq_prefill_scratch_bytes(int nkv, int max_seq) {
 
 // K and V of a chunk of one sequence into its cache slot, as tq_prep_launch does for any step.
 int tq_prompt_encode_launch(const Tq *tq, const TqPrep &p, int slot, cudaStream_t st) {
+    if (tq->hd != kHd) return fail(IM_ERR_INVALID, "the prompt's cache write is built for head_dim 128 (got %d)", tq->hd);
     PromptEncode a{};
     a.kv = p.kv ? p.kv : p.qkv; a.stride = p.kv ? p.kv_stride : p.stride; a.k_off = p.k_off; a.v_off = p.v_off;
     a.kw = p.with_norm ? p.kw : nullptr; a.eps = p.eps;
