@@ -186,7 +186,8 @@ __global__ void __launch_bounds__(kHd) tq_reduce_kernel(const float *__restrict_
 // The warps of a CTA take the tiles of one (KV head, token, split) in turn and merge their results in shared
 // memory, so the number of partials per head is the same as with the kernel above.  Two CTAs per SM walk all (KV head, token, split) items
 // with one table.  mma.sync issue bounds it (48 products per tile, one per 32 clocks and SM quarter).  16 sequences of 1024 .. 8192
-// positions, 32 / 8 heads: 166 us with eight warps, rows loaded where they were used and a CTA per item.
+// positions, 32 / 8 heads: 166 us with eight warps, rows loaded where they were used and a CTA per item of one
+// split; 126 us with this form and one split, 83 us with parts for every SM.
 constexpr int kTcWarps = 6;  // two CTAs per SM: 168 registers a thread, for a tile's V rows and the next tile's K rows in flight
 __device__ __forceinline__ void mma_f16(float (&c)[4], unsigned a0, unsigned a1, unsigned a2, unsigned a3, unsigned b0, unsigned b1) {
     asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
