@@ -220,9 +220,12 @@ int im_cuda_tq_encode(const im_tq *tq, const void *kv_dev, int is_k, void *cache
 /* turboquant_attention in split mode + fused_sdpa_reduce (.../turboquant/turboquant.metal:202-462,
  * .../attention/flash_decode.metal:163-215; dispatch crates/ironmill-inference/src/metal/attention.rs:394-489).
  * q, out fp16 [nseq, T, nh, hd]; causal length of token t = base_pos + pos_dev[s] + t + 1.
- * num_splits 0 = chosen from the device size and the sequence length.  The split partials live in
- * scratch memory owned by the handle (grown on demand; reserve it up front to keep this call
- * allocation-free). */
+ * num_splits 0 = chosen from the device size and the longest context that the call can meet (max_seq when positions are
+ * on the device).  The split partials live in scratch memory owned by the handle.  A count chosen here fits what the handle
+ * holds (a new handle: about 33 KB per SM); the call allocates only for more than that with a count that the caller gave,
+ * or where one split of every head does not fit: reserve im_cuda_tq_scratch_bytes(nseq, T, nh, hd, num_splits or 1) bytes
+ * up front to keep it allocation-free.  Memory that a launch has used stays with the handle when it grows, so a
+ * captured call can be replayed until im_cuda_tq_free. */
 int im_cuda_tq_attention(im_tq *tq, const void *q_dev, const void *k_cache_dev, const void *v_cache_dev,
                          const float *k_scale_dev, const float *v_scale_dev, const float *k_rnorm_dev, float attn_scale,
                          void *out_dev, int nseq, int nh, int nkv, int max_seq, int base_pos, const int *pos_dev, int T,
@@ -265,7 +268,7 @@ int im_cuda_tq_prefill_attention(im_tq *tq, const void *q_dev, const void *k_cac
                                  const float *v_scale_dev, const float *k_rnorm_dev, float attn_scale, void *out_dev, int nh, int nkv,
                                  int max_seq, int base_pos, int T, void *dq_dev, void *stream);
 /* Scratch im_cuda_tq_attention needs for a launch: split partials (nseq*T*nh*splits*(head_dim+2) floats) plus the
- * rotated queries of its pre-pass (nseq*T*nh*2*head_dim floats).  The handle grows its scratch on demand. */
+ * rotated queries of its pre-pass (nseq*T*nh*2*head_dim floats). */
 size_t im_cuda_tq_scratch_bytes(int nseq, int T, int nh, int head_dim, int splits);
 int im_cuda_tq_reserve_scratch(im_tq *tq, size_t bytes);
 

@@ -6,6 +6,8 @@
 #include <stdio.h>
 #include <atomic>
 #include <string>
+#include <utility>
+#include <vector>
 
 #include "../../include/ironmill_cuda.h"
 
@@ -212,6 +214,8 @@ struct Tq {
     float *signs = nullptr, *qjl = nullptr, *qjl_t = nullptr, *k_cb = nullptr, *k_bd = nullptr, *v_cb = nullptr, *v_bd = nullptr;
     float *scratch = nullptr;
     size_t scratch_bytes = 0;
+    bool scratch_used = false;  // some launch, perhaps a captured one, holds its address: outgrown, it stays until the handle goes
+    std::vector<std::pair<float *, size_t>> outgrown;
     size_t const_bytes = 0;
 };
 

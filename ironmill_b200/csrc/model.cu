@@ -1274,7 +1274,8 @@ int Model::finalize() {
         IM_TRY(m->alloc(&m->pf_dq, tq_prefill_scratch_bytes(m->nkv_l, c.max_seq_len)));
     IM_TRY(im_cuda_tq_reserve_scratch(m->tq, need));
     m->scratch_ref = reinterpret_cast<Tq *>(m->tq)->scratch;
-    m->bytes += need + reinterpret_cast<Tq *>(m->tq)->const_bytes;
+    reinterpret_cast<Tq *>(m->tq)->scratch_used = true;
+    m->bytes += reinterpret_cast<Tq *>(m->tq)->scratch_bytes + reinterpret_cast<Tq *>(m->tq)->const_bytes;
     IM_CUDA_CHECK(cudaDeviceSynchronize());
     IM_TRY(mega_prepare(m));
     return IM_OK;

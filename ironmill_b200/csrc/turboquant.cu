@@ -474,6 +474,10 @@ __global__ void __launch_bounds__(kHd) tq_qrot_kernel(const __half *__restrict__
 using namespace im;
 struct im_tq : im::Tq {};
 
+// Scratch of a new handle: what automatic counts of more than one part take with up to four query heads per KV head (8 parts per SM; at most 4
+// (sequence, token, KV head) triples per SM and their queries). 4.9 MB with 148 SMs.
+static size_t tq_auto_scratch_bytes(const Device *dev) { return (size_t)dev->sm_count * 4 * (8 * (kHd + 2) + 4 * 2 * kHd) * sizeof(float); }
+
 IM_EXPORT int im_cuda_tq_lloyd_max(int dim, int n_bits, float *levels_out_host, float *bounds_out_host) {
     IM_GUARD_BEGIN
     IM_REQUIRE(dim > 0 && n_bits >= 1 && n_bits <= 8 && levels_out_host && bounds_out_host, "bad argument");
@@ -525,6 +529,7 @@ IM_EXPORT void im_cuda_tq_free(im_tq *tq) {
     dev_free(tq->dev, tq->v_cb, (size_t)tq->v_levels * 4);
     dev_free(tq->dev, tq->v_bd, (size_t)tq->v_levels * 4);
     dev_free(tq->dev, tq->scratch, tq->scratch_bytes);
+    for (const auto &o : tq->outgrown) dev_free(tq->dev, o.first, o.second);
     delete tq;
 }
 
@@ -582,6 +587,11 @@ IM_EXPORT int im_cuda_tq_create(im_device *dev, int head_dim, int n_bits, const 
         }
         tq->const_bytes += u.alloc * 4;
     }
+    if (head_dim == kHd)
+        if (const int rc = im_cuda_tq_reserve_scratch(tq, tq_auto_scratch_bytes(dev)); rc != IM_OK) {
+            im_cuda_tq_free(tq);
+            return rc;
+        }
     *out = tq;
     return IM_OK;
     IM_GUARD_END
@@ -613,24 +623,23 @@ IM_EXPORT size_t im_cuda_tq_scratch_bytes(int nseq, int T, int nh, int head_dim,
     return tq_partial_bytes(nseq, T, nh, head_dim, splits) + (size_t)nseq * T * nh * 2 * head_dim * sizeof(float);
 }
 
-namespace im {
-// Automatic split count of a call: from the longest context that it can meet (positions on the device: the cache's length), and scratch for it.  Inside a
-// capture the scratch cannot grow: fewer splits then, if those fit.
-static int tq_call_scratch(im_tq *tq, int num_splits, int nseq, int T, int nh, int nkv, int max_seq, int base_pos, const int *pos_dev, cudaStream_t st, int *out);
-}  // namespace im
-
+// A buffer that a launch has used is kept when it is outgrown: a captured graph may write to it again. Each one is at least twice as large as the
+// one before, so that they never hold more than twice the largest request.
 IM_EXPORT int im_cuda_tq_reserve_scratch(im_tq *tq, size_t bytes) {
     IM_GUARD_BEGIN
     IM_REQUIRE(tq, "bad argument");
     if (bytes <= tq->scratch_bytes) return IM_OK;
     IM_CUDA_CHECK(cudaSetDevice(tq->dev->ordinal));
-    IM_CUDA_CHECK(cudaDeviceSynchronize());  // earlier launches may still use the old buffer
-    dev_free(tq->dev, tq->scratch, tq->scratch_bytes);
-    tq->scratch = nullptr;
-    tq->scratch_bytes = 0;
-    int rc = dev_malloc(tq->dev, (void **)&tq->scratch, bytes);
+    if (tq->scratch_used) bytes = std::max(bytes, 2 * tq->scratch_bytes);
+    float *grown = nullptr;
+    tq->outgrown.reserve(tq->outgrown.size() + 1);
+    int rc = dev_malloc(tq->dev, (void **)&grown, bytes);
     if (rc != IM_OK) return rc;
+    if (tq->scratch_used) tq->outgrown.emplace_back(tq->scratch, tq->scratch_bytes);
+    else dev_free(tq->dev, tq->scratch, tq->scratch_bytes);
+    tq->scratch = grown;
     tq->scratch_bytes = bytes;
+    tq->scratch_used = false;
     return IM_OK;
     IM_GUARD_END
 }
@@ -655,11 +664,22 @@ int tq_prep_launch(const Tq *tq, const TqPrep &a, cudaStream_t st) {
 }
 
 // Parts that the positions of a (sequence, token, KV head) are cut into: enough for two CTAs per SM with one tile per warp of a part; and where parts
-// can hold three tiles per warp, four times as many as CTAs, so that sequences of different lengths share the GPU evenly.
+// can hold three tiles per warp, up to four times as many as CTAs, so that sequences of different lengths share the GPU evenly.
 int tq_auto_splits(const Device *dev, int nseq, int T, int nkv, int seq_len) {
     const long long ctas = (long long)nseq * T * nkv, fill = 2 * dev->sm_count, run = kTcWarps * kTile;
-    const long long a = std::min((fill + ctas - 1) / ctas, (seq_len + run - 1) / run), b = std::min((4 * fill + ctas - 1) / ctas, seq_len / (3 * run));
+    const long long a = std::min((fill + ctas - 1) / ctas, (seq_len + run - 1) / run), b = std::min(4 * fill / ctas, seq_len / (3 * run));
     return (int)std::max(1ll, std::min(128ll, std::max(a, b)));
+}
+
+// Split count of a call and scratch for it. An automatic count (the longest context that the call can meet decides: with positions on the device, the
+// cache's length) takes what the scratch holds: it grows only for a count that the caller gave or where one part of each does not fit.
+static int tq_call_scratch(im_tq *tq, int num_splits, int nseq, int T, int nh, int nkv, int max_seq, int base_pos, const int *pos_dev, int *out) {
+    int splits = num_splits > 0 ? num_splits : tq_auto_splits(tq->dev, nseq, T, nkv, pos_dev ? max_seq : base_pos + T);
+    while (num_splits <= 0 && splits > 1 && im_cuda_tq_scratch_bytes(nseq, T, nh, kHd, splits) > tq->scratch_bytes) splits--;
+    *out = splits;
+    const int rc = im_cuda_tq_reserve_scratch(tq, im_cuda_tq_scratch_bytes(nseq, T, nh, kHd, splits));
+    if (rc == IM_OK) tq->scratch_used = true;
+    return rc;
 }
 
 int tq_attention_launch(const Tq *tq, float *scratch, const __half *q, const uint8_t *kc, const uint8_t *vc, const float *ks,
@@ -729,31 +749,14 @@ IM_EXPORT int im_cuda_tq_prefill_attention(im_tq *tq, const void *q_dev, const v
     IM_REQUIRE(T >= 0 && max_seq > 0 && base_pos >= 0, "bad shape");
     if (T == 0) return IM_OK;
     if (base_pos + T > max_seq) return fail(IM_ERR_BOUNDS, "sequence position %d + %d tokens exceeds max_seq_len %d", base_pos, T, max_seq);
-    const size_t need = im_cuda_tq_scratch_bytes(1, T, nh, kHd, 1);
-    if (need > tq->scratch_bytes) {
-        int rc = im_cuda_tq_reserve_scratch(tq, need);
-        if (rc != IM_OK) return rc;
-    }
+    if (const int grc = im_cuda_tq_reserve_scratch(tq, im_cuda_tq_scratch_bytes(1, T, nh, kHd, 1)); grc != IM_OK) return grc;
+    tq->scratch_used = true;
     const int rc = tq_prefill_attention_launch(tq, tq->scratch, dq_dev, TqPromptQuery{static_cast<const __half *>(q_dev), nh * kHd}, static_cast<const uint8_t *>(k_cache_dev),
                                                static_cast<const uint8_t *>(v_cache_dev), k_scale_dev, v_scale_dev, k_rnorm_dev, attn_scale, static_cast<__half *>(out_dev), 0, nh,
                                                nkv, max_seq, nullptr, T, base_pos + T, as_stream(stream), base_pos);
     if (rc == IM_ERR_BOUNDS) return fail(IM_ERR_INVALID, "query heads per KV head must be 1, 2, 4 or 8 (got %d/%d)", nh, nkv);
     return rc;
     IM_GUARD_END
-}
-
-int im::tq_call_scratch(im_tq *tq, int num_splits, int nseq, int T, int nh, int nkv, int max_seq, int base_pos, const int *pos_dev, cudaStream_t st, int *out) {
-    int splits = num_splits > 0 ? num_splits : tq_auto_splits(tq->dev, nseq, T, nkv, pos_dev ? max_seq : base_pos + T);
-    if (im_cuda_tq_scratch_bytes(nseq, T, nh, kHd, splits) > tq->scratch_bytes) {
-        cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-        if (num_splits <= 0 && cudaStreamIsCapturing(st, &cs) == cudaSuccess && cs != cudaStreamCaptureStatusNone)
-            while (splits > 1 && im_cuda_tq_scratch_bytes(nseq, T, nh, kHd, splits) > tq->scratch_bytes) splits--;
-        const size_t need = im_cuda_tq_scratch_bytes(nseq, T, nh, kHd, splits);
-        if (need > tq->scratch_bytes)
-            if (const int rc = im_cuda_tq_reserve_scratch(tq, need); rc != IM_OK) return rc;
-    }
-    *out = splits;
-    return IM_OK;
 }
 
 IM_EXPORT int im_cuda_tq_attention(im_tq *tq, const void *q_dev, const void *k_cache_dev, const void *v_cache_dev,
@@ -770,7 +773,7 @@ IM_EXPORT int im_cuda_tq_attention(im_tq *tq, const void *q_dev, const void *k_c
         return fail(IM_ERR_BOUNDS, "sequence position %d + %d tokens exceeds max_seq_len %d", base_pos, T, max_seq);
     IM_REQUIRE(num_splits <= 1024, "too many splits");
     int splits = 0;
-    if (const int rc = tq_call_scratch(tq, num_splits, nseq, T, nh, nkv, max_seq, base_pos, pos_dev, as_stream(stream), &splits); rc != IM_OK) return rc;
+    if (const int rc = tq_call_scratch(tq, num_splits, nseq, T, nh, nkv, max_seq, base_pos, pos_dev, &splits); rc != IM_OK) return rc;
     // rotate the queries once (every split of a head would otherwise redo the rotation and the 128 x 128 projection)
     float *qrot = tq->scratch + tq_partial_bytes(nseq, T, nh, kHd, splits) / sizeof(float);
     IM_CUDA_CHECK(launch_k(tq_qrot_kernel, dim3(nseq * T, nh), dim3(kHd), 0, as_stream(stream), static_cast<const __half *>(q_dev),
@@ -799,7 +802,7 @@ IM_EXPORT int im_cuda_tq_fused_attention(im_tq *tq, const void *qkv_dev, int qkv
     if (!pos_dev && base_pos + T > max_seq)
         return fail(IM_ERR_BOUNDS, "sequence position %d + %d tokens exceeds max_seq_len %d", base_pos, T, max_seq);
     int splits = 0;
-    if (const int src = tq_call_scratch(tq, num_splits, nseq, T, nh, nkv, max_seq, base_pos, pos_dev, as_stream(stream), &splits); src != IM_OK) return src;
+    if (const int src = tq_call_scratch(tq, num_splits, nseq, T, nh, nkv, max_seq, base_pos, pos_dev, &splits); src != IM_OK) return src;
     TqPrep a{};
     a.qkv = static_cast<const __half *>(qkv_dev); a.stride = qkv_stride; a.k_off = k_offset; a.v_off = v_offset;
     a.qw = static_cast<const __half *>(q_norm_w_dev); a.kw = static_cast<const __half *>(k_norm_w_dev);

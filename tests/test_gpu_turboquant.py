@@ -182,6 +182,48 @@ def test_device_side_position_past_the_cache_is_clamped(tq, tqc):
     assert np.isfinite(out).all() and H.rel_err(out[1], q1.reshape(nh, 128)) <= 2e-3
 
 
+def test_scratch_of_a_handle_outlives_captured_calls(tqc):
+    """A captured call writes to the scratch that the handle had at that time. Automatic split counts never outgrow it (smaller batches
+    wanted more than larger ones here), and where a count given by the caller does, the old memory stays until the handle goes."""
+    from ironmill_b200 import ops
+    from ironmill_b200._lib import C, check, lib
+    dev = ops.Device(0)
+    start = dev.allocated_bytes()
+    tq = ops.TurboQuant(dev, 128, 8, tqc.signs, tqc.qjl, tqc.k_levels, tqc.k_bounds, tqc.v_levels, tqc.v_bounds)
+    nh, nkv, max_seq, n = 32, 8, 1024, 32
+    kc, ks, kr, vc, vs = _fill_cache(tq, tqc, nkv, max_seq, max_seq, seed=8, nseq=n)
+    q = _c(H.make_x(n, nh * 128, seed=8, name="q"))
+    pos = torch.tensor([(i * 677 + 5) % max_seq for i in range(n)], dtype=torch.int32, device="cuda")
+
+    def call(m, splits=0):
+        return tq.attention(q[:m], kc[:m], vc[:m], ks[:m], vs[:m], kr[:m], 0.0884, nh, nkv, max_seq, 0, nseq=m, pos_dev=pos[:m], num_splits=splits)
+
+    check(lib().im_cuda_tq_reserve_scratch(tq.handle, C.c_size_t(lib().im_cuda_tq_scratch_bytes(C.c_int(n), C.c_int(1), C.c_int(nh), C.c_int(128), C.c_int(1)))))
+    held = dev.allocated_bytes()
+    one = call(n, 1)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        captured = call(n)
+    for m in (n, 29, 28, 17, 1):
+        eager = call(m)
+        assert dev.allocated_bytes() == held
+        captured.zero_()
+        graph.replay()
+        assert m < n or torch.equal(captured, eager)
+        assert H.rel_err(captured.cpu().numpy(), one.cpu().numpy()) <= 2e-3
+        assert H.rel_err(eager.cpu().numpy(), one[:m].cpu().numpy()) <= 2e-3
+    want = captured.clone()
+    many = call(n, 40)  # 22 MB of partials
+    assert dev.allocated_bytes() > held and H.rel_err(many.cpu().numpy(), one.cpu().numpy()) <= 2e-3
+    captured.zero_()
+    graph.replay()
+    assert torch.equal(captured, want)
+    del graph
+    torch.cuda.synchronize()
+    tq.free()
+    assert dev.allocated_bytes() == start
+
+
 def test_sequence_overflow_is_reported(tq):
     from ironmill_b200 import CudaSysError
     z8 = torch.zeros((1, 8, 16, 128), dtype=torch.uint8, device="cuda")
