@@ -221,7 +221,7 @@ int im_cuda_tq_encode(const im_tq *tq, const void *kv_dev, int is_k, void *cache
  * .../attention/flash_decode.metal:163-215; dispatch crates/ironmill-inference/src/metal/attention.rs:394-489).
  * q, out fp16 [nseq, T, nh, hd]; causal length of token t = base_pos + pos_dev[s] + t + 1.
  * num_splits 0 = chosen from the device size and the longest context that the call can meet (max_seq when positions are
- * on the device).  The split partials live in scratch memory owned by the handle.  A count chosen here fits what the handle
+ * on the device); each token's context is cut into as many of them as its own length fills.  The split partials live in scratch memory owned by the handle.  A count chosen here fits what the handle
  * holds (a new handle: about 33 KB per SM); the call allocates only for more than that with a count that the caller gave,
  * or where one split of every head does not fit: reserve im_cuda_tq_scratch_bytes(nseq, T, nh, hd, num_splits or 1) bytes
  * up front to keep it allocation-free.  Memory that a launch has used stays with the handle when it grows, so a
@@ -253,8 +253,8 @@ int im_cuda_tq_fused_attention(im_tq *tq, const void *qkv_dev, int qkv_stride, i
  *  - the device of `tq` must be the current device;
  *  - the first call on a device looks the array's device address up (cudaGetSymbolAddress); make that first call
  *    before any stream capture;
- *  - all calls share the one array, which keeps whatever the last call left in it (nothing needs clearing: every
- *    split writes its whole partial before it is read); two calls whose kernels overlap on the GPU race. */
+ *  - all calls share the one array, which keeps whatever the last call left in it (nothing needs clearing:
+ *    only partials that the call itself has written are read); two calls whose kernels overlap on the GPU race. */
 int im_cuda_tq_attention_static(const im_tq *tq, const void *q_dev, const void *k_cache_dev, const void *v_cache_dev,
                                 const float *k_scale_dev, const float *v_scale_dev, const float *k_rnorm_dev, float attn_scale,
                                 void *out_dev, int nseq, int nh, int nkv, int max_seq, int base_pos, const int *pos_dev, int T,

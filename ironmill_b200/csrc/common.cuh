@@ -255,8 +255,8 @@ struct TqPrep {
 int tq_prep_launch(const Tq *tq, const TqPrep &a, cudaStream_t st);
 int tq_attention_launch(const Tq *tq, float *scratch, const __half *q, const uint8_t *kc, const uint8_t *vc, const float *ks,
                         const float *vs, const float *krn, float attn_scale, __half *out, int nseq, int nh, int nkv, int max_seq,
-                        int base_pos, const int *pos_dev, int T, int splits, cudaStream_t st, const float *qrot = nullptr,
-                        const int *slot_map = nullptr);
+                        int base_pos, const int *pos_dev, int T, int splits, bool own_parts, cudaStream_t st, const float *qrot = nullptr,
+                        const int *slot_map = nullptr);  // own_parts: splits is an automatic count, each token takes what its context fills
 
 // ---- fp16 (unquantized) KV cache: kv_f16.cu ----
 struct Kv16Prep {

@@ -466,7 +466,7 @@ static int attention_block(Model *m, int part, const TqPrep &a, __half *q_buf, L
                                            TqPromptQuery{a.qkv, a.stride, a.with_norm ? a.qw : nullptr, a.eps, a.cosc, a.sinc, a.rotary_dim}, L.kc, L.vc, L.ks, L.vs, L.krn,
                                            attn_scale, m->attn_out, m->prefill_slot_id, a.nh, a.nkv, c.max_seq_len, m->pos_dev, T, m->prefill_ctx_end, st);
     return tq_attention_launch(reinterpret_cast<const Tq *>(m->tq), m->scratch_ref, nullptr, L.kc, L.vc, L.ks, L.vs, L.krn, attn_scale, m->attn_out,
-                               nseq, a.nh, a.nkv, c.max_seq_len, 0, m->pos_dev, T, attn_splits, st, m->qrot, slots);
+                               nseq, a.nh, a.nkv, c.max_seq_len, 0, m->pos_dev, T, attn_splits, true, st, m->qrot, slots);
 }
 
 // Logits of `rows` normed rows. The matvec reads the whole table for every four rows (up to 64 rows per call); from five rows on one pass on the

@@ -227,7 +227,22 @@ struct AttnParams {
     const int *pos_dev;      // optional per-slot positions (added to base_pos)
     const int *slot_map;     // optional: sequence index of this launch -> cache slot (nullptr: identity)
     int bits;                // cache bits per element (8 or 4); rows hold tq_row_bytes(bits, hd) bytes
+    int own_parts;           // `splits` is the most that a token may use: its context is cut into parts of at least one run of tiles
 };
+constexpr int kTcWarps = 6, kTcRun = kTcWarps * kTile;  // a run: a tile for each warp of tq_attention_tc_kernel
+// Positions that token st (sequence-major) of a launch sees and positions of a part of them (whole tiles). Part i is there if i chunk < len; of the
+// rest of `splits` only the maximum is written, minus infinity (100 positions in a cache of 65536 cut into 113 parts took 32 us, 25 in one).
+struct TqSpan {
+    int len, chunk;
+};
+__device__ __forceinline__ TqSpan tq_span(const AttnParams &p, int st, int slot) {
+    TqSpan s;
+    // never past the end of the head's rows, whatever a device-side position says (the host can only check base_pos)
+    s.len = max(min(p.base_pos + (p.pos_dev ? p.pos_dev[slot] : 0) + st % p.T + 1, p.max_seq), 0);
+    const int n = p.own_parts ? max(min(p.splits, (s.len + kTcRun - 1) / kTcRun), 1) : p.splits;
+    s.chunk = max((int)((unsigned)(s.len + n - 1) / (unsigned)n + kTile - 1) / kTile, 1) * kTile;
+    return s;
+}
 // Eight 4-bit elements of a cache word -> two words of one byte per element (the 8-bit layout the score and value
 // loops read).  K: the 3-bit index stays in bits 0-2, the QJL sign moves from bit 3 to bit 7; V: the byte is the index.
 __device__ __forceinline__ unsigned tq_spread4(unsigned x) {  // nibbles 0-3 of x (low 16 bits) -> bytes
@@ -587,40 +602,64 @@ __device__ __forceinline__ void tq_prep_item(const Scope &sc, const PrepArgs &a,
     tq_prep_item(sc, a, sh, slot, st, pj);
 }
 
-// Combine the splits of one (token, head), normalise, rotate back, write fp16.
+// Combine the parts of one (token, head), normalise, rotate back, write fp16.
 // The inverse rotation is linear, so applying it once after the combination equals the
-// reference's per-split rotation up to float rounding.  x: 128 floats of shared memory.
+// reference's per-split rotation up to float rounding.  x: 128 floats of shared memory.  Parts that are not there have a maximum of minus infinity
+// and leave the rest of their place as it was: the first eight are requested as they are, of the others only those up to the last that is there.
 template <class Scope>
 __device__ __forceinline__ void tq_reduce_item(const Scope &sc, float *x, const float *__restrict__ po, const float *__restrict__ pm,
                                                const float *__restrict__ pl, const float *__restrict__ signs, __half *__restrict__ out,
-                                               size_t head_index, int splits_stride, int splits_used) {
+                                               size_t head_index, int splits) {
     const int d = sc.d;
-    const size_t base = head_index * splits_stride;
+    const size_t base = head_index * splits;
     const float sg = signs[d];
-    float gm = -INFINITY;
-    for (int s0 = 0; s0 < splits_used; s0 += 8) {  // eight loads in flight at a time; combined in split order
-        float m[8];
-#pragma unroll
-        for (int j = 0; j < 8; j++) m[j] = s0 + j < splits_used ? pm[base + s0 + j] : -INFINITY;
-#pragma unroll
-        for (int j = 0; j < 8; j++) gm = fmaxf(gm, m[j]);
-    }
-    float acc = 0.0f, lsum = 0.0f;
-    for (int s0 = 0; s0 < splits_used; s0 += 8) {
-        float m[8], l[8], o[8];
+    float m[8], l[8], o[8];
+    auto load = [&](int s0, int n) {
 #pragma unroll
         for (int j = 0; j < 8; j++) {
-            const bool live = s0 + j < splits_used;
+            const bool live = s0 + j < n;
             m[j] = live ? pm[base + s0 + j] : -INFINITY;
             l[j] = live ? pl[base + s0 + j] : 0.0f;
             o[j] = live ? po[(base + s0 + j) * kHd + d] : 0.0f;
         }
+    };
+    load(0, splits);
+    float gm = -INFINITY;
 #pragma unroll
-        for (int j = 0; j < 8; j++) {
-            const float corr = m[j] == -INFINITY ? 0.0f : __expf(m[j] - gm);
-            lsum += l[j] * corr;
-            acc += o[j] * corr;
+    for (int j = 0; j < 8; j++) gm = fmaxf(gm, m[j]);
+    int used = min(splits, 8);
+    if (splits > 8) {  // a thread per part
+        int last = 0;
+        for (int s = 8 + d; s < splits; s += kHd) {
+            const float t = pm[base + s];
+            if (t != -INFINITY) last = s + 1;
+            gm = fmaxf(gm, t);
         }
+        gm = warp_max(gm);
+        last = __reduce_max_sync(0xffffffffu, last);
+        if ((d & 31) == 0) {
+            x[d >> 5] = gm;
+            x[4 + (d >> 5)] = __int_as_float(last);
+        }
+        sc.sync();
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            gm = fmaxf(gm, x[i]);
+            used = max(used, __float_as_int(x[4 + i]));
+        }
+        sc.sync();  // x is used again below
+    }
+    float acc = 0.0f, lsum = 0.0f;
+    for (int s0 = 0;;) {  // in the order of the parts
+#pragma unroll
+        for (int j = 0; j < 8; j++)
+            if (m[j] != -INFINITY) {
+                const float corr = __expf(m[j] - gm);
+                lsum += l[j] * corr;
+                acc += o[j] * corr;
+            }
+        if ((s0 += 8) >= used) break;
+        load(s0, used);
     }
     const float r = hadamard_thread(sc, acc / fmaxf(lsum, 1e-10f), sg, x, kHd);
     out[head_index * kHd + d] = __float2half_rn(r);

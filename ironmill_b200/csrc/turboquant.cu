@@ -128,11 +128,12 @@ __global__ void __launch_bounds__(kAttnThreads) tq_attention_kernel(const AttnPa
     const int kvh = blockIdx.x, st = blockIdx.y, split = blockIdx.z;
     pdl_trigger();
     pdl_wait();
-    const int seq = st / p.T, t = st % p.T;
-    // never past the end of the head's rows, whatever a device-side position says (the host can only check base_pos)
-    const int seq_len = min(p.base_pos + (p.pos_dev ? p.pos_dev[cache_slot(p.slot_map, seq)] : 0) + t + 1, p.max_seq);
-    const int chunk = (seq_len + p.splits - 1) / p.splits;
-    const int r0 = split * chunk, r1 = min(r0 + chunk, seq_len);
+    const TqSpan span = tq_span(p, st, cache_slot(p.slot_map, st / p.T));
+    if (split * span.chunk >= span.len) {  // (the whole CTA)
+        if (tid < GQ) p.pm[((size_t)st * p.nh + kvh * GQ + tid) * p.splits + split] = -INFINITY;
+        return;
+    }
+    const int r0 = split * span.chunk, r1 = min(r0 + span.chunk, span.len);
     const int kl = 1 << (p.bits - 1), vl = 1 << p.bits;  // codebook sizes: K keeps one bit for the QJL sign
     cbk[tid] = tid < kl ? p.k_cb[tid] : 0.0f;
     cbv[tid] = tid < vl ? p.v_cb[tid] : 0.0f;
@@ -158,14 +159,13 @@ __global__ void __launch_bounds__(kHd) tq_qkv_prep_kernel(const PrepArgs a_in) {
 }
 
 // grid (nseq*T, nh), hd threads.
-__global__ void __launch_bounds__(kHd) tq_reduce_kernel(const float *__restrict__ po, const float *__restrict__ pm,
-                                                        const float *__restrict__ pl, const float *__restrict__ signs,
-                                                        __half *__restrict__ out, int nh, int splits) {
+__global__ void __launch_bounds__(kHd) tq_reduce_kernel(const AttnParams p, __half *__restrict__ out) {
     __shared__ float x[kHd];
     pdl_trigger();
     pdl_wait();
     const CtaScope sc{(int)threadIdx.x, kHd};
-    tq_reduce_item(sc, x, po, pm, pl, signs, out, (size_t)blockIdx.x * nh + blockIdx.y, splits, splits);
+    const int st = blockIdx.x;
+    tq_reduce_item(sc, x, p.po, p.pm, p.pl, p.signs, out, (size_t)st * p.nh + blockIdx.y, p.splits);
 }
 
 
@@ -183,12 +183,11 @@ __global__ void __launch_bounds__(kHd) tq_reduce_kernel(const float *__restrict_
 //     against the signs, columns 4-7 = S q with zeros against the centroids; outputs as [16 dims x 16 positions] x
 //     [16 positions x 8 heads].  The fragment <-> (dimension, position) assignment is chosen so that a fragment
 //     register is built from bytes the lane already holds.
-// The warps of a CTA take the tiles of one (KV head, token, split) in turn and merge their results in shared
+// The six warps of a CTA (two CTAs per SM: 168 registers a thread, for a tile's V rows and the next tile's K rows in flight) take the tiles of one (KV head, token, split) in turn and merge their results in shared
 // memory, so the number of partials per head is the same as with the kernel above.  Two CTAs per SM walk all (KV head, token, split) items
 // with one table.  mma.sync issue bounds it (48 products per tile, one per 32 clocks and SM quarter).  16 sequences of 1024 .. 8192
 // positions, 32 / 8 heads: 166 us with eight warps, rows loaded where they were used and a CTA per item of one
 // split; 126 us with this form and one split, 83 us with parts for every SM.
-constexpr int kTcWarps = 6;  // two CTAs per SM: 168 registers a thread, for a tile's V rows and the next tile's K rows in flight
 __device__ __forceinline__ void mma_f16(float (&c)[4], unsigned a0, unsigned a1, unsigned a2, unsigned a3, unsigned b0, unsigned b1) {
     asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
                  : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
@@ -237,13 +236,15 @@ __global__ void __launch_bounds__(kTcWarps * 32, 2) tq_attention_tc_kernel(const
 
     for (int item = blockIdx.x; item < items; item += gridDim.x) {
         const int kvh = item % p.nkv, rest = item / p.nkv, split = rest % p.splits, st = rest / p.splits;
-        const int seq = st / p.T, tt = st % p.T;
-        const int slot = cache_slot(p.slot_map, seq);
-        const int seq_len = min(p.base_pos + (p.pos_dev ? p.pos_dev[slot] : 0) + tt + 1, p.max_seq);  // see tq_attention_kernel
-        const int chunk = ((seq_len + p.splits - 1) / p.splits + kTile - 1) / kTile * kTile;
-        const int c0 = split * chunk, c1 = min(c0 + chunk, seq_len);
+        const int slot = cache_slot(p.slot_map, st / p.T);
+        const TqSpan span = tq_span(p, st, slot);
+        if (split * span.chunk >= span.len) {  // (the whole CTA)
+            if (tid < GQ) p.pm[((size_t)st * p.nh + kvh * GQ + tid) * p.splits + split] = -INFINITY;
+            continue;
+        }
+        const int c0 = split * span.chunk, c1 = min(c0 + span.chunk, span.len);
         // this warp's tiles of the split's range: every kTcWarps-th
-        const int tiles = (max(c1 - c0, 0) + kTile - 1) / kTile;
+        const int tiles = (c1 - c0 + kTile - 1) / kTile;
         const int h0 = kvh * GQ;
         const size_t head_base = ((size_t)slot * p.nkv + kvh) * p.max_seq;
         const uint8_t *krow = p.kc + head_base * kRowB, *vrow = p.vc + head_base * kRowB;
@@ -666,7 +667,7 @@ int tq_prep_launch(const Tq *tq, const TqPrep &a, cudaStream_t st) {
 // Parts that the positions of a (sequence, token, KV head) are cut into: enough for two CTAs per SM with one tile per warp of a part; and where parts
 // can hold three tiles per warp, up to four times as many as CTAs, so that sequences of different lengths share the GPU evenly.
 int tq_auto_splits(const Device *dev, int nseq, int T, int nkv, int seq_len) {
-    const long long ctas = (long long)nseq * T * nkv, fill = 2 * dev->sm_count, run = kTcWarps * kTile;
+    const long long ctas = (long long)nseq * T * nkv, fill = 2 * dev->sm_count, run = kTcRun;
     const long long a = std::min((fill + ctas - 1) / ctas, (seq_len + run - 1) / run), b = std::min(4 * fill / ctas, seq_len / (3 * run));
     return (int)std::max(1ll, std::min(128ll, std::max(a, b)));
 }
@@ -684,8 +685,9 @@ static int tq_call_scratch(im_tq *tq, int num_splits, int nseq, int T, int nh, i
 
 int tq_attention_launch(const Tq *tq, float *scratch, const __half *q, const uint8_t *kc, const uint8_t *vc, const float *ks,
                         const float *vs, const float *krn, float attn_scale, __half *out, int nseq, int nh, int nkv, int max_seq,
-                        int base_pos, const int *pos_dev, int T, int splits, cudaStream_t st, const float *qrot, const int *slot_map) {
+                        int base_pos, const int *pos_dev, int T, int splits, bool own_parts, cudaStream_t st, const float *qrot, const int *slot_map) {
     AttnParams p{};
+    p.own_parts = own_parts;
     p.qrot = qrot;
     p.slot_map = slot_map;
     p.bits = tq->n_bits;
@@ -728,8 +730,7 @@ int tq_attention_launch(const Tq *tq, float *scratch, const __half *q, const uin
         }
     }
     dim3 rgrid(nseq * T, nh);
-    IM_CUDA_CHECK(launch_k(tq_reduce_kernel, rgrid, dim3(kHd), 0, st, (const float *)p.po, (const float *)p.pm, (const float *)p.pl,
-                           (const float *)tq->signs, out, nh, splits));
+    IM_CUDA_CHECK(launch_k(tq_reduce_kernel, rgrid, dim3(kHd), 0, st, p, out));
     return IM_OK;
 }
 }  // namespace im
@@ -780,7 +781,7 @@ IM_EXPORT int im_cuda_tq_attention(im_tq *tq, const void *q_dev, const void *k_c
                            (const float *)tq->signs, (const float *)tq->qjl_t, qrot, nh));
     return tq_attention_launch(tq, tq->scratch, nullptr, static_cast<const uint8_t *>(k_cache_dev),
                                static_cast<const uint8_t *>(v_cache_dev), k_scale_dev, v_scale_dev, k_rnorm_dev, attn_scale,
-                               static_cast<__half *>(out_dev), nseq, nh, nkv, max_seq, base_pos, pos_dev, T, splits, as_stream(stream), qrot);
+                               static_cast<__half *>(out_dev), nseq, nh, nkv, max_seq, base_pos, pos_dev, T, splits, num_splits <= 0, as_stream(stream), qrot);
     IM_GUARD_END
 }
 
@@ -815,7 +816,7 @@ IM_EXPORT int im_cuda_tq_fused_attention(im_tq *tq, const void *qkv_dev, int qkv
     int rc = tq_prep_launch(tq, a, st);
     if (rc != IM_OK) return rc;
     return tq_attention_launch(tq, tq->scratch, nullptr, a.kc, a.vc, a.ks, a.vs, a.krn, attn_scale, static_cast<__half *>(out_dev), nseq,
-                               nh, nkv, max_seq, base_pos, pos_dev, T, splits, st, qrot_dev);
+                               nh, nkv, max_seq, base_pos, pos_dev, T, splits, num_splits <= 0, st, qrot_dev);
     IM_GUARD_END
 }
 
@@ -861,13 +862,13 @@ IM_EXPORT int im_cuda_tq_attention_static(const im_tq *tq, const void *q_dev, co
                     "%d sequence(s) x %d token(s) x %d heads x %d splits need %zu bytes of split partials and rotated queries; the built-in "
                     "scratch holds %zu (use fewer splits or im_cuda_tq_attention)",
                     nseq, T, nh, splits, need, kStaticScratchFloats * sizeof(float));
-    // Nothing has to start at zero: every split, empty ones included, writes its whole partial before the reduce reads it.
+    // Nothing has to start at zero: the reduce reads only parts that have been written whole.
     float *scratch = g_static_attn_ptr[cur];
     float *qrot = scratch + tq_partial_bytes(nseq, T, nh, kHd, splits) / sizeof(float);
     IM_CUDA_CHECK(launch_k(tq_qrot_kernel, dim3(nseq * T, nh), dim3(kHd), 0, as_stream(stream), static_cast<const __half *>(q_dev),
                            (const float *)tq->signs, (const float *)tq->qjl_t, qrot, nh));
     return tq_attention_launch(tq, scratch, nullptr, static_cast<const uint8_t *>(k_cache_dev),
                                static_cast<const uint8_t *>(v_cache_dev), k_scale_dev, v_scale_dev, k_rnorm_dev, attn_scale,
-                               static_cast<__half *>(out_dev), nseq, nh, nkv, max_seq, base_pos, pos_dev, T, splits, as_stream(stream), qrot);
+                               static_cast<__half *>(out_dev), nseq, nh, nkv, max_seq, base_pos, pos_dev, T, splits, num_splits <= 0, as_stream(stream), qrot);
     IM_GUARD_END
 }

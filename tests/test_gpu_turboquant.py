@@ -182,6 +182,26 @@ def test_device_side_position_past_the_cache_is_clamped(tq, tqc):
     assert np.isfinite(out).all() and H.rel_err(out[1], q1.reshape(nh, 128)) <= 2e-3
 
 
+@pytest.mark.parametrize("nh,nkv", [(2, 2), (4, 2), (8, 2), (16, 2)])
+def test_parts_of_ragged_contexts_with_positions_on_the_device(tq, tqc, nh, nkv):
+    """Contexts around one and three runs of tiles (192 positions each) and at the ends of the cache, many parts and few, an empty one; longest
+    first, so that later calls find other calls' partials where they write none."""
+    max_seq, lengths = 2305, [2305, 2304, 577, 576, 575, 193, 192, 33, 32, 1, 0]
+    n = len(lengths)
+    kc, ks, kr, vc, vs = _fill_cache(tq, tqc, nkv, max_seq, max_seq, seed=nh, nseq=n)
+    q = H.make_x(n, nh * 128, seed=nh, name="q")
+    kcn, vcn, ksn, vsn, krn = (a.cpu().numpy() for a in (kc, vc, ks, vs, kr))
+    ref = [orc.tq_attention(q[i:i + 1], kcn[i], vcn[i], tqc, ksn[i], vsn[i], krn[i], 0.0884, nh, nkv, max_seq, m - 1, num_splits=0).reshape(-1) if m else
+           np.zeros(nh * 128) for i, m in enumerate(lengths)]
+    pos = torch.tensor([m - 1 for m in lengths], dtype=torch.int32, device="cuda")
+    for splits in (0, 1, 5, 90):
+        for first in range(0, n, 1 if splits == 0 else 5):
+            out = tq.attention(_c(q[first:]), kc[first:], vc[first:], ks[first:], vs[first:], kr[first:], 0.0884, nh, nkv, max_seq, 0, nseq=n - first,
+                               pos_dev=pos[first:], num_splits=splits).cpu().numpy()
+            for i in range(first, n):
+                assert np.abs(out[i - first] - ref[i]).max() <= 2e-3 * max(np.abs(ref[i]).max(), 1e-6), (splits, first, lengths[i])
+
+
 def test_scratch_of_a_handle_outlives_captured_calls(tqc):
     """A captured call writes to the scratch that the handle had at that time. Automatic split counts never outgrow it (smaller batches
     wanted more than larger ones here), and where a count given by the caller does, the old memory stays until the handle goes."""
