@@ -319,22 +319,20 @@ __global__ void __launch_bounds__(kGThreads, 1) gemm_int4_tc_kernel(const GemmPa
     }
 }
 
-// xs[m, k] = f16(x[m, k] / awq[k]) (or a copy when there are no activation scales)
-__global__ void act_scale_kernel(const __half *__restrict__ x, const __half *__restrict__ awq, __half *__restrict__ xs, size_t n, int K) {
+// xs[m, k] = f16(x[m, k] / awq[k]); xs may be x
+__global__ void act_scale_kernel(const __half *x, const __half *__restrict__ awq, __half *xs, size_t n, int K) {
     pdl_trigger();
     pdl_wait();
     const size_t i = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * 8;
     if (i >= n) return;
     uint4 v = *reinterpret_cast<const uint4 *>(x + i);
-    if (awq) {
-        const uint4 a = *reinterpret_cast<const uint4 *>(awq + (i % (size_t)K));
-        __half2 *hv = reinterpret_cast<__half2 *>(&v);
-        const __half2 *ha = reinterpret_cast<const __half2 *>(&a);
+    const uint4 a = *reinterpret_cast<const uint4 *>(awq + (i % (size_t)K));
+    __half2 *hv = reinterpret_cast<__half2 *>(&v);
+    const __half2 *ha = reinterpret_cast<const __half2 *>(&a);
 #pragma unroll
-        for (int j = 0; j < 4; j++) {
-            const float2 fx = __half22float2(hv[j]), fa = __half22float2(ha[j]);
-            hv[j] = __floats2half2_rn(fx.x / fa.x, fx.y / fa.y);
-        }
+    for (int j = 0; j < 4; j++) {
+        const float2 fx = __half22float2(hv[j]), fa = __half22float2(ha[j]);
+        hv[j] = __floats2half2_rn(fx.x / fa.x, fx.y / fa.y);
     }
     *reinterpret_cast<uint4 *>(xs + i) = v;
 }
@@ -404,12 +402,12 @@ int gemm_launch(const GemmParams &p, const Device *dev, cudaStream_t st) {
 
 static bool gemm_takes(const AffineWeight *w) { return (w->bits == 4 || w->bits == 8) && w->group_size == 128 && w->K % 128 == 0; }
 
-// The tokens as the projection reads them: x itself, or f16(x / awq) in the scratch.
+// The tokens as the projection reads them: x itself, or f16(x / awq) in the scratch (both 16-byte aligned).
 static int scaled_tokens(const AffineWeight *w, const __half *x, int M, __half *xs_scratch, bool scaled, cudaStream_t st, const __half **out) {
     *out = x;
-    if ((scaled || !w->awq) && reinterpret_cast<uintptr_t>(x) % 16 == 0) return IM_OK;
+    if (scaled || !w->awq) return IM_OK;
     const size_t n = (size_t)M * w->K;
-    IM_CUDA_CHECK(launch_k(act_scale_kernel, dim3((unsigned)((n / 8 + 255) / 256)), dim3(256), 0, st, x, (const __half *)(scaled ? nullptr : w->awq), xs_scratch, n, w->K));
+    IM_CUDA_CHECK(launch_k(act_scale_kernel, dim3((unsigned)((n / 8 + 255) / 256)), dim3(256), 0, st, x, (const __half *)w->awq, xs_scratch, n, w->K));
     *out = xs_scratch;
     return IM_OK;
 }
@@ -433,7 +431,7 @@ int gemm_affine_tc(const AffineWeight *w, const __half *x, __half *y, int M, __h
     // Few tokens and few row tiles (decode batches of 16-64 against 4096-6144 rows: 32-48 CTAs of 32-112 sequential
     // stages): split K so that the grid covers the GPU.  At least four groups per slice; the slices' f32 sums go through
     // the device handle's scratch (one GEMM in flight per handle, like the tiled matvec).
-    if (M <= 64 && w->N % 4 == 0 && w->dev->gemm_partial) {
+    if (M <= 64 && w->N % 4 == 0 && reinterpret_cast<uintptr_t>(y) % 8 == 0 && w->dev->gemm_partial) {
         const int tiles = (w->N + kGM - 1) / kGM;
         int splits = std::min(w->dev->sm_count / tiles, w->G / 4);
         while (splits > 1 && (size_t)splits * M * w->N * sizeof(float) > kGemmPartialBytes) splits--;

@@ -92,6 +92,32 @@ def test_unusual_zero_points_take_the_f32_path(dev):
     _check(dev, qw, 40)
 
 
+@pytest.mark.parametrize("awq", [False, True])
+@pytest.mark.parametrize("K,M", [(512, 16), (512, 130), (4096, 300)])
+def test_result_over_the_tokens(dev, K, M, awq):
+    # out may be x: K split over the grid, whole tiles, CTA pairs
+    from ironmill_b200 import ops
+    w = H.QWeight(K, K, awq=awq, seed=K + M, name="gi").gpu(dev)
+    x = torch.from_numpy(H.rng_for("gi-x", M).standard_normal((M, K)).astype(np.float16)).cuda()
+    want = ops.matmul_affine(w, x)
+    assert torch.equal(ops.matmul_affine(w, x, out=x), want)
+
+
+@pytest.mark.parametrize("awq", [False, True])
+@pytest.mark.parametrize("K,M", [(512, 16), (512, 130), (4096, 300)])
+def test_rows_that_are_not_aligned(dev, K, M, awq):
+    from ironmill_b200 import CudaSysError, ops
+    w = H.QWeight(K, K, awq=awq, seed=K + M, name="gu").gpu(dev)
+    x = torch.from_numpy(H.rng_for("gu-x", M).standard_normal((M, K)).astype(np.float16)).cuda()
+    want = ops.matmul_affine(w, x)
+    far = torch.empty(2, M * K + 8, dtype=torch.float16, device="cuda")
+    xo, yo = far[0, 1:1 + M * K].view(M, K), far[1, 3:3 + M * K].view(M, K)
+    xo.copy_(x)
+    assert H.rel_err(ops.matmul_affine(w, xo, out=yo).cpu().numpy(), want.cpu().numpy()) <= TOL  # (K may be split for one and not the other)
+    with pytest.raises(CudaSysError):
+        ops.matmul_affine(w, xo, scratch=yo)
+
+
 def test_matches_the_matvec_kernel_rows(dev):
     # the same weight through the decode matvec (24-bit integer activations) and the GEMM: both within their tolerance of the oracle
     from ironmill_b200 import ops
