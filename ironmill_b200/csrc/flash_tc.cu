@@ -20,6 +20,8 @@
 #include <cuda_bf16.h>
 #include <math.h>
 
+#include <type_traits>
+
 #include "flash_tc.cuh"
 #include "tmap.cuh"
 #include "v2_device.cuh"
@@ -368,12 +370,14 @@ __global__ void __launch_bounds__(kFThreads, 1)
                 fence_after();
                 const int p0 = n_begin + it * PN;
                 float s[PN], lazy = kLazy;
+                bool odd = false;  // (quantized caches) a factor of this tile is not finite
                 const float *ks = Fs + (it % ST) * 3 * PN, *kr = ks + PN, *vs = kr + PN;
                 if constexpr (TQ) {
                     if (ok && !wait_for(&vfull[it % ST], (it / ST) & 1, a.err)) ok = false;
                     // a weight times vs has to stay in fp16's range: where vs is large the maximum follows at once
                     const unsigned vm = __reduce_max_sync(0xffffffffu, max(__float_as_uint(fabsf(vs[lane])), __float_as_uint(fabsf(vs[lane + 32]))));
                     if (vm > __float_as_uint(128.0f)) lazy = 0.0f;
+                    odd = vm >= 0x7f800000u;
 #pragma unroll
                     for (int c = 0; c < PN; c += 32) {
                         float t[32];
@@ -432,29 +436,38 @@ __global__ void __launch_bounds__(kFThreads, 1)
                 }
                 const float base = m == -INFINITY ? 0.0f : m;
                 float sum[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-                // 64 columns at a time: 32 words of weights and, with two terms, 32 words of what their rounding left
+                // 64 columns at a time: 32 words of weights and, with two terms, 32 words of what their rounding left. ODD: zero times a factor that is
+                // not finite would be a NaN in rows that do not see its position
+                auto weights = [&](auto ODD) {
 #pragma unroll
-                for (int c = 0; c < PN; c += 64) {
-                    uint32_t w[32], w2[32];
+                    for (int c = 0; c < PN; c += 64) {
+                        uint32_t w[32], w2[32];
 #pragma unroll
-                    for (int j = 0; j < 32; j++) {
-                        const float x0 = ex2(fmaf(s[c + 2 * j], p.scale2, -base)), x1 = ex2(fmaf(s[c + 2 * j + 1], p.scale2, -base));
-                        sum[(2 * j) & 3] += x0;
-                        sum[(2 * j + 1) & 3] += x1;
-                        if constexpr (TQ) {
-                            const float2 v2 = *reinterpret_cast<const float2 *>(vs + c + 2 * j);
-                            w[j] = pack2<BF16>(x0 * v2.x, x1 * v2.y);
-                        } else {
-                            w[j] = pack2<BF16>(x0, x1);
+                        for (int j = 0; j < 32; j++) {
+                            const float x0 = ex2(fmaf(s[c + 2 * j], p.scale2, -base)), x1 = ex2(fmaf(s[c + 2 * j + 1], p.scale2, -base));
+                            sum[(2 * j) & 3] += x0;
+                            sum[(2 * j + 1) & 3] += x1;
+                            if constexpr (TQ) {
+                                float2 v2 = *reinterpret_cast<const float2 *>(vs + c + 2 * j);
+                                if constexpr (ODD) {
+                                    if (p0 + c + 2 * j > lim) v2.x = 0.0f;
+                                    if (p0 + c + 2 * j + 1 > lim) v2.y = 0.0f;
+                                }
+                                w[j] = pack2<BF16>(x0 * v2.x, x1 * v2.y);
+                            } else {
+                                w[j] = pack2<BF16>(x0, x1);
+                            }
+                            if (TERMS > 1) {
+                                const float2 r = unpack2<BF16>(w[j]);
+                                w2[j] = pack2<BF16>(x0 - r.x, x1 - r.y);
+                            }
                         }
-                        if (TERMS > 1) {
-                            const float2 r = unpack2<BF16>(w[j]);
-                            w2[j] = pack2<BF16>(x0 - r.x, x1 - r.y);
-                        }
+                        st32(ts + (uint32_t)(c / 2), w);
+                        if (TERMS > 1) st32(ts + (uint32_t)(PN / 2 + c / 2), w2);
                     }
-                    st32(ts + (uint32_t)(c / 2), w);
-                    if (TERMS > 1) st32(ts + (uint32_t)(PN / 2 + c / 2), w2);
-                }
+                };
+                if (TQ && odd) weights(std::bool_constant<TQ>());
+                else weights(std::false_type());
                 l += (sum[0] + sum[1]) + (sum[2] + sum[3]);
                 tmem_wait_st();
                 fence_before();

@@ -340,6 +340,26 @@ def test_prefill_flash_attention_against_the_oracle(tq, tqc, nh, nkv, base, T):
     assert e_new <= 2e-3, (e_new, e_tok)
 
 
+@pytest.mark.parametrize("bad", [np.inf, -np.inf, np.nan])
+@pytest.mark.parametrize("which", ["ks", "kr", "vs"])
+def test_prompt_pass_keeps_a_poisoned_token_to_those_that_see_it(tq, tqc, which, bad):
+    """A factor of a cached row that is not finite reaches the tokens from its own on, none before it: in the first half of a block of 256
+    tokens, in the second and in the next block."""
+    nh, nkv, base, T = 4, 2, 20, 400
+    n = base + T
+    kc, ks, kr, vc, vs = _fill_cache(tq, tqc, nkv, n, n, seed=6)
+    q = H.make_x(T, nh * 128, seed=6, name="qq")
+    want = orc.tq_attention(q, kc[0].cpu().numpy(), vc[0].cpu().numpy(), tqc, ks[0].cpu().numpy(), vs[0].cpu().numpy(), kr[0].cpu().numpy(),
+                            0.0884, nh, nkv, n, base).reshape(T, nh * 128)
+    for at in (130, 250, 391):
+        f = {"ks": ks.clone(), "kr": kr.clone(), "vs": vs.clone()}
+        f[which][:, :, base + at] = bad
+        out = tq.prefill_attention(_c(q), kc, vc, f["ks"], f["vs"], f["kr"], 0.0884, nh, nkv, n, base).cpu().numpy()
+        assert H.rel_err(out[:at], want[:at]) <= 2e-3, at
+        if which == "vs":
+            assert not np.isfinite(out[at:]).any()
+
+
 @pytest.mark.parametrize("base,T", [(0, 40), (130, 70)])
 def test_prefill_flash_attention_4bit(tq4, tqc4, base, T):
     nh, nkv = 16, 4
