@@ -262,7 +262,7 @@ int im_cuda_tq_attention_static(const im_tq *tq, const void *q_dev, const void *
                                 int num_splits, void *stream);
 /* Prefill form for one sequence (T tokens at positions base_pos .. base_pos + T - 1, rows already in the cache, the
  * reference's turboquant_attention with token_count > 1, turboquant.metal:202-462): the cached rows are dequantised once
- * into dq_dev (im_cuda_tq_prefill_scratch_bytes(nkv, max_seq) bytes) and scored by a causal tensor-core pass.  Caches of
+ * into dq_dev (im_cuda_tq_prefill_scratch_bytes(nkv, max_seq) bytes, 16-byte aligned) and scored by a causal tensor-core pass.  Caches of
  * one sequence: [nkv, max_seq, ...].  Same results as im_cuda_tq_attention within its tolerance. */
 size_t im_cuda_tq_prefill_scratch_bytes(int nkv, int max_seq);
 int im_cuda_tq_prefill_attention(im_tq *tq, const void *q_dev, const void *k_cache_dev, const void *v_cache_dev, const float *k_scale_dev,

@@ -750,12 +750,19 @@ IM_EXPORT int im_cuda_tq_prefill_attention(im_tq *tq, const void *q_dev, const v
     IM_REQUIRE(T >= 0 && max_seq > 0 && base_pos >= 0, "bad shape");
     if (T == 0) return IM_OK;
     if (base_pos + T > max_seq) return fail(IM_ERR_BOUNDS, "sequence position %d + %d tokens exceeds max_seq_len %d", base_pos, T, max_seq);
+    IM_REQUIRE(reinterpret_cast<uintptr_t>(dq_dev) % 16 == 0, "the buffer for dequantised rows must be 16-byte aligned");
+    if (!tq_prefill_takes(nh, nkv)) return fail(IM_ERR_INVALID, "query heads per KV head must be 1, 2, 4 or 8 (got %d/%d)", nh, nkv);
+    // 1544 bytes per (token, head): the query rows take 512, results for a place that is not aligned 256 behind them
     if (const int grc = im_cuda_tq_reserve_scratch(tq, im_cuda_tq_scratch_bytes(1, T, nh, kHd, 1)); grc != IM_OK) return grc;
     tq->scratch_used = true;
+    const size_t results = (size_t)T * nh * kHd;
+    const bool move = reinterpret_cast<uintptr_t>(out_dev) % 16 != 0;
+    __half *out = move ? reinterpret_cast<__half *>(tq->scratch) + 2 * results : static_cast<__half *>(out_dev);
     const int rc = tq_prefill_attention_launch(tq, tq->scratch, dq_dev, TqPromptQuery{static_cast<const __half *>(q_dev), nh * kHd}, static_cast<const uint8_t *>(k_cache_dev),
-                                               static_cast<const uint8_t *>(v_cache_dev), k_scale_dev, v_scale_dev, k_rnorm_dev, attn_scale, static_cast<__half *>(out_dev), 0, nh,
+                                               static_cast<const uint8_t *>(v_cache_dev), k_scale_dev, v_scale_dev, k_rnorm_dev, attn_scale, out, 0, nh,
                                                nkv, max_seq, nullptr, T, base_pos + T, as_stream(stream), base_pos);
-    if (rc == IM_ERR_BOUNDS) return fail(IM_ERR_INVALID, "query heads per KV head must be 1, 2, 4 or 8 (got %d/%d)", nh, nkv);
+    if (rc == IM_ERR_BOUNDS) return fail(IM_ERR_INVALID, "the prompt pass does not take %d tokens of %d heads", T, nh);
+    if (rc == IM_OK && move) IM_CUDA_CHECK(cudaMemcpyAsync(out_dev, out, results * sizeof(__half), cudaMemcpyDeviceToDevice, as_stream(stream)));
     return rc;
     IM_GUARD_END
 }

@@ -360,6 +360,23 @@ def test_prompt_pass_keeps_a_poisoned_token_to_those_that_see_it(tq, tqc, which,
             assert not np.isfinite(out[at:]).any()
 
 
+def test_prompt_pass_into_a_place_that_is_not_aligned(tq, tqc, monkeypatch):
+    from ironmill_b200 import ops
+    nh, nkv, T = 8, 2, 300
+    kc, ks, kr, vc, vs = _fill_cache(tq, tqc, nkv, T, T, seed=9)
+    q = _c(H.make_x(T, nh * 128, seed=9, name="q"))
+    args = (kc, vc, ks, vs, kr, 0.0884, nh, nkv, T, 0)
+    want = tq.prefill_attention(q, *args)
+    place = torch.full((T * nh * 128 + 16,), 7.0, dtype=torch.float16, device="cuda")
+    for off in (1, 4, 7):
+        place.fill_(7.0)
+        got = place[off:off + T * nh * 128].view(T, nh * 128)
+        with monkeypatch.context() as m:
+            m.setattr(ops.torch, "empty_like", lambda t: got)
+            assert tq.prefill_attention(q, *args).data_ptr() == got.data_ptr()
+        assert torch.equal(got, want) and bool((place[:off] == 7).all()) and bool((place[off + T * nh * 128:] == 7).all())
+
+
 @pytest.mark.parametrize("base,T", [(0, 40), (130, 70)])
 def test_prefill_flash_attention_4bit(tq4, tqc4, base, T):
     nh, nkv = 16, 4
