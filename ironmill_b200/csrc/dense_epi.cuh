@@ -10,8 +10,8 @@ namespace im {
 template <>
 __device__ __forceinline__ __half from_f<__half>(float v) { return __float2half_rn(v); }
 
-// z sigmoid(z), and gelu_tanh(z) = z / (1 + exp(-2 u)), u = sqrt(2 / pi) (z + 0.044715 z^3); the error of the
-// fast exponential and quotient (about 1e-6) is far below the 16-bit result's rounding
+// bf16 epilogues: z sigmoid(z), and gelu_tanh(z) = z / (1 + exp(-2 u)), u = sqrt(2 / pi) (z + 0.044715 z^3); the error of the
+// fast exponential and quotient (about 1e-6) is far below the bf16 result's rounding
 __device__ __forceinline__ float silu_fast(float z) { return __fdividef(z, 1.0f + __expf(-z)); }
 template <typename T>
 __device__ __forceinline__ float pair_act(float z, float up, bool silu) {
@@ -22,7 +22,7 @@ __device__ __forceinline__ float pair_act(float z, float up, bool silu) {
 // fp16 (quantized blocks): gate and up are rounded before the activation, as the reference's separate kernels do
 template <>
 __device__ __forceinline__ float pair_act<__half>(float z, float up, bool) {
-    return silu_fast(__half2float(__float2half_rn(z))) * __half2float(__float2half_rn(up));
+    return silu_f(__half2float(__float2half_rn(z))) * __half2float(__float2half_rn(up));
 }
 
 // One round of a transposition between lanes: of every two values the lane with bit X clear keeps the first and gets its

@@ -193,3 +193,34 @@ def test_prompt_with_gate_and_up_in_one_projection(awq, bits):
     eng.load_weights(DictProvider(cfg, tensors))
     prompt = H.rng_for("kv16-joint").integers(0, 400, 203).astype(np.uint32)
     assert np.abs(eng.prefill(prompt) - OracleModel(cfg, tensors, None, 256, kv_f16=True).forward(prompt)).max() <= 5e-2
+
+
+def test_activation_in_the_joint_projection_is_that_of_the_separate_pass():
+    """Gate, up and down with one element per row: their sums are single products, exact in any order, so the activation alone can tell the prompt of 256 tokens (gate
+    and up joint, SiLU in the epilogue) from the one of 100 (two projections, then the activation). Attention adds nothing (o is zero)."""
+    from ironmill_b200.bundle import ModelConfig, WeightTensor
+    from ironmill_b200.engine import CudaConfig, CudaInference
+    from tests.oracle_model import DictProvider, synth_model
+    I, Hd = 4096, 256
+    cfg = ModelConfig(architecture="llama", hidden_size=Hd, intermediate_size=I, num_hidden_layers=1, num_attention_heads=2,
+                      num_key_value_heads=1, head_dim=128, vocab_size=300, max_position_embeddings=512, rms_norm_eps=1e-5, rope_theta=5e5,
+                      tie_word_embeddings=False)
+    tensors = synth_model(cfg, seed=8)
+    r = H.rng_for("one-per-row")
+
+    def one_per_row(name, N, K, scale, on=1):
+        codes = np.zeros((N, K), dtype=np.uint8)
+        codes[np.arange(N), r.permutation(K)[:N] if N <= K else r.integers(0, K, N)] = on
+        sc = (scale * r.uniform(0.4, 1.6, (N, K // 128)) * r.choice([-1.0, 1.0], (N, K // 128))).astype(np.float16)
+        tensors["model.layers.0." + name] = WeightTensor(orc.pack_int4(codes.reshape(-1)), (N, K), "uint8", sc, np.zeros_like(sc), 4, 128, 1, None)
+
+    one_per_row("self_attn.o_proj.weight", Hd, 256, 1.0, on=0)
+    one_per_row("mlp.gate_proj.weight", I, Hd, 2.0)
+    one_per_row("mlp.up_proj.weight", I, Hd, 1.0)
+    one_per_row("mlp.down_proj.weight", Hd, I, 1.0)
+    eng = CudaInference(CudaConfig(max_seq_len=256).without_turboquant())
+    eng.load_weights(DictProvider(cfg, tensors))
+    prompt = r.integers(0, 300, 256).astype(np.uint32)
+    joint = eng.prefill_all_logits(prompt)
+    eng.reset()
+    assert np.array_equal(joint[:100], eng.prefill_all_logits(prompt[:100]))
