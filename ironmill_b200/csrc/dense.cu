@@ -322,10 +322,10 @@ struct DenseGemm {
 };
 
 // 16 tokens m .. m + 15 of row n (one per lane) of the f32 sums
-template <typename T>
+template <typename T, int TN>
 __device__ __forceinline__ void dense_store16(const DenseGemm &p, int z, int n, int n_warp, int m, const float (&v)[16]) {
     if (!p.partial) {
-        epi_store16<T>(p.epi, p.N, p.M, n, n_warp, m, v);
+        epi_store16<T>(p.epi, p.N, p.M, n, n_warp, m, v, TN == 32 && p.M < kDenseGemmMinF32);
     } else if (n < p.N) {
         float *dst = p.partial + ((size_t)z * p.M + m) * p.N + n;
 #pragma unroll
@@ -423,7 +423,7 @@ __global__ void __launch_bounds__(kDThreads, kDCtasPerSm) dense_gemm_tc_kernel(c
                 for (int c = c_begin; c < c_begin + TN / 2 && m0 + c < p.M; c += 16) {
                     float v[16];
                     dense_tmem_ld16(tmem_d + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(acc * TN + c), v);
-                    dense_store16<T>(p, z, n_warp + lane, n_warp, m0 + c, v);
+                    dense_store16<T, TN>(p, z, n_warp + lane, n_warp, m0 + c, v);
                 }
             }
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");

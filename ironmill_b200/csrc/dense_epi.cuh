@@ -11,17 +11,19 @@ template <>
 __device__ __forceinline__ __half from_f<__half>(float v) { return __float2half_rn(v); }
 
 // bf16 epilogues: z sigmoid(z), and gelu_tanh(z) = z / (1 + exp(-2 u)), u = sqrt(2 / pi) (z + 0.044715 z^3); the error of the
-// fast exponential and quotient (about 1e-6) is far below the bf16 result's rounding
+// fast exponential and quotient (about 1e-6) is far below the bf16 result's rounding. few: fewer rows than kDenseGemmMinF32, for which
+// the activations are those of the matvec (epi_pair), so that a row's result is as exact whichever kernel a batch takes.
 __device__ __forceinline__ float silu_fast(float z) { return __fdividef(z, 1.0f + __expf(-z)); }
 template <typename T>
-__device__ __forceinline__ float pair_act(float z, float up, bool silu) {
+__device__ __forceinline__ float pair_act(float z, float up, bool silu, bool few) {
+    if (few) return (silu ? silu_f(z) : gelu_tanh_f(z)) * up;
     if (silu) return silu_fast(z) * up;
     const float w = -1.5957691216057308f * z * fmaf(0.044715f * z, z, 1.0f);
     return __fdividef(z * up, 1.0f + __expf(fminf(w, 80.0f)));
 }
 // fp16 (quantized blocks): gate and up are rounded before the activation, as the reference's separate kernels do
 template <>
-__device__ __forceinline__ float pair_act<__half>(float z, float up, bool) {
+__device__ __forceinline__ float pair_act<__half>(float z, float up, bool, bool) {
     return silu_f(__half2float(__float2half_rn(z))) * __half2float(__float2half_rn(up));
 }
 
@@ -69,7 +71,7 @@ __device__ __forceinline__ bool aligned16(const void *p, long long row_bytes) { 
 // carries 16 bytes.  A two-byte store per lane takes the SM 13 clocks however narrow it is: 128 x 256 results as such took 14000 clocks, most of a
 // tile's products (gemm_pair.cu, 2048 tokens x 4096 x 512: 20.8 us, now 17.4 us with the activation branch below, 9.7 us without any store).  false: not such a warp, nothing stored.
 template <typename T>
-__device__ __forceinline__ bool epi_store16_wide(const DenseEpi &e, int N, int M, int n, int n_warp, int m, const float (&v)[16]) {
+__device__ __forceinline__ bool epi_store16_wide(const DenseEpi &e, int N, int M, int n, int n_warp, int m, const float (&v)[16], bool few) {
     const int lane = threadIdx.x & 31, left = M - m, end = n_warp + 32;
     if (end > N) return false;
     const bool proj = e.kind == kEpiProj;
@@ -82,7 +84,7 @@ __device__ __forceinline__ bool epi_store16_wide(const DenseEpi &e, int N, int M
 #pragma unroll
         for (int i = 0; i < 16; i += 2) {  // (gate, up) in neighbouring lanes: the even lane takes token i, the odd lane token i + 1
             const float got = __shfl_xor_sync(0xffffffffu, odd ? v[i] : v[i + 1], 1);
-            r[i / 2] = odd ? pair_act<T>(got, v[i + 1], e.pair_silu) : pair_act<T>(v[i], got, e.pair_silu);
+            r[i / 2] = odd ? pair_act<T>(got, v[i + 1], e.pair_silu, few) : pair_act<T>(v[i], got, e.pair_silu, few);
         }
         const uint4 q = gather8<T, 2>(r);
         const int tok = lane & 15;
@@ -97,7 +99,7 @@ __device__ __forceinline__ bool epi_store16_wide(const DenseEpi &e, int N, int M
         for (int i = 0; i < 16; i++) r[i] = v[i];
         if (n_warp < e.silu_end)  // a branch: evaluated for every value and then dropped, it took more time than the stores
 #pragma unroll
-            for (int i = 0; i < 16; i++) r[i] = n < e.silu_end ? silu_fast(v[i]) : v[i];
+            for (int i = 0; i < 16; i++) r[i] = n < e.silu_end ? few ? silu_f(v[i]) : silu_fast(v[i]) : v[i];
 #pragma unroll
         for (int k = 0; k < 2; k++) {
             const uint4 q = gather8<T, 1>(r + 8 * k);
@@ -143,8 +145,8 @@ __device__ __forceinline__ bool epi_store16_wide(const DenseEpi &e, int N, int M
 
 // 16 tokens m .. m + 15 of row n (one per lane; n_warp: that of lane 0) of a result of N rows and M tokens
 template <typename T>
-__device__ __forceinline__ void epi_store16(const DenseEpi &e, int N, int M, int n, int n_warp, int m, const float (&v)[16]) {
-    if (epi_store16_wide<T>(e, N, M, n, n_warp, m, v)) return;
+__device__ __forceinline__ void epi_store16(const DenseEpi &e, int N, int M, int n, int n_warp, int m, const float (&v)[16], bool few = false) {
+    if (epi_store16_wide<T>(e, N, M, n, n_warp, m, v, few)) return;
     const int lane = threadIdx.x & 31, left = M - m;
     if (e.kind == kEpiProj) {
         if (n_warp + 31 >= e.pair0) {
@@ -157,14 +159,14 @@ __device__ __forceinline__ void epi_store16(const DenseEpi &e, int N, int M, int
             for (int i = 0; i < 16; i += 2) {
                 const float got = __shfl_xor_sync(0xffffffffu, odd ? v[i] : v[i + 1], 1);
                 if (pair) {
-                    const float r = odd ? pair_act<T>(got, v[i + 1], e.pair_silu) : pair_act<T>(v[i], got, e.pair_silu);
+                    const float r = odd ? pair_act<T>(got, v[i + 1], e.pair_silu, few) : pair_act<T>(v[i], got, e.pair_silu, few);
                     if (n < N && i + odd < left) act[(size_t)(i + odd) * e.ldact] = from_f<T>(r);
                 } else {
 #pragma unroll
                     for (int j = 0; j < 2; j++)
                         if (i + j < left) {
                             if (n >= e.f0) e.xf[(size_t)(m + i + j) * e.ldx + (n - e.f0)] = v[i + j];
-                            else y[(size_t)(i + j) * e.ldy] = from_f<T>(n < e.silu_end ? silu_fast(v[i + j]) : v[i + j]);
+                            else y[(size_t)(i + j) * e.ldy] = from_f<T>(n < e.silu_end ? few ? silu_f(v[i + j]) : silu_fast(v[i + j]) : v[i + j]);
                         }
                 }
             }
@@ -179,7 +181,7 @@ __device__ __forceinline__ void epi_store16(const DenseEpi &e, int N, int M, int
             } else if (n < N) {
 #pragma unroll
                 for (int i = 0; i < 16; i++)
-                    if (i < left) y[(size_t)i * e.ldy] = from_f<T>(act ? silu_fast(v[i]) : v[i]);
+                    if (i < left) y[(size_t)i * e.ldy] = from_f<T>(act ? few ? silu_f(v[i]) : silu_fast(v[i]) : v[i]);
             }
         }
     } else if (n < N) {
