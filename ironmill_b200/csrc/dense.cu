@@ -432,7 +432,7 @@ __global__ void __launch_bounds__(kDThreads, kDCtasPerSm) dense_gemm_tc_kernel(c
         }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
+    sync_and_settle(ok);
     if (warp == kDEpi + 1) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_d), "r"(kCols) : "memory");

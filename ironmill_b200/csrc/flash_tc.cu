@@ -544,7 +544,7 @@ __global__ void __launch_bounds__(kFThreads, 1)
         }
     }
     fence_before();
-    __syncthreads();
+    sync_and_settle(ok);
     if (warp == kFMmaWarp) {
         fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");

@@ -115,7 +115,7 @@ __device__ __forceinline__ bool pair_wait_warp(uint64_t *bar, uint32_t parity, i
 // (whole 32-byte sectors of codes, one (scale, zero) pair); in the upper 64 columns the words are taken in the order 2, 3, 0, 1,
 // so that the eight lanes of a store phase hit eight different 16-byte columns of the swizzle.
 template <int TN, int BITS>
-__device__ __forceinline__ void weight_warps(const PairGemm &p, unsigned char *As, uint64_t *full, uint64_t *empty, int rank, int pair, int npairs) {
+__device__ __forceinline__ bool weight_warps(const PairGemm &p, unsigned char *As, uint64_t *full, uint64_t *empty, int rank, int pair, int npairs) {
     using S = PairShape<TN, BITS>;
     constexpr int kAhead = BITS == 4 ? kPAhead4 : kPAhead8, kVec = BITS == 4 ? 1 : 2;
     const int tid = threadIdx.x, lane = tid & 31, r = tid >> 2, q = tid & 3, G = p.kstages;
@@ -207,6 +207,7 @@ __device__ __forceinline__ void weight_warps(const PairGemm &p, unsigned char *A
         }
     }
     if (total > 0) hand_over(prev);
+    return ok;
 }
 
 template <typename T, int TN, int BITS>
@@ -244,12 +245,12 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PairShape<TN, BITS>:
     const uint32_t tmem_d = *tmem_slot;
     if (warp >= S::kWeightWarps) pdl_wait();  // the weight warps read constants and write shared memory only
 
+    bool ok = true;
     if (warp < S::kWeightWarps) {
-        if constexpr (BITS != 0) weight_warps<TN, BITS>(p, As, full, empty, rank, pair, npairs);
+        if constexpr (BITS != 0) ok = weight_warps<TN, BITS>(p, As, full, empty, rank, pair, npairs);
     } else if (warp == kCopyWarp) {
         if (lane == 0) {
             const uint32_t full0 = leader_addr(full);
-            bool ok = true;
             int s = 0, use = 0;
             for (int w = pair; w < tiles; w += npairs) {
                 const int m0 = w % p.mtiles * TN + rank * (TN / 2), n0 = w / p.mtiles * (2 * kPRows) + rank * kPRows;
@@ -265,9 +266,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PairShape<TN, BITS>:
                     if (++s == S::kStages) s = 0, use++;
                 }
             }
-            // after a wait that ran out: the copies in flight land before the shared memory is given back
-            if (!ok)
-                for (const unsigned long long t0 = global_ns(); global_ns() - t0 < 1000000ull;) __nanosleep(1000);
         }
         __syncwarp();
     } else if (warp == kMmaWarp) {
@@ -275,7 +273,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PairShape<TN, BITS>:
             // f32 accumulator, fp16 (0) or bf16 (1) operands, both K-major, N >> 3 in bits 17-22, M = 256: M >> 4 in bits 24-28
             constexpr uint32_t fmt = BITS ? 0u : 1u;
             constexpr uint32_t idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)(TN >> 3) << 17) | ((uint32_t)(2 * kPRows >> 4) << 24);
-            bool ok = true;
             int s = 0, ph = 0, cnt = 0;
             for (int w = pair; w < tiles; w += npairs, cnt++) {
                 const int acc = cnt & 1, use = cnt >> 1;
@@ -302,7 +299,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PairShape<TN, BITS>:
         const int ew = warp - S::kWeightWarps, lanes = (warp & 3) * 32, half = ew >> 2;  // a warp reads tensor-memory lanes 32 (warp % 4) ..
         constexpr int kSpan = TN / (S::kEpiWarps / 4);
         const uint32_t tempty0 = leader_addr(tempty);
-        bool ok = true;
         int cnt = 0;
         for (int w = pair; w < tiles; w += npairs, cnt++) {
             const int m0 = w % p.mtiles * TN, n_warp = w / p.mtiles * (2 * kPRows) + rank * kPRows + lanes, acc = cnt & 1;
@@ -322,7 +318,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PairShape<TN, BITS>:
         }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
+    sync_and_settle(ok);
     cluster_sync();  // neither CTA leaves while the other may still signal it or read its operands
     if (warp == kMmaWarp) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");

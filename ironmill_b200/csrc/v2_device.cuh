@@ -46,6 +46,16 @@ __device__ __forceinline__ unsigned long long global_ns() {
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
     return t;
 }
+// End of a kernel that feeds the tensor cores by the copy engine, instead of its last __syncthreads(): where one of the block's waits ran out, copies
+// and products may still be in flight to shared and tensor memory that the next block on the SM gets. They land within microseconds of being able to at all; the
+// block stays a millisecond.
+__device__ __forceinline__ void sync_and_settle(bool ok) {
+    if (!__syncthreads_or(!ok)) return;
+    if (threadIdx.x == 0)
+        for (const unsigned long long t0 = global_ns(); global_ns() - t0 < 1000000ull;) __nanosleep(1000);
+    __syncthreads();
+}
+
 // limit_ms: patience of this wait (default: kWaitLimitNs); a kernel that may legitimately sit behind another GPU passes more
 __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, int *err, unsigned limit_ms = (unsigned)(kWaitLimitNs / 1000000ull)) {
     if (mbar_try_wait(bar, parity)) return true;
