@@ -847,8 +847,7 @@ int latent_attention_run(const Device *dev, const LatentArgs &a, cudaStream_t st
     const int M = a.nseq * a.T;
     const int dv = prefill_dv(s);
     const size_t per_head = (size_t)(s.dimP + s.vP) * 2;
-    if (!a.f32 && a.nseq == 1 && a.host_slot >= 0 && (a.T >= kLatentExpandMin || (a.T >= kLatentExpandShort && a.host_pos <= 3 * a.T)) &&
-        latent_expands(s) && a.kv) {
+    if (!a.f32 && a.nseq == 1 && a.host_slot >= 0 && a.T >= kLatentExpandMin && latent_expands(s) && a.kv) {
         const int ctx = a.host_pos + a.T;
         const int group = (int)std::min<size_t>(s.heads, a.kv_bytes / (per_head * ctx));
         if (group >= 1) {

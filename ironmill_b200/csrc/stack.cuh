@@ -106,9 +106,9 @@ struct LatentArgs {
     int host_slot;
     int splits_ctx;          // context length the split count is chosen for
 };
-// Tokens of one sequence from which keys and values are expanded per head; and where the portion is at least a quarter of the context, so that
-// expanding it costs no more than a few of its own projections (a prompt of 50 tokens, 16 heads: 19 + 13 + 41 us absorbed, 20 + 12 us expanded).
-constexpr int kLatentExpandMin = 64, kLatentExpandShort = 16;
+// Tokens of one sequence from which keys and values are expanded per head. (A prompt of 50 tokens takes 19 + 13 + 41 us in absorbed form and 20 + 12 us
+// expanded, but the absorbed form keeps weighted sums of latents and W_uv's products in f32 where the expanded one rounds every value to bf16.)
+constexpr int kLatentExpandMin = 64;
 int latent_attention_run(const Device *dev, const LatentArgs &a, cudaStream_t st, int *launches);
 size_t latent_part_bytes(const Device *dev, const LatentShape &s, int tokens, int nseq);
 bool latent_expands(const LatentShape &s);  // prompt chunks of this shape can take the expanded form
