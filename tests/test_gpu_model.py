@@ -74,6 +74,35 @@ def test_prompt_chunks_with_qk_norm(n_bits, nh, nkv, prompt_len):
     assert err <= 5e-2, err
 
 
+@pytest.mark.parametrize("n_bits", [8, 4])
+@pytest.mark.parametrize("arch,rotary_dim", [("llama", 0), ("qwen3", 0), ("qwen3", 64), ("llama", 96)])
+def test_prompt_leaves_the_cache_rows_of_single_tokens(arch, rotary_dim, n_bits):
+    """With one layer, keys and values depend on the tokens alone: prompts in one portion (the encoder of 16 tokens and more) and in portions of 14
+    (the per-token one) leave the same bytes, norms and residual norms, so steps that read them give the same logits, bit for bit. Token
+    counts around the four rows of an encoding warp, in the second slot, behind a cached prefix, beside a sequence that has to stay as it was."""
+    from ironmill_b200.engine import CudaConfig, CudaInference
+    cfg = _cfg(arch, 1, 256, 512, 4, 2, 500, 1e6, 1e-6)
+    cfg.extra["rotary_dim"] = rotary_dim
+    tensors = synth_model(cfg, seed=23, gamma_jitter=0.2)
+    tqc = orc.TqConstants(128, n_bits, seed=3)
+    engines = [CudaInference(CudaConfig(max_seq_len=200, max_batch=2, n_bits=n_bits, prefill_chunk_size=c)) for c in (200, 14)]
+    for e in engines:
+        e.load_weights(DictProvider(cfg, tensors), tq_signs=tqc.signs, tq_qjl=tqc.qjl)
+    rng = H.rng_for("rows")
+    for n in (16, 17, 18, 19, 131):
+        first, prefix, rest, fed = (rng.integers(0, 500, k).astype(np.uint32) for k in (9, 21, n, 16))
+        logits = []
+        for e in engines:
+            e.reset()
+            a, b = e.add_sequence(first), e.add_sequence(prefix)
+            steps = [e.batch_decode_step({a: int(fed[0])})]
+            e.extend_sequence(b, rest, [n - 1])
+            steps += [e.batch_decode_step({a: int(x), b: int(y)}) for x, y in fed[2:].reshape(-1, 2)]
+            logits.append([lg for step in steps for _, lg in step])
+        for x, y in zip(*logits):
+            assert np.array_equal(x, y), n
+
+
 def test_tiny_llama_shape_awq_int8_parity():
     # no QK-norm (plain RoPE), AWQ scales, GQA 4, tied embeddings, INT8 weights
     cfg = _cfg("llama", 2, 512, 1024, 8, 2, 777, 5e5, 1e-5, tie=True)
