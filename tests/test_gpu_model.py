@@ -103,6 +103,40 @@ def test_prompt_leaves_the_cache_rows_of_single_tokens(arch, rotary_dim, n_bits)
             assert np.array_equal(x, y), n
 
 
+@pytest.mark.parametrize("n_bits", [16, 8, 4])
+@pytest.mark.parametrize("arch,rotary_dim", [("qwen3", 64), ("llama", 96)])
+def test_partial_rotation(arch, rotary_dim, n_bits, monkeypatch):
+    """Queries and keys of which the first 64 or 96 dimensions are rotated (d with d + rotary_dim / 2), in a prompt's kernels and a step's. The weights are large
+    enough for scores that a wrong rotation would change."""
+    from ironmill_b200.engine import CudaConfig, CudaInference
+    cfg = _cfg(arch, 1, 256, 512, 4, 2, 500, 1e4, 1e-6)
+    cfg.extra["rotary_dim"] = rotary_dim
+    tensors = synth_model(cfg, seed=24, gamma_jitter=0.2)
+    for n in ("q_proj", "k_proj"):
+        t = tensors["model.layers.0.self_attn.%s.weight" % n]
+        t.scale = (np.asarray(t.scale) * 3).astype(np.asarray(t.scale).dtype)
+    norm_rope = orc.qk_norm_rope
+    monkeypatch.setattr(orc, "qk_norm_rope", lambda *a: norm_rope(*a, rotary_dim=rotary_dim))
+
+    def rope(x, cos, sin, heads, hd, off):
+        v = np.asarray(x, dtype=np.float32).reshape(-1, heads, hd).copy()
+        h = rotary_dim // 2
+        c, s = (np.asarray(t, dtype=np.float32)[off:off + len(v), None, :h] for t in (cos, sin))
+        lo, hi = v[..., :h].copy(), v[..., h:2 * h].copy()
+        v[..., :h], v[..., h:2 * h] = lo * c - hi * s, lo * s + hi * c
+        return v.astype(np.float16).reshape(np.shape(x))
+
+    monkeypatch.setattr(orc, "rope", rope)
+    if n_bits == 16:
+        eng, ref = CudaInference(CudaConfig(max_seq_len=128).without_turboquant()), OracleModel(cfg, tensors, None, 128, kv_f16=True)
+        eng.load_weights(DictProvider(cfg, tensors))
+    else:
+        eng, ref = _engines(cfg, tensors, 128, n_bits=n_bits)
+    prompt = H.rng_for("partial").integers(0, 500, 83).astype(np.uint32)
+    errs = [np.abs(eng.prefill(prompt) - ref.forward(prompt)).max()] + [np.abs(eng.decode_step(t) - ref.forward([t])).max() for t in (1, 77, 400)]
+    assert max(errs) <= (1e-2 if n_bits == 16 else 5e-2), errs
+
+
 def test_tiny_llama_shape_awq_int8_parity():
     # no QK-norm (plain RoPE), AWQ scales, GQA 4, tied embeddings, INT8 weights
     cfg = _cfg("llama", 2, 512, 1024, 8, 2, 777, 5e5, 1e-5, tie=True)
