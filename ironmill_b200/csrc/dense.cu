@@ -612,10 +612,6 @@ int dense_prepare(const Device *dev) {
     return IM_OK;
 }
 
-int dense_launches(int M, int f32, int src_kind) {
-    return M >= (f32 ? kDenseGemmMinF32 : kDenseGemmMin) ? 1 + (src_kind != kSrcPlain) : (M + kDenseMaxRows - 1) / kDenseMaxRows;
-}
-
 int dense_project(const Device *dev, const DenseWeight &w, const DenseSrc &src, const DenseEpi &epi, int M, void *h_scratch, cudaStream_t st) {
     if (M <= 0) return IM_OK;
     const int ldv = 16 / (int)elem_size(w.f32);

@@ -736,14 +736,13 @@ static FlashArgs grouped_flash_args(const Device *dev, const GroupedArgs &a) {
     return f;
 }
 
-int grouped_attention_run(const Device *dev, const GroupedArgs &a, cudaStream_t st, int *launches) {
+int grouped_attention_run(const Device *dev, const GroupedArgs &a, cudaStream_t st) {
     const GroupedShape &s = a.s;
     const int M = a.nseq * a.T;
     int rc;
     if (!a.f32 && a.nseq == 1 && a.host_slot >= 0 && a.T >= kGroupedPrefillMin && grouped_prefills(s)) {
         rc = rows_launch<__nv_bfloat16>(a, st);
         if (rc != IM_OK) return rc;
-        *launches += 2;
         rc = flash_run(grouped_flash_args(dev, a), st);
         if (rc != IM_ERR_BOUNDS) return rc;
         const int dv = prefill_dv(s);
@@ -762,13 +761,10 @@ int grouped_attention_run(const Device *dev, const GroupedArgs &a, cudaStream_t 
     if (!tc || a.T > 1) {
         rc = a.f32 ? rows_launch<float>(a, st) : rows_launch<__nv_bfloat16>(a, st);
         if (rc != IM_OK) return rc;
-        *launches += 1;
     }
     if (tc) {
-        *launches += 1;
         return head_tiles(s) == 2 ? decode_any<2>(a, p, st) : decode_any<1>(a, p, st);
     }
-    *launches += 2;
     return a.f32 ? simt_launch<float>(a, p, st) : simt_launch<__nv_bfloat16>(a, p, st);
 }
 

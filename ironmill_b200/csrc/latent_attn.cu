@@ -842,7 +842,7 @@ static FlashArgs expanded_flash_args(const Device *dev, const LatentArgs &a, con
     return f;
 }
 
-int latent_attention_run(const Device *dev, const LatentArgs &a, cudaStream_t st, int *launches) {
+int latent_attention_run(const Device *dev, const LatentArgs &a, cudaStream_t st) {
     const LatentShape &s = a.s;
     const int M = a.nseq * a.T;
     const int dv = prefill_dv(s);
@@ -852,7 +852,6 @@ int latent_attention_run(const Device *dev, const LatentArgs &a, cudaStream_t st
         const int group = (int)std::min<size_t>(s.heads, a.kv_bytes / (per_head * ctx));
         if (group >= 1) {
             IM_CUDA_CHECK(launch_k(latent_rows_kernel<__nv_bfloat16>, dim3(M), dim3(256), 0, st, a));
-            *launches += 1;
             const __nv_bfloat16 *lat = static_cast<const __nv_bfloat16 *>(a.cache) + (size_t)a.host_slot * a.max_seq * s.rowP;
             for (int h0 = 0; h0 < s.heads; h0 += group) {
                 const int nh = std::min(group, s.heads - h0), ldkv = nh * (s.dimP + s.vP);
@@ -869,13 +868,11 @@ int latent_attention_run(const Device *dev, const LatentArgs &a, cudaStream_t st
                 rc = flash_run(expanded_flash_args(dev, a, kv, ldkv, h0, nh, ctx), st);
                 if (rc != IM_ERR_BOUNDS) {
                     if (rc != IM_OK) return rc;
-                    *launches += 2;
                     continue;
                 }
                 rc = dv == 32 ? prefill_launch<32>(a, kv, ldkv, h0, nh, st) : dv == 64 ? prefill_launch<64>(a, kv, ldkv, h0, nh, st)
                      : dv == 128 ? prefill_launch<128>(a, kv, ldkv, h0, nh, st) : prefill_launch<256>(a, kv, ldkv, h0, nh, st);
                 if (rc != IM_OK) return rc;
-                *launches += 2;
             }
             return IM_OK;
         }
@@ -911,11 +908,9 @@ int latent_attention_run(const Device *dev, const LatentArgs &a, cudaStream_t st
         if (splits > 32) IM_CUDA_CHECK(launch_k(latent_combine_kernel<4>, grid, dim3(512), 0, st, p, a.sink, s.heads, s.latP, comb));
         else IM_CUDA_CHECK(launch_k(latent_combine_kernel<1>, grid, dim3(128), 0, st, p, a.sink, s.heads, s.latP, comb));
         src = comb;
-        *launches += 1;
     }
     if (a.f32) rc = M >= 4 ? out_launch<float, 4>(a, p, src, splits > 1, M, st) : out_launch<float, 1>(a, p, src, splits > 1, M, st);
     else rc = M >= 4 ? out_launch<__nv_bfloat16, 4>(a, p, src, splits > 1, M, st) : out_launch<__nv_bfloat16, 1>(a, p, src, splits > 1, M, st);
-    *launches += 3;
     return rc;
 }
 

@@ -402,16 +402,15 @@ int linear_prepare(const Device *dev) {
     return gated_prepare();
 }
 
-int linear_attention_run(const Device *dev, const LinearArgs &a, cudaStream_t st, int *launches) {
+int linear_attention_run(const Device *dev, const LinearArgs &a, cudaStream_t st) {
     const int dimK = round_up(a.s.dimP, 16), M = a.nseq * a.T;
     int rc = IM_ERR_BOUNDS;
     if (a.s.gated) {
         if (a.T == 1 && gated_decode_takes(a.s)) {
-            *launches += 1;
             return gated_decode_run(a, st);
         }
         if (!a.f32 && a.nseq == 1 && a.T >= kGatedChunkMin && gated_chunk_takes(a.s)) {
-            rc = gated_chunk_run(a, st, launches);
+            rc = gated_chunk_run(a, st);
             if (rc != IM_ERR_BOUNDS) return rc;
         }
     } else if (!a.f32 && a.T >= 16 && dimK <= 256 && linear_chunk_smem(64, dimK, 1) <= kLinearSmemMax) {
@@ -426,7 +425,6 @@ int linear_attention_run(const Device *dev, const LinearArgs &a, cudaStream_t st
             }
         }
         if (sg.count > 1) {
-            *launches += 1;
             rc = chunk_any(a, dimK, 1, sg, st);
         } else if (a.T > 64 && dimK <= 128 && linear_chunk_smem(128, dimK, 2) <= kLinearSmemMax) {
             rc = chunk_launch<128, 1>(a, dimK, 2, sg, st);
@@ -438,7 +436,6 @@ int linear_attention_run(const Device *dev, const LinearArgs &a, cudaStream_t st
     if (rc != IM_OK) return rc;
     if (a.f32) IM_CUDA_CHECK(launch_k(linear_finish_kernel<float>, dim3(M), dim3(256), 0, st, a));
     else IM_CUDA_CHECK(launch_k(linear_finish_kernel<__nv_bfloat16>, dim3(M), dim3(256), 0, st, a));
-    *launches += 2;
     return IM_OK;
 }
 

@@ -546,7 +546,7 @@ int gated_decode_run(const LinearArgs &a, cudaStream_t st) {
     return a.f32 ? decode_any<float>(a, p, st) : decode_any<__nv_bfloat16>(a, p, st);
 }
 
-int gated_chunk_run(const LinearArgs &a, cudaStream_t st, int *launches) {
+int gated_chunk_run(const LinearArgs &a, cudaStream_t st) {
     const LinearShape &s = a.s;
     const GatedSizes z = chunk_sizes(s, a.T);
     if (!a.decays || !a.chunk_states || (size_t)z.nchunks * s.heads * s.dim * s.vS * 4 > a.chunk_bytes) return IM_ERR_BOUNDS;
@@ -556,7 +556,6 @@ int gated_chunk_run(const LinearArgs &a, cudaStream_t st, int *launches) {
     if (s.vP <= 64) IM_CUDA_CHECK(launch_k(gated_output_kernel<4>, grid, block, gated_output_smem(64), st, a));
     else if (s.vP <= 128) IM_CUDA_CHECK(launch_k(gated_output_kernel<8>, grid, block, gated_output_smem(128), st, a));
     else IM_CUDA_CHECK(launch_k(gated_output_kernel<16>, grid, block, gated_output_smem(256), st, a));
-    *launches += 3;
     return IM_OK;
 }
 

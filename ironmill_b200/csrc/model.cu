@@ -229,7 +229,7 @@ struct Model : im_model {
     PeerAllreduce xar;
 
     ~Model() override;
-    int forward(int nseq, int T, cudaStream_t st, int *launches, Prof *prof, bool all_logits, const int *slots) override;
+    int forward(int nseq, int T, cudaStream_t st, Prof *prof, bool all_logits, const int *slots) override;
     int finalize() override;
     // the matvec kernels take at most 64 rows per call
     int prefill_chunk() const override { return gemm_ok ? cfg.prefill_chunk_size : std::min(cfg.prefill_chunk_size, 64); }
@@ -471,34 +471,28 @@ static int attention_block(Model *m, int part, const TqPrep &a, __half *q_buf, L
 
 // Logits of `rows` normed rows. The matvec reads the whole table for every four rows (up to 64 rows per call); from five rows on one pass on the
 // tensor cores reads it once (24 rows, 32768 x 4096: six passes of 65 us, one of 50).
-static int head_rows(Model *m, const __half *x, __half *out, int rows, cudaStream_t st, int *nl) {
+static int head_rows(Model *m, const __half *x, __half *out, int rows, cudaStream_t st) {
     const int H = m->cfg.hidden_size;
     if (rows > 4) {
         const int rc = dense_rows_f16(m->dev, m->lm_head, m->vocab_l, H, x, out, rows, st);
-        if (rc != IM_ERR_BOUNDS) {
-            ++*nl;
-            return rc;
-        }
+        if (rc != IM_ERR_BOUNDS) return rc;
     }
     for (int r = 0; r < rows; r += 64) {
         const int nb = rows - r < 64 ? rows - r : 64;
         IM_TRY(im_cuda_matvec_f16(m->lm_head, x + (size_t)r * H, out + (size_t)r * m->vocab_l, m->vocab_l, H, nb, st));
-        *nl += (nb + 3) / 4;
     }
     return IM_OK;
 }
 
-int Model::forward(int nseq, int T, cudaStream_t st, int *launches, Prof *prof, bool all_logits, const int *slots) {
+int Model::forward(int nseq, int T, cudaStream_t st, Prof *prof, bool all_logits, const int *slots) {
     Model *const m = this;
     const im_model_config &c = m->cfg;
     const int attn_splits = m->prefill_slot_id >= 0 ? tq_auto_splits(m->dev, 1, T, m->nkv_l, m->prefill_ctx_end) : decode_splits(m, nseq);
     const int H = c.hidden_size, hd = c.head_dim, MT = nseq * T;
     const float eps = c.rms_eps;
     const float attn_scale = c.attn_scale != 0.0f ? c.attn_scale : 1.0f / sqrtf((float)hd);
-    int nl = 0;
     IM_TRY(im_cuda_embedding_norm(m->tokens_dev, m->embed, m->layers[0].input_ln, m->norm_out, m->hidden, H, MT, (uint32_t)c.vocab_size, eps,
                                   c.embed_scale != 0.0f ? c.embed_scale : 1.0f, st));
-    nl++;
     IM_MARK(kCatEmbed);
     const bool mega = MT == 1 && m->mega_ready && !prof && !slots;  // the whole-token kernel works on slot 0
     if (mega) {  // every layer in one persistent launch (decode_mega.cu); leaves the same buffers as the loop below
@@ -507,7 +501,6 @@ int Model::forward(int nseq, int T, cudaStream_t st, int *launches, Prof *prof, 
         IM_TRY(rc);
         IM_TRY(tp_allreduce(m, m->ffn_down, (size_t)H, st));  // tensor parallel: the last layer's down projection
         IM_TRY(im_cuda_residual_add(m->residual, m->ffn_down, m->hidden, (size_t)H, st));
-        nl += 2 + (m->world > 1 ? 1 : 0);
     }
     // More than one token per sequence is the reference's prefill form (its matmul kernels round x / awq and the
     // dequantised weights to fp16: affine_matmul.metal:44-74), whatever the count; so are decode batches of 16 and more.
@@ -518,7 +511,6 @@ int Model::forward(int nseq, int T, cudaStream_t st, int *launches, Prof *prof, 
         Layer &L = m->layers[l];
         if (l == 0) {
             IM_TRY(gemm_affine_tc(L.qkv, m->norm_out, m->qkv, MT, m->xs_scratch, st));
-            nl += 2;
             IM_MARK(kCatQkv);
         }
         TqPrep a{};
@@ -531,7 +523,6 @@ int Model::forward(int nseq, int T, cudaStream_t st, int *launches, Prof *prof, 
         IM_TRY(attention_block(m, 0, a, m->qkv, L, nseq, T, attn_scale, attn_splits, slots, st));
         IM_MARK(kCatKvWrite);
         IM_TRY(attention_block(m, 1, a, m->qkv, L, nseq, T, attn_scale, attn_splits, slots, st));
-        nl += 3;
         IM_MARK(kCatAttn);
         IM_TRY(gemm_affine_tc(L.o, m->attn_out, m->ffn_down, MT, m->xs_scratch, st));
         IM_MARK(kCatOProj);
@@ -557,7 +548,6 @@ int Model::forward(int nseq, int T, cudaStream_t st, int *launches, Prof *prof, 
         IM_MARK(kCatDown);
         IM_TRY(tp_allreduce(m, m->ffn_down, (size_t)MT * H, st));  // tensor parallel: down is row-split
         if (m->world > 1) IM_MARK(kCatComm);
-        nl += 7 + (m->world > 1 ? 2 : 0);
         if (l + 1 < c.num_layers) {
             Layer &Nx = m->layers[l + 1];
             rc = residual_norm_scaled(m->residual, m->ffn_down, Nx.input_ln, Nx.qkv->awq, m->norm_out, m->hidden, H, MT, eps, st);
@@ -565,11 +555,9 @@ int Model::forward(int nseq, int T, cudaStream_t st, int *launches, Prof *prof, 
             if (rc == IM_ERR_BOUNDS) rc = im_cuda_fused_residual_rms_norm(m->residual, m->ffn_down, Nx.input_ln, m->norm_out, m->hidden, H, MT, eps, st);
             IM_TRY(rc);
             IM_TRY(gemm_affine_tc(Nx.qkv, m->norm_out, m->qkv, MT, m->xs_scratch, st, qkv_scaled));
-            nl += 2;
             IM_MARK(kCatQkv);
         } else {
             IM_TRY(im_cuda_residual_add(m->residual, m->ffn_down, m->hidden, (size_t)MT * H, st));
-            nl++;
             IM_MARK(kCatResNorm);
         }
     }
@@ -581,11 +569,9 @@ int Model::forward(int nseq, int T, cudaStream_t st, int *launches, Prof *prof, 
     for (int l = 0; l < c.num_layers && !mega && !gemm; l++) {
         Layer &L = m->layers[l];
         const bool fused4 = L.qkv->bits == 4 && L.gate->bits == 4 && L.up->bits == 4;
-        const int nmv = (MT + 3) / 4;
         if (l == 0) {
             IM_TRY(im_cuda_matvec_affine(static_cast<const im_affine_weight *>(&L.q_rows), m->norm_out, m->q_d, MT, st));
             IM_TRY(im_cuda_matvec_affine(static_cast<const im_affine_weight *>(&L.kv_rows), m->norm_out, m->k_d, MT, st));
-            nl += 2 * nmv;
             IM_MARK(kCatQkv);
         }
         // (QK-norm +) RoPE, K/V cache write and query rotation in one launch, then split attention + reduce
@@ -599,7 +585,6 @@ int Model::forward(int nseq, int T, cudaStream_t st, int *launches, Prof *prof, 
         IM_TRY(attention_block(m, 0, a, m->q_d, L, nseq, T, attn_scale, attn_splits, slots, st));
         IM_MARK(kCatKvWrite);
         IM_TRY(attention_block(m, 1, a, m->q_d, L, nseq, T, attn_scale, attn_splits, slots, st));
-        nl += 3;
         IM_MARK(kCatAttn);
         IM_TRY(im_cuda_matvec_affine(static_cast<im_affine_weight *>(L.o), m->attn_out, m->ffn_down, MT, st));
         IM_MARK(kCatOProj);
@@ -610,7 +595,6 @@ int Model::forward(int nseq, int T, cudaStream_t st, int *launches, Prof *prof, 
         if (fused4) {
             IM_TRY(im_cuda_ffn_gate_up_act(static_cast<im_affine_weight *>(L.gate), static_cast<im_affine_weight *>(L.up), m->norm_out,
                                            m->ffn_gate, MT, st));
-            nl += nmv;
         } else {
             IM_TRY(im_cuda_matvec_affine(static_cast<im_affine_weight *>(L.gate), m->norm_out, m->ffn_gate, MT, st));
             IM_TRY(im_cuda_matvec_affine(static_cast<im_affine_weight *>(L.up), m->norm_out, m->ffn_up, MT, st));
@@ -618,14 +602,12 @@ int Model::forward(int nseq, int T, cudaStream_t st, int *launches, Prof *prof, 
             cudaError_t le = launch_k(silu_mul_kernel, dim3((unsigned)((n / 2 + 255) / 256)), dim3(256), 0, st, (const __half *)m->ffn_gate,
                                       (const __half *)m->ffn_up, m->ffn_gate, n);
             if (le != cudaSuccess) return fail(IM_ERR_CUDA, "launch failed: %s", cudaGetErrorString(le));
-            nl += 2 * nmv + 1;
         }
         IM_MARK(kCatFfn);
         IM_TRY(im_cuda_matvec_affine(static_cast<im_affine_weight *>(L.down), m->ffn_gate, m->ffn_down, MT, st));
         IM_MARK(kCatDown);
         IM_TRY(tp_allreduce(m, m->ffn_down, (size_t)MT * H, st));
         if (m->world > 1) IM_MARK(kCatComm);
-        nl += 2 * nmv + 1 + (m->world > 1 ? 2 : 0);
         if (l + 1 < c.num_layers) {
             Layer &Nx = m->layers[l + 1];
             if (Nx.qkv->bits == 4) {
@@ -634,49 +616,39 @@ int Model::forward(int nseq, int T, cudaStream_t st, int *launches, Prof *prof, 
             } else {
                 IM_TRY(im_cuda_fused_residual_rms_norm(m->residual, m->ffn_down, Nx.input_ln, m->norm_out, m->hidden, H, MT, eps, st));
                 IM_TRY(im_cuda_matvec_affine(static_cast<const im_affine_weight *>(&Nx.q_rows), m->norm_out, m->q_d, MT, st));
-                nl++;
             }
             IM_TRY(im_cuda_matvec_affine(static_cast<const im_affine_weight *>(&Nx.kv_rows), m->norm_out, m->k_d, MT, st));
-            nl += 2 * nmv;
             IM_MARK(kCatQkv);
         } else {
             IM_TRY(im_cuda_residual_add(m->residual, m->ffn_down, m->hidden, (size_t)MT * H, st));
-            nl++;
             IM_MARK(kCatResNorm);
         }
     }
     if (all_logits) {  // final norm + lm_head on every token of the (single) sequence: prefill_all_logits
         IM_TRY(im_cuda_rms_norm(m->hidden, m->final_norm, m->norm_out, H, MT, eps, st));
-        IM_TRY(head_rows(m, m->norm_out, m->logits_seq, MT, st, &nl));
-        nl++;
+        IM_TRY(head_rows(m, m->norm_out, m->logits_seq, MT, st));
         if (m->world > 1) {
 #if IM_HAVE_NCCL_H
             IM_NCCL_CHECK(nccl()->AllGather(m->logits_seq, m->logits_seq_all, (size_t)MT * m->vocab_l, ncclHalf, m->comm, st));
-            nl++;
 #endif
         }
-        if (launches) *launches = nl;
         return IM_OK;
     }
     // final norm + lm_head on the last token of each sequence
     if (T == 1) {  // one row per sequence: one launch
         IM_TRY(im_cuda_rms_norm(m->hidden, m->final_norm, m->norm_out, H, nseq, eps, st));
-        nl++;
     }
     for (int s = 0; s < nseq && T > 1; s++) {
         const __half *last = m->hidden + ((size_t)s * T + (T - 1)) * H;
         IM_TRY(im_cuda_rms_norm(last, m->final_norm, m->norm_out + (size_t)s * H, H, 1, eps, st));
-        nl++;
     }
-    IM_TRY(head_rows(m, m->norm_out, m->logits, nseq, st, &nl));
+    IM_TRY(head_rows(m, m->norm_out, m->logits, nseq, st));
     if (m->world > 1) {
 #if IM_HAVE_NCCL_H
         IM_NCCL_CHECK(nccl()->AllGather(m->logits, m->logits_all, (size_t)nseq * m->vocab_l, ncclHalf, m->comm, st));
-        nl++;
 #endif
     }
     IM_MARK(kCatHead);
-    if (launches) *launches = nl;
     return IM_OK;
 }
 

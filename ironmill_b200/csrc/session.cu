@@ -120,14 +120,13 @@ static int get_graph(im_model *m, int batch, cudaGraphExec_t *out, bool mapped =
     cudaStream_t st = m->stream;
     // one eager pass first: sets function attributes and warms NCCL outside the capture
     m->uncounted = true;
-    int rc = m->forward(batch, 1, st, nullptr, nullptr, false, slots);
+    int rc = m->forward(batch, 1, st, nullptr, false, slots);
     m->uncounted = false;
     IM_TRY(rc);
     IM_CUDA_CHECK(cudaStreamSynchronize(st));
     cudaGraph_t g = nullptr;
     IM_CUDA_CHECK(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-    int nl = 0;
-    rc = m->forward(batch, 1, st, &nl, nullptr, false, slots);
+    rc = m->forward(batch, 1, st, nullptr, false, slots);
     if (rc == IM_OK) {
         const int vp = m->cfg.vocab_size / m->logit_parts;
         const dim3 grid(kArgmaxCtas, batch);
@@ -140,7 +139,6 @@ static int get_graph(im_model *m, int batch, cudaGraphExec_t *out, bool mapped =
         if (le == cudaSuccess) le = launch_k(bump_kernel, dim3(1), dim3(1), 0, st, m->step_dev);
         if (le == cudaSuccess) le = launch_k(advance_pos_kernel, dim3(1), dim3(64), 0, st, m->pos_dev, slots, batch, 1);
         if (le != cudaSuccess) rc = fail(IM_ERR_CUDA, "launch failed: %s", cudaGetErrorString(le));
-        nl += 3;
     }
     cudaError_t e = cudaStreamEndCapture(st, &g);
     if (rc != IM_OK) {
@@ -148,12 +146,26 @@ static int get_graph(im_model *m, int batch, cudaGraphExec_t *out, bool mapped =
         return rc;
     }
     if (e != cudaSuccess) return fail(IM_ERR_CUDA, "graph capture failed: %s", cudaGetErrorString(e));
+    size_t nodes = 0;
+    int kernels = 0;
+    e = cudaGraphGetNodes(g, nullptr, &nodes);
+    std::vector<cudaGraphNode_t> all(nodes);
+    if (e == cudaSuccess && nodes > 0) e = cudaGraphGetNodes(g, all.data(), &nodes);
+    for (size_t i = 0; i < nodes && e == cudaSuccess; i++) {
+        cudaGraphNodeType type;
+        e = cudaGraphNodeGetType(all[i], &type);
+        kernels += e == cudaSuccess && type == cudaGraphNodeTypeKernel;
+    }
+    if (e != cudaSuccess) {
+        cudaGraphDestroy(g);
+        return fail(IM_ERR_CUDA, "graph inspection failed: %s", cudaGetErrorString(e));
+    }
     cudaGraphExec_t ge = nullptr;
     e = cudaGraphInstantiate(&ge, g, 0);
     cudaGraphDestroy(g);
     if (e != cudaSuccess) return fail(IM_ERR_CUDA, "graph instantiate failed: %s", cudaGetErrorString(e));
     m->graphs[key] = ge;
-    m->launches_per_step = nl;
+    m->launches_per_step = kernels;
     *out = ge;
     return IM_OK;
 }
@@ -232,7 +244,7 @@ static int prefill_slot(im_model *m, int slot, const uint32_t *tokens_host, int 
         m->prefill_slot_id = slot;
         m->prefill_ctx_begin = m->slot_pos[slot];
         m->prefill_ctx_end = m->slot_pos[slot] + T;
-        const int frc = m->forward(1, T, st, nullptr, nullptr, rows_here, slots);
+        const int frc = m->forward(1, T, st, nullptr, rows_here, slots);
         m->prefill_slot_id = -1;
         IM_TRY(frc);
         advance_pos_kernel<<<1, 64, 0, st>>>(m->pos_dev, slots, 1, T);
@@ -572,11 +584,11 @@ IM_EXPORT int im_cuda_model_profile_step(im_model *m, int batch, float *ms_by_ca
     IM_CUDA_CHECK(cudaSetDevice(m->dev->ordinal));
     cudaStream_t st = m->stream;
     m->uncounted = true;
-    int rc = m->forward(batch, 1, st, nullptr, nullptr, false, nullptr);  // warm
+    int rc = m->forward(batch, 1, st, nullptr, false, nullptr);  // warm
     Prof prof;
     prof.st = st;
     prof.mark(-1);
-    if (rc == IM_OK) rc = m->forward(batch, 1, st, nullptr, &prof, false, nullptr);
+    if (rc == IM_OK) rc = m->forward(batch, 1, st, &prof, false, nullptr);
     m->uncounted = false;
     cudaError_t e = cudaStreamSynchronize(st);
     for (int i = 0; i < n_categories; i++) ms_by_category[i] = 0.0f;

@@ -77,7 +77,7 @@ struct im_model {
     // One forward pass over nseq sequences x T tokens each (decode: T = 1; prefill: nseq = 1), tokens in tokens_dev.
     // Logits of the last token of every sequence go to logits_dev, or of every token to logits_rows.
     // slots: device array naming the cache slot of each sequence (nullptr: slots 0 .. nseq - 1).
-    virtual int forward(int nseq, int T, cudaStream_t st, int *launches, im::Prof *prof, bool all_logits, const int *slots) = 0;
+    virtual int forward(int nseq, int T, cudaStream_t st, im::Prof *prof, bool all_logits, const int *slots) = 0;
     virtual int finalize() = 0;
     virtual int prefill_chunk() const { return cfg.prefill_chunk_size; }
     virtual int alloc_logits_rows() = 0;

@@ -91,7 +91,7 @@ struct StackModel : im_model {
     int last_rows = 0;
     std::map<std::array<double, 8>, std::pair<float *, float *>> rot_tables;
 
-    int forward(int nseq, int T, cudaStream_t st, int *launches, Prof *prof, bool all_logits, const int *slots) override;
+    int forward(int nseq, int T, cudaStream_t st, Prof *prof, bool all_logits, const int *slots) override;
     int finalize() override;
     int alloc_logits_rows() override {
         IM_TRY(alloc((void **)&rows, (size_t)kAllLogitsChunk * cfg.vocab_size * 4));
@@ -112,8 +112,8 @@ struct StackModel : im_model {
     }
     int load(const std::string &name, const void *data, int dtype, const std::vector<int64_t> &shape);
     int rot_table(const im_stack_layer &c, const float **cosc, const float **sinc);
-    int mix(const StackRun &r, int nseq, int T, const int *slots, cudaStream_t st, int *nl);
-    int logits_of(DenseSrc src, int row, int n, float *out, cudaStream_t st, int *nl);
+    int mix(const StackRun &r, int nseq, int T, const int *slots, cudaStream_t st);
+    int logits_of(DenseSrc src, int row, int n, float *out, cudaStream_t st);
 };
 
 namespace {
@@ -454,7 +454,7 @@ int StackModel::finalize() {
 
 // cap tanh(head rms(x) g / cap) of n consecutive rows of the residual, from `row` on.  src: the residual, a sublayer's output that
 // is still to be added included; leaves its rows in last_x.
-int StackModel::logits_of(DenseSrc src, int row, int n, float *out, cudaStream_t st, int *nl) {
+int StackModel::logits_of(DenseSrc src, int row, int n, float *out, cudaStream_t st) {
     const size_t off = (size_t)row * W;
     src.xf += off;
     last_x = src.xf;
@@ -470,12 +470,11 @@ int StackModel::logits_of(DenseSrc src, int row, int n, float *out, cudaStream_t
     }
     DenseEpi e;
     e.kind = kEpiF32; e.xf = out; e.ldx = cfg.vocab_size; e.cap = sc.logit_softcap;
-    *nl += dense_launches(n, f32, src.kind);
     return dense_project(dev, sc.tied_head ? embed : head, src, e, n, h, st);
 }
 
 // The mixer of a run: projected rows in y (and a1), heads to cat.
-int StackModel::mix(const StackRun &r, int nseq, int T, const int *slots, cudaStream_t st, int *nl) {
+int StackModel::mix(const StackRun &r, int nseq, int T, const int *slots, cudaStream_t st) {
     const StackLayer &L = layers[(size_t)r.layer];
     const int host_pos = prefill_slot_id >= 0 ? prefill_ctx_begin : -1, splits_ctx = prefill_slot_id >= 0 ? prefill_ctx_end : cfg.max_seq_len;
     if (L.c.mixer == IM_MIXER_LATENT) {
@@ -484,7 +483,7 @@ int StackModel::mix(const StackRun &r, int nseq, int T, const int *slots, cudaSt
         a.cosc = L.cosc; a.sinc = L.sinc; a.cache = r.cache; a.max_seq = cfg.max_seq_len; a.nseq = nseq; a.T = T; a.pos_dev = pos_dev; a.slot_map = slots;
         a.out = cat; a.ldo = ldcat; a.qabs = qabs; a.part = part; a.part_bytes = part_bytes; a.kv = kv; a.kv_bytes = kv_bytes;
         a.host_slot = prefill_slot_id; a.host_pos = host_pos; a.splits_ctx = splits_ctx;
-        return latent_attention_run(dev, a, st, nl);
+        return latent_attention_run(dev, a, st);
     }
     if (L.c.mixer == IM_MIXER_GROUPED) {
         GroupedArgs a{};
@@ -492,18 +491,17 @@ int StackModel::mix(const StackRun &r, int nseq, int T, const int *slots, cudaSt
         a.kcache = r.cache; a.vcache = r.vcache; a.max_seq = cfg.max_seq_len; a.nseq = nseq; a.T = T; a.pos_dev = pos_dev; a.slot_map = slots;
         a.out = cat; a.ldo = ldcat; a.part = part; a.part_bytes = part_bytes; a.counters = counters;
         a.host_slot = prefill_slot_id; a.host_pos = host_pos; a.splits_ctx = splits_ctx;
-        return grouped_attention_run(dev, a, st, nl);
+        return grouped_attention_run(dev, a, st);
     }
     LinearArgs a{};
     a.s = L.ns; a.f32 = f32; a.y = y; a.ldy = ldy; a.norm = L.o_norm; a.pows = L.pows; a.state = static_cast<float *>(r.cache);
     a.a1 = a1; a.a2 = L.a2; a.a2b = L.a2b; a.decays = decays; a.chunk_states = chunk_states; a.chunk_bytes = chunk_bytes;
     a.nseq = nseq; a.T = T; a.pos_dev = pos_dev; a.slot_map = slots; a.keep_state = uncounted ? 1 : 0; a.o = rec_o; a.seg_sums = seg_sums; a.out = cat; a.ldo = ldcat;
-    return linear_attention_run(dev, a, st, nl);
+    return linear_attention_run(dev, a, st);
 }
 
-int StackModel::forward(int nseq, int T, cudaStream_t st, int *launches, Prof *prof, bool all_logits, const int *slots) {
+int StackModel::forward(int nseq, int T, cudaStream_t st, Prof *prof, bool all_logits, const int *slots) {
     const int M = nseq * T;
-    int nl = 1;
     IM_TRY(stack_embed(tokens_dev, embed.w, f32, embed.ld, embed_norm, sc.embed_scale, x, x0, W, (uint32_t)sc.vocab, sc.norm_eps, M, st));
     IM_MARK(kCatEmbed);
     float *cur = x, *other = x_alt;
@@ -512,7 +510,6 @@ int StackModel::forward(int nseq, int T, cudaStream_t st, int *launches, Prof *p
     res.kind = post ? kSrcAddNorm : kSrcNorm;
     auto read_residual = [&](const DenseWeight &w, const DenseEpi &e) -> int {
         IM_TRY(dense_project(dev, w, res, e, M, h, st));
-        nl += dense_launches(M, f32, res.kind);
         if (res.xf2) {  // the sum has been written to `other`
             std::swap(cur, other);
             res.xf = cur; res.xf2 = nullptr; res.gamma = nullptr; res.xout = nullptr;
@@ -525,7 +522,6 @@ int StackModel::forward(int nseq, int T, cudaStream_t st, int *launches, Prof *p
         DenseEpi e;
         e.kind = post ? kEpiF32 : kEpiResidual; e.xf = post ? sub : cur; e.ldx = W;
         IM_TRY(dense_project(dev, w, s, e, M, nullptr, st));
-        nl += dense_launches(M, f32, s.kind);
         if (post) {
             res.xf2 = sub; res.gamma = gamma; res.xout = other;
         }
@@ -539,7 +535,6 @@ int StackModel::forward(int nseq, int T, cudaStream_t st, int *launches, Prof *p
             DenseEpi e;
             e.kind = kEpiF32; e.xf = other; e.ldx = W; e.bias = loop_step + (size_t)r.pass * W;
             IM_TRY(dense_project(dev, loop_in, s, e, M, h, st));
-            nl += dense_launches(M, f32, s.kind);
             std::swap(cur, other);
             res.xf = cur;
             IM_MARK(kCatResNorm);
@@ -552,7 +547,7 @@ int StackModel::forward(int nseq, int T, cudaStream_t st, int *launches, Prof *p
         if (!post) res.gamma = L.norm1;
         IM_TRY(read_residual(L.w_in, e));
         IM_MARK(kCatQkv);
-        IM_TRY(mix(r, nseq, T, slots, st, &nl));
+        IM_TRY(mix(r, nseq, T, slots, st));
         IM_MARK(kCatAttn);
         IM_TRY(sublayer_out(L.w_out, L.norm1));
         IM_MARK(post ? kCatOProj : kCatDown);
@@ -566,14 +561,13 @@ int StackModel::forward(int nseq, int T, cudaStream_t st, int *launches, Prof *p
         }
     }
     if (all_logits) {
-        IM_TRY(logits_of(res, 0, M, rows, st, &nl));
+        IM_TRY(logits_of(res, 0, M, rows, st));
     } else if (T == 1) {
-        IM_TRY(logits_of(res, 0, M, logits, st, &nl));
+        IM_TRY(logits_of(res, 0, M, logits, st));
     } else {
-        for (int s = 0; s < nseq; s++) IM_TRY(logits_of(res, s * T + T - 1, 1, logits + (size_t)s * cfg.vocab_size, st, &nl));
+        for (int s = 0; s < nseq; s++) IM_TRY(logits_of(res, s * T + T - 1, 1, logits + (size_t)s * cfg.vocab_size, st));
     }
     IM_MARK(kCatHead);
-    if (launches) *launches = nl;
     return IM_OK;
 }
 

@@ -63,7 +63,6 @@ constexpr int kDenseMaxRows = 8;   // tokens per matvec launch
 int dense_project(const Device *dev, const DenseWeight &w, const DenseSrc &src, const DenseEpi &epi, int M, void *h_scratch, cudaStream_t st);
 // Sets every launch attribute of this file's kernels on the current device (so that a capture can be their first use).
 int dense_prepare(const Device *dev);
-int dense_launches(int M, int f32, int src_kind);
 
 // x[m] = x0[m] = rms(table[token]) * gamma, or without gamma table[token] * scale (f32); tokens past the vocabulary read as zeros.
 int stack_embed(const uint32_t *tokens, const void *table, int f32, int ld, const float *gamma, float scale, float *x, float *x0, int width, uint32_t vocab, float eps,
@@ -109,7 +108,7 @@ struct LatentArgs {
 // Tokens of one sequence from which keys and values are expanded per head. (A prompt of 50 tokens takes 19 + 13 + 41 us in absorbed form and 20 + 12 us
 // expanded, but the absorbed form keeps weighted sums of latents and W_uv's products in f32 where the expanded one rounds every value to bf16.)
 constexpr int kLatentExpandMin = 64;
-int latent_attention_run(const Device *dev, const LatentArgs &a, cudaStream_t st, int *launches);
+int latent_attention_run(const Device *dev, const LatentArgs &a, cudaStream_t st);
 size_t latent_part_bytes(const Device *dev, const LatentShape &s, int tokens, int nseq);
 bool latent_expands(const LatentShape &s);  // prompt chunks of this shape can take the expanded form
 int latent_prepare(const Device *dev);
@@ -145,7 +144,7 @@ struct GroupedArgs {
     int host_pos, host_slot; // as in LatentArgs
     int splits_ctx;
 };
-int grouped_attention_run(const Device *dev, const GroupedArgs &a, cudaStream_t st, int *launches);
+int grouped_attention_run(const Device *dev, const GroupedArgs &a, cudaStream_t st);
 size_t grouped_part_bytes(const Device *dev, const GroupedShape &s, int f32, int tokens);
 int grouped_counters(const GroupedShape &s, int tokens);
 constexpr int kGroupedPrefillMin = 16;  // tokens of one sequence from which the prompt kernel runs (bf16)
@@ -187,13 +186,13 @@ struct LinearArgs {
 constexpr int kLinearPow = 128;
 constexpr int kLinearSegMax = 8;
 constexpr int kGatedChunk = 64, kGatedChunkMin = 16;  // tokens of a chunk; shortest portion that runs in chunks (bf16)
-int linear_attention_run(const Device *dev, const LinearArgs &a, cudaStream_t st, int *launches);
+int linear_attention_run(const Device *dev, const LinearArgs &a, cudaStream_t st);
 int linear_prepare(const Device *dev);
 // linear_gated.cu, called by linear_attention_run: IM_ERR_BOUNDS when the shape or the scratch does not allow it
 bool gated_decode_takes(const LinearShape &s);
 bool gated_chunk_takes(const LinearShape &s);
 int gated_decode_run(const LinearArgs &a, cudaStream_t st);
-int gated_chunk_run(const LinearArgs &a, cudaStream_t st, int *launches);
+int gated_chunk_run(const LinearArgs &a, cudaStream_t st);
 int gated_prepare();
 
 #ifdef __CUDACC__

@@ -137,6 +137,21 @@ def test_partial_rotation(arch, rotary_dim, n_bits, monkeypatch):
     assert max(errs) <= (1e-2 if n_bits == 16 else 5e-2), errs
 
 
+@pytest.mark.parametrize("awq", [False, True])
+def test_launches_of_a_step_are_counted(awq):
+    # 16 sequences in lockstep. Embedding; QKV, cache write, attention, its reduction, o, norm, gate, up, activation, down and the sum of its two K slices (8 groups);
+    # residual; norm, head; argmax and two counters. Activation scales: a pass before the first QKV and before o (the others are folded in)
+    from ironmill_b200.engine import CudaConfig, CudaInference
+    cfg = _cfg("llama", 1, 512, 1024, 4, 2, 500, 5e5, 1e-5)
+    tqc = orc.TqConstants(128, 8, seed=1)
+    eng = CudaInference(CudaConfig(max_seq_len=32, max_batch=16))
+    eng.load_weights(DictProvider(cfg, synth_model(cfg, seed=3, awq=awq)), tq_signs=tqc.signs, tq_qjl=tqc.qjl)
+    for _ in range(16):
+        eng.add_sequence(np.arange(1, 6, dtype=np.uint32))
+    eng.batch_decode_step()
+    assert eng.step_launches() == 18 + 2 * awq
+
+
 def test_tiny_llama_shape_awq_int8_parity():
     # no QK-norm (plain RoPE), AWQ scales, GQA 4, tied embeddings, INT8 weights
     cfg = _cfg("llama", 2, 512, 1024, 8, 2, 777, 5e5, 1e-5, tie=True)
