@@ -1,9 +1,10 @@
 // Dense projections (bf16 with f32 accumulation, or true f32) with fused prologues and epilogues.
-//   up to 15 tokens   dense_matvec_kernel: a warp (or several, K split) per pair of weight rows, 16-byte weight loads
+//   up to 4 tokens (f32: 15)   dense_matvec_kernel: a warp (or several, K split) per pair of weight rows, 16-byte weight loads
 //                     requested one step ahead, the activations staged once per CTA in shared memory; the staging can be
 //                     the RMS norm of the f32 residual or the concatenation of two f32 vectors
-//   16 tokens and more, bf16   dense_gemm_tc_kernel: tcgen05.mma, both operands by TMA into the 128-byte swizzle, f32
-//                     accumulator in tensor memory, K split over the grid for few tokens
+//   5 tokens and more, bf16    dense_gemm_tc_kernel: tcgen05.mma, both operands by TMA into the 128-byte swizzle, f32
+//                     accumulator in tensor memory, K split over the grid for few tokens; more than 128 tokens with enough
+//                     tiles: CTA pairs (gemm_pair.cu)
 //   16 tokens and more, f32    dense_gemm_f32_kernel: register-tiled f32 FMA
 // The epilogues (activation of some rows, gate * up pairs, residual add, bias, soft cap) work on the f32 sums.
 #include <cuda.h>
@@ -571,7 +572,7 @@ int matvec_any(const Device *dev, const DenseWeight &w, const DenseSrc &src, con
     for (int m0 = 0; m0 < M;) {
         const int B = std::min(M - m0, cap);
         int rc;
-        if (B > 4) rc = matvec_launch<T, 8>(dev, w, src, epi, m0, B, st);
+        if (sizeof(T) == 4 && B > 4) rc = matvec_launch<float, 8>(dev, w, src, epi, m0, B, st);  // (bf16 batches of five rows and more are a GEMM)
         else if (B > 2) rc = matvec_launch<T, 4>(dev, w, src, epi, m0, B, st);
         else if (B > 1) rc = matvec_launch<T, 2>(dev, w, src, epi, m0, B, st);
         else rc = matvec_launch<T, 1>(dev, w, src, epi, m0, B, st);
@@ -601,7 +602,7 @@ int dense_prepare(const Device *dev) {
     const int mv = (int)kMvSmemMax;
 #define IM_SMEM(k, b) IM_CUDA_CHECK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, b))
     IM_SMEM((dense_matvec_kernel<__nv_bfloat16, 1>), mv); IM_SMEM((dense_matvec_kernel<__nv_bfloat16, 2>), mv);
-    IM_SMEM((dense_matvec_kernel<__nv_bfloat16, 4>), mv); IM_SMEM((dense_matvec_kernel<__nv_bfloat16, 8>), mv);
+    IM_SMEM((dense_matvec_kernel<__nv_bfloat16, 4>), mv);
     IM_SMEM((dense_matvec_kernel<float, 1>), mv); IM_SMEM((dense_matvec_kernel<float, 2>), mv);
     IM_SMEM((dense_matvec_kernel<float, 4>), mv); IM_SMEM((dense_matvec_kernel<float, 8>), mv);
     IM_SMEM((dense_gemm_tc_kernel<128, __nv_bfloat16>), dense_gemm_smem<128>());

@@ -263,8 +263,8 @@ int kv16_prep_launch(const Kv16Prep &a, cudaStream_t st) {
     return IM_OK;
 }
 
-// Rows of an fp16 cache as the prompt kernel takes them (also of a quantized cache written out as fp16 rows: tq_prefill.cu).
-FlashArgs kv16_flash_args(const Device *dev, const __half *q, int q_stride, const __half *kc, const __half *vc, float scale, __half *out, int nh, int nkv, int max_seq,
+// Rows of an fp16 cache as the prompt kernel takes them.
+static FlashArgs kv16_flash_args(const Device *dev, const __half *q, int q_stride, const __half *kc, const __half *vc, float scale, __half *out, int nh, int nkv, int max_seq,
                           int base_pos, const int *pos_dev, int T, int slot) {
     FlashArgs f;
     f.T = T; f.heads = nh; f.group = nh / nkv;

@@ -57,7 +57,7 @@ struct DenseEpi {
 // Tokens from which a projection is a dense contraction. bf16: the matvec's multiply-adds grow with the rows (2048-wide model, 12 MB to 82 MB of weights: 15 us
 // a launch for one row, 30 for three or four, 71 for eight) while the tensor-core pass takes 19 to 21 us up to 32 rows. f32 has no tensor-core pass.
 constexpr int kDenseGemmMin = 5, kDenseGemmMinF32 = 16;
-constexpr int kDenseMaxRows = 8;   // tokens per matvec launch
+constexpr int kDenseMaxRows = 8;   // tokens per matvec launch (f32)
 
 // y = W x for M tokens.  h_scratch: M x round_up(K, 8) elements, used when the source is not plain and M >= kDenseGemmMin (kDenseGemmMinF32).
 int dense_project(const Device *dev, const DenseWeight &w, const DenseSrc &src, const DenseEpi &epi, int M, void *h_scratch, cudaStream_t st);
