@@ -9,7 +9,8 @@
 //     O += P V     A operand P from tensor memory, B operand V with the head dimension contiguous (MN-major), f32 accumulator
 // The two halves take turns: while one half's four warps exponentiate, the other half's products run. Tensor memory is full:
 // scores / weights of two halves in 256 columns, outputs in 256 more. An accumulator is rescaled only when a row's maximum has grown by
-// more than 2^8 since the last time (weights up to 2^8 are representable and the normalisation uses the same maximum).
+// more than 2^8 since the last time (weights up to 2^8 are representable and the normalisation uses the same maximum; the scheme, like that of two
+// halves in turns, is known from published attention kernels for this architecture, FlashAttention-4).
 //
 // Order: every product is issued by one thread, so S of the next tile cannot overtake the P V product that still reads the same
 // columns, and a score barrier (tcgen05.commit) says that the half's earlier P V product is complete too: its softmax warps may

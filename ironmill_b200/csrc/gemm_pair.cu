@@ -16,8 +16,12 @@
 //
 // Bound: the tensor pipe (512 clocks per 64 columns of a 128 x 256 half tile).  Measured back to back, bf16 2048 tokens x
 // 28672 x 4096: 343 us, 1404 TFLOP/s; 20032 x 2048: 131 us (128-row kernel 164 us alone); 4-bit codes 28672 x 4096: 411 us, 1172 TFLOP/s, 4096 x 14336: 216 us;
-// there the weight warps bound: without any epilogue the same launches reach 1240 TFLOP/s. A full proxy fence and cluster-scope
-// barrier semantics in the weight warps made them wait for their own loads in flight: 1.5 times the time.
+// there the weight warps bound: without any epilogue the same launches reach 1240 TFLOP/s.
+//
+// The weight warps of the second CTA arrive at the leader's barrier with the default scope. What that barrier has to order is the issue of the products: a
+// weight tile lies in the shared memory of the CTA that converted it, only that SM's tensor core reads it, and fence.proxy.async.shared::cta, which every
+// lane executes before its warp arrives, is complete when the stores are visible there. A proxy fence for all spaces and cluster-scope semantics made the warps wait
+// for their own loads of codes in flight: 1.5 times the time.
 #include <cuda.h>
 
 #include <algorithm>

@@ -1,7 +1,7 @@
 // Latent attention: one cached row per token, [normed latent c | rotated key part], shared by all heads; the keys of head h
 // are W_uk[h] c next to the rotated part, its values W_uv[h] c; softmax with an optional keyless sink logit per head.
 //
-// Two equal forms:
+// Two forms of the same sums (the expanded one rounds keys and values to bf16, the absorbed one q'):
 //   absorbed   q' = W_uk^T q is a query against the latents themselves, the weighted sum of latents goes through W_uv at
 //              the end: every head reads the same cached row.  Decode, batches and short chunks.
 //                latent_absorb_kernel   q', the rotated query part, the token's cache row
@@ -9,7 +9,8 @@
 //                                       the grid (bf16);  latent_attn_simt_kernel: the same in f32 FMA
 //                latent_combine_kernel, latent_out_kernel   splits and sink, then W_uv
 //   expanded   keys and values of a group of heads by one GEMM over the cached latents, then a causal tensor-core pass
-//              (latent_prefill_kernel).  Prompt chunks in bf16, where it is 3-4 times fewer operations.
+//              (flash_tc.cu; head sizes that it does not take: latent_prefill_kernel).  Prompt chunks of 64 tokens and
+//              more in bf16, where it is 3-4 times fewer operations.
 // Scores, softmax and sums are f32; on the tensor cores a softmax weight enters the second product as two bf16 terms.
 #include <math.h>
 
