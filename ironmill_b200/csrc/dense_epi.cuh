@@ -26,6 +26,22 @@ template <>
 __device__ __forceinline__ float pair_act<__half>(float z, float up, bool, bool) {
     return silu_f(__half2float(__float2half_rn(z))) * __half2float(__float2half_rn(up));
 }
+// The same for the values of a lane side by side: the general quotient's branches keep them apart (a prompt of 5003 tokens through four layers of a 2048-wide model
+// took 5.21 ms with them, 4.84 with the fast exponential and quotient, which are less exact, 4.93 like this). Quotient by Markstein's method (IBM J. Res. Dev. 34, 1990):
+// reciprocal refined by Newton steps, remainder by fma, one correction; equal to silu_f, bit for bit, for every fp16 gate but those that set odd (zeros, -80 and less, infinities, NaN).
+template <typename T>
+__device__ __forceinline__ float pair_act_side(float z, float up, bool silu, bool few, bool &) { return pair_act<T>(z, up, silu, few); }
+template <>
+__device__ __forceinline__ float pair_act_side<__half>(float z, float up, bool, bool, bool &odd) {
+    const float g = __half2float(__float2half_rn(z)), d = 1.0f + expf(-g);
+    odd = odd || !(g > -80.0f && g < INFINITY) || g == 0.0f;
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(d));
+    y = fmaf(y, fmaf(-d, y, 1.0f), y);
+    y = fmaf(y, fmaf(-d, y, 1.0f), y);
+    const float q = g * y;
+    return fmaf(fmaf(-d, q, g), y, q) * __half2float(__float2half_rn(up));
+}
 
 // One round of a transposition between lanes: of every two values the lane with bit X clear keeps the first and gets its
 // partner's first, the other lane the second ones; the results lie in the order of the lanes.
@@ -80,12 +96,19 @@ __device__ __forceinline__ bool epi_store16_wide(const DenseEpi &e, int N, int M
         T *act = static_cast<T *>(e.act) + (size_t)m * e.ldact + col;
         if (!aligned16(act, 2ll * e.ldact)) return false;
         const bool odd = lane & 1;
-        float r[8];
+        float r[8], z[8], u[8];
+        bool other = false;
 #pragma unroll
         for (int i = 0; i < 16; i += 2) {  // (gate, up) in neighbouring lanes: the even lane takes token i, the odd lane token i + 1
             const float got = __shfl_xor_sync(0xffffffffu, odd ? v[i] : v[i + 1], 1);
-            r[i / 2] = odd ? pair_act<T>(got, v[i + 1], e.pair_silu, few) : pair_act<T>(v[i], got, e.pair_silu, few);
+            z[i / 2] = odd ? got : v[i];
+            u[i / 2] = odd ? v[i + 1] : got;
         }
+#pragma unroll
+        for (int i = 0; i < 8; i++) r[i] = pair_act_side<T>(z[i], u[i], e.pair_silu, few, other);
+        if (other)
+#pragma unroll
+            for (int i = 0; i < 8; i++) r[i] = pair_act<T>(z[i], u[i], e.pair_silu, few);
         const uint4 q = gather8<T, 2>(r);
         const int tok = lane & 15;
         if (tok < left) *reinterpret_cast<uint4 *>(act + (size_t)tok * e.ldact + (lane >> 4) * 8) = q;
