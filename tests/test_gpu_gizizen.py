@@ -400,18 +400,19 @@ def test_prompts_on_cta_pairs(width, ff, n):
 def test_activations_of_a_batch_are_those_of_single_rows():
     """Gate, up, down and head with one element per row: their sums are single products, exact in any order, so the activation alone can tell a row of a batch (tensor
     cores from five rows on) from the same row by itself (matvec). The mixer adds nothing (o is zero)."""
-    cfg = G.config([G.latent(ff=8192)], width=256, vocab=256, cap=None)
+    cfg = G.config([G.latent(ff=8192)], width=448, vocab=448, cap=None)
     w = G.weights(cfg, 16)
     r = np.random.default_rng(17)
     for name in ("l0.mlp.gate", "l0.mlp.up", "l0.mlp.down", "head", "l0.mix.o"):
         N, K = w[name].shape
         a = np.zeros((N, K), dtype=np.float32)
         if name != "l0.mix.o":
-            a[np.arange(N), r.permutation(K)[:N] if N <= K else r.integers(0, K, N)] = r.choice([-1.0, 1.0], N) * r.uniform(0.5, 2.0, N)
+            # (down is large, so that what a row carries on is the activation rather than the embedding)
+            a[np.arange(N), r.permutation(K)[:N] if N <= K else r.integers(0, K, N)] = r.choice([-1.0, 1.0], N) * r.uniform(0.5, 2.0, N) * (64 if "down" in name else 1)
         w[name] = G.bf16(a)
-    n, steps = 15, 40
-    both = [engine(cfg, w, "bfloat16", max_seq_len=64, max_batch=n) for _ in range(2)]
-    toks = np.random.default_rng(18).integers(0, 256, (steps + 1, n)).astype(np.uint32)
+    n, steps = 15, 150
+    both = [engine(cfg, w, "bfloat16", max_seq_len=160, max_batch=n) for _ in range(2)]
+    toks = np.random.default_rng(18).integers(0, 448, (steps + 1, n)).astype(np.uint32)
     ids = [[e.add_sequence(toks[0, i:i + 1]) for i in range(n)] for e in both]
     for k in range(1, steps + 1):
         batch = dict(both[0].batch_decode_step({s: int(toks[k, i]) for i, s in enumerate(ids[0])}))
