@@ -56,7 +56,7 @@ struct Device {
     // device handle at a time.
     float *gemm_partial = nullptr;
 };
-constexpr size_t kGemmPartialBytes = (size_t)8 << 20;
+constexpr size_t kGemmPartialBytes = (size_t)10 << 20;
 constexpr int kSkMaxBlocks = 1 << 17;  // row blocks the counters cover (2M rows)
 
 // cudaFuncSetAttribute applies to the current device: remember per device ordinal (not per thread) whether a
@@ -114,16 +114,17 @@ struct V2Params {
 };
 
 // INT4 g128 GEMM on tcgen05 / TMEM (gemm_tc.cu): y[M, N] = f16(x / awq) * dequant(w)^T; xs_scratch holds M * K halves.
-// IM_ERR_BOUNDS when the weight is not INT4 group-128.  scaled: x holds f16(x / awq) already.
-int gemm_affine_tc(const AffineWeight *w, const __half *x, __half *y, int M, __half *xs_scratch, cudaStream_t st, bool scaled = false);
+// IM_ERR_BOUNDS when the weight is not INT4 or INT8 group-128.
+enum TokenForm { kTokensRaw, kTokensScaled, kTokensPacked };  // x as it is; f16(x / awq); that, packed for gemm_rows.cu (where gemm_rows_takes says so)
+int gemm_affine_tc(const AffineWeight *w, const __half *x, __half *y, int M, __half *xs_scratch, cudaStream_t st, TokenForm form = kTokensRaw);
 // The gated activation y[M, N] = f16(silu(f16(gate x)) f16(up x)) in one launch, for two weights of the same form and activation scales;
 // only where gemm_affine_joins() says so.
 bool gemm_affine_joins(const AffineWeight *gate, int M);
-int gemm_affine_gate_up(const AffineWeight *gate, const AffineWeight *up, const __half *x, __half *y, int M, __half *xs_scratch, cudaStream_t st, bool scaled);
+int gemm_affine_gate_up(const AffineWeight *gate, const AffineWeight *up, const __half *x, __half *y, int M, __half *xs_scratch, cudaStream_t st, TokenForm form);
 // y[M, N] = f16(x w^T) for fp16 weights [N, K] and rows x [M, K] on the tensor cores (dense.cu); IM_ERR_BOUNDS for rows that are not 16-byte aligned
 int dense_rows_f16(const Device *dev, const __half *w, int N, int K, const __half *x, __half *y, int M, cudaStream_t st);
 int residual_norm_scaled(const __half *a, const __half *b, const __half *gamma, const __half *scale, __half *out, __half *residual, int H, int T, float eps,
-                         cudaStream_t st);
+                         cudaStream_t st, bool packed = false);
 // Gate/up pair as one tile stream (matvec.cu); built on first use.
 int ensure_pair(const AffineWeight *gate, const AffineWeight *up, cudaStream_t st);
 int v2_run(int mode, int nb, const V2Params &p, const Device *dev, cudaStream_t st, int bits = 4);

@@ -1,0 +1,28 @@
+// Projections of few tokens over quantized weights (gemm_rows.cu) and the token layout that they read.
+#pragma once
+#include "common.cuh"
+
+namespace im {
+
+constexpr int kRowsMaxTokens = 48, kRowsMaxTokens8 = 32;  // 4-bit, 8-bit codes
+
+// Packed tokens, in 16-byte chunks of eight columns: [group of 128][eight columns i of a run of 32][token][run t].
+// Chunk c of token m of M lies at this place; its halves in the order 0, 4, 1, 5, 2, 6, 3, 7.
+__host__ __device__ __forceinline__ size_t token_chunk(int c, int m, int M) {
+    const int grp = c >> 4, t = (c >> 2) & 3, i = c & 3;
+    return ((size_t)(grp * 4 + i) * M + m) * 4 + t;
+}
+#ifdef __CUDACC__
+__device__ __forceinline__ uint4 pack_chunk(const __half (&h)[8]) {
+    auto two = [](__half a, __half b) { return (uint32_t)__half_as_ushort(a) | ((uint32_t)__half_as_ushort(b) << 16); };
+    return make_uint4(two(h[0], h[4]), two(h[1], h[5]), two(h[2], h[6]), two(h[3], h[7]));
+}
+#endif
+
+bool gemm_rows_takes(const AffineWeight *w, int M);
+// f16(x / awq) (awq may be null) of M rows of K = a multiple of 128, packed; x anywhere, out 16-byte aligned and apart from it
+int token_pack(const __half *x, const __half *awq, __half *out, int M, int K, cudaStream_t st);
+// y[M, N] = packed tokens times w; with `up` (of w's form) the gated activation of both, divided by `div` if given; pack_out: packed for the next projection
+int gemm_rows(const AffineWeight *w, const AffineWeight *up, const __half *packed, __half *y, int M, const __half *div, bool pack_out, cudaStream_t st);
+
+}  // namespace im

@@ -1,5 +1,5 @@
 // INT4 group-128 GEMM on the 5th-generation tensor cores (tcgen05 + TMEM) for the dense-contraction cases of the
-// hot path: decode batches of 16 tokens and more and prefill chunks that do not fill CTA pairs (gemm_pair.cu).
+// hot path: decode batches and prompt portions that are too many tokens for gemm_rows.cu and do not fill CTA pairs (gemm_pair.cu).
 //   crates/ironmill-inference/src/metal/shaders/quantized/affine_matmul.metal:10-152 (superblock_matmul_int4):
 //   C[m, n] = sum_k f16(A[m, k] / awq[k]) * f16((q[n, k] - z) * s), f32 accumulation, fp16 result.
 //
@@ -26,6 +26,7 @@
 #include "common.cuh"
 #include "dequant.cuh"
 #include "gemm_pair.cuh"
+#include "gemm_rows.cuh"
 #include "v2_device.cuh"
 
 namespace im {
@@ -414,18 +415,26 @@ static int scaled_tokens(const AffineWeight *w, const __half *x, int M, __half *
 
 bool gemm_affine_joins(const AffineWeight *gate, int M) { return gemm_takes(gate) && pair_gemm_takes(gate->dev, 2 * gate->N, M); }
 
-int gemm_affine_gate_up(const AffineWeight *gate, const AffineWeight *up, const __half *x, __half *y, int M, __half *xs_scratch, cudaStream_t st, bool scaled) {
+int gemm_affine_gate_up(const AffineWeight *gate, const AffineWeight *up, const __half *x, __half *y, int M, __half *xs_scratch, cudaStream_t st, TokenForm form) {
     const __half *xs;
-    const int rc = scaled_tokens(gate, x, M, xs_scratch, scaled, st, &xs);
+    const int rc = scaled_tokens(gate, x, M, xs_scratch, form != kTokensRaw, st, &xs);
     return rc != IM_OK ? rc : pair_gemm_affine(gate, up, xs, y, M, st);
 }
 
 // Y[M, N] = f16(X / awq) * dequant(W)^T for M tokens.  xs_scratch: M * K halves.  IM_ERR_BOUNDS when the weight is not
 // INT4 group-128 with K a multiple of 128 (the caller falls back to the matvec kernels).
-int gemm_affine_tc(const AffineWeight *w, const __half *x, __half *y, int M, __half *xs_scratch, cudaStream_t st, bool scaled) {
+int gemm_affine_tc(const AffineWeight *w, const __half *x, __half *y, int M, __half *xs_scratch, cudaStream_t st, TokenForm form) {
     if (!gemm_takes(w) || M < 1) return IM_ERR_BOUNDS;
+    // Up to 64 tokens over tiled weights: gemm_rows.cu (the tokens are packed in the scratch unless they come packed).
+    if (gemm_rows_takes(w, M) && (form == kTokensPacked || (x != xs_scratch && reinterpret_cast<uintptr_t>(xs_scratch) % 16 == 0))) {
+        if (form != kTokensPacked) {
+            if (const int rc = token_pack(x, form == kTokensRaw ? w->awq : nullptr, xs_scratch, M, w->K, st); rc != IM_OK) return rc;
+            x = xs_scratch;
+        }
+        return gemm_rows(w, nullptr, x, y, M, nullptr, false, st);
+    }
     const __half *xs;
-    if (const int rc = scaled_tokens(w, x, M, xs_scratch, scaled, st, &xs); rc != IM_OK) return rc;
+    if (const int rc = scaled_tokens(w, x, M, xs_scratch, form != kTokensRaw, st, &xs); rc != IM_OK) return rc;
     if (pair_gemm_takes(w->dev, w->N, M)) return pair_gemm_affine(w, nullptr, xs, y, M, st);
     GemmParams p{w->codes, w->sz, xs, y, w->N, w->K, w->G, M, w->dev->err_flag, nullptr, w->G};
     // Few tokens and few row tiles (decode batches of 16-64 against 4096-6144 rows: 32-48 CTAs of 32-112 sequential

@@ -21,6 +21,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "gemm_rows.cuh"
 #include "mega.cuh"
 #include "session.cuh"
 
@@ -530,31 +531,37 @@ int Model::forward(int nseq, int T, cudaStream_t st, Prof *prof, bool all_logits
         if (m->world > 1) IM_MARK(kCatComm);
         // what a projection with activation scales reads, f16(x / awq), is written by the norm and by the activation's own kernel; in the epilogues of
         // attention and of the joint projection the divisions took more time than the pass that they would save
-        int rc = L.ffn_joint ? residual_norm_scaled(m->hidden, m->ffn_down, L.post_ln, L.gate->awq, m->norm_out, m->residual, H, MT, eps, st) : IM_ERR_BOUNDS;
-        const bool scaled = rc == IM_OK;
+        // (few tokens: packed, as is the activation; gemm_rows.cu)
+        const bool rows = L.ffn_joint && gemm_rows_takes(L.gate, MT) && gemm_rows_takes(L.up, MT) && gemm_rows_takes(L.down, MT);
+        int rc = L.ffn_joint ? residual_norm_scaled(m->hidden, m->ffn_down, L.post_ln, L.gate->awq, m->norm_out, m->residual, H, MT, eps, st, rows) : IM_ERR_BOUNDS;
+        TokenForm form = rc == IM_OK ? (rows ? kTokensPacked : kTokensScaled) : kTokensRaw;
         if (rc == IM_ERR_BOUNDS) rc = im_cuda_fused_residual_rms_norm(m->hidden, m->ffn_down, L.post_ln, m->norm_out, m->residual, H, MT, eps, st);
         IM_TRY(rc);
         IM_MARK(kCatResNorm);
-        const bool joint = L.ffn_joint && gemm_affine_joins(L.gate, MT);
-        if (joint) {
-            IM_TRY(gemm_affine_gate_up(L.gate, L.up, m->norm_out, m->ffn_gate, MT, m->xs_scratch, st, scaled));
+        if (form == kTokensPacked) {
+            IM_TRY(gemm_rows(L.gate, L.up, m->norm_out, m->ffn_gate, MT, L.down->awq, true, st));
+        } else if (L.ffn_joint && gemm_affine_joins(L.gate, MT)) {
+            IM_TRY(gemm_affine_gate_up(L.gate, L.up, m->norm_out, m->ffn_gate, MT, m->xs_scratch, st, form));
+            form = kTokensRaw;
         } else {
-            IM_TRY(gemm_affine_tc(L.gate, m->norm_out, m->ffn_gate, MT, m->xs_scratch, st, scaled));
-            IM_TRY(gemm_affine_tc(L.up, m->norm_out, m->ffn_up, MT, m->xs_scratch, st, scaled));
+            IM_TRY(gemm_affine_tc(L.gate, m->norm_out, m->ffn_gate, MT, m->xs_scratch, st, form));
+            IM_TRY(gemm_affine_tc(L.up, m->norm_out, m->ffn_up, MT, m->xs_scratch, st, form));
             IM_TRY(silu_mul_rows(m->ffn_gate, m->ffn_up, L.down->awq, m->ffn_gate, MT, m->I_l, st));
+            form = kTokensScaled;
         }
         IM_MARK(kCatFfn);
-        IM_TRY(gemm_affine_tc(L.down, m->ffn_gate, m->ffn_down, MT, m->xs_scratch, st, !joint));
+        IM_TRY(gemm_affine_tc(L.down, m->ffn_gate, m->ffn_down, MT, m->xs_scratch, st, form));
         IM_MARK(kCatDown);
         IM_TRY(tp_allreduce(m, m->ffn_down, (size_t)MT * H, st));  // tensor parallel: down is row-split
         if (m->world > 1) IM_MARK(kCatComm);
         if (l + 1 < c.num_layers) {
             Layer &Nx = m->layers[l + 1];
-            rc = residual_norm_scaled(m->residual, m->ffn_down, Nx.input_ln, Nx.qkv->awq, m->norm_out, m->hidden, H, MT, eps, st);
-            const bool qkv_scaled = rc == IM_OK;
+            const bool qkv_rows = gemm_rows_takes(Nx.qkv, MT);
+            rc = residual_norm_scaled(m->residual, m->ffn_down, Nx.input_ln, Nx.qkv->awq, m->norm_out, m->hidden, H, MT, eps, st, qkv_rows);
+            form = rc == IM_OK ? (qkv_rows ? kTokensPacked : kTokensScaled) : kTokensRaw;
             if (rc == IM_ERR_BOUNDS) rc = im_cuda_fused_residual_rms_norm(m->residual, m->ffn_down, Nx.input_ln, m->norm_out, m->hidden, H, MT, eps, st);
             IM_TRY(rc);
-            IM_TRY(gemm_affine_tc(Nx.qkv, m->norm_out, m->qkv, MT, m->xs_scratch, st, qkv_scaled));
+            IM_TRY(gemm_affine_tc(Nx.qkv, m->norm_out, m->qkv, MT, m->xs_scratch, st, form));
             IM_MARK(kCatQkv);
         } else {
             IM_TRY(im_cuda_residual_add(m->residual, m->ffn_down, m->hidden, (size_t)MT * H, st));

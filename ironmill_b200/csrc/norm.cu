@@ -16,6 +16,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "gemm_rows.cuh"
 
 namespace im {
 
@@ -67,7 +68,7 @@ constexpr int kRowVecs = 4;  // 16-byte vectors of a thread
 template <int MODE>
 __global__ void __launch_bounds__(kNormThreads) rms_rows_kernel(const __half *__restrict__ a, const __half *__restrict__ b, const uint32_t *__restrict__ tokens,
                                                                 const __half *__restrict__ gamma, const __half *__restrict__ scale, __half *__restrict__ normed,
-                                                                __half *__restrict__ residual, int H, uint32_t vocab, float eps, float embed_scale) {
+                                                                __half *__restrict__ residual, int H, uint32_t vocab, float eps, float embed_scale, int packed) {
     __shared__ float sh[32];
     const int nv = H / 8, tid = threadIdx.x, nt = blockDim.x;
     pdl_trigger();
@@ -130,7 +131,8 @@ __global__ void __launch_bounds__(kNormThreads) rms_rows_kernel(const __half *__
                     ho[i] = __floats2half2_rn(n.x / f.x, n.y / f.y);
                 }
             }
-            reinterpret_cast<uint4 *>(normed)[base + tid + j * nt] = out;
+            if (packed) reinterpret_cast<uint4 *>(normed)[token_chunk(tid + j * nt, blockIdx.x, gridDim.x)] = pack_chunk(reinterpret_cast<const __half(&)[8]>(out));
+            else reinterpret_cast<uint4 *>(normed)[base + tid + j * nt] = out;
         }
 }
 
@@ -250,12 +252,12 @@ int launch_qk_rope(const QkRopeArgs &a, int T, cudaStream_t st) {
     return IM_OK;
 }
 
-// fused_residual_rms_norm whose result is left as a projection with activation scales `scale` (or none) reads it; IM_ERR_BOUNDS for rows the
-// kernel does not take.
+// fused_residual_rms_norm whose result is left as a projection with activation scales `scale` (or none) reads it, packed if it reads packed tokens;
+// IM_ERR_BOUNDS for rows the kernel does not take.
 int residual_norm_scaled(const __half *a, const __half *b, const __half *gamma, const __half *scale, __half *out, __half *residual, int H, int T, float eps,
-                         cudaStream_t st) {
+                         cudaStream_t st, bool packed) {
     if (!rows_fit(H, {a, b, gamma, scale, out, residual})) return IM_ERR_BOUNDS;
-    IM_CUDA_CHECK(launch_k(rms_rows_kernel<1>, dim3(T), rows_block(H), 0, st, a, b, (const uint32_t *)nullptr, gamma, scale, out, residual, H, 0u, eps, 1.0f));
+    IM_CUDA_CHECK(launch_k(rms_rows_kernel<1>, dim3(T), rows_block(H), 0, st, a, b, (const uint32_t *)nullptr, gamma, scale, out, residual, H, 0u, eps, 1.0f, packed ? 1 : 0));
     return IM_OK;
 }
 
@@ -271,7 +273,7 @@ IM_EXPORT int im_cuda_rms_norm(const void *x_dev, const void *gamma_dev, void *o
     if (rows_fit(H, {x_dev, gamma_dev, out_dev})) {
         IM_CUDA_CHECK(launch_k(rms_rows_kernel<0>, dim3(T), rows_block(H), 0, as_stream(stream), static_cast<const __half *>(x_dev), (const __half *)nullptr,
                                (const uint32_t *)nullptr, static_cast<const __half *>(gamma_dev), (const __half *)nullptr, static_cast<__half *>(out_dev),
-                               (__half *)nullptr, H, 0u, eps, 1.0f));
+                               (__half *)nullptr, H, 0u, eps, 1.0f, 0));
         return IM_OK;
     }
     IM_CUDA_CHECK(launch_k(rms_norm_kernel<0>, dim3(T), dim3(kNormThreads), 0, as_stream(stream), static_cast<const __half *>(x_dev),
@@ -321,7 +323,7 @@ IM_EXPORT int im_cuda_embedding_norm(const uint32_t *tokens_dev, const void *tab
     if (rows_fit(H, {table_dev, gamma_dev, normed_dev, raw_dev})) {
         IM_CUDA_CHECK(launch_k(rms_rows_kernel<2>, dim3(T), rows_block(H), 0, as_stream(stream), static_cast<const __half *>(table_dev), (const __half *)nullptr,
                                tokens_dev, static_cast<const __half *>(gamma_dev), (const __half *)nullptr, static_cast<__half *>(normed_dev),
-                               static_cast<__half *>(raw_dev), H, vocab, eps, embed_scale));
+                               static_cast<__half *>(raw_dev), H, vocab, eps, embed_scale, 0));
         return IM_OK;
     }
     IM_CUDA_CHECK(launch_k(embedding_norm_kernel, dim3(T), dim3(kNormThreads), 0, as_stream(stream), tokens_dev,

@@ -1,0 +1,57 @@
+"""Projections of few tokens (converted fragments on mma.sync) against the CPU oracle's matmul, and the forms of a model that chain them."""
+import numpy as np
+import pytest
+
+from oracle import oracle as orc
+from tests import helpers as H
+from tests.test_gpu_model import DictProvider, _cfg, synth_model
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+TOL = 2e-3  # same fp16 operands, f32 accumulation in a different order, one fp16 rounding of the result
+
+
+@pytest.fixture(scope="module")
+def dev():
+    from ironmill_b200 import ops
+    return ops.Device(0)
+
+
+# token counts around the eight tokens of an instruction and at the ends of both ranges; row counts that leave a row tile, a row block or eight
+# rows incomplete; eight groups (one stage of a slice), an uneven number in slices, a long sum; more row tiles than CTAs (shares cut inside a tile)
+@pytest.mark.parametrize("bits", [4, 8])
+@pytest.mark.parametrize("N,K,M", [(16, 1024, 1), (120, 1024, 7), (200, 1408, 8), (1000, 1024, 9), (2056, 1152, 16), (136, 14336, 17), (6144, 1024, 24), (260, 2176, 25),
+                                   (19208, 1024, 31), (24584, 1152, 12), (640, 4224, 32), (250, 1024, 33), (19000, 1280, 48), (512, 1024, 41)])
+def test_few_tokens(dev, N, K, M, bits):
+    from ironmill_b200 import ops
+    qw = H.QWeight(N, K, bits=bits, awq=M % 2 == 0, seed=N + M + bits, name="gr")
+    qw.zps = qw.zps.copy()
+    qw.zps[3::397] += 0.25  # zero points that are no integer: the f32 path
+    qw.zps[5::911] = -700.0  # and one past the range of the packed one
+    qw.zps_f16 = orc.f32_to_f16(qw.zps)
+    w = qw.gpu(dev)
+    x = (H.rng_for("gr-x", M).standard_normal((M, K))).astype(np.float16)
+    ref = orc.matmul_affine(qw.packed, qw.scales_f16, qw.zps_f16, x, N, K, 128, bits, awq=qw.awq, threads=8)
+    for _ in range(2):  # the counters of cut tiles are back at zero after a launch
+        y = ops.matmul_affine(w, torch.from_numpy(x).cuda()).cpu().numpy()
+        assert H.rel_err(y, ref) <= TOL, (N, K, M)
+
+
+@pytest.mark.parametrize("chunk", [9, 24, 33])
+def test_prompt_in_short_portions(chunk):
+    """Portions of few tokens (packed norms, joint gate and up, packed activation) against the whole prompt at once (the kernels of many tokens):
+    the same operands and rounding points, sums in another order, an fp16 cache.  Each of the layer's seven roundings to fp16 may fall the other way,
+    2^-11 of a value each, two layers deep: sqrt(14) 2^-11 = 1.8e-3 of the logits' norm, doubled."""
+    from ironmill_b200.engine import CudaConfig, CudaInference
+    cfg = _cfg("llama", 2, 1024, 1152, 8, 4, 500, 1e6, 1e-6)
+    tensors = synth_model(cfg, seed=31, gamma_jitter=0.2)
+    tokens = H.rng_for("rows-prompt").integers(0, 500, 99).astype(np.uint32)
+    out = []
+    for c in (99, chunk):
+        conf = CudaConfig(max_seq_len=128, max_batch=1, prefill_chunk_size=c)
+        conf.without_turboquant()
+        eng = CudaInference(conf)
+        eng.load_weights(DictProvider(cfg, tensors))
+        out.append(eng.prefill(tokens).astype(np.float64))
+    assert np.linalg.norm(out[1] - out[0]) / np.linalg.norm(out[0]) <= 3.6e-3
