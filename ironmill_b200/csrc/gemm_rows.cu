@@ -6,9 +6,9 @@
 // On tcgen05 the converted weights have to pass through shared memory (store, proxy fence, barrier, one MMA thread), which left a stage of
 // 128 x 128 codes at 1 us and SM whatever the token count: five times its bytes' time.  Here a lane converts the codes of
 // its own mma.sync fragment in registers and multiplies them at once: no store, no fence, no hand-over.  Back to back with the packing of
-// the tokens, 4-bit, 24 tokens, tcgen05 -> here: 14336 x 4096 32.4 -> 19.9 us, 4096 x 14336 30.2 -> 21.2, 4096 x 4096 12.3 -> 10.4.  What is left
-// of a launch: 5 us of start and end, the rest at 50 % of the issue slots (460 instructions for two tiles, a third of them the conversion).  An
-// instruction serves eight tokens, so the gain ends at about 48 (14336 x 4096: 31.0 against 33.2 us; 64 tokens 36 against 33.3) and,
+// the tokens, 4-bit, 24 tokens, tcgen05 -> here: 14336 x 4096 32.4 -> 20.1 us, 4096 x 14336 30.2 -> 20.8, 4096 x 4096 12.3 -> 9.9.  What is left
+// of a launch: 4 us of start and end, the rest at 50 % of the issue slots (460 instructions for two tiles, a third of them the conversion).  An
+// instruction serves eight tokens, so the gain ends at about 48 (14336 x 4096: 30.4 against 33.2 us; 64 tokens 36 against 33.3) and,
 // with 8-bit codes, 32 (28.2 against 29.3; 48 tokens 32.5 against 30.5): more tokens stay on tcgen05 (gemm_tc.cu).
 //   * weights: the tiles of the matvec (16 rows x 128 columns, matvec_v2.cu); lane (g, t) owns columns 32 t .. 32 t + 31 of rows g
 //     and g + 8, so that 16 contiguous bytes are its fragments of eight k-steps.  A warp multiplies two row blocks (they share
@@ -22,6 +22,12 @@
 //     CTAs arrives last (a counter, nobody waits), adding the parts in CTA order.
 // The joint form multiplies gate rows and up rows as the pair of row blocks and leaves f16(silu(f16 gate) f16(up)), if asked
 // divided by the next projection's activation scales and packed for it.
+//
+// Batches of up to 15 rows keep the matvec's arithmetic (matvec_v2.cu: activations as 24-bit integers per group of 128, three byte planes, exact integer
+// sums, u8 x s8 products): the same kernel with INT = true, two rows to an instruction.  The matvec stages the planes again in every CTA, which
+// for four rows of 4096 values took 20 of a launch's 30 us, and passes over the weights once per four rows.  Here the kernel in front writes the planes
+// (rows_planes_kernel, norm_planes_kernel), one pass serves the batch, and gate, up and their activation or Q, K and V are one launch: a step of four
+// sequences through four 8B layers 690 -> 495 us, projections 24 -> 14 us a launch on average.
 #include <algorithm>
 
 #include "common.cuh"
@@ -37,18 +43,23 @@ constexpr int kRPad = 132;      // floats of a token's row of sums in shared mem
 constexpr int kRBStages = 3;    // token slabs: in use, on their way, and one that its slowest reader may still hold
 
 // More than 24 tokens: half the warps, so that their sums fit a thread's registers (16 with 8-bit codes, whose rings are twice as large).
-template <int NT, int BITS>
-constexpr int rows_warps() { return NT <= (BITS == 4 ? 3 : 2) ? 16 : 8; }
-template <int NT, int BITS>
-constexpr int rows_klanes() { return rows_warps<NT, BITS>() / 4; }
-template <int NT, int BITS>
-constexpr int rows_depth() { return rows_warps<NT, BITS>() == 16 ? (BITS == 4 ? 3 : 2) : BITS == 4 ? 4 : 3; }  // units (two tiles) in flight per warp
+template <int NT, int BITS, bool INT>
+constexpr int rows_warps() { return INT || NT <= (BITS == 4 ? 3 : 2) ? 16 : 8; }
+template <int NT, int BITS, bool INT>
+constexpr int rows_klanes() { return rows_warps<NT, BITS, INT>() / 4; }
+template <int NT, int BITS, bool INT>
+constexpr int rows_depth() { return rows_warps<NT, BITS, INT>() == 16 ? (BITS == 4 ? 3 : 2) : BITS == 4 ? 4 : 3; }  // units (two tiles) in flight per warp
+template <int NT, bool INT>
+constexpr int rows_tokens() { return INT ? NT * 2 : NT * 8; }  // tokens that NT instructions of eight columns take: four columns a row of integers
+template <int NT, bool INT>
+constexpr int rows_slab_max() { return INT ? planes_slab(NT * 2) : NT * 8 * 256; }
 template <int BITS>
 constexpr int rows_unit_bytes() { return 2 * TileGeom<BITS>::kTileBytes; }
 
 struct RowsParams {
     const uint8_t *tiles[2];  // joint: gate, up; else both the matrix
-    const __half *xs;         // packed tokens
+    const uint8_t *xs[2];     // packed tokens or planes, [group][slab]; the second set for rows from split_row on
+    int slab, split_row;
     __half *y;
     const __half *div;        // joint: activation scales of the next projection, or none
     float *partial;           // [grid][2][tokens][128]
@@ -56,7 +67,7 @@ struct RowsParams {
     int *err;
     int N, G, M, nblk, total;
     int slices;               // CTAs of a cluster that share a row tile (1: equal shares of the whole list)
-    int joint, packed, wide;  // packed: the result as the next projection reads it; wide: 16-byte stores of the result
+    int joint, packed, wide;  // joint: 1 rounds gate and up before the activation, 2 does not; packed: the result as the next projection reads it; wide: 8-byte stores of the result
 };
 
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void *src) {
@@ -151,20 +162,21 @@ struct Runs {
     }
 };
 
-template <int NT, int BITS>
-__global__ void __launch_bounds__(rows_warps<NT, BITS>() * 32, 1) gemm_rows_kernel(const RowsParams p) {
-    constexpr int NW = rows_warps<NT, BITS>(), KQ = rows_klanes<NT, BITS>(), D = rows_depth<NT, BITS>(), MP = NT * 8;
+template <int NT, int BITS, bool INT>
+__global__ void __launch_bounds__(rows_warps<NT, BITS, INT>() * 32, 1) gemm_rows_kernel(const RowsParams p) {
+    constexpr int NW = rows_warps<NT, BITS, INT>(), KQ = rows_klanes<NT, BITS, INT>(), D = rows_depth<NT, BITS, INT>(), MP = rows_tokens<NT, INT>();
     constexpr int kTile = TileGeom<BITS>::kTileBytes, kCodes = TileGeom<BITS>::kCodeBytes, kUnit = rows_unit_bytes<BITS>();
+    constexpr int kStage = KQ * rows_slab_max<NT, INT>();
     constexpr int CV = BITS == 4 ? 2 : 4;         // 16-byte vectors of codes per lane and tile
     constexpr int kCopies = KQ / 2;               // sums of warps on different groups, halved once in registers
     extern __shared__ __align__(128) unsigned char rows_smem[];
     unsigned char *ring = rows_smem;                                              // [warp][D][unit]
-    unsigned char *bs = ring + NW * D * kUnit;                                    // [stage][KQ groups][tokens * 256 bytes], read up to seven tokens past the end
-    float *red = reinterpret_cast<float *>(bs + kRBStages * KQ * MP * 256 + 512);  // [copies][MP][kRPad]
+    unsigned char *bs = ring + NW * D * kUnit;                                    // [stage][KQ groups][slab], read up to seven tokens past the end
+    float *red = reinterpret_cast<float *>(bs + kRBStages * kStage + 512);  // [copies][MP][kRPad]
     uint64_t *full = reinterpret_cast<uint64_t *>(red + kCopies * MP * kRPad), *empty = full + kRBStages;
     int *flag = reinterpret_cast<int *>(empty + kRBStages);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int G = p.G, M = p.M, slab = M * 256, stage_bytes = KQ * MP * 256;
+    const int G = p.G, M = p.M, slab = p.slab;
     int u0 = (int)((long long)p.total * blockIdx.x / gridDim.x), u1 = (int)((long long)p.total * (blockIdx.x + 1) / gridDim.x), rank = 0;
     if (p.slices > 1) {  // a row tile per cluster, a slice of K per CTA
         const int tile = blockIdx.x / p.slices;
@@ -232,7 +244,7 @@ __global__ void __launch_bounds__(rows_warps<NT, BITS>() * 32, 1) gemm_rows_kern
         }
         if (lane == 0) {
             mbar_expect_tx(&full[sl], (uint32_t)(n * slab));
-            bulk_g2s(bs + sl * stage_bytes, reinterpret_cast<const unsigned char *>(p.xs) + (size_t)bg * slab, (uint32_t)(n * slab), &full[sl]);
+            bulk_g2s(bs + sl * kStage, (br.tile * kRRows >= p.split_row ? p.xs[1] : p.xs[0]) + (size_t)bg * slab, (uint32_t)(n * slab), &full[sl]);
         }
         __syncwarp();
         bit++;
@@ -246,7 +258,8 @@ __global__ void __launch_bounds__(rows_warps<NT, BITS>() * 32, 1) gemm_rows_kern
 
     uint32_t e;
     asm volatile("mov.b32 %0, 0x64006400;" : "=r"(e));
-    float acc[2][NT][4];
+    constexpr int A = INT ? 2 : 4;
+    float acc[2][NT][A];
     int s = 0, par = 0, slot = 0, nrun = 0;
     for (Runs r(u0, u1, G); r.next(); nrun++) {
 #pragma unroll
@@ -254,71 +267,124 @@ __global__ void __launch_bounds__(rows_warps<NT, BITS>() * 32, 1) gemm_rows_kern
 #pragma unroll
             for (int n = 0; n < NT; n++)
 #pragma unroll
-                for (int i = 0; i < 4; i++) acc[b][n][i] = 0.0f;
+                for (int i = 0; i < A; i++) acc[b][n][i] = 0.0f;
         for (int g0 = r.g0; g0 < r.g1; g0 += KQ) {
             bring();
             if (!dead && !mbar_wait_warp(&full[s], par, p.err)) dead = true;
             if (g0 + kq < r.g1) {
                 cp_wait<D - 1>();
                 __syncwarp();
-                const unsigned char *tp = mine + slot * kUnit, *bp = bs + s * stage_bytes + kq * slab + g8 * 64 + t * 16;
-                uint32_t sz[2][2];
-                RowScale rs[2][2];
-                bool fast = true;
-#pragma unroll
-                for (int b = 0; b < 2; b++) {
-#pragma unroll
-                    for (int h = 0; h < 2; h++) sz[b][h] = *reinterpret_cast<const uint32_t *>(tp + b * kTile + kCodes + g8 * 4 + 32 * h);
-                    fast = row_scales(sz[b][0], sz[b][1], rs[b]) && fast;
-                }
-                // eight columns: two k-steps of both row blocks
-                auto multiply = [&](int i, const uint32_t (&a)[2][2][4]) {
-#pragma unroll
-                    for (int n = 0; n < NT; n++) {
-                        const uint4 x = *reinterpret_cast<const uint4 *>(bp + i * (M * 64) + n * 512);
-#pragma unroll
-                        for (int b = 0; b < 2; b++) mma_f16(acc[b][n], a[b][0][0], a[b][1][0], a[b][0][1], a[b][1][1], x.x, x.y);
-#pragma unroll
-                        for (int b = 0; b < 2; b++) mma_f16(acc[b][n], a[b][0][2], a[b][1][2], a[b][0][3], a[b][1][3], x.z, x.w);
-                    }
-                };
-                uint32_t a[2][2][4];
-                if (__builtin_expect(__all_sync(0xffffffffu, fast), 1)) {
+                const unsigned char *tp = mine + slot * kUnit, *bp = bs + s * kStage + kq * slab;
+                if constexpr (INT) {
                     uint4 w[2][CV];
+                    float2 sz[2][2];
 #pragma unroll
-                    for (int b = 0; b < 2; b++)
+                    for (int b = 0; b < 2; b++) {
 #pragma unroll
                         for (int v = 0; v < CV; v++) w[b][v] = *reinterpret_cast<const uint4 *>(tp + b * kTile + v * 512 + lane * 16);
+#pragma unroll
+                        for (int h = 0; h < 2; h++) sz[b][h] = __half22float2(*reinterpret_cast<const __half2 *>(tp + b * kTile + kCodes + g8 * 4 + 32 * h));
+                    }
                     __syncwarp();
-                    request_next(slot);  // every lane has its codes in registers
+                    request_next(slot);
                     if (!dead)
 #pragma unroll
+                        for (int n = 0; n < NT; n++) {
+                            // this lane's column: byte plane g % 4 of batch row 2 n + g / 4 (plane 3: zeros), its 32 columns as two vectors
+                            uint4 x0 = make_uint4(0, 0, 0, 0), x1 = x0;
+                            if ((g8 & 3) < 3) {
+                                const unsigned char *xp = bp + (2 * n + (g8 >> 2)) * 192 + (g8 & 3) * 64 + t * 16;
+                                x0 = *reinterpret_cast<const uint4 *>(xp);
+                                x1 = *reinterpret_cast<const uint4 *>(xp + M * 192);
+                            }
+                            // constants of (group, row 2 n + t / 2): even lanes hold the high and middle planes' sums, odd ones the low plane's
+                            const float2 m = *reinterpret_cast<const float2 *>(bp + M * 384 + (2 * n + (t >> 1)) * 8);
+                            const float mx = t & 1 ? m.x * 0x1p-16f : m.x, my = t & 1 ? 0.0f : m.y;
+#pragma unroll
+                            for (int b = 0; b < 2; b++) {
+                                int lo[4], hi[4];
+                                float f[2];
+                                if (BITS == 4) {
+                                    constexpr unsigned ML = 0x0F0F0F0Fu, MH = 0xF0F0F0F0u;
+                                    const uint4 a0 = w[b][0], a1 = w[b][1];
+                                    mma_u8s8_z(lo, a0.x & ML, a1.x & ML, a0.y & ML, a1.y & ML, x0.x, x0.z);
+                                    mma_u8s8_z(hi, a0.x & MH, a1.x & MH, a0.y & MH, a1.y & MH, x0.y, x0.w);
+                                    mma_u8s8(lo, a0.z & ML, a1.z & ML, a0.w & ML, a1.w & ML, x1.x, x1.z);
+                                    mma_u8s8(hi, a0.z & MH, a1.z & MH, a0.w & MH, a1.w & MH, x1.y, x1.w);
+#pragma unroll
+                                    for (int h = 0; h < 2; h++) f[h] = fmaf((float)(lo[2 * h] * 16 + hi[2 * h]), 256.0f, (float)(lo[2 * h + 1] * 16 + hi[2 * h + 1]));
+                                } else {
+                                    const uint4 a0 = w[b][0], a1 = w[b][1], c0 = w[b][2 % CV], c1 = w[b][3 % CV];
+                                    mma_u8s8_z(lo, a0.x, c0.x, a0.z, c0.z, x0.x, x0.z);
+                                    mma_u8s8_z(hi, a0.y, c0.y, a0.w, c0.w, x0.y, x0.w);
+                                    mma_u8s8(lo, a1.x, c1.x, a1.z, c1.z, x1.x, x1.z);
+                                    mma_u8s8(hi, a1.y, c1.y, a1.w, c1.w, x1.y, x1.w);
+#pragma unroll
+                                    for (int h = 0; h < 2; h++) f[h] = fmaf((float)(lo[2 * h] + hi[2 * h]), 4096.0f, (float)(lo[2 * h + 1] + hi[2 * h + 1]) * 16.0f);
+                                }
+#pragma unroll
+                                for (int h = 0; h < 2; h++) acc[b][n][h] = fmaf(sz[b][h].x * mx, fmaf(-sz[b][h].y, my, f[h]), acc[b][n][h]);
+                            }
+                        }
+                } else {
+                    uint32_t sz[2][2];
+                    RowScale rs[2][2];
+                    bool fast = true;
+#pragma unroll
+                    for (int b = 0; b < 2; b++) {
+#pragma unroll
+                        for (int h = 0; h < 2; h++) sz[b][h] = *reinterpret_cast<const uint32_t *>(tp + b * kTile + kCodes + g8 * 4 + 32 * h);
+                        fast = row_scales(sz[b][0], sz[b][1], rs[b]) && fast;
+                    }
+                    // eight columns: two k-steps of both row blocks
+                    auto multiply = [&](int i, const uint32_t (&a)[2][2][4]) {
+#pragma unroll
+                        for (int n = 0; n < NT; n++) {
+                            const uint4 x = *reinterpret_cast<const uint4 *>(bp + g8 * 64 + t * 16 + i * (M * 64) + n * 512);
+#pragma unroll
+                            for (int b = 0; b < 2; b++) mma_f16(acc[b][n], a[b][0][0], a[b][1][0], a[b][0][1], a[b][1][1], x.x, x.y);
+#pragma unroll
+                            for (int b = 0; b < 2; b++) mma_f16(acc[b][n], a[b][0][2], a[b][1][2], a[b][0][3], a[b][1][3], x.z, x.w);
+                        }
+                    };
+                    uint32_t a[2][2][4];
+                    if (__builtin_expect(__all_sync(0xffffffffu, fast), 1)) {
+                        uint4 w[2][CV];
+#pragma unroll
+                        for (int b = 0; b < 2; b++)
+#pragma unroll
+                            for (int v = 0; v < CV; v++) w[b][v] = *reinterpret_cast<const uint4 *>(tp + b * kTile + v * 512 + lane * 16);
+                        __syncwarp();
+                        request_next(slot);  // every lane has its codes in registers
+                        if (!dead)
+#pragma unroll
+                            for (int i = 0; i < 4; i++) {
+#pragma unroll
+                                for (int b = 0; b < 2; b++)
+#pragma unroll
+                                    for (int h = 0; h < 2; h++) {
+                                        const uint4 q = BITS == 4 ? w[b][h] : w[b][(2 * h + (i >> 1)) % CV];
+                                        if (BITS == 4) rows_dequant<BITS>(i == 0 ? q.x : i == 1 ? q.y : i == 2 ? q.z : q.w, 0u, rs[b][h], e, a[b][h]);
+                                        else rows_dequant<BITS>(i & 1 ? q.z : q.x, i & 1 ? q.w : q.y, rs[b][h], e, a[b][h]);
+                                    }
+                                multiply(i, a);
+                            }
+                    } else {
+#pragma unroll 1
                         for (int i = 0; i < 4; i++) {
 #pragma unroll
                             for (int b = 0; b < 2; b++)
 #pragma unroll
                                 for (int h = 0; h < 2; h++) {
-                                    const uint4 q = BITS == 4 ? w[b][h] : w[b][(2 * h + (i >> 1)) % CV];
-                                    if (BITS == 4) rows_dequant<BITS>(i == 0 ? q.x : i == 1 ? q.y : i == 2 ? q.z : q.w, 0u, rs[b][h], e, a[b][h]);
-                                    else rows_dequant<BITS>(i & 1 ? q.z : q.x, i & 1 ? q.w : q.y, rs[b][h], e, a[b][h]);
+                                    const uint32_t *w = reinterpret_cast<const uint32_t *>(tp + b * kTile + (BITS == 4 ? h : 2 * h + (i >> 1)) * 512 + lane * 16);
+                                    if (BITS == 4) rows_dequant_any<BITS>(w[i], 0u, sz[b][h], a[b][h]);
+                                    else rows_dequant_any<BITS>(w[2 * (i & 1)], w[2 * (i & 1) + 1], sz[b][h], a[b][h]);
                                 }
-                            multiply(i, a);
+                            if (!dead) multiply(i, a);
                         }
-                } else {
-#pragma unroll 1
-                    for (int i = 0; i < 4; i++) {
-#pragma unroll
-                        for (int b = 0; b < 2; b++)
-#pragma unroll
-                            for (int h = 0; h < 2; h++) {
-                                const uint32_t *w = reinterpret_cast<const uint32_t *>(tp + b * kTile + (BITS == 4 ? h : 2 * h + (i >> 1)) * 512 + lane * 16);
-                                if (BITS == 4) rows_dequant_any<BITS>(w[i], 0u, sz[b][h], a[b][h]);
-                                else rows_dequant_any<BITS>(w[2 * (i & 1)], w[2 * (i & 1) + 1], sz[b][h], a[b][h]);
-                            }
-                        if (!dead) multiply(i, a);
+                        __syncwarp();
+                        request_next(slot);
                     }
-                    __syncwarp();
-                    request_next(slot);
                 }
                 if (++slot == D) slot = 0;
             }
@@ -329,13 +395,21 @@ __global__ void __launch_bounds__(rows_warps<NT, BITS>() * 32, 1) gemm_rows_kern
         // ---- the run's sums: warps on different groups together, through shared memory as [token][row]
         auto sync = [&]() { asm volatile("bar.sync 1, %0;" ::"n"(NW * 32) : "memory"); };
         auto each = [&](auto f) {
+            float *at = red + (kq % kCopies) * MP * kRPad + rp * (p.joint ? 16 : 32) + g8;
+            const int second = p.joint ? 64 : 16;  // rows from the pair's first block to its second
 #pragma unroll
             for (int b = 0; b < 2; b++)
 #pragma unroll
                 for (int n = 0; n < NT; n++)
 #pragma unroll
-                    for (int i = 0; i < 4; i++)
-                        f(acc[b][n][i], red + ((kq % kCopies) * MP + n * 8 + 2 * t + (i & 1)) * kRPad + (p.joint ? b * 64 + rp * 16 : rp * 32 + b * 16) + g8 + 8 * (i >> 1));
+                    for (int i = 0; i < A; i++) {
+                        if constexpr (INT) {
+                            const float v = acc[b][n][i] + __shfl_xor_sync(0xffffffffu, acc[b][n][i], 1);
+                            if (!(t & 1)) f(v, at + (2 * n + (t >> 1)) * kRPad + b * second + 8 * i);
+                        } else {
+                            f(acc[b][n][i], at + (n * 8 + 2 * t + (i & 1)) * kRPad + b * second + 8 * (i >> 1));
+                        }
+                    }
         };
         if (kq >= kCopies) each([](float v, float *q) { *q = v; });
         sync();
@@ -370,66 +444,80 @@ __global__ void __launch_bounds__(rows_warps<NT, BITS>() * 32, 1) gemm_rows_kern
             finish = *flag != 0;
         }
         if (finish && !dead) {
-            // a task: eight neighbouring rows of a token; the CTAs of a cluster share them
-            const int chunks = p.joint ? 8 : 16, share = (M * chunks + p.slices - 1) / p.slices, end = min((rank + 1) * share, M * chunks);
-            for (int i = rank * share + tid; i < end; i += NW * 32) {
-                const int m = i / chunks, c = i - m * chunks;
-                float v[2][8];
+            // a task: four neighbouring rows of a token; the CTAs of a cluster share them
+            const int sh = p.joint ? 4 : 5, share = ((M << sh) + p.slices - 1) / p.slices + 1 & ~1, end = min((rank + 1) * share, M << sh);
+            for (int i0 = rank * share; i0 < end; i0 += NW * 32) {  // whole warps: two lanes hold eight rows
+                const int i = min(i0 + tid, end - 1), m = i >> sh, c = i - (m << sh);
+                const bool mine_too = i0 + tid < end;
+                float4 v[2];
 #pragma unroll
                 for (int b = 0; b < 2; b++) {
+                    v[b] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
                     if (b && !p.joint) break;
-                    const int row = b * 64 + c * 8;
-                    float4 lo = make_float4(0.0f, 0.0f, 0.0f, 0.0f), hi = lo;
+                    const int row = b * 64 + c * 4;
                     if (parts) {
                         constexpr int kAtOnce = 4;  // parts on their way together
                         for (int c0 = c_first; c0 <= c_last; c0 += kAtOnce) {
-                            float4 x[kAtOnce], z[kAtOnce];
+                            float4 x[kAtOnce];
 #pragma unroll
                             for (int k = 0; k < kAtOnce; k++) {
                                 const int cc = min(c0 + k, c_last), first_tile = (int)((long long)p.total * cc / gridDim.x) / G;
-                                const float4 *q =
-                                    reinterpret_cast<const float4 *>(p.partial + ((size_t)cc * 2 + (first_tile == r.tile ? 0 : 1)) * (MP * kRRows) + m * kRRows + row);
-                                x[k] = __ldcg(q);
-                                z[k] = __ldcg(q + 1);
+                                x[k] = __ldcg(reinterpret_cast<const float4 *>(p.partial + ((size_t)cc * 2 + (first_tile == r.tile ? 0 : 1)) * (MP * kRRows) + m * kRRows + row));
                             }
 #pragma unroll
                             for (int k = 0; k < kAtOnce; k++)
-                                if (c0 + k <= c_last) {
-                                    add4(lo, x[k]);
-                                    add4(hi, z[k]);
-                                }
+                                if (c0 + k <= c_last) add4(v[b], x[k]);
                         }
                     } else {
-                        const uint32_t q = smem_u32(red + m * kRPad + row);
-                        for (int k = 0; k < p.slices; k++) {
-                            const uint32_t qk = p.slices > 1 ? cluster_addr(q, k) : q;
+                        const float *q = red + m * kRPad + row;
+                        if (p.slices == 1) {
+                            v[b] = *reinterpret_cast<const float4 *>(q);
+                            if (kCopies > 1) add4(v[b], *reinterpret_cast<const float4 *>(q + MP * kRPad));
+                        } else {
+                            const uint32_t qs = smem_u32(q);
+                            constexpr int kAtOnce = 4;  // CTAs whose sums are on their way together
+                            int k0 = 0;
+                            for (; k0 + kAtOnce <= p.slices; k0 += kAtOnce) {
+                                float4 x[kAtOnce][kCopies];
 #pragma unroll
-                            for (int j = 0; j < kCopies; j++) {
-                                add4(lo, ld_cluster(qk + j * MP * kRPad * 4));
-                                add4(hi, ld_cluster(qk + j * MP * kRPad * 4 + 16));
+                                for (int k = 0; k < kAtOnce; k++)
+#pragma unroll
+                                    for (int j = 0; j < kCopies; j++) x[k][j] = ld_cluster(cluster_addr(qs, k0 + k) + j * MP * kRPad * 4);
+#pragma unroll
+                                for (int k = 0; k < kAtOnce; k++)
+#pragma unroll
+                                    for (int j = 0; j < kCopies; j++) add4(v[b], x[k][j]);
                             }
+                            for (; k0 < p.slices; k0++)
+#pragma unroll
+                                for (int j = 0; j < kCopies; j++) add4(v[b], ld_cluster(cluster_addr(qs, k0) + j * MP * kRPad * 4));
                         }
                     }
-                    v[b][0] = lo.x; v[b][1] = lo.y; v[b][2] = lo.z; v[b][3] = lo.w;
-                    v[b][4] = hi.x; v[b][5] = hi.y; v[b][6] = hi.z; v[b][7] = hi.w;
                 }
-                const int n = r.tile * (p.joint ? 64 : 128) + c * 8;
-                __half h[8];
+                const int n = r.tile * (p.joint ? 64 : 128) + c * 4;
+                const float f[2][4] = {{v[0].x, v[0].y, v[0].z, v[0].w}, {v[1].x, v[1].y, v[1].z, v[1].w}};
+                __half h[4];
 #pragma unroll
-                for (int j = 0; j < 8; j++) {
-                    h[j] = __float2half_rn(v[0][j]);
-                    if (p.joint) {
-                        const float gv = __half2float(h[j]), uv = __half2float(__float2half_rn(v[1][j]));
+                for (int j = 0; j < 4; j++) {
+                    h[j] = __float2half_rn(f[0][j]);
+                    if (p.joint == 2) {
+                        h[j] = __float2half_rn((f[0][j] / (1.0f + expf(-f[0][j]))) * f[1][j]);
+                    } else if (p.joint) {
+                        const float gv = __half2float(h[j]), uv = __half2float(__float2half_rn(f[1][j]));
                         h[j] = __float2half_rn((gv / (1.0f + expf(-gv))) * uv);
                         if (p.div && n + j < p.N) h[j] = __float2half_rn(__half2float(h[j]) / __half2float(p.div[n + j]));
                     }
                 }
-                if (p.packed) {
-                    if (n < p.N) *reinterpret_cast<uint4 *>(p.y + token_chunk(n >> 3, m, M) * 8) = pack_chunk(h);
+                auto two = [](__half a, __half b) { return (uint32_t)__half_as_ushort(a) | ((uint32_t)__half_as_ushort(b) << 16); };
+                uint2 w = make_uint2(two(h[0], h[1]), two(h[2], h[3]));
+                if (p.packed) {  // rows c .. c + 3 and c + 4 .. c + 7 of a chunk of eight, interleaved: the even lane writes the first two words of four
+                    const uint2 o = make_uint2(__shfl_xor_sync(0xffffffffu, w.x, 1), __shfl_xor_sync(0xffffffffu, w.y, 1));
+                    w = lane & 1 ? make_uint2(__byte_perm(o.y, w.y, 0x5410), __byte_perm(o.y, w.y, 0x7632)) : make_uint2(__byte_perm(w.x, o.x, 0x5410), __byte_perm(w.x, o.x, 0x7632));
+                    if (mine_too && n < p.N) *reinterpret_cast<uint2 *>(p.y + token_chunk(n >> 3, m, M) * 8 + (lane & 1) * 4) = w;
                 } else if (p.wide) {
-                    if (n < p.N) *reinterpret_cast<uint4 *>(p.y + (size_t)m * p.N + n) = *reinterpret_cast<const uint4 *>(h);
-                } else {
-                    for (int j = 0; j < 8; j++)
+                    if (mine_too && n < p.N) *reinterpret_cast<uint2 *>(p.y + (size_t)m * p.N + n) = w;
+                } else if (mine_too) {
+                    for (int j = 0; j < 4; j++)
                         if (n + j < p.N) p.y[(size_t)m * p.N + n + j] = h[j];
                 }
             }
@@ -441,6 +529,123 @@ __global__ void __launch_bounds__(rows_warps<NT, BITS>() * 32, 1) gemm_rows_kern
     // token copies that nobody waited for (a wait ran out) must land before the block leaves
     if (warp == 0 && dead)
         for (int i = max(0, bit - kRBStages); i < bit; i++) mbar_wait_warp(&full[i % kRBStages], (i / kRBStages) & 1, p.err);
+}
+
+// Eight values of a group of 128 (its sixteen chunks in sixteen consecutive lanes, chunk hl) of row m as 24-bit integers against the group's largest
+// magnitude: rounding and digits of stage_chunk24 (v2_device.cuh), laid out for the fragments above.  scale: a factor of the row, into the constants.
+__device__ __forceinline__ void plane_chunk(const float (&v)[8], bool live, int grp, int m, int M, int hl, float scale, uint8_t *__restrict__ out) {
+    float amax = 0.0f;
+#pragma unroll
+    for (int i = 0; i < 8; i++) amax = fmaxf(amax, fabsf(v[i]));
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+    const float sx = amax > 0.0f ? amax * (1.0f / (float)kActTop) : 1.0f, inv = amax > 0.0f ? (float)kActTop / amax : 0.0f;
+    unsigned y[8];
+    int lsum = 0;
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+        const int xi = max(-kActTop, min(kActTop, __float2int_rn(v[i] * inv)));
+        lsum += xi;
+        y[i] = (unsigned)(xi + 0x808080) ^ 0x808080u;
+    }
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) lsum += __shfl_xor_sync(0xffffffffu, lsum, o);
+    if (!live) return;
+    uint8_t *slab = out + (size_t)grp * planes_slab(M);
+    const int t = hl >> 2, j = hl & 3;
+#pragma unroll
+    for (int c = 0; c < 3; c++) {  // plane c: 0 high, 1 middle, 2 low = byte 2 - c of y; the even columns, then the odd ones
+        const unsigned sel = (unsigned)(2 - c) | ((unsigned)(6 - c) << 4);
+        const unsigned e = __byte_perm(__byte_perm(y[0], y[2], sel), __byte_perm(y[4], y[6], sel), 0x5410);
+        const unsigned o = __byte_perm(__byte_perm(y[1], y[3], sel), __byte_perm(y[5], y[7], sel), 0x5410);
+        *reinterpret_cast<uint2 *>(slab + (j >> 1) * (M * 192) + m * 192 + c * 64 + t * 16 + (j & 1) * 8) = make_uint2(e, o);
+    }
+    if (hl == 0) *reinterpret_cast<float2 *>(slab + M * 384 + m * 8) = make_float2(sx * 16.0f * scale, (float)lsum * 0.0625f);
+}
+__device__ __forceinline__ void half8(const __half *p, float (&v)[8]) {
+    const uint4 raw = *reinterpret_cast<const uint4 *>(p);
+    const __half2 *h = reinterpret_cast<const __half2 *>(&raw);
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const float2 f = __half22float2(h[i]);
+        v[2 * i] = f.x;
+        v[2 * i + 1] = f.y;
+    }
+}
+
+// Planes of x / awq (or x): grid (rows, groups / 8), two groups a warp.
+__global__ void __launch_bounds__(128) rows_planes_kernel(const __half *__restrict__ x, const __half *__restrict__ awq, uint8_t *__restrict__ out, int G) {
+    pdl_trigger();
+    const int lane = threadIdx.x & 31, hl = lane & 15, m = blockIdx.x, want = blockIdx.y * 8 + (threadIdx.x >> 5) * 2 + (lane >> 4), grp = min(want, G - 1), k = grp * 128 + hl * 8;
+    float v[8], a[8];
+    if (awq) half8(awq + k, a);
+    pdl_wait();
+    half8(x + (size_t)m * G * 128 + k, v);
+    if (awq)
+#pragma unroll
+        for (int i = 0; i < 8; i++) v[i] = __fdiv_rn(v[i], a[i]);
+    plane_chunk(v, want < G, grp, m, gridDim.x, hl, 1.0f, out);
+}
+
+// r = a + b, residual = f16(r), and r normed, as planes of what the next projections read (the reference's two forms, matvec.cu):
+//   u: the unrounded r gamma / awq, the norm's factor in the constants;   n: f16(r rms_inv gamma) / awq.
+// One CTA per row; a half-warp holds a group (two for rows longer than 4096) from the sums on.
+constexpr int kNormPlaneChunks = 2;
+__global__ void __launch_bounds__(512) norm_planes_kernel(const __half *__restrict__ a, const __half *__restrict__ b, const __half *__restrict__ gamma,
+                                                          const __half *__restrict__ awq, __half *__restrict__ residual, uint8_t *__restrict__ u, uint8_t *__restrict__ n,
+                                                          int G, float eps) {
+    __shared__ float sh[16];
+    pdl_trigger();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, hl = lane & 15, m = blockIdx.x, M = gridDim.x, K = G * 128;
+    float r[kNormPlaneChunks][8], ss = 0.0f;
+    pdl_wait();
+#pragma unroll
+    for (int c = 0; c < kNormPlaneChunks; c++) {
+        const int grp = c * 32 + warp * 2 + (lane >> 4), k = grp * 128 + hl * 8;
+        if (grp < G) {
+            float v[8];
+            half8(a + (size_t)m * K + k, r[c]);
+            half8(b + (size_t)m * K + k, v);
+            uint4 out;
+            __half2 *ho = reinterpret_cast<__half2 *>(&out);
+#pragma unroll
+            for (int i = 0; i < 8; i++) {
+                r[c][i] += v[i];
+                ss = fmaf(r[c][i], r[c][i], ss);
+            }
+#pragma unroll
+            for (int i = 0; i < 4; i++) ho[i] = __floats2half2_rn(r[c][2 * i], r[c][2 * i + 1]);
+            *reinterpret_cast<uint4 *>(residual + (size_t)m * K + k) = out;
+        }
+    }
+    ss = warp_sum(ss);
+    if (lane == 0) sh[warp] = ss;
+    __syncthreads();
+    float tot = 0.0f;
+    for (int w = 0; w < (int)(blockDim.x >> 5); w++) tot += sh[w];
+    const float ri = rsqrtf(tot / (float)K + eps);
+#pragma unroll
+    for (int c = 0; c < kNormPlaneChunks; c++) {
+        if (c * 32 + warp * 2 >= G) break;  // warp-uniform
+        const int want = c * 32 + warp * 2 + (lane >> 4), grp = min(want, G - 1), k = grp * 128 + hl * 8;
+        float g[8], q[8], v[8];
+        half8(gamma + k, g);
+        if (awq) half8(awq + k, q);
+        if (u) {
+#pragma unroll
+            for (int i = 0; i < 8; i++) {
+                v[i] = r[c][i] * g[i];
+                if (awq) v[i] = __fdiv_rn(v[i], q[i]);
+            }
+            plane_chunk(v, want < G, grp, m, M, hl, ri, u);
+        }
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+            v[i] = __half2float(__float2half_rn(r[c][i] * ri * g[i]));
+            if (awq) v[i] = __fdiv_rn(v[i], q[i]);
+        }
+        plane_chunk(v, want < G, grp, m, M, hl, 1.0f, n);
+    }
 }
 
 // Packed tokens f16(x / awq) (or x): one thread per eight columns of a token.
@@ -511,14 +716,14 @@ int rows_clusters(void (*kern)(RowsParams), int size, int threads, size_t smem, 
     return n;
 }
 
-template <int NT, int BITS>
+template <int NT, int BITS, bool INT>
 int rows_launch(RowsParams p, const Device *dev, cudaStream_t st) {
-    constexpr int NW = rows_warps<NT, BITS>(), KQ = rows_klanes<NT, BITS>(), MP = NT * 8;
-    constexpr size_t smem = (size_t)NW * rows_depth<NT, BITS>() * rows_unit_bytes<BITS>() + (size_t)kRBStages * KQ * MP * 256 + 512 +
+    constexpr int NW = rows_warps<NT, BITS, INT>(), KQ = rows_klanes<NT, BITS, INT>(), MP = rows_tokens<NT, INT>();
+    constexpr size_t smem = (size_t)NW * rows_depth<NT, BITS, INT>() * rows_unit_bytes<BITS>() + (size_t)kRBStages * KQ * rows_slab_max<NT, INT>() + 512 +
                             (size_t)(KQ / 2) * MP * kRPad * 4 + 2 * kRBStages * 8 + 16;
     static_assert(smem <= 227 * 1024, "the rings of this form do not fit");
     if (smem > dev->smem_optin) return IM_ERR_BOUNDS;
-    auto kern = gemm_rows_kernel<NT, BITS>;
+    auto kern = gemm_rows_kernel<NT, BITS, INT>;
     static DeviceOnce once;  // per instantiation
     if (once.first(dev->ordinal)) IM_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     // Few row tiles: a cluster of CTAs per tile, as many as the GPU holds (at least one stage of groups each).  Otherwise equal shares of the
@@ -537,11 +742,18 @@ int rows_launch(RowsParams p, const Device *dev, cudaStream_t st) {
 template <int BITS>
 int rows_run(const RowsParams &p, const Device *dev, cudaStream_t st) {
     const int nt = (p.M + 7) / 8;
-    if (nt <= 1) return rows_launch<1, BITS>(p, dev, st);
-    if (nt == 2) return rows_launch<2, BITS>(p, dev, st);
-    if (nt == 3) return rows_launch<3, BITS>(p, dev, st);
-    if (nt == 4) return rows_launch<4, BITS>(p, dev, st);
-    return rows_launch<6, 4>(p, dev, st);
+    if (nt <= 1) return rows_launch<1, BITS, false>(p, dev, st);
+    if (nt == 2) return rows_launch<2, BITS, false>(p, dev, st);
+    if (nt == 3) return rows_launch<3, BITS, false>(p, dev, st);
+    if (nt == 4) return rows_launch<4, BITS, false>(p, dev, st);
+    return rows_launch<6, 4, false>(p, dev, st);
+}
+template <int BITS>
+int planes_run(const RowsParams &p, const Device *dev, cudaStream_t st) {
+    if (p.M <= 2) return rows_launch<1, BITS, true>(p, dev, st);
+    if (p.M <= 4) return rows_launch<2, BITS, true>(p, dev, st);
+    if (p.M <= 8) return rows_launch<4, BITS, true>(p, dev, st);
+    return rows_launch<8, BITS, true>(p, dev, st);
 }
 
 }  // namespace
@@ -559,15 +771,46 @@ int token_pack(const __half *x, const __half *awq, __half *out, int M, int K, cu
     return IM_OK;
 }
 
-int gemm_rows(const AffineWeight *w, const AffineWeight *up, const __half *packed, __half *y, int M, const __half *div, bool pack_out, cudaStream_t st) {
+static RowsParams rows_params(const AffineWeight *w, const AffineWeight *up, __half *y, int M, int joint) {
     RowsParams p{};
     p.tiles[0] = w->tiles;
     p.tiles[1] = up ? up->tiles : w->tiles;
-    p.xs = packed; p.y = y; p.div = div; p.partial = w->dev->gemm_partial; p.counters = w->dev->sk_counters; p.err = w->dev->err_flag;
-    p.N = w->N; p.G = w->G; p.M = M; p.nblk = w->nblk; p.joint = up ? 1 : 0; p.packed = pack_out ? 1 : 0;
-    p.wide = w->N % 8 == 0 && reinterpret_cast<uintptr_t>(y) % 16 == 0;
+    p.y = y; p.partial = w->dev->gemm_partial; p.counters = w->dev->sk_counters; p.err = w->dev->err_flag;
+    p.N = w->N; p.G = w->G; p.M = M; p.nblk = w->nblk; p.joint = up ? joint : 0;
+    p.wide = w->N % 4 == 0 && reinterpret_cast<uintptr_t>(y) % 8 == 0;
     p.total = (up ? (w->nblk + 3) / 4 : (w->nblk + 7) / 8) * w->G;
+    return p;
+}
+
+int gemm_rows(const AffineWeight *w, const AffineWeight *up, const __half *packed, __half *y, int M, const __half *div, bool pack_out, cudaStream_t st) {
+    RowsParams p = rows_params(w, up, y, M, 1);
+    p.xs[0] = p.xs[1] = reinterpret_cast<const uint8_t *>(packed);
+    p.slab = M * 256; p.split_row = 1 << 30; p.div = div; p.packed = pack_out ? 1 : 0;
     return w->bits == 8 ? rows_run<8>(p, w->dev, st) : rows_run<4>(p, w->dev, st);
+}
+
+bool planes_take(const AffineWeight *w, int M) { return M >= 1 && M <= kPlanesMaxRows && gemm_rows_takes(w, M); }
+
+int rows_planes(const __half *x, const __half *awq, uint8_t *planes, int M, int K, cudaStream_t st) {
+    const int G = K / 128;
+    IM_CUDA_CHECK(launch_k(rows_planes_kernel, dim3(M, (G + 7) / 8), dim3(128), 0, st, x, awq, planes, G));
+    return IM_OK;
+}
+
+int norm_planes(const __half *a, const __half *b, const __half *gamma, const __half *awq, __half *residual, uint8_t *u, uint8_t *n, int H, int M, float eps, cudaStream_t st) {
+    const int G = H / 128;
+    if (H % 128 != 0 || G > 32 * kNormPlaneChunks) return IM_ERR_BOUNDS;
+    IM_CUDA_CHECK(launch_k(norm_planes_kernel, dim3(M), dim3(32 * std::min(16, (G + 1) / 2)), 0, st, a, b, gamma, awq, residual, u, n, G, eps));
+    return IM_OK;
+}
+
+int matvec_planes(const AffineWeight *w, const AffineWeight *up, const uint8_t *planes, const uint8_t *planes_from, int split_row, __half *y, int M, bool round_gate_up,
+                  cudaStream_t st) {
+    RowsParams p = rows_params(w, up, y, M, round_gate_up ? 1 : 2);
+    p.xs[0] = planes;
+    p.xs[1] = planes_from ? planes_from : planes;
+    p.slab = planes_slab(M); p.split_row = planes_from ? split_row : 1 << 30;
+    return w->bits == 8 ? planes_run<8>(p, w->dev, st) : planes_run<4>(p, w->dev, st);
 }
 
 }  // namespace im

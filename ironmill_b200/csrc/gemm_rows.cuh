@@ -19,10 +19,24 @@ __device__ __forceinline__ uint4 pack_chunk(const __half (&h)[8]) {
 }
 #endif
 
+// Byte planes of M rows for one group of 128 columns: [16 of a run of 32 columns][row][plane][run] x 16 bytes, then two constants a row.
+__host__ __device__ constexpr int planes_slab(int M) { return M * 384 + (M + 1) / 2 * 16; }
+constexpr int kPlanesMaxRows = 15;  // from 16 rows on a decode step's projections are the reference's matmul form (gemm_rows, gemm_affine_tc)
+
 bool gemm_rows_takes(const AffineWeight *w, int M);
 // f16(x / awq) (awq may be null) of M rows of K = a multiple of 128, packed; x anywhere, out 16-byte aligned and apart from it
 int token_pack(const __half *x, const __half *awq, __half *out, int M, int K, cudaStream_t st);
 // y[M, N] = packed tokens times w; with `up` (of w's form) the gated activation of both, divided by `div` if given; pack_out: packed for the next projection
 int gemm_rows(const AffineWeight *w, const AffineWeight *up, const __half *packed, __half *y, int M, const __half *div, bool pack_out, cudaStream_t st);
+
+// The same for rows as 24-bit integers.
+bool planes_take(const AffineWeight *w, int M);
+int rows_planes(const __half *x, const __half *awq, uint8_t *planes, int M, int K, cudaStream_t st);
+// residual = f16(a + b); planes of the normed sum as the next projections read it: u (may be null) unrounded, n rounded.  IM_ERR_BOUNDS: H is not
+// a multiple of 128 or too long.
+int norm_planes(const __half *a, const __half *b, const __half *gamma, const __half *awq, __half *residual, uint8_t *u, uint8_t *n, int H, int M, float eps, cudaStream_t st);
+// y[M, N]; rows from split_row on read planes_from (null: all read planes); with `up` the gated activation, of rounded or of f32 products
+int matvec_planes(const AffineWeight *w, const AffineWeight *up, const uint8_t *planes, const uint8_t *planes_from, int split_row, __half *y, int M, bool round_gate_up,
+                  cudaStream_t st);
 
 }  // namespace im

@@ -212,6 +212,7 @@ struct Model : im_model {
            *attn_out = nullptr, *ffn_down = nullptr, *ffn_gate = nullptr, *ffn_up = nullptr, *xs_scratch = nullptr, *logits = nullptr,
            *logits_all = nullptr;
     bool gemm_ok = false;  // every projection is INT4 or INT8 group-128: forwards of 16 tokens and more run the tensor-core GEMM
+    uint8_t *planes[2] = {nullptr, nullptr};  // activations of up to 15 rows as byte planes, unrounded and rounded norms (null: some weight is not tiled for it)
     float *qrot = nullptr;  // [MT, nh_l, 2, hd] rotated queries
     float *scratch_ref = nullptr;
     void *pf_dq = nullptr;          // dequantised K' / V' rows of one sequence for prefill chunks (tq_prefill.cu)
@@ -568,12 +569,59 @@ int Model::forward(int nseq, int T, cudaStream_t st, Prof *prof, bool all_logits
             IM_MARK(kCatResNorm);
         }
     }
+    // The schedule below for up to 15 rows of tiled weights: activations as byte planes written by the kernel in front of each projection, Q | K | V and
+    // gate | up joint (gemm_rows.cu).  The same rounding points.
+    const bool planes = !mega && !gemm && m->planes[0] && MT <= kPlanesMaxRows;
+    for (int l = 0; l < c.num_layers && planes; l++) {
+        Layer &L = m->layers[l];
+        const bool fused4 = L.qkv->bits == 4 && L.gate->bits == 4 && L.up->bits == 4;
+        if (l == 0) {
+            IM_TRY(rows_planes(m->norm_out, L.qkv->awq, m->planes[0], MT, H, st));
+            IM_TRY(matvec_planes(L.qkv, nullptr, m->planes[0], nullptr, 0, m->qkv, MT, false, st));
+            IM_MARK(kCatQkv);
+        }
+        TqPrep a{};
+        a.qkv = m->qkv; a.stride = m->qkv_dim; a.k_off = m->q_dim; a.v_off = m->q_dim + m->kv_dim;
+        a.qw = L.q_norm; a.kw = L.k_norm; a.cosc = m->cosc; a.sinc = m->sinc;
+        a.nh = m->nh_l; a.nkv = m->nkv_l; a.rotary_dim = c.rotary_dim ? c.rotary_dim : hd; a.with_norm = c.qk_norm ? 1 : 0;
+        a.T = T; a.nseq = nseq; a.max_seq = c.max_seq_len; a.base_pos = 0; a.eps = eps; a.pos_dev = m->pos_dev; a.slot_map = slots;
+        a.qrot = m->qrot; a.q_out = nullptr;
+        a.kc = L.kc; a.vc = L.vc; a.ks = L.ks; a.vs = L.vs; a.krn = L.krn;
+        IM_TRY(attention_block(m, 0, a, m->qkv, L, nseq, T, attn_scale, attn_splits, slots, st));
+        IM_MARK(kCatKvWrite);
+        IM_TRY(attention_block(m, 1, a, m->qkv, L, nseq, T, attn_scale, attn_splits, slots, st));
+        IM_MARK(kCatAttn);
+        IM_TRY(rows_planes(m->attn_out, L.o->awq, m->planes[0], MT, m->q_dim, st));
+        IM_TRY(matvec_planes(L.o, nullptr, m->planes[0], nullptr, 0, m->ffn_down, MT, false, st));
+        IM_MARK(kCatOProj);
+        IM_TRY(tp_allreduce(m, m->ffn_down, (size_t)MT * H, st));
+        if (m->world > 1) IM_MARK(kCatComm);
+        IM_TRY(norm_planes(m->hidden, m->ffn_down, L.post_ln, L.gate->awq, m->residual, nullptr, m->planes[0], H, MT, eps, st));
+        IM_MARK(kCatResNorm);
+        IM_TRY(matvec_planes(L.gate, L.up, m->planes[0], nullptr, 0, m->ffn_gate, MT, !fused4, st));
+        IM_MARK(kCatFfn);
+        IM_TRY(rows_planes(m->ffn_gate, L.down->awq, m->planes[0], MT, m->I_l, st));
+        IM_TRY(matvec_planes(L.down, nullptr, m->planes[0], nullptr, 0, m->ffn_down, MT, false, st));
+        IM_MARK(kCatDown);
+        IM_TRY(tp_allreduce(m, m->ffn_down, (size_t)MT * H, st));
+        if (m->world > 1) IM_MARK(kCatComm);
+        if (l + 1 < c.num_layers) {
+            Layer &Nx = m->layers[l + 1];
+            const bool unrounded = Nx.qkv->bits == 4;  // Q's form; K and V read the rounded one
+            IM_TRY(norm_planes(m->residual, m->ffn_down, Nx.input_ln, Nx.qkv->awq, m->hidden, unrounded ? m->planes[0] : nullptr, m->planes[1], H, MT, eps, st));
+            IM_TRY(matvec_planes(Nx.qkv, nullptr, unrounded ? m->planes[0] : m->planes[1], m->planes[1], m->q_dim, m->qkv, MT, false, st));
+            IM_MARK(kCatQkv);
+        } else {
+            IM_TRY(im_cuda_residual_add(m->residual, m->ffn_down, m->hidden, (size_t)MT * H, st));
+            IM_MARK(kCatResNorm);
+        }
+    }
     // Launch-per-kernel schedule with the reference's decode-time rounding points (one token per sequence):
     //   4-bit weights: Q of layers >= 1 comes out of the fused residual + norm + projection kernel (unrounded
     //   normalised vector), K and V read norm_out (metal/attention.rs:616-702); gate/up read norm_out and keep their
     //   f32 dot products for SiLU(g) * u (metal/ffn.rs:25-54).  Other widths have no fused kernels in the reference:
     //   every projection reads the fp16 buffers, gate and up are rounded before the activation (ffn.rs:58-150).
-    for (int l = 0; l < c.num_layers && !mega && !gemm; l++) {
+    for (int l = 0; l < c.num_layers && !mega && !gemm && !planes; l++) {
         Layer &L = m->layers[l];
         const bool fused4 = L.qkv->bits == 4 && L.gate->bits == 4 && L.up->bits == 4;
         if (l == 0) {
@@ -1228,6 +1276,17 @@ int Model::finalize() {
     for (Layer &L : m->layers)
         for (AffineWeight *w : {L.qkv, L.o, L.gate, L.up, L.down})
             if (!w || (w->bits != 4 && w->bits != 8) || w->group_size != 128 || w->K % 128 != 0 || w->N % 8 != 0) m->gemm_ok = false;
+    bool tiled = H % 128 == 0 && H <= 8192 && m->q_dim % 128 == 0;
+    size_t groups = 0;
+    for (Layer &L : m->layers) {
+        tiled = tiled && L.ffn_joint;
+        for (AffineWeight *w : {L.qkv, L.o, L.gate, L.up, L.down}) {
+            tiled = tiled && w && planes_take(w, 1);
+            if (w) groups = std::max(groups, (size_t)w->G);
+        }
+    }
+    for (uint8_t *&b : m->planes)
+        if (tiled) IM_TRY(m->alloc((void **)&b, groups * planes_slab(kPlanesMaxRows)));
     IM_TRY(m->alloc((void **)&m->logits, (size_t)c.max_batch * m->vocab_l * 2));
     if (m->world > 1) IM_TRY(m->alloc((void **)&m->logits_all, (size_t)c.max_batch * c.vocab_size * 2));
     m->logits_dev = m->world > 1 ? m->logits_all : m->logits;

@@ -55,3 +55,28 @@ def test_prompt_in_short_portions(chunk):
         eng.load_weights(DictProvider(cfg, tensors))
         out.append(eng.prefill(tokens).astype(np.float64))
     assert np.linalg.norm(out[1] - out[0]) / np.linalg.norm(out[0]) <= 3.6e-3
+
+
+@pytest.mark.parametrize("bits,awq,batch", [(4, True, 1), (4, True, 2), (4, False, 3), (8, True, 5), (4, True, 9), (8, False, 15)])
+def test_decode_batches_over_planes(bits, awq, batch):
+    """Steps of a few sequences (planes written by the norms, Q | K | V and gate | up joint) against the oracle model of the first ones, at the gate of decode
+    logits: row counts around the two rows of an instruction, both code widths and their rounding points."""
+    from ironmill_b200.engine import CudaConfig, CudaInference
+    from tests.oracle_model import OracleModel
+    cfg = _cfg("llama", 2, 1024, 1152, 8, 4, 300, 1e6, 1e-6)
+    tensors = synth_model(cfg, seed=41, awq=awq, gamma_jitter=0.2, bits=bits)
+    tqc = orc.TqConstants(128, 8, seed=4)
+    eng = CudaInference(CudaConfig(max_seq_len=64, max_batch=max(batch, 2), n_bits=8))
+    eng.load_weights(DictProvider(cfg, tensors), tq_signs=tqc.signs, tq_qjl=tqc.qjl)
+    rng = H.rng_for("planes")
+    prompts = [rng.integers(0, 300, 3 + i % 5).astype(np.uint32) for i in range(batch)]
+    ids = [eng.add_sequence(p) for p in prompts]
+    refs = [OracleModel(cfg, tensors, tqc, 64) for _ in prompts[:3]]
+    for ref, p in zip(refs, prompts):
+        ref.forward(p)
+    for _ in range(3):
+        fed = rng.integers(0, 300, batch)
+        got = eng.batch_decode_step(dict(zip(ids, fed.tolist())))
+        for i, ref in enumerate(refs):
+            want = ref.forward([int(fed[i])])
+            assert float(np.abs(got[i][1] - want).max()) <= 5e-2, (bits, batch, i)
