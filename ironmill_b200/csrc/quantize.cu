@@ -19,125 +19,195 @@ __device__ __forceinline__ float load_weight(const __half *w, const __half *awq,
 }
 
 // ---- one pass over the weights: groups of 8 * L columns, rows a multiple of 8 columns, 16-byte aligned ------------------
-// Bound: HBM (2 bytes in, 0.5 or 1 byte and 8 bytes per group out).  A thread owns the same eight columns of kQRows
-// consecutive rows, so that its loads are in flight together and one index division and one load of the AWQ vector serve
-// them all; the L = group / 8 lanes of a group find its extrema by shuffles and the codes are formed from the values still in
-// registers.  14336 x 4096, 4-bit with AWQ: 406 -> 90 us (1.7 TB/s; issue bounds it: about eight instructions per element).
+// Bound: HBM (2 bytes in, 0.5 or 1 byte and 8 bytes per group out), as long as issue keeps up: at 14336 x 4096 an instruction per element is
+// 1.7 us of a floor of 23.  A lane owns C octets of a group (every P = L / C-th, so that neighbouring lanes read neighbouring octets): the
+// group's scale and zero point - two divisions, and shuffles among P lanes - are worked out for 32 elements at a time.  (Two rows to a lane, so that a
+// vector of AWQ factors serves both: 16 warps an SM instead of 32, 55 us against 47.)  Octets past the end of a row and rows past the last repeat the
+// last one and are not stored.  4-bit with AWQ, 14336 x 4096: 90 us with one octet to a lane (about 27 instructions per element) -> 52 (about 17; issue slots 57 % busy).
 //
 // Codes without a division per element: t = x * (1 / scale) + zp differs from the defining fl(fl(x / scale) + zp) by less
-// than 2^-20 (|x / scale| + |zp| + 1), so the two round to the same integer unless t lies that close to a half; a thread
-// that meets such a value (or a non-finite one, or a magnitude past 2^21) recomputes its eight by the definition.
-constexpr int kQRows = 4;
+// than 2^-20 (|x / scale| + |zp| + 1), so the two round to the same integer unless t lies that close to a half; an octet
+// with such a value (or a magnitude past 2^21) is recomputed by the definition.  An octet without one needs no clamp: x lies between the group's
+// extrema, so t is at most a half outside 0 .. qmax, give or take that error.  Groups with a value that is not finite, or whose minimum is a zero
+// (of equal extrema the first counts, and the sign of a zero shows in the zero point), take quantize_row_any.
 
 __device__ __forceinline__ unsigned quantize_one(float x, float scale, float zp, float qmax);
 
+__device__ __forceinline__ float min3(float a, float b, float c) {  // NaN if one of them is
+    float d;
+    asm("min.NaN.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+    return d;
+}
+__device__ __forceinline__ float max3(float a, float b, float c) {
+    float d;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+    return d;
+}
+// Weight times AWQ factor: a product of two fp16 values is exact in f32.
+template <bool AWQ>
+__device__ __forceinline__ void quantize_values(const uint4 w, const uint4 a, float (&x)[8]) {
+    const unsigned u[4] = {w.x, w.y, w.z, w.w}, v[4] = {a.x, a.y, a.z, a.w};
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+        const float2 f = __half22float2(*reinterpret_cast<const __half2 *>(&u[j]));
+        x[2 * j] = f.x;
+        x[2 * j + 1] = f.y;
+        if (AWQ) {
+            const float2 g = __half22float2(*reinterpret_cast<const __half2 *>(&v[j]));
+            x[2 * j] = __fmul_rn(f.x, g.x);
+            x[2 * j + 1] = __fmul_rn(f.y, g.y);
+        }
+    }
+}
+__device__ __forceinline__ void quantize_scale(float mn, float mx, bool finite, float qmax, float &scale, float &zp) {
+    if (!finite) {  // no finite value in the group
+        scale = 1.0f;
+        zp = 0.0f;
+    } else if (fabsf(__fsub_rn(mx, mn)) < FLT_EPSILON) {
+        scale = 1.0f;
+        zp = roundf(-mn);
+    } else {
+        scale = __fdiv_rn(__fsub_rn(mx, mn), qmax);
+        zp = roundf(__fdiv_rn(-mn, scale));
+    }
+}
 template <int BITS>
-__global__ void __launch_bounds__(256) quantize_groups_kernel(const __half *__restrict__ w, const __half *__restrict__ awq, size_t rows, unsigned K, int L,
-                                                              unsigned G, float *__restrict__ scales, float *__restrict__ zps, uint8_t *__restrict__ packed) {
+__device__ __forceinline__ void store_codes(uint8_t *packed, size_t octet, const float (&c)[8]) {
+    if (BITS == 4) {
+        // four codes in one exact f32 sum, the lower column in the lower nibble
+        const float lo = fmaf(fmaf(fmaf(c[3], 16.0f, c[2]), 16.0f, c[1]), 16.0f, c[0]), hi = fmaf(fmaf(fmaf(c[7], 16.0f, c[6]), 16.0f, c[5]), 16.0f, c[4]);
+        reinterpret_cast<unsigned *>(packed)[octet] = __byte_perm(__float_as_uint(lo + 8388608.0f), __float_as_uint(hi + 8388608.0f), 0x5410);
+    } else {
+        const float s0 = fmaf(c[1], 256.0f, c[0]) + 8388608.0f, s1 = fmaf(c[3], 256.0f, c[2]) + 8388608.0f, s2 = fmaf(c[5], 256.0f, c[4]) + 8388608.0f,
+                    s3 = fmaf(c[7], 256.0f, c[6]) + 8388608.0f;
+        reinterpret_cast<uint2 *>(packed)[octet] = make_uint2(__byte_perm(__float_as_uint(s0), __float_as_uint(s1), 0x5410), __byte_perm(__float_as_uint(s2), __float_as_uint(s3), 0x5410));
+    }
+}
+
+// A row's share of a lane by the definition, whatever its values: all lanes of the warp.  octets: where the lane's octets lie, dead ones negative.
+template <int BITS, int C, bool AWQ>
+__device__ __noinline__ void quantize_row_any(const uint4 (&w)[C], const uint4 (&a)[C], int lane_of_group, int P, int live, size_t octet0, bool store, float *scale_out,
+                                              float *zp_out, uint8_t *packed) {
+    constexpr float qmax = BITS == 4 ? 15.0f : 255.0f;
+    float mn = INFINITY, mx = -INFINITY;
+    unsigned imn = 0xffffffffu, imx = 0xffffffffu;
+#pragma unroll
+    for (int i = 0; i < C; i++) {
+        float x[8];
+        quantize_values<AWQ>(w[i], a[i], x);
+        const unsigned at = (unsigned)(lane_of_group + i * P) * 8;
+        for (int j = 0; j < 8; j++)
+            if (isfinite(x[j])) {
+                if (x[j] < mn) { mn = x[j]; imn = at + j; }
+                if (x[j] > mx) { mx = x[j]; imx = at + j; }
+            }
+    }
+    for (int o = P >> 1; o > 0; o >>= 1) {
+        const float omn = __shfl_xor_sync(0xffffffffu, mn, o), omx = __shfl_xor_sync(0xffffffffu, mx, o);
+        const unsigned oimn = __shfl_xor_sync(0xffffffffu, imn, o), oimx = __shfl_xor_sync(0xffffffffu, imx, o);
+        if (omn < mn || (omn == mn && oimn < imn)) { mn = omn; imn = oimn; }
+        if (omx > mx || (omx == mx && oimx < imx)) { mx = omx; imx = oimx; }
+    }
+    const bool finite = isfinite(mn) && isfinite(mx);
+    float scale, zp;
+    quantize_scale(mn, mx, finite, qmax, scale, zp);
+    if (!store) return;
+    if (lane_of_group == 0) {
+        *scale_out = scale;
+        *zp_out = zp;
+    }
+#pragma unroll
+    for (int i = 0; i < C; i++) {
+        float x[8], c[8];
+        quantize_values<AWQ>(w[i], a[i], x);
+        for (int j = 0; j < 8; j++) c[j] = finite ? (float)quantize_one(x[j], scale, zp, qmax) : 0.0f;
+        if (i < live) store_codes<BITS>(packed, octet0 + i * P, c);
+    }
+}
+
+template <int BITS, int C, bool AWQ>
+__global__ void __launch_bounds__(256, C == 8 ? 2 : 4) quantize_groups_kernel(const __half *__restrict__ w, const __half *__restrict__ awq, size_t rows, unsigned K, int P,
+                                                                              unsigned G, float *__restrict__ scales, float *__restrict__ zps, uint8_t *__restrict__ packed) {
     constexpr float qmax = BITS == 4 ? 15.0f : 255.0f;
     constexpr float kMagic = 12582912.0f;  // 1.5 * 2^23: adding it rounds to an integer in the low mantissa bits
-    const unsigned per_row = G * (unsigned)L;  // octets of a row, the short last group padded
-    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const size_t rb = (i >> 32) == 0 ? (unsigned)i / per_row : i / per_row;
-    const unsigned o = (unsigned)(i - rb * per_row), g = o >> (__ffs(L) - 1), col = o * 8;
-    const size_t r0 = rb * kQRows;
-    const int lane = threadIdx.x & 31;
-    const unsigned seg = (L == 32 ? 0xffffffffu : ((1u << L) - 1u)) << (lane & ~(L - 1));  // the lanes of this group
-    const bool in_row = col < K;  // a group is 8 L columns and K a multiple of 8: an octet is inside or outside
-    float a[8];
+    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x, at = i >> (__ffs(P) - 1);  // the group's number
+    const size_t row = (at >> 32) == 0 ? (unsigned)at / G : at / G;
+    const unsigned g = (unsigned)(at - row * G), p = (unsigned)i & (unsigned)(P - 1);
+    const bool store = row < rows;
+    const unsigned octets = K / 8, o0 = g * (unsigned)(P * C) + p;  // this lane's octets of the row: o0, o0 + P, ...
+    const int live = o0 >= octets ? 0 : min(C, (int)((octets - 1 - o0) / (unsigned)P) + 1);
+    const uint4 *src = reinterpret_cast<const uint4 *>(w) + min(row, rows - 1) * octets;
+    const size_t octet0 = row * octets + o0;
+    uint4 a[C], raw[C];
 #pragma unroll
-    for (int j = 0; j < 8; j++) a[j] = 1.0f;
-    unsigned bad_awq = 0;
-    if (awq && in_row) {
-        const uint4 v = *reinterpret_cast<const uint4 *>(awq + col);
-        const unsigned u[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-        for (int j = 0; j < 4; j++) {
-            const float2 f = __half22float2(*reinterpret_cast<const __half2 *>(&u[j]));
-            a[2 * j] = f.x;
-            a[2 * j + 1] = f.y;
-            bad_awq |= ((u[j] & 0x7fff7fffu) + 0x04000400u) & 0x80008000u;  // an exponent of all ones
-        }
+    for (int c = 0; c < C; c++) {
+        raw[c] = ldg_stream_v4(src + min(o0 + c * (unsigned)P, octets - 1));
+        a[c] = make_uint4(0, 0, 0, 0);
+        if (AWQ) a[c] = __ldg(reinterpret_cast<const uint4 *>(awq) + min(o0 + c * (unsigned)P, octets - 1));
     }
-    uint4 raw[kQRows];
+    float mn = INFINITY, mx = -INFINITY;  // NaN or infinite with a value that is not finite
 #pragma unroll
-    for (int r = 0; r < kQRows; r++) {
-        raw[r] = make_uint4(0, 0, 0, 0);
-        if (in_row && r0 + r < rows) raw[r] = ldg_stream_v4(w + (r0 + r) * K + col);
-    }
-#pragma unroll
-    for (int r = 0; r < kQRows; r++) {
-        const bool live = in_row && r0 + r < rows;
-        const unsigned u[4] = {raw[r].x, raw[r].y, raw[r].z, raw[r].w};
+    for (int c = 0; c < C; c++) {
         float x[8];
-        unsigned bad = bad_awq;
+        quantize_values<AWQ>(raw[c], a[c], x);
 #pragma unroll
-        for (int j = 0; j < 4; j++) {
-            const float2 f = __half22float2(*reinterpret_cast<const __half2 *>(&u[j]));
-            x[2 * j] = awq ? __fmul_rn(f.x, a[2 * j]) : f.x;
-            x[2 * j + 1] = awq ? __fmul_rn(f.y, a[2 * j + 1]) : f.y;
-            bad |= ((u[j] & 0x7fff7fffu) + 0x04000400u) & 0x80008000u;
-        }
-        // extrema of the finite values; of equal extrema the first counts (the sign of a zero can tell them apart)
-        float mn = INFINITY, mx = -INFINITY;
-        if (live) {
-#pragma unroll
-            for (int j = 0; j < 8; j++)
-                if (!bad || isfinite(x[j])) {
-                    if (x[j] < mn) mn = x[j];
-                    if (x[j] > mx) mx = x[j];
-                }
-        }
-        float gmn = mn, gmx = mx;
-        for (int d = L >> 1; d > 0; d >>= 1) {
-            gmn = fminf(gmn, __shfl_xor_sync(0xffffffffu, gmn, d));
-            gmx = fmaxf(gmx, __shfl_xor_sync(0xffffffffu, gmx, d));
-        }
-        const unsigned at_mn = __ballot_sync(0xffffffffu, mn == gmn) & seg, at_mx = __ballot_sync(0xffffffffu, mx == gmx) & seg;
-        mn = __shfl_sync(0xffffffffu, mn, __ffs(at_mn) - 1);
-        mx = __shfl_sync(0xffffffffu, mx, __ffs(at_mx) - 1);
-        float scale, zp;
-        const bool finite = isfinite(mn) && isfinite(mx);  // false: no finite value in the group
-        if (!finite) {
-            scale = 1.0f;
-            zp = 0.0f;
-        } else if (fabsf(__fsub_rn(mx, mn)) < FLT_EPSILON) {
-            scale = 1.0f;
-            zp = roundf(-mn);
-        } else {
-            scale = __fdiv_rn(__fsub_rn(mx, mn), qmax);
-            zp = roundf(__fdiv_rn(-mn, scale));
-        }
-        if (!live) continue;
-        if ((o & (unsigned)(L - 1)) == 0) {
-            scales[(r0 + r) * G + g] = scale;
-            zps[(r0 + r) * G + g] = zp;
-        }
-        const float inv = __fdividef(1.0f, scale);
-        // t is within [mn, mx] / scale + zp; the largest magnitude on the way bounds the rounding of both forms
-        const float mag = fmaxf(fabsf(mn), fabsf(mx)) * inv + fabsf(zp) + 1.0f;
-        const float near_half = 0.5f - mag * 0x1p-20f;
-        float c[8], far = 0.0f;
-#pragma unroll
-        for (int j = 0; j < 8; j++) {
-            const float t = fmaf(x[j], inv, zp), rr = __fsub_rn(__fadd_rn(t, kMagic), kMagic);
-            far = fmaxf(far, fabsf(t - rr));
-            c[j] = fminf(fmaxf(rr, 0.0f), qmax);
-        }
-        if (bad || !finite || !(far < near_half) || !(mag < 2097152.0f)) {
-#pragma unroll
-            for (int j = 0; j < 8; j++) c[j] = finite ? (float)quantize_one(x[j], scale, zp, qmax) : 0.0f;
-        }
-        if (BITS == 4) {
-            // four codes in one exact f32 sum, the lower column in the lower nibble
-            const float lo = fmaf(fmaf(fmaf(c[3], 16.0f, c[2]), 16.0f, c[1]), 16.0f, c[0]), hi = fmaf(fmaf(fmaf(c[7], 16.0f, c[6]), 16.0f, c[5]), 16.0f, c[4]);
-            reinterpret_cast<unsigned *>(packed)[((r0 + r) * K + col) >> 3] = (unsigned)lo | ((unsigned)hi << 16);
-        } else {
-            const float lo = fmaf(c[1], 256.0f, c[0]), lo2 = fmaf(c[3], 256.0f, c[2]), hi = fmaf(c[5], 256.0f, c[4]), hi2 = fmaf(c[7], 256.0f, c[6]);
-            reinterpret_cast<uint2 *>(packed)[((r0 + r) * K + col) >> 3] =
-                make_uint2((unsigned)lo | ((unsigned)lo2 << 16), (unsigned)hi | ((unsigned)hi2 << 16));
+        for (int j = 0; j < 8; j += 2) {
+            mn = min3(mn, x[j], x[j + 1]);
+            mx = max3(mx, x[j], x[j + 1]);
         }
     }
+    for (int o = P >> 1; o > 0; o >>= 1) {
+        mn = min3(mn, mn, __shfl_xor_sync(0xffffffffu, mn, o));
+        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    }
+    if (__any_sync(0xffffffffu, !isfinite(mn) || !isfinite(mx) || mn == 0.0f)) {
+        quantize_row_any<BITS, C, AWQ>(raw, a, (int)p, P, live, octet0, store, scales + at, zps + at, packed);
+        return;
+    }
+    float scale, zp;
+    quantize_scale(mn, mx, true, qmax, scale, zp);
+    if (!store) return;
+    if (p == 0) {
+        scales[at] = scale;
+        zps[at] = zp;
+    }
+    const float inv = __fdividef(1.0f, scale);
+    // t is within [mn, mx] / scale + zp; the largest magnitude on the way bounds the rounding of both forms
+    const float mag = fmaxf(fabsf(mn), fabsf(mx)) * inv + fabsf(zp) + 1.0f;
+    const float near_half = mag < 2097152.0f ? 0.5f - mag * 0x1p-20f : 0.0f;
+#pragma unroll
+    for (int c = 0; c < C; c++) {
+        float x[8], q[8], far = 0.0f;
+        quantize_values<AWQ>(raw[c], a[c], x);
+#pragma unroll
+        for (int j = 0; j < 8; j += 2) {
+            const float t0 = fmaf(x[j], inv, zp), t1 = fmaf(x[j + 1], inv, zp);
+            q[j] = __fsub_rn(__fadd_rn(t0, kMagic), kMagic);
+            q[j + 1] = __fsub_rn(__fadd_rn(t1, kMagic), kMagic);
+            far = max3(far, fabsf(t0 - q[j]), fabsf(t1 - q[j + 1]));
+        }
+        if (!(far < near_half)) {
+#pragma unroll
+            for (int j = 0; j < 8; j++) q[j] = (float)quantize_one(x[j], scale, zp, qmax);
+        }
+        if (c < live) store_codes<BITS>(packed, octet0 + c * (unsigned)P, q);
+    }
+}
+
+template <int BITS, int C>
+static int quantize_groups(const __half *w, const __half *awq, size_t rows, size_t K, int P, size_t G, float *scales, float *zps, uint8_t *packed, cudaStream_t st) {
+    const size_t blocks = (rows * G * P + 255) / 256;
+    if (blocks > 0x7fffffff) return IM_ERR_BOUNDS;
+    if (awq) quantize_groups_kernel<BITS, C, true><<<(unsigned)blocks, 256, 0, st>>>(w, awq, rows, (unsigned)K, P, (unsigned)G, scales, zps, packed);
+    else quantize_groups_kernel<BITS, C, false><<<(unsigned)blocks, 256, 0, st>>>(w, awq, rows, (unsigned)K, P, (unsigned)G, scales, zps, packed);
+    IM_CUDA_CHECK(cudaGetLastError());
+    return IM_OK;
+}
+template <int BITS>
+static int quantize_groups(const __half *w, const __half *awq, size_t rows, size_t K, int L, size_t G, float *scales, float *zps, uint8_t *packed, cudaStream_t st) {
+    if (L >= 4) return quantize_groups<BITS, 4>(w, awq, rows, K, L / 4, G, scales, zps, packed, st);
+    if (L == 2) return quantize_groups<BITS, 2>(w, awq, rows, K, 1, G, scales, zps, packed, st);
+    return quantize_groups<BITS, 1>(w, awq, rows, K, 1, G, scales, zps, packed, st);
 }
 
 // ---- any other shape: parameters first, then the codes -------------------------------------------------------------------
@@ -270,17 +340,10 @@ IM_EXPORT int im_cuda_quantize_affine(const void *w_dev, const void *awq_dev, si
     const int L = group_size / 8;
     if (group_size % 8 == 0 && L <= 32 && (L & (L - 1)) == 0 && K % 8 == 0 && K < ((size_t)1 << 31) && reinterpret_cast<uintptr_t>(w_dev) % 16 == 0 &&
         reinterpret_cast<uintptr_t>(awq_dev) % 16 == 0 && reinterpret_cast<uintptr_t>(packed_dev) % (bit_width == 4 ? 4 : 8) == 0) {
-        const size_t threads = (rows + im::kQRows - 1) / im::kQRows * G * L, blocks = (threads + 255) / 256;
-        if (blocks <= 0x7fffffff) {
-            if (bit_width == 4)
-                im::quantize_groups_kernel<4><<<(unsigned)blocks, 256, 0, st>>>(w, awq, rows, (unsigned)K, L, (unsigned)G, scales_dev, zps_dev,
-                                                                               static_cast<uint8_t *>(packed_dev));
-            else
-                im::quantize_groups_kernel<8><<<(unsigned)blocks, 256, 0, st>>>(w, awq, rows, (unsigned)K, L, (unsigned)G, scales_dev, zps_dev,
-                                                                               static_cast<uint8_t *>(packed_dev));
-            IM_CUDA_CHECK(cudaGetLastError());
-            return IM_OK;
-        }
+        uint8_t *packed = static_cast<uint8_t *>(packed_dev);
+        const int rc = bit_width == 4 ? im::quantize_groups<4>(w, awq, rows, K, L, G, scales_dev, zps_dev, packed, st)
+                                      : im::quantize_groups<8>(w, awq, rows, K, L, G, scales_dev, zps_dev, packed, st);
+        if (rc != IM_ERR_BOUNDS) return rc;
     }
     size_t ngroups = rows * G;
     const int warps_per_block = 8;

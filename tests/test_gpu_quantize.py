@@ -120,3 +120,26 @@ def test_full_size_property_dequant_error_bound():
     err = (deq - w.float().reshape(28672, 32, 128)).abs()
     assert bool((err <= s[..., None] * 0.5001 + 1e-7).all())
     assert int(q.max()) <= 15 and int(q.min()) >= 0
+
+
+@pytest.mark.parametrize("gs", [8, 16, 32, 64, 128, 256])
+@pytest.mark.parametrize("bits", [4, 8])
+def test_lanes_of_a_group(gs, bits):
+    # one to eight lanes to a group, one to four octets a lane, a short last group, the last block partly empty; groups whose minimum is a zero of
+    # either sign (the first one counts), equal values, values half way between two codes, and rows that are not finite beside ordinary ones
+    rng = H.rng_for("lanes", gs + bits)
+    K = 3 * gs + 8 if gs > 8 else 40
+    w = (rng.standard_normal((37, K)) * 0.02).astype(np.float16)
+    w[1] = np.abs(w[1])
+    w[1, ::5], w[1, 2::5] = 0.0, -0.0
+    w[2] = np.abs(w[2])
+    w[2, 1::4], w[2, 3::4] = -0.0, 0.0
+    w[3] = 0.125
+    w[4] = (np.arange(K) % 31 * 0.5).astype(np.float16)   # scale 1 at 4 bits: halves
+    w[5, 7] = np.inf
+    w[6, K - 1] = np.nan
+    w[7] = np.nan
+    w[8] = -np.abs(w[8])
+    w[8, 4] = 0.0
+    for awq in (None, (rng.random(K) * 1.5 + 0.5).astype(np.float16)):
+        _check(w, gs, bits, awq)
