@@ -163,7 +163,7 @@ __device__ __forceinline__ bool weight_warps(const PairGemm &p, unsigned char *A
     if (total > 0) point();
 #pragma unroll
     for (int u = 0; u < kAhead; u++) request(u);
-    const uint32_t full0 = leader_addr(full);
+    const uint32_t full0 = leader_addr(full), e = half_exponent();
     auto hand_over = [&](int stage) {
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // generic-proxy writes -> visible to the tensor cores
         __syncwarp();
@@ -189,13 +189,13 @@ __device__ __forceinline__ bool weight_warps(const PairGemm &p, unsigned char *A
                     const uint4 a = swap ? cw[kVec - 1] : cw[0], b = swap ? cw[0] : cw[kVec - 1];
                     in[0] = make_uint2(a.x, a.y); in[1] = make_uint2(a.z, a.w); in[2] = make_uint2(b.x, b.y); in[3] = make_uint2(b.z, b.w);
                 }
-                const float zf = __high2float(sz), sf = __low2float(sz);
+                const GroupScale gs = BITS == 4 ? group_scale(sz) : group_scale_f32(sz);
                 uint4 v[4];
-                if (__builtin_expect(zf == rintf(zf) && zf >= -1024.0f && zf <= 1023.0f, 1)) {
-                    const __half2 c2 = __float2half2_rn(1024.0f + zf), s2 = __half2half2(__low2half(sz));
+                if (__builtin_expect(gs.plain, 1)) {
 #pragma unroll
-                    for (int i = 0; i < 4; i++) v[i] = BITS == 4 ? dequant8_fast(in[i].x, c2, s2) : dequant8b_fast(in[i].x, in[i].y, c2, s2);
+                    for (int i = 0; i < 4; i++) v[i] = BITS == 4 ? dequant8_fast(in[i].x, gs, e) : dequant8b_fast(in[i].x, in[i].y, gs);
                 } else {
+                    const float zf = __high2float(sz), sf = __low2float(sz);
 #pragma unroll
                     for (int i = 0; i < 4; i++) v[i] = BITS == 4 ? dequant8_slow(in[i].x, zf, sf) : dequant8b_slow(in[i].x, in[i].y, zf, sf);
                 }
@@ -254,7 +254,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PairShape<TN, BITS>:
         if constexpr (BITS != 0) ok = weight_warps<TN, BITS>(p, As, full, empty, rank, pair, npairs);
     } else if (warp == kCopyWarp) {
         if (lane == 0) {
-            const uint32_t full0 = leader_addr(full);
+            const uint32_t full0 = leader_addr(full), e = half_exponent();
             int s = 0, use = 0;
             for (int w = pair; w < tiles; w += npairs) {
                 const int m0 = w % p.mtiles * TN + rank * (TN / 2), n0 = w / p.mtiles * (2 * kPRows) + rank * kPRows;

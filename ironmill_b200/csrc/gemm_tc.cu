@@ -145,6 +145,7 @@ __device__ __forceinline__ void gemm_weight_warps(const GemmParams &p, unsigned 
         __syncwarp();
         if (lane == 0) mbar_arrive(&full[stage]);
     };
+    const uint32_t e = half_exponent();
     int s = 0, use = 0, prev = 0;  // ring slot, how often it has been used, the slot before
     for (int kt0 = 0; kt0 < G; kt0 += kAheadA) {
 #pragma unroll
@@ -166,18 +167,17 @@ __device__ __forceinline__ void gemm_weight_warps(const GemmParams &p, unsigned 
                     szb[u] = szrow[kt + kAheadA];
                 }
                 // convert into registers first: only the eight stores wait for the slot to be free
-                const float zf = __high2float(szc), sf = __low2float(szc);
-                const bool fast = zf == rintf(zf) && zf >= -1024.0f && zf <= 1023.0f;
+                const GroupScale gs = group_scale(szc);
                 uint4 v0, v1, v2, v3;
                 // Two real branches (not a select): the f32 path costs three times the packed one and almost no group
                 // needs it.  Rows past N carry zero codes and a zero scale, which dequantise to zero.
-                if (__builtin_expect(fast, 1)) {
-                    const __half2 c2 = __float2half2_rn(1024.0f + zf), s2 = __half2half2(__low2half(szc));
+                const float zf = __high2float(szc), sf = __low2float(szc);
+                if (__builtin_expect(gs.plain, 1)) {
                     if (BITS == 4) {
-                        v0 = dequant8_fast(cw[0].x, c2, s2); v1 = dequant8_fast(cw[0].y, c2, s2); v2 = dequant8_fast(cw[0].z, c2, s2); v3 = dequant8_fast(cw[0].w, c2, s2);
+                        v0 = dequant8_fast(cw[0].x, gs, e); v1 = dequant8_fast(cw[0].y, gs, e); v2 = dequant8_fast(cw[0].z, gs, e); v3 = dequant8_fast(cw[0].w, gs, e);
                     } else {
-                        v0 = dequant8b_fast(cw[0].x, cw[0].y, c2, s2); v1 = dequant8b_fast(cw[0].z, cw[0].w, c2, s2);
-                        v2 = dequant8b_fast(cw[kCodeVec - 1].x, cw[kCodeVec - 1].y, c2, s2); v3 = dequant8b_fast(cw[kCodeVec - 1].z, cw[kCodeVec - 1].w, c2, s2);
+                        v0 = dequant8b_fast(cw[0].x, cw[0].y, gs); v1 = dequant8b_fast(cw[0].z, cw[0].w, gs);
+                        v2 = dequant8b_fast(cw[kCodeVec - 1].x, cw[kCodeVec - 1].y, gs); v3 = dequant8b_fast(cw[kCodeVec - 1].z, cw[kCodeVec - 1].w, gs);
                     }
                 } else if (BITS == 4) {
                     v0 = dequant8_slow(cw[0].x, zf, sf); v1 = dequant8_slow(cw[0].y, zf, sf); v2 = dequant8_slow(cw[0].z, zf, sf); v3 = dequant8_slow(cw[0].w, zf, sf);
