@@ -437,10 +437,10 @@ int gemm_affine_tc(const AffineWeight *w, const __half *x, __half *y, int M, __h
     if (const int rc = scaled_tokens(w, x, M, xs_scratch, form != kTokensRaw, st, &xs); rc != IM_OK) return rc;
     if (pair_gemm_takes(w->dev, w->N, M)) return pair_gemm_affine(w, nullptr, xs, y, M, st);
     GemmParams p{w->codes, w->sz, xs, y, w->N, w->K, w->G, M, w->dev->err_flag, nullptr, w->G};
-    // Few tokens and few row tiles (decode batches of 16-64 against 4096-6144 rows: 32-48 CTAs of 32-112 sequential
-    // stages): split K so that the grid covers the GPU.  At least four groups per slice; the slices' f32 sums go through
+    // One token tile and few row tiles (4096-6144 rows: 32-48 CTAs of 32-112 sequential stages): split K so that the grid covers the GPU.  100 tokens over
+    // 4096 x 14336: 97 -> 35 us, over 6144 x 4096 32 -> 19.  More tokens are more tiles, or CTA pairs.  At least four groups per slice; the slices' f32 sums go through
     // the device handle's scratch (one GEMM in flight per handle, like the tiled matvec).
-    if (M <= 64 && w->N % 4 == 0 && reinterpret_cast<uintptr_t>(y) % 8 == 0 && w->dev->gemm_partial) {
+    if (M <= 128 && w->N % 4 == 0 && reinterpret_cast<uintptr_t>(y) % 8 == 0 && w->dev->gemm_partial) {
         const int tiles = (w->N + kGM - 1) / kGM;
         int splits = std::min(w->dev->sm_count / tiles, w->G / 4);
         while (splits > 1 && (size_t)splits * M * w->N * sizeof(float) > kGemmPartialBytes) splits--;

@@ -38,6 +38,17 @@ def test_few_tokens(dev, N, K, M, bits):
         assert H.rel_err(y, ref) <= TOL, (N, K, M)
 
 
+@pytest.mark.parametrize("N,K,M", [(512, 2048, 65), (384, 1792, 128), (260, 14336, 100), (6144, 1024, 97)])
+def test_one_token_tile_over_slices_of_k(dev, N, K, M):
+    # the tcgen05 kernel's full token tile with K cut along the grid: ragged rows, an uneven last slice, both ends of the token range
+    from ironmill_b200 import ops
+    qw = H.QWeight(N, K, awq=True, seed=N + M, name="gs")
+    x = (H.rng_for("gs-x", M).standard_normal((M, K))).astype(np.float16)
+    y = ops.matmul_affine(qw.gpu(dev), torch.from_numpy(x).cuda()).cpu().numpy()
+    ref = orc.matmul_affine(qw.packed, qw.scales_f16, qw.zps_f16, x, N, K, 128, 4, awq=qw.awq, threads=8)
+    assert H.rel_err(y, ref) <= TOL, (N, K, M)
+
+
 @pytest.mark.parametrize("chunk", [9, 24, 33])
 def test_prompt_in_short_portions(chunk):
     """Portions of few tokens (packed norms, joint gate and up, packed activation) against the whole prompt at once (the kernels of many tokens):
