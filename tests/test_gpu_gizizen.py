@@ -93,6 +93,28 @@ def test_portions_of_every_size(dtype):
         e.remove_sequence(sid)
 
 
+@pytest.mark.parametrize("rank,dim,vdim", [(128, 16, 32), (256, 48, 64), (512, 128, 128), (1024, 32, 96)])
+def test_absorbed_portions_of_whole_tiles(rank, dim, vdim):
+    """The tensor-core forms of absorbing queries and of W_uv (every column count they are built for): portions around the sixteen tokens of a tile, one split and
+    several, then a batch of sequences of different lengths."""
+    cfg = G.config([G.latent(heads=3, dim=dim, rot_dim=16, vdim=vdim, kv_rank=rank, ff=0)], width=96, vocab=90)
+    w = G.weights(cfg, 15)
+    toks = tokens(260, 90)
+    want = OracleGizizen(cfg, w).forward(toks)
+    e = engine(cfg, w, "bfloat16", max_seq_len=280, max_batch=6)
+    sid, at, rows = e.open_sequence(), 0, []
+    for n in (4, 15, 16, 17, 33, 48, 5, 122):
+        rows.append(e.extend_sequence(sid, toks[at:at + n], range(n)))
+        at += n
+    assert G.error(np.concatenate(rows), want) < G.TOL["bfloat16"]
+    e.remove_sequence(sid)
+    lengths = (3, 40, 17, 90, 200, 64)
+    ids = [e.add_sequence(toks[:n]) for n in lengths]
+    for k in range(3):
+        got = dict(e.batch_decode_step({i: int(toks[n + k]) for i, n in zip(ids, lengths)}))
+        assert G.error(np.stack([got[i] for i in ids]), np.stack([want[n + k] for n in lengths])) < G.TOL["bfloat16"]
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 def test_long_prompts_in_internal_chunks(dtype):
     """The engine's own chunk size must not show; only some places are asked for."""
