@@ -228,7 +228,10 @@ struct AttnParams {
     const int *slot_map;     // optional: sequence index of this launch -> cache slot (nullptr: identity)
     int bits;                // cache bits per element (8 or 4); rows hold tq_row_bytes(bits, hd) bytes
     int own_parts;           // `splits` is the most that a token may use: its context is cut into parts of at least one run of tiles
+    int shares;              // number of tokens whose contexts tq_attention_tc_kernel deals out as equal shares (0: item by item)
 };
+constexpr int kTcShareTiles = 16;    // least tiles of a share
+constexpr int kTcShareTokens = 64;  // most (sequence, token) pairs whose contexts are dealt out as equal shares
 constexpr int kTcWarps = 6, kTcRun = kTcWarps * kTile;  // a run: a tile for each warp of tq_attention_tc_kernel
 // Positions that token st (sequence-major) of a launch sees and positions of a part of them (whole tiles). Part i is there if i chunk < len; of the
 // rest of `splits` only the maximum is written, minus infinity (100 positions in a cache of 65536 cut into 113 parts took 32 us, 25 in one).

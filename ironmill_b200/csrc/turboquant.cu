@@ -184,8 +184,11 @@ __global__ void __launch_bounds__(kHd) tq_reduce_kernel(const AttnParams p, __ha
 //     [16 positions x 8 heads].  The fragment <-> (dimension, position) assignment is chosen so that a fragment
 //     register is built from bytes the lane already holds.
 // The six warps of a CTA (two CTAs per SM: 168 registers a thread, for a tile's V rows and the next tile's K rows in flight) take the tiles of one (KV head, token, split) in turn and merge their results in shared
-// memory, so the number of partials per head is the same as with the kernel above.  Two CTAs per SM walk all (KV head, token, split) items
-// with one table.  mma.sync issue bounds it (48 products per tile, one per 32 clocks and SM quarter).  16 sequences of 1024 .. 8192
+// memory, so the number of partials per head is the same as with the kernel above.  Two CTAs per SM with one table each.  With an automatic split count
+// and up to 64 contexts, each takes an equal run of the list of all their tiles: dealt out as (KV head, token, split) items, whose sizes follow their
+// contexts', SMs idled 18 % of the time and an item's start and merge came four times a CTA (16 sequences of 1024 .. 8192 positions, the whole call:
+// 86.9 -> 76.7 us, 4-bit 76.5 -> 62; two of 7500 .. 60000: 109 -> 89).  Shares of less than
+// 16 tiles: items, each of which fits one context (tq_shares).  mma.sync issue bounds it (48 products per tile, one per 32 clocks and SM quarter).  16 sequences of 1024 .. 8192
 // positions, 32 / 8 heads: 166 us with eight warps, rows loaded where they were used and a CTA per item of one
 // split; 126 us with this form and one split, 83 us with parts for every SM.
 __device__ __forceinline__ void mma_f16(float (&c)[4], unsigned a0, unsigned a1, unsigned a2, unsigned a3, unsigned b0, unsigned b1) {
@@ -234,15 +237,85 @@ __global__ void __launch_bounds__(kTcWarps * 32, 2) tq_attention_tc_kernel(const
     const unsigned sel0 = g < 4 ? 0x4410u : 0x1044u, sel1 = g < 4 ? 0x4432u : 0x3244u;
     __half *pwarp = pw + warp * 4 * 32;
 
-    for (int item = blockIdx.x; item < items; item += gridDim.x) {
-        const int kvh = item % p.nkv, rest = item / p.nkv, split = rest % p.splits, st = rest / p.splits;
-        const int slot = cache_slot(p.slot_map, st / p.T);
-        const TqSpan span = tq_span(p, st, slot);
-        if (split * span.chunk >= span.len) {  // (the whole CTA)
-            if (tid < GQ) p.pm[((size_t)st * p.nh + kvh * GQ + tid) * p.splits + split] = -INFINITY;
-            continue;
+    // Shares (p.shares): the tiles of all (token, KV head) contexts in one list, an equal run of it per CTA; a context's parts are the CTAs
+    // that its tiles fall to.  So few CTAs that no context has more than p.splits of them.
+    __shared__ int before[kTcShareTokens + 1], plan[4];  // tiles x KV heads of the tokens in front; where this CTA's run ends and goes on, all tiles, CTAs
+    bool flat = false;                                   // (in shared memory: the registers are the tiles')
+    if (p.shares) {
+        if (warp == 0) {
+            int v[2], sum = 0, most = 0;
+#pragma unroll
+            for (int i = 0; i < 2; i++) {
+                const int st = 2 * lane + i;
+                const int tiles = st < p.shares ? (tq_span(p, st, cache_slot(p.slot_map, st / p.T)).len + kTile - 1) / kTile : 0;
+                v[i] = tiles * p.nkv;
+                sum += v[i];
+                most = max(most, tiles);
+            }
+            int upto = sum;
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1) {
+                const int o = __shfl_up_sync(0xffffffffu, upto, d);
+                if (lane >= d) upto += o;
+            }
+            before[2 * lane] = upto - sum;
+            before[2 * lane + 1] = upto - sum + v[0];
+            const int all = __shfl_sync(0xffffffffu, upto, 31), total = max(all, 1);
+            most = __reduce_max_sync(0xffffffffu, most);
+            // tiles of a share: a context of L tiles touches at most (L - 1) / least + 2 shares
+            const int least = max((most + p.splits - 2) / (p.splits - 1), 1), ctas = max(min((int)gridDim.x, total / least), 1);
+            const bool mine = (int)blockIdx.x < ctas && all > 0;
+            if (lane == 0) {
+                before[kTcShareTokens] = all;
+                plan[0] = mine ? (int)((long long)total * (blockIdx.x + 1) / ctas) : 0;
+                plan[1] = mine ? (int)((long long)total * blockIdx.x / ctas) : 0;
+                plan[2] = total;
+                plan[3] = ctas;
+            }
         }
-        const int c0 = split * span.chunk, c1 = min(c0 + span.chunk, span.len);
+        __syncthreads();
+        flat = plan[2] >= kTcShareTiles * (int)gridDim.x;
+        if (flat && blockIdx.x == 0)  // tokens that see nothing
+            for (int st = warp; st < p.shares; st += kTcWarps)
+                if (before[st + 1] == before[st])
+                    for (int i = lane; i < p.nh * p.splits; i += 32) p.pm[(size_t)st * p.nh * p.splits + i] = -INFINITY;
+    }
+    for (int item = blockIdx.x;;) {
+        int kvh, split, st, slot, c0, c1;
+        if (flat) {
+            const int u = plan[1], u1 = plan[0], total = plan[2], ctas = plan[3];
+            if (u >= u1) break;
+            __syncthreads();  // everyone has read where the run goes on
+            st = 0;
+#pragma unroll
+            for (int d = kTcShareTokens / 2; d > 0; d >>= 1)
+                if (before[st + d] <= u) st += d;
+            slot = cache_slot(p.slot_map, st / p.T);
+            const int len = tq_span(p, st, slot).len, tl = (len + kTile - 1) / kTile, at = u - before[st], t0 = at % tl, t1 = min(tl, t0 + u1 - u), b0 = u - t0;
+            kvh = at / tl;
+            if (tid == 0) plan[1] = u + t1 - t0;  // (read after the item's barriers)
+            c0 = t0 * kTile;
+            c1 = min(t1 * kTile, len);
+            const int first = (int)((((long long)b0 + 1) * ctas + total - 1) / total) - 1, last = (int)(((long long)(b0 + tl) * ctas + total - 1) / total) - 1;
+            split = blockIdx.x - first;
+            if (split == 0)  // places of parts that this context does not have
+                for (int i = tid; i < GQ * (p.splits - 1 - (last - first)); i += kTcWarps * 32)
+                    p.pm[((size_t)st * p.nh + kvh * GQ + i % GQ) * p.splits + last - first + 1 + i / GQ] = -INFINITY;
+        } else {
+            if (item >= items) break;
+            kvh = item % p.nkv;
+            split = item / p.nkv % p.splits;
+            st = item / p.nkv / p.splits;
+            item += gridDim.x;
+            slot = cache_slot(p.slot_map, st / p.T);
+            const TqSpan span = tq_span(p, st, slot);
+            if (split * span.chunk >= span.len) {  // (the whole CTA)
+                if (tid < GQ) p.pm[((size_t)st * p.nh + kvh * GQ + tid) * p.splits + split] = -INFINITY;
+                continue;
+            }
+            c0 = split * span.chunk;
+            c1 = min(c0 + span.chunk, span.len);
+        }
         // this warp's tiles of the split's range: every kTcWarps-th
         const int tiles = (c1 - c0 + kTile - 1) / kTile;
         const int h0 = kvh * GQ;
@@ -666,8 +739,18 @@ int tq_prep_launch(const Tq *tq, const TqPrep &a, cudaStream_t st) {
 
 // Parts that the positions of a (sequence, token, KV head) are cut into: enough for two CTAs per SM with one tile per warp of a part; and where parts
 // can hold three tiles per warp, up to four times as many as CTAs, so that sequences of different lengths share the GPU evenly.
+// Contexts that can fill shares of kTcShareTiles tiles for two CTAs per SM (the kernel looks again at what they are: the looking and the larger number of
+// parts cost shorter ones 5 %, a step of four sequences of 1024 positions 991 -> 1051 us)
+static bool tq_shares(const Device *dev, int nseq, int T, int nkv, int seq_len) {
+    return (long long)nseq * T <= kTcShareTokens && (long long)nseq * T * nkv * ((seq_len + kTile - 1) / kTile) >= 2ll * dev->sm_count * kTcShareTiles;
+}
 int tq_auto_splits(const Device *dev, int nseq, int T, int nkv, int seq_len) {
     const long long ctas = (long long)nseq * T * nkv, fill = 2 * dev->sm_count, run = kTcRun;
+    if (tq_shares(dev, nseq, T, nkv, seq_len)) {
+        // equal shares of all contexts' tiles (at least a tile per warp): as many parts as the longest context can fall to where the others are half as long on average
+        const long long tiles = (seq_len + kTile - 1) / kTile, share = std::max(ctas * tiles / fill, (long long)kTcWarps);
+        return (int)std::max(1ll, std::min(128ll, ((nseq > 1 ? 2 : 1) * tiles + share - 1) / share + 1));
+    }
     const long long a = std::min((fill + ctas - 1) / ctas, (seq_len + run - 1) / run), b = std::min(4 * fill / ctas, seq_len / (3 * run));
     return (int)std::max(1ll, std::min(128ll, std::max(a, b)));
 }
@@ -716,8 +799,9 @@ int tq_attention_launch(const Tq *tq, float *scratch, const __half *q, const uin
         auto kern = tq->n_bits == 4 ? (gq == 1 ? tq_attention_tc_kernel<1, 4> : (gq == 2 ? tq_attention_tc_kernel<2, 4> : tq_attention_tc_kernel<4, 4>))
                                     : (gq == 1 ? tq_attention_tc_kernel<1, 8> : (gq == 2 ? tq_attention_tc_kernel<2, 8> : tq_attention_tc_kernel<4, 8>));
         const long long items = (long long)nkv * nseq * T * splits;
+        if (own_parts && splits > 1 && tq_shares(tq->dev, nseq, T, nkv, pos_dev ? max_seq : base_pos + T)) p.shares = nseq * T;
         if (items > 0x7fffffffll) return fail(IM_ERR_BOUNDS, "attention over %lld parts", items);
-        IM_CUDA_CHECK(launch_k(kern, dim3((unsigned)std::min(items, 2ll * tq->dev->sm_count)), dim3(kTcWarps * 32), kTcSmem, st, p, (int)items));
+        IM_CUDA_CHECK(launch_k(kern, dim3((unsigned)p.shares ? 2ll * tq->dev->sm_count : std::min(items, 2ll * tq->dev->sm_count)), dim3(kTcWarps * 32), kTcSmem, st, p, (int)items));
     } else
     {
         const bool b4 = tq->n_bits == 4;
