@@ -160,8 +160,8 @@ int im_cuda_fused_residual_norm_ffn(const im_affine_weight *gate, const im_affin
  * w_dev fp16 [N,K] row-major, x_dev fp16 [B,K], y_dev fp16 [B,N]. */
 int im_cuda_matvec_f16(const void *w_dev, const void *x_dev, void *y_dev, int N, int K, int B, void *stream);
 /* superblock_matmul_int4 (.../shaders/quantized/affine_matmul.metal:10-152), the dense-contraction case (prefill,
- * decode batches >= 16): y[M,N] = sum_k f16(x[m,k] / awq[k]) * f16((q - z) * s), f32 accumulation on the tcgen05
- * tensor cores, fp16 result.  INT4 or INT8 group-128 weights; scratch_dev, 16-byte aligned, holds M*K halves (the activations, scaled or
+ * decode batches >= 16): y[M,N] = sum_k f16(x[m,k] / awq[k]) * f16((q - z) * s), f32 accumulation on the
+ * tensor cores (tcgen05; few tokens over K >= 1024: mma.sync), fp16 result.  INT4 or INT8 group-128 weights; scratch_dev, 16-byte aligned, holds M*K halves (the activations, scaled or
  * moved: x_dev may lie anywhere and y_dev over it). */
 int im_cuda_matmul_affine(const im_affine_weight *w, const void *x_dev, void *y_dev, int M, void *scratch_dev, void *stream);
 
