@@ -161,8 +161,9 @@ int im_cuda_fused_residual_norm_ffn(const im_affine_weight *gate, const im_affin
 int im_cuda_matvec_f16(const void *w_dev, const void *x_dev, void *y_dev, int N, int K, int B, void *stream);
 /* superblock_matmul_int4 (.../shaders/quantized/affine_matmul.metal:10-152), the dense-contraction case (prefill,
  * decode batches >= 16): y[M,N] = sum_k f16(x[m,k] / awq[k]) * f16((q - z) * s), f32 accumulation on the
- * tensor cores (tcgen05; few tokens over K >= 1024: mma.sync), fp16 result.  INT4 or INT8 group-128 weights; scratch_dev, 16-byte aligned, holds M*K halves (the activations, scaled or
- * moved: x_dev may lie anywhere and y_dev over it). */
+ * tensor cores (tcgen05; few tokens over K >= 1024: mma.sync), fp16 result.  INT4 or INT8 group-128 weights; scratch_dev, 16-byte aligned, holds M*K halves (the activations,
+ * scaled, packed or moved: x_dev may lie anywhere and y_dev over it).  x_dev and y_dev may share memory with the scratch where the tokens can be read
+ * where they are: no activation scales, x_dev 16-byte aligned, y_dev not over it. */
 int im_cuda_matmul_affine(const im_affine_weight *w, const void *x_dev, void *y_dev, int M, void *scratch_dev, void *stream);
 
 /* ------------------------------------------------------------------ norms, embedding, RoPE

@@ -114,9 +114,10 @@ struct V2Params {
 };
 
 // INT4 g128 GEMM on tcgen05 / TMEM (gemm_tc.cu): y[M, N] = f16(x / awq) * dequant(w)^T; xs_scratch holds M * K halves.
-// IM_ERR_BOUNDS when the weight is not INT4 or INT8 group-128.
+// IM_ERR_BOUNDS when the weight is not INT4 or INT8 group-128.  pack: the scratch is 16-byte aligned and shares no memory with x and y.
 enum TokenForm { kTokensRaw, kTokensScaled, kTokensPacked };  // x as it is; f16(x / awq); that, packed for gemm_rows.cu (where gemm_rows_takes says so)
-int gemm_affine_tc(const AffineWeight *w, const __half *x, __half *y, int M, __half *xs_scratch, cudaStream_t st, TokenForm form = kTokensRaw);
+int gemm_affine_tc(const AffineWeight *w, const __half *x, __half *y, int M, __half *xs_scratch, cudaStream_t st, TokenForm form = kTokensRaw,
+                   bool pack = true);
 // The gated activation y[M, N] = f16(silu(f16(gate x)) f16(up x)) in one launch, for two weights of the same form and activation scales;
 // only where gemm_affine_joins() says so.
 bool gemm_affine_joins(const AffineWeight *gate, int M);

@@ -423,10 +423,10 @@ int gemm_affine_gate_up(const AffineWeight *gate, const AffineWeight *up, const 
 
 // Y[M, N] = f16(X / awq) * dequant(W)^T for M tokens.  xs_scratch: M * K halves.  IM_ERR_BOUNDS when the weight is not
 // INT4 group-128 with K a multiple of 128 (the caller falls back to the matvec kernels).
-int gemm_affine_tc(const AffineWeight *w, const __half *x, __half *y, int M, __half *xs_scratch, cudaStream_t st, TokenForm form) {
+int gemm_affine_tc(const AffineWeight *w, const __half *x, __half *y, int M, __half *xs_scratch, cudaStream_t st, TokenForm form, bool pack) {
     if (!gemm_takes(w) || M < 1) return IM_ERR_BOUNDS;
-    // Up to 64 tokens over tiled weights: gemm_rows.cu (the tokens are packed in the scratch unless they come packed).
-    if (gemm_rows_takes(w, M) && (form == kTokensPacked || (x != xs_scratch && reinterpret_cast<uintptr_t>(xs_scratch) % 16 == 0))) {
+    // Few tokens over tiled weights: gemm_rows.cu (the tokens are packed in the scratch unless they come packed).
+    if (gemm_rows_takes(w, M) && (form == kTokensPacked || pack)) {
         if (form != kTokensPacked) {
             if (const int rc = token_pack(x, form == kTokensRaw ? w->awq : nullptr, xs_scratch, M, w->K, st); rc != IM_OK) return rc;
             x = xs_scratch;

@@ -881,20 +881,20 @@ IM_EXPORT int im_cuda_matmul_affine(const im_affine_weight *w, const void *x_dev
     if (M == 0) return IM_OK;
     IM_CUDA_CHECK(cudaSetDevice(w->dev->ordinal));
     // Without activation scales the tokens are read where they are: not if the result is written over them, nor if the copies cannot
-    // start there. They move to the scratch then, which has to be aligned itself if it is used.
+    // start there. They move to the scratch then, which has to be aligned itself if it is used.  Few tokens are packed in the scratch whatever they are
+    // (gemm_rows.cu): only if it shares no memory with them, which other threads of the packing still read, nor with the result, which is written while
+    // packed tokens are read.
     const size_t nx = (size_t)M * w->K * sizeof(__half), ny = (size_t)M * w->N * sizeof(__half);
-    const uintptr_t x0 = reinterpret_cast<uintptr_t>(x_dev), y0 = reinterpret_cast<uintptr_t>(y_dev);
-    // (few tokens are packed in the scratch whatever they are: gemm_rows.cu)
-    const uintptr_t s0 = reinterpret_cast<uintptr_t>(scratch_dev);
-    const bool rows = gemm_rows_takes(w, M) && s0 % 16 == 0 && (s0 >= x0 + nx || x0 >= s0 + nx);
-    const bool move = rows ? false : x0 % 16 != 0 || (!w->awq && x0 < y0 + ny && y0 < x0 + nx);
+    const uintptr_t x0 = reinterpret_cast<uintptr_t>(x_dev), y0 = reinterpret_cast<uintptr_t>(y_dev), s0 = reinterpret_cast<uintptr_t>(scratch_dev);
+    const bool pack = s0 % 16 == 0 && (s0 >= x0 + nx || x0 >= s0 + nx) && (s0 >= y0 + ny || y0 >= s0 + nx);
+    const bool move = !(pack && gemm_rows_takes(w, M)) && (x0 % 16 != 0 || (!w->awq && x0 < y0 + ny && y0 < x0 + nx));
     IM_REQUIRE((!move && !w->awq) || reinterpret_cast<uintptr_t>(scratch_dev) % 16 == 0, "the scratch must be 16-byte aligned");
     if (move) {
         IM_CUDA_CHECK(cudaMemcpyAsync(scratch_dev, x_dev, nx, cudaMemcpyDeviceToDevice, as_stream(stream)));
         x_dev = scratch_dev;
     }
     const int rc = gemm_affine_tc(w, static_cast<const __half *>(x_dev), static_cast<__half *>(y_dev), M, static_cast<__half *>(scratch_dev),
-                                  as_stream(stream));
+                                  as_stream(stream), kTokensRaw, pack);
     if (rc == IM_ERR_BOUNDS) return fail(IM_ERR_INVALID, "the tensor-core GEMM takes INT4 or INT8 group-128 weights with K a multiple of 128");
     return rc;
     IM_GUARD_END

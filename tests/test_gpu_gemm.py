@@ -118,6 +118,43 @@ def test_rows_that_are_not_aligned(dev, K, M, awq):
         ops.matmul_affine(w, xo, scratch=yo)
 
 
+@pytest.mark.parametrize("bits", [4, 8])
+@pytest.mark.parametrize("K,M", [(1024, 7), (2048, 32), (1024, 48)])
+def test_scratch_that_shares_memory(dev, K, M, bits):
+    # without activation scales, tokens that can be read where they are stay there: a view at an offset into the scratch, and the result in the scratch
+    from ironmill_b200 import ops
+    w = H.QWeight(K, K, bits=bits, seed=K + M, name="gs").gpu(dev)
+    x = torch.from_numpy(H.rng_for("gs-x", M).standard_normal((M, K)).astype(np.float16)).cuda()
+    want = ops.matmul_affine(w, x).cpu().numpy()
+    for at in (0, 8, 5 * K // 2, M * K - 8):  # from the same place to all but sixteen bytes apart
+        buf = torch.zeros(2 * M * K, dtype=torch.float16, device="cuda")
+        view = buf[at:at + M * K].view(M, K)
+        view.copy_(x)
+        assert H.rel_err(ops.matmul_affine(w, view, scratch=buf[:M * K]).cpu().numpy(), want) <= TOL, at
+        assert torch.equal(view, x), at
+        buf.zero_()
+        out = ops.matmul_affine(w, x, out=buf[at:at + M * K].view(M, K), scratch=buf[:M * K])
+        assert H.rel_err(out.cpu().numpy(), want) <= TOL, at
+
+
+@pytest.mark.parametrize("awq", [False, True])
+@pytest.mark.parametrize("K,M", [(1024, 5), (2048, 24), (1024, 48)])
+def test_few_tokens_anywhere(dev, K, M, awq):
+    # few tokens over a long sum: the result over the tokens, tokens and result at places that no vector reaches
+    from ironmill_b200 import CudaSysError, ops
+    w = H.QWeight(K, K, awq=awq, seed=K + M, name="gu").gpu(dev)
+    x = torch.from_numpy(H.rng_for("gu-x", M).standard_normal((M, K)).astype(np.float16)).cuda()
+    want = ops.matmul_affine(w, x)
+    far = torch.empty(2, M * K + 8, dtype=torch.float16, device="cuda")
+    xo, yo = far[0, 1:1 + M * K].view(M, K), far[1, 3:3 + M * K].view(M, K)
+    xo.copy_(x)
+    assert torch.equal(ops.matmul_affine(w, xo, out=yo), want)
+    assert torch.equal(ops.matmul_affine(w, xo, out=xo), want)
+    with pytest.raises(CudaSysError):
+        ops.matmul_affine(w, yo, scratch=far[0, 1:1 + M * K].view(M, K))
+    assert torch.equal(ops.matmul_affine(w, x, out=x), want)
+
+
 def test_matches_the_matvec_kernel_rows(dev):
     # the same weight through the decode matvec (24-bit integer activations) and the GEMM: both within their tolerance of the oracle
     from ironmill_b200 import ops
