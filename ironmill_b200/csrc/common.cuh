@@ -221,7 +221,7 @@ struct Tq {
     size_t const_bytes = 0;
 };
 
-int tq_auto_splits(const Device *dev, int nseq, int T, int nkv, int seq_len);
+int tq_auto_splits(const Device *dev, int nseq, int T, int nh, int nkv, int seq_len);
 // Prefill chunks of one sequence: dequantise the cached rows once, causal flash attention on the tensor cores (tq_prefill.cu).
 size_t tq_prefill_scratch_bytes(int nkv, int max_seq);
 struct TqPromptQuery {       // query rows as projected: head h at column 128 h

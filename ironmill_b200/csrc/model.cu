@@ -436,7 +436,7 @@ static int tp_allreduce(Model *m, __half *buf, size_t count, cudaStream_t st) {
 
 
 static int decode_splits(const Model *m, int batch) {
-    return tq_auto_splits(m->dev, batch, 1, m->nkv_l, m->cfg.max_seq_len);
+    return tq_auto_splits(m->dev, batch, 1, m->nh_l, m->nkv_l, m->cfg.max_seq_len);
 }
 
 // One forward pass over nseq sequences x T tokens each (decode: T = 1; prefill: nseq = 1).
@@ -489,7 +489,7 @@ static int head_rows(Model *m, const __half *x, __half *out, int rows, cudaStrea
 int Model::forward(int nseq, int T, cudaStream_t st, Prof *prof, bool all_logits, const int *slots) {
     Model *const m = this;
     const im_model_config &c = m->cfg;
-    const int attn_splits = m->prefill_slot_id >= 0 ? tq_auto_splits(m->dev, 1, T, m->nkv_l, m->prefill_ctx_end) : decode_splits(m, nseq);
+    const int attn_splits = m->prefill_slot_id >= 0 ? tq_auto_splits(m->dev, 1, T, m->nh_l, m->nkv_l, m->prefill_ctx_end) : decode_splits(m, nseq);
     const int H = c.hidden_size, hd = c.head_dim, MT = nseq * T;
     const float eps = c.rms_eps;
     const float attn_scale = c.attn_scale != 0.0f ? c.attn_scale : 1.0f / sqrtf((float)hd);
@@ -1298,7 +1298,7 @@ int Model::finalize() {
         if (s > need) need = s;
     }
     for (int t = 1; t <= m->MT; t++) {
-        const size_t s = im_cuda_tq_scratch_bytes(1, t, m->nh_l, hd, tq_auto_splits(m->dev, 1, t, m->nkv_l, c.max_seq_len));
+        const size_t s = im_cuda_tq_scratch_bytes(1, t, m->nh_l, hd, tq_auto_splits(m->dev, 1, t, m->nh_l, m->nkv_l, c.max_seq_len));
         if (s > need) need = s;
     }
     if (c.tq_bits == 16) {

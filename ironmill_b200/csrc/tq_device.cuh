@@ -227,7 +227,7 @@ struct AttnParams {
     const int *pos_dev;      // optional per-slot positions (added to base_pos)
     const int *slot_map;     // optional: sequence index of this launch -> cache slot (nullptr: identity)
     int bits;                // cache bits per element (8 or 4); rows hold tq_row_bytes(bits, hd) bytes
-    int own_parts;           // `splits` is the most that a token may use: its context is cut into parts of at least one run of tiles
+    int own_parts;           // not 0: the most parts of `splits` that a token may use; its context is cut into parts of at least one run of tiles
     int shares;              // number of tokens whose contexts tq_attention_tc_kernel deals out as equal shares (0: item by item)
 };
 constexpr int kTcShareTiles = 16;    // least tiles of a share
@@ -242,7 +242,7 @@ __device__ __forceinline__ TqSpan tq_span(const AttnParams &p, int st, int slot)
     TqSpan s;
     // never past the end of the head's rows, whatever a device-side position says (the host can only check base_pos)
     s.len = max(min(p.base_pos + (p.pos_dev ? p.pos_dev[slot] : 0) + st % p.T + 1, p.max_seq), 0);
-    const int n = p.own_parts ? max(min(p.splits, (s.len + kTcRun - 1) / kTcRun), 1) : p.splits;
+    const int n = p.own_parts ? max(min(p.own_parts, (s.len + kTcRun - 1) / kTcRun), 1) : p.splits;
     s.chunk = max((int)((unsigned)(s.len + n - 1) / (unsigned)n + kTile - 1) / kTile, 1) * kTile;
     return s;
 }

@@ -737,28 +737,32 @@ int tq_prep_launch(const Tq *tq, const TqPrep &a, cudaStream_t st) {
     return IM_OK;
 }
 
+// Contexts that can fill shares of kTcShareTiles tiles for two CTAs per SM (the kernel looks again at what they are: the looking costs shorter ones 5 %, a
+// step of four sequences of 1024 positions 991 -> 1051 us)
+static bool tq_shares(const Device *dev, int nseq, int T, int nh, int nkv, int seq_len) {
+    const int gq = nkv > 0 ? nh / nkv : 0;
+    return (gq == 1 || gq == 2 || gq == 4) && (long long)nseq * T <= kTcShareTokens &&
+           (long long)nseq * T * nkv * ((seq_len + kTile - 1) / kTile) >= 2ll * dev->sm_count * kTcShareTiles;
+}
 // Parts that the positions of a (sequence, token, KV head) are cut into: enough for two CTAs per SM with one tile per warp of a part; and where parts
 // can hold three tiles per warp, up to four times as many as CTAs, so that sequences of different lengths share the GPU evenly.
-// Contexts that can fill shares of kTcShareTiles tiles for two CTAs per SM (the kernel looks again at what they are: the looking and the larger number of
-// parts cost shorter ones 5 %, a step of four sequences of 1024 positions 991 -> 1051 us)
-static bool tq_shares(const Device *dev, int nseq, int T, int nkv, int seq_len) {
-    return (long long)nseq * T <= kTcShareTokens && (long long)nseq * T * nkv * ((seq_len + kTile - 1) / kTile) >= 2ll * dev->sm_count * kTcShareTiles;
-}
-int tq_auto_splits(const Device *dev, int nseq, int T, int nkv, int seq_len) {
+static int tq_parts(const Device *dev, int nseq, int T, int nkv, int seq_len) {
     const long long ctas = (long long)nseq * T * nkv, fill = 2 * dev->sm_count, run = kTcRun;
-    if (tq_shares(dev, nseq, T, nkv, seq_len)) {
-        // equal shares of all contexts' tiles (at least a tile per warp): as many parts as the longest context can fall to where the others are half as long on average
-        const long long tiles = (seq_len + kTile - 1) / kTile, share = std::max(ctas * tiles / fill, (long long)kTcWarps);
-        return (int)std::max(1ll, std::min(128ll, ((nseq > 1 ? 2 : 1) * tiles + share - 1) / share + 1));
-    }
     const long long a = std::min((fill + ctas - 1) / ctas, (seq_len + run - 1) / run), b = std::min(4 * fill / ctas, seq_len / (3 * run));
     return (int)std::max(1ll, std::min(128ll, std::max(a, b)));
+}
+// Places for parts: with shares also as many as the longest context falls to where the others are half as long on average.  Never fewer for a longer
+// seq_len: scratch that was sized for the longest one holds those of all.
+int tq_auto_splits(const Device *dev, int nseq, int T, int nh, int nkv, int seq_len) {
+    const long long ctas = (long long)nseq * T * nkv, fill = 2 * dev->sm_count;
+    const int n = tq_parts(dev, nseq, T, nkv, seq_len);
+    return tq_shares(dev, nseq, T, nh, nkv, seq_len) ? std::max(n, (int)std::min(128ll, ((nseq > 1 ? 2 : 1) * fill + ctas - 1) / ctas + 1)) : n;
 }
 
 // Split count of a call and scratch for it. An automatic count (the longest context that the call can meet decides: with positions on the device, the
 // cache's length) takes what the scratch holds: it grows only for a count that the caller gave or where one part of each does not fit.
 static int tq_call_scratch(im_tq *tq, int num_splits, int nseq, int T, int nh, int nkv, int max_seq, int base_pos, const int *pos_dev, int *out) {
-    int splits = num_splits > 0 ? num_splits : tq_auto_splits(tq->dev, nseq, T, nkv, pos_dev ? max_seq : base_pos + T);
+    int splits = num_splits > 0 ? num_splits : tq_auto_splits(tq->dev, nseq, T, nh, nkv, pos_dev ? max_seq : base_pos + T);
     while (num_splits <= 0 && splits > 1 && im_cuda_tq_scratch_bytes(nseq, T, nh, kHd, splits) > tq->scratch_bytes) splits--;
     *out = splits;
     const int rc = im_cuda_tq_reserve_scratch(tq, im_cuda_tq_scratch_bytes(nseq, T, nh, kHd, splits));
@@ -770,7 +774,7 @@ int tq_attention_launch(const Tq *tq, float *scratch, const __half *q, const uin
                         const float *vs, const float *krn, float attn_scale, __half *out, int nseq, int nh, int nkv, int max_seq,
                         int base_pos, const int *pos_dev, int T, int splits, bool own_parts, cudaStream_t st, const float *qrot, const int *slot_map) {
     AttnParams p{};
-    p.own_parts = own_parts;
+    p.own_parts = own_parts ? std::min(splits, tq_parts(tq->dev, nseq, T, nkv, pos_dev ? max_seq : base_pos + T)) : 0;
     p.qrot = qrot;
     p.slot_map = slot_map;
     p.bits = tq->n_bits;
@@ -799,9 +803,9 @@ int tq_attention_launch(const Tq *tq, float *scratch, const __half *q, const uin
         auto kern = tq->n_bits == 4 ? (gq == 1 ? tq_attention_tc_kernel<1, 4> : (gq == 2 ? tq_attention_tc_kernel<2, 4> : tq_attention_tc_kernel<4, 4>))
                                     : (gq == 1 ? tq_attention_tc_kernel<1, 8> : (gq == 2 ? tq_attention_tc_kernel<2, 8> : tq_attention_tc_kernel<4, 8>));
         const long long items = (long long)nkv * nseq * T * splits;
-        if (own_parts && splits > 1 && tq_shares(tq->dev, nseq, T, nkv, pos_dev ? max_seq : base_pos + T)) p.shares = nseq * T;
+        if (own_parts && splits > 1 && tq_shares(tq->dev, nseq, T, nh, nkv, pos_dev ? max_seq : base_pos + T)) p.shares = nseq * T;
         if (items > 0x7fffffffll) return fail(IM_ERR_BOUNDS, "attention over %lld parts", items);
-        IM_CUDA_CHECK(launch_k(kern, dim3((unsigned)p.shares ? 2ll * tq->dev->sm_count : std::min(items, 2ll * tq->dev->sm_count)), dim3(kTcWarps * 32), kTcSmem, st, p, (int)items));
+        IM_CUDA_CHECK(launch_k(kern, dim3((unsigned)(p.shares ? 2ll * tq->dev->sm_count : std::min(items, 2ll * tq->dev->sm_count))), dim3(kTcWarps * 32), kTcSmem, st, p, (int)items));
     } else
     {
         const bool b4 = tq->n_bits == 4;
@@ -945,7 +949,7 @@ IM_EXPORT int im_cuda_tq_attention_static(const im_tq *tq, const void *q_dev, co
     // The array holds what im_cuda_tq_attention keeps in its allocated scratch: the split partials, then the rotated
     // queries of the pre-pass (so both entry points run the same kernels).  A split count chosen here shrinks until
     // the request fits; one given by the caller is taken as it is or refused.
-    int splits = num_splits > 0 ? num_splits : tq_auto_splits(tq->dev, nseq, T, nkv, pos_dev ? max_seq : base_pos + T);
+    int splits = num_splits > 0 ? num_splits : tq_auto_splits(tq->dev, nseq, T, nh, nkv, pos_dev ? max_seq : base_pos + T);
     while (num_splits <= 0 && splits > 1 && im_cuda_tq_scratch_bytes(nseq, T, nh, kHd, splits) > kStaticScratchFloats * sizeof(float)) splits--;
     const size_t need = im_cuda_tq_scratch_bytes(nseq, T, nh, kHd, splits);
     if (need > kStaticScratchFloats * sizeof(float))
