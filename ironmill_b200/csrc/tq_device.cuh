@@ -228,10 +228,11 @@ struct AttnParams {
     const int *slot_map;     // optional: sequence index of this launch -> cache slot (nullptr: identity)
     int bits;                // cache bits per element (8 or 4); rows hold tq_row_bytes(bits, hd) bytes
     int own_parts;           // not 0: the most parts of `splits` that a token may use; its context is cut into parts of at least one run of tiles
-    int shares;              // number of tokens whose contexts tq_attention_tc_kernel deals out as equal shares (0: item by item)
+    int shares;              // number of tokens whose contexts tq_attention_tc_kernel may deal out as equal shares (0: none)
 };
-constexpr int kTcShareTiles = 16;    // least tiles of a share
-constexpr int kTcShareTokens = 64;  // most (sequence, token) pairs whose contexts are dealt out as equal shares
+constexpr int kTcShareTiles = 8;     // least tiles of a share
+constexpr int kTcShareContexts = 5;  // most of the shortest context that a share may hold
+constexpr int kTcShareTokens = 64;   // most (sequence, token) pairs whose contexts are dealt out as equal shares: two to a lane
 constexpr int kTcWarps = 6, kTcRun = kTcWarps * kTile;  // a run: a tile for each warp of tq_attention_tc_kernel
 // Positions that token st (sequence-major) of a launch sees and positions of a part of them (whole tiles). Part i is there if i chunk < len; of the
 // rest of `splits` only the maximum is written, minus infinity (100 positions in a cache of 65536 cut into 113 parts took 32 us, 25 in one).
@@ -626,6 +627,7 @@ __device__ __forceinline__ void tq_reduce_item(const Scope &sc, float *x, const 
             o[j] = live ? po[(base + s0 + j) * kHd + d] : 0.0f;
         }
     };
+    const float beyond = 8 + d < splits ? pm[base + 8 + d] : -INFINITY;  // (with the first ones' loads)
     load(0, splits);
     float gm = -INFINITY;
 #pragma unroll
@@ -634,7 +636,7 @@ __device__ __forceinline__ void tq_reduce_item(const Scope &sc, float *x, const 
     if (splits > 8) {  // a thread per part
         int last = 0;
         for (int s = 8 + d; s < splits; s += kHd) {
-            const float t = pm[base + s];
+            const float t = s < 8 + kHd ? beyond : pm[base + s];
             if (t != -INFINITY) last = s + 1;
             gm = fmaxf(gm, t);
         }

@@ -183,14 +183,19 @@ __global__ void __launch_bounds__(kHd) tq_reduce_kernel(const AttnParams p, __ha
 //     against the signs, columns 4-7 = S q with zeros against the centroids; outputs as [16 dims x 16 positions] x
 //     [16 positions x 8 heads].  The fragment <-> (dimension, position) assignment is chosen so that a fragment
 //     register is built from bytes the lane already holds.
-// The six warps of a CTA (two CTAs per SM: 168 registers a thread, for a tile's V rows and the next tile's K rows in flight) take the tiles of one (KV head, token, split) in turn and merge their results in shared
-// memory, so the number of partials per head is the same as with the kernel above.  Two CTAs per SM with one table each.  With an automatic split count
-// and up to 64 contexts, each takes an equal run of the list of all their tiles: dealt out as (KV head, token, split) items, whose sizes follow their
-// contexts', SMs idled 18 % of the time and an item's start and merge came four times a CTA (16 sequences of 1024 .. 8192 positions, the whole call:
-// 86.9 -> 76.7 us, 4-bit 76.5 -> 62; two of 7500 .. 60000: 109 -> 89).  Shares of less than
-// 16 tiles: items, each of which fits one context (tq_shares).  mma.sync issue bounds it (48 products per tile, one per 32 clocks and SM quarter).  16 sequences of 1024 .. 8192
-// positions, 32 / 8 heads: 166 us with eight warps, rows loaded where they were used and a CTA per item of one
-// split; 126 us with this form and one split, 83 us with parts for every SM.
+// The six warps of a CTA (two CTAs per SM: 168 registers a thread, for a tile's V rows and the next tile's K rows in flight) take the tiles of one (KV head,
+// token, part) in turn and merge their results in shared memory, so the number of partials per head is the same as with the kernel above.  Two CTAs per SM
+// with one table each.  mma.sync issue bounds it (48 products per tile, one per 32 clocks and SM quarter).  16 sequences of 1024 .. 8192 positions, 32 / 8
+// heads, the whole call: 166 us with eight warps, rows loaded where they were used and a CTA per item of one split; 85 us with parts for every SM.
+//
+// SHARES (tq_shares): each CTA takes an equal run of the list of all contexts' tiles (a context's parts are the CTAs that its tiles fall to) or, item by item,
+// its turn of the list of their parts.  In parts, whose sizes follow their contexts', SMs idle 18 % of the time and a start and a merge come four times a
+// CTA; in shares, a run of short contexts is a start and a merge for each.  So: shares where they hold eight tiles (kTcShareTiles) and no more than five of
+// the shortest context (kTcShareContexts), unless the longest context has too few places for parts and ties them to few CTAs (a share a quarter longer
+// than the longest part), or the parts are about as long and all at work at once.  8-bit cache, in parts / in shares: 16 of 1024 .. 8192 positions 86 / 69
+// us, two of 7500 and 60000 77 / 63, one of 10000 in a cache of 65536 32 / 27; one of 30000 among fifteen of 500 97 / 122, one of 60000 among 31 of 400
+// 269 / 570; 4-bit, one of 20000 31 / 36.  Each form is a loop of its own, and launches that cannot take shares have neither: in one loop for
+// both, the registers of one spilled in the other (two of 7500 and 60000: 67 us; 24 of 600: 35 -> 37).
 __device__ __forceinline__ void mma_f16(float (&c)[4], unsigned a0, unsigned a1, unsigned a2, unsigned a3, unsigned b0, unsigned b1) {
     asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
                  : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
@@ -208,16 +213,239 @@ __device__ __forceinline__ unsigned pack_h2(float a, float b) {
     return *reinterpret_cast<const unsigned *>(&h);
 }
 
+// One part: positions c0 .. c1 of token st and KV head kvh as part `split` of p.splits.
 template <int GQ, int BITS>
-__global__ void __launch_bounds__(kTcWarps * 32, 2) tq_attention_tc_kernel(const AttnParams p, int items) {
+__device__ __forceinline__ void tc_part(const AttnParams &p, const unsigned char *lut, __half *pw, float *comb, int st, int kvh, int split, int slot, int c0, int c1) {
     constexpr int kRowB = BITS == 4 ? kHd / 2 : kHd;  // bytes of a cached row
     constexpr int kKV = BITS == 8 ? 2 : 1;            // 16-byte vectors of a lane's piece of a K row
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
+    const unsigned lane_k = lane * 4u, lane_v = 128u + lane * 4u;
+    // halves of a packed query pair as B operand words against (centroid, sign) pairs: (q, 0) for the columns of centroid sums (g < 4),
+    // (0, S q) for the columns of sign sums
+    const unsigned sel0 = g < 4 ? 0x4410u : 0x1044u, sel1 = g < 4 ? 0x4432u : 0x3244u;
+    __half *pwarp = pw + warp * 4 * 32;
+    // this warp's tiles of the split's range: every kTcWarps-th
+    const int tiles = (c1 - c0 + kTile - 1) / kTile;
+    const int h0 = kvh * GQ;
+    const size_t head_base = ((size_t)slot * p.nkv + kvh) * p.max_seq;
+    const uint8_t *krow = p.kc + head_base * kRowB, *vrow = p.vc + head_base * kRowB;
+
+    // B fragments of the score products: lane (n = g, t) holds dims 32 t + 2 i, + 1 of column n: the rotated query
+    // of head n (n < GQ) or S q of head n - 4 (4 <= n < 4 + GQ); zero otherwise
+    unsigned bx[16];
+#pragma unroll
+    for (int i = 0; i < 16; i++) bx[i] = 0u;
+    if (g < GQ || (g >= 4 && g < 4 + GQ)) {
+        const float *src = p.qrot + ((size_t)st * p.nh + h0 + (g < 4 ? g : g - 4)) * 2 * kHd + (g < 4 ? 0 : kHd) + 32 * t;
+#pragma unroll
+        for (int j = 0; j < 8; j++) {
+            const float4 v = *reinterpret_cast<const float4 *>(src + 4 * j);
+            bx[2 * j] = pack_h2(v.x, v.y);
+            bx[2 * j + 1] = pack_h2(v.z, v.w);
+        }
+    }
+
+    float m_run[2] = {-INFINITY, -INFINITY}, l_run[2] = {0.0f, 0.0f};  // lanes t < 2: heads 2t, 2t + 1
+    float o[8][4];                                                       // o[mb]: dims 16g + 2mb, +1 (rows) x heads 2t, 2t+1
+#pragma unroll
+    for (int i = 0; i < 8; i++) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.0f;
+
+    // K rows g, g+8, g+16, g+24 of a tile: dims 32t .. 32t+31 each (32 bytes, or 16 bytes of nibbles), and the rows' factors
+    uint4 kq[4][kKV];
+    float ksv[4], rwv[4], vsv[4];
+    auto request = [&](int ts) {
+#pragma unroll
+        for (int r = 0; r < 4; r++) {
+            const int pos = ts + g + 8 * r;
+            ksv[r] = rwv[r] = vsv[r] = 0.0f;
+#pragma unroll
+            for (int v = 0; v < kKV; v++) kq[r][v] = make_uint4(0, 0, 0, 0);
+            if (pos < c1) {
+                const uint4 *src = reinterpret_cast<const uint4 *>(krow + (size_t)pos * kRowB + (kRowB / 4) * t);
+#pragma unroll
+                for (int v = 0; v < kKV; v++) kq[r][v] = __ldcs(src + v);
+                ksv[r] = p.ks[head_base + pos];
+                rwv[r] = p.krn[head_base + pos];
+                vsv[r] = p.vs[head_base + pos];
+            }
+        }
+    };
+    request(c0 + warp * kTile);
+    for (int tile = warp; tile < tiles; tile += kTcWarps) {
+        const int ts = c0 + tile * kTile, nt = min(kTile, c1 - ts);
+        // ---- V rows 2t, 2t+1, 2t+8, 2t+9 (+16): dims 16g .. 16g+15 each (16 bytes, or 8 bytes of nibbles in .x/.y), in flight during the scores ----
+        uint4 vq[8];
+#pragma unroll
+        for (int r = 0; r < 8; r++) {
+            const int pos = 2 * t + (r & 1) + 8 * ((r >> 1) & 1) + 16 * (r >> 2);
+            vq[r] = make_uint4(0, 0, 0, 0);
+            if (pos < nt) {
+                if (BITS == 8) {
+                    vq[r] = __ldcs(reinterpret_cast<const uint4 *>(vrow + (size_t)(ts + pos) * kRowB + 16 * g));
+                } else {
+                    const uint2 v2 = __ldcs(reinterpret_cast<const uint2 *>(vrow + (size_t)(ts + pos) * kRowB + 8 * g));
+                    vq[r].x = v2.x;
+                    vq[r].y = v2.y;
+                }
+            }
+        }
+        // ---- scores: a product of 16 positions x (centroid, sign) of eight dimensions per step, two row blocks ----
+        float sc[2][4];  // [row block][c0..c3]
+#pragma unroll
+        for (int rb = 0; rb < 2; rb++) sc[rb][0] = sc[rb][1] = sc[rb][2] = sc[rb][3] = 0.0f;
+#pragma unroll
+        for (int i = 0; i < 16; i++) {  // dims 32 t + 2 i, + 1
+            const unsigned b0 = __byte_perm(bx[i], 0, sel0), b1 = __byte_perm(bx[i], 0, sel1);
+            const int w = BITS == 8 ? i >> 1 : i >> 2, e = BITS == 8 ? 2 * (i & 1) : 2 * (i & 3);
+#pragma unroll
+            for (int rb = 0; rb < 2; rb++) {
+                const unsigned a = reinterpret_cast<const unsigned *>(&kq[2 * rb][0])[w], b = reinterpret_cast<const unsigned *>(&kq[2 * rb + 1][0])[w];  // rows g, g + 8 (+ 16 rb)
+                mma_f16(sc[rb], lut_at<BITS>(lut, lane_k, a, e), lut_at<BITS>(lut, lane_k, b, e), lut_at<BITS>(lut, lane_k, a, e + 1), lut_at<BITS>(lut, lane_k, b, e + 1),
+                        b0, b1);
+            }
+        }
+        // lanes t < 2 hold the centroid sums of heads 2t, 2t+1; lanes t + 2 the sign sums of the same heads
+        float s[4][2], vw[4];  // [position g + 8 r][head 2t + i]
+#pragma unroll
+        for (int rb = 0; rb < 2; rb++)
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                const float other = __shfl_xor_sync(0xffffffffu, sc[rb][q], 2);
+                const int r = 2 * rb + (q >> 1), i = q & 1;  // c0,c1: row g ; c2,c3: row g + 8
+                const bool live = t < 2 && g + 8 * r < nt;  // lanes t >= 2 only feed the shuffle above
+                s[r][i] = live ? p.attn_scale * (ksv[r] * (sc[rb][q] + rwv[r] * p.qjl_factor * other)) : -INFINITY;
+            }
+#pragma unroll
+        for (int r = 0; r < 4; r++) vw[r] = vsv[r];
+        request(tile + kTcWarps < tiles ? ts + kTcWarps * kTile : c1);  // the next tile's K rows travel during the rest of this one
+        // ---- online softmax over the tile (meaningful on lanes t < 2; the others carry copies of no use) ----
+        float wgt[4][2];
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+            float mx = fmaxf(fmaxf(s[0][i], s[1][i]), fmaxf(s[2][i], s[3][i]));
+            mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 4));
+            mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 8));
+            mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 16));
+            const float m_new = fmaxf(m_run[i], mx);
+            const float corr = m_new == -INFINITY ? 1.0f : __expf(m_run[i] - m_new);
+            float sum = 0.0f;
+#pragma unroll
+            for (int r = 0; r < 4; r++) {
+                wgt[r][i] = s[r][i] == -INFINITY ? 0.0f : __expf(s[r][i] - m_new);
+                sum += wgt[r][i];
+            }
+            l_run[i] = l_run[i] * corr + sum;  // this lane's own positions; added up over the lanes at the end
+            m_run[i] = m_new;
+            if (__any_sync(0xffffffffu, corr != 1.0f)) {
+#pragma unroll
+                for (int mb = 0; mb < 8; mb++) {  // heads 2t + i live in accumulator columns i (rows d0) and i + 2 (rows d1)
+                    o[mb][i] *= corr;
+                    o[mb][i + 2] *= corr;
+                }
+            }
+        }
+        // weights x V scale, as fp16, to this warp's P[head][position] for the output products
+        __syncwarp();
+        if (t < 2) {
+#pragma unroll
+            for (int r = 0; r < 4; r++)
+#pragma unroll
+                for (int i = 0; i < 2; i++)
+                    if (2 * t + i < 4) pwarp[(2 * t + i) * 32 + g + 8 * r] = __float2half_rn(wgt[r][i] * vw[r]);
+        }
+        __syncwarp();
+        // ---- outputs: O^T[dims][heads] += V^T[dims][positions] P^T[positions][heads] ----
+#pragma unroll
+        for (int kb = 0; kb < 2; kb++) {
+            unsigned b0 = 0u, b1 = 0u;  // lane (n = g): P[head g][16 kb + 2t, +1] and [.. + 8, + 9]
+            if (g < GQ) {
+                b0 = *reinterpret_cast<const unsigned *>(pwarp + g * 32 + 16 * kb + 2 * t);
+                b1 = *reinterpret_cast<const unsigned *>(pwarp + g * 32 + 16 * kb + 2 * t + 8);
+            }
+            const unsigned *v0 = reinterpret_cast<const unsigned *>(&vq[4 * kb + 0]);  // position 16 kb + 2t
+            const unsigned *v1 = reinterpret_cast<const unsigned *>(&vq[4 * kb + 1]);  // + 1
+            const unsigned *v2 = reinterpret_cast<const unsigned *>(&vq[4 * kb + 2]);  // + 8
+            const unsigned *v3 = reinterpret_cast<const unsigned *>(&vq[4 * kb + 3]);  // + 9
+#pragma unroll
+            for (int mb = 0; mb < 8; mb++) {  // rows g, g + 8 of the block: dims 16 g + 2 mb, + 1
+                const int w = BITS == 8 ? mb >> 1 : mb >> 2, by = BITS == 8 ? 2 * (mb & 1) : 2 * (mb & 3);
+                auto pair = [&](unsigned x, unsigned y, int e) {
+                    return __byte_perm(lut_at<BITS>(lut, lane_v, x, e), lut_at<BITS>(lut, lane_v, y, e), 0x5410);
+                };
+                mma_f16(o[mb], pair(v0[w], v1[w], by), pair(v0[w], v1[w], by + 1), pair(v2[w], v3[w], by), pair(v2[w], v3[w], by + 1), b0, b1);
+            }
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < 2; i++)
+#pragma unroll
+        for (int d = 4; d < 32; d <<= 1) l_run[i] += __shfl_xor_sync(0xffffffffu, l_run[i], d);
+
+    // ---- merge the warps: comb[warp][head][130] = o (dims 0..127), m, l ----
+    __syncthreads();  // the previous item's sums have been read
+    if (t < 2) {
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+            const int h = 2 * t + i;
+            if (h < 4) {
+                float *dst = comb + (warp * 4 + h) * 130;
+#pragma unroll
+                for (int mb = 0; mb < 8; mb++) {
+                    dst[16 * g + 2 * mb] = o[mb][i];
+                    dst[16 * g + 2 * mb + 1] = o[mb][i + 2];
+                }
+                if (g == 0) {
+                    dst[128] = m_run[i];
+                    dst[129] = l_run[i];
+                }
+            }
+        }
+    }
+    __syncthreads();
+    for (int idx = tid; idx < GQ * kHd; idx += kTcWarps * 32) {
+        const int h = idx >> 7, d = idx & 127;
+        float gm = -INFINITY;
+#pragma unroll
+        for (int w = 0; w < kTcWarps; w++) gm = fmaxf(gm, comb[(w * 4 + h) * 130 + 128]);
+        float acc = 0.0f, lsum = 0.0f;
+#pragma unroll
+        for (int w = 0; w < kTcWarps; w++) {
+            const float m = comb[(w * 4 + h) * 130 + 128];
+            const float corr = m == -INFINITY ? 0.0f : __expf(m - gm);
+            acc += comb[(w * 4 + h) * 130 + d] * corr;
+            lsum += comb[(w * 4 + h) * 130 + 129] * corr;
+        }
+        const size_t pi = ((size_t)st * p.nh + h0 + h) * p.splits + split;
+        p.po[pi * kHd + d] = acc;
+        if (d == 0) {
+            p.pm[pi] = gm;
+            p.pl[pi] = lsum;
+        }
+    }
+}
+
+// SHARES: the lists that CTAs take their work from, in shared memory.
+struct TcPlan {
+    int tiles[kTcShareTokens + 1], parts[kTcShareTokens + 1];  // tiles and parts (times KV heads) of the tokens in front
+    int len[kTcShareTokens], chunk[kTcShareTokens];            // positions that a token sees and those of a part of them
+    int next, end;                                             // where this CTA's share goes on and ends
+    int ctas, equal;                                           // shares, and whether they are taken
+};
+__device__ __forceinline__ int plan_token(const int *upto, int u) {  // the token whose run of the list holds u
+    int st = 0;
+#pragma unroll
+    for (int d = kTcShareTokens / 2; d > 0; d >>= 1)
+        if (upto[st + d] <= u) st += d;
+    return st;
+}
+template <int GQ, int BITS, bool SHARES>
+__global__ void __launch_bounds__(kTcWarps * 32, 2) tq_attention_tc_kernel(const AttnParams p, int items) {
     extern __shared__ __align__(256) unsigned char tc_smem[];
     unsigned char *lut = tc_smem;                                  // [256][K of 32 lanes | V of 32 lanes] (16 entries for 4-bit caches)
     __half *pw = reinterpret_cast<__half *>(lut + 256 * 256);      // [warps][4 heads][32 positions] softmax weights x v scale
     float *comb = reinterpret_cast<float *>(pw + kTcWarps * 4 * 32);  // [warps][4 heads][130]: o, m, l of each warp
 
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     pdl_trigger();
     {   // tables (constants): before the dependency wait
         constexpr int kSign = 1 << (BITS - 1), kVals = 1 << BITS;
@@ -230,288 +458,90 @@ __global__ void __launch_bounds__(kTcWarps * 32, 2) tq_attention_tc_kernel(const
         }
     }
     pdl_wait();
-    __syncthreads();
-    const unsigned lane_k = lane * 4u, lane_v = 128u + lane * 4u;
-    // halves of a packed query pair as B operand words against (centroid, sign) pairs: (q, 0) for the columns of centroid sums (g < 4),
-    // (0, S q) for the columns of sign sums
-    const unsigned sel0 = g < 4 ? 0x4410u : 0x1044u, sel1 = g < 4 ? 0x4432u : 0x3244u;
-    __half *pwarp = pw + warp * 4 * 32;
-
-    // Shares (p.shares): the tiles of all (token, KV head) contexts in one list, an equal run of it per CTA; a context's parts are the CTAs
-    // that its tiles fall to.  So few CTAs that no context has more than p.splits of them.
-    __shared__ int before[kTcShareTokens + 1], plan[4];  // tiles x KV heads of the tokens in front; where this CTA's run ends and goes on, all tiles, CTAs
-    bool flat = false;                                   // (in shared memory: the registers are the tiles')
-    if (p.shares) {
-        if (warp == 0) {
-            int v[2], sum = 0, most = 0;
-#pragma unroll
-            for (int i = 0; i < 2; i++) {
-                const int st = 2 * lane + i;
-                const int tiles = st < p.shares ? (tq_span(p, st, cache_slot(p.slot_map, st / p.T)).len + kTile - 1) / kTile : 0;
-                v[i] = tiles * p.nkv;
-                sum += v[i];
-                most = max(most, tiles);
-            }
-            int upto = sum;
-#pragma unroll
-            for (int d = 1; d < 32; d <<= 1) {
-                const int o = __shfl_up_sync(0xffffffffu, upto, d);
-                if (lane >= d) upto += o;
-            }
-            before[2 * lane] = upto - sum;
-            before[2 * lane + 1] = upto - sum + v[0];
-            const int all = __shfl_sync(0xffffffffu, upto, 31), total = max(all, 1);
-            most = __reduce_max_sync(0xffffffffu, most);
-            // tiles of a share: a context of L tiles touches at most (L - 1) / least + 2 shares
-            const int least = max((most + p.splits - 2) / (p.splits - 1), 1), ctas = max(min((int)gridDim.x, total / least), 1);
-            const bool mine = (int)blockIdx.x < ctas && all > 0;
-            if (lane == 0) {
-                before[kTcShareTokens] = all;
-                plan[0] = mine ? (int)((long long)total * (blockIdx.x + 1) / ctas) : 0;
-                plan[1] = mine ? (int)((long long)total * blockIdx.x / ctas) : 0;
-                plan[2] = total;
-                plan[3] = ctas;
-            }
-        }
+    if constexpr (!SHARES) {
         __syncthreads();
-        flat = plan[2] >= kTcShareTiles * (int)gridDim.x;
-        if (flat && blockIdx.x == 0)  // tokens that see nothing
-            for (int st = warp; st < p.shares; st += kTcWarps)
-                if (before[st + 1] == before[st])
-                    for (int i = lane; i < p.nh * p.splits; i += 32) p.pm[(size_t)st * p.nh * p.splits + i] = -INFINITY;
-    }
-    for (int item = blockIdx.x;;) {
-        int kvh, split, st, slot, c0, c1;
-        if (flat) {
-            const int u = plan[1], u1 = plan[0], total = plan[2], ctas = plan[3];
-            if (u >= u1) break;
-            __syncthreads();  // everyone has read where the run goes on
-            st = 0;
-#pragma unroll
-            for (int d = kTcShareTokens / 2; d > 0; d >>= 1)
-                if (before[st + d] <= u) st += d;
-            slot = cache_slot(p.slot_map, st / p.T);
-            const int len = tq_span(p, st, slot).len, tl = (len + kTile - 1) / kTile, at = u - before[st], t0 = at % tl, t1 = min(tl, t0 + u1 - u), b0 = u - t0;
-            kvh = at / tl;
-            if (tid == 0) plan[1] = u + t1 - t0;  // (read after the item's barriers)
-            c0 = t0 * kTile;
-            c1 = min(t1 * kTile, len);
-            const int first = (int)((((long long)b0 + 1) * ctas + total - 1) / total) - 1, last = (int)(((long long)(b0 + tl) * ctas + total - 1) / total) - 1;
-            split = blockIdx.x - first;
-            if (split == 0)  // places of parts that this context does not have
-                for (int i = tid; i < GQ * (p.splits - 1 - (last - first)); i += kTcWarps * 32)
-                    p.pm[((size_t)st * p.nh + kvh * GQ + i % GQ) * p.splits + last - first + 1 + i / GQ] = -INFINITY;
-        } else {
-            if (item >= items) break;
-            kvh = item % p.nkv;
-            split = item / p.nkv % p.splits;
-            st = item / p.nkv / p.splits;
-            item += gridDim.x;
-            slot = cache_slot(p.slot_map, st / p.T);
+        for (int item = blockIdx.x; item < items; item += gridDim.x) {
+            const int kvh = item % p.nkv, rest = item / p.nkv, split = rest % p.splits, st = rest / p.splits;
+            const int slot = cache_slot(p.slot_map, st / p.T);
             const TqSpan span = tq_span(p, st, slot);
             if (split * span.chunk >= span.len) {  // (the whole CTA)
                 if (tid < GQ) p.pm[((size_t)st * p.nh + kvh * GQ + tid) * p.splits + split] = -INFINITY;
                 continue;
             }
-            c0 = split * span.chunk;
-            c1 = min(c0 + span.chunk, span.len);
+            const int c0 = split * span.chunk;
+            tc_part<GQ, BITS>(p, lut, pw, comb, st, kvh, split, slot, c0, min(c0 + span.chunk, span.len));
         }
-        // this warp's tiles of the split's range: every kTcWarps-th
-        const int tiles = (c1 - c0 + kTile - 1) / kTile;
-        const int h0 = kvh * GQ;
-        const size_t head_base = ((size_t)slot * p.nkv + kvh) * p.max_seq;
-        const uint8_t *krow = p.kc + head_base * kRowB, *vrow = p.vc + head_base * kRowB;
-
-        // B fragments of the score products: lane (n = g, t) holds dims 32 t + 2 i, + 1 of column n: the rotated query
-        // of head n (n < GQ) or S q of head n - 4 (4 <= n < 4 + GQ); zero otherwise
-        unsigned bx[16];
-#pragma unroll
-        for (int i = 0; i < 16; i++) bx[i] = 0u;
-        if (g < GQ || (g >= 4 && g < 4 + GQ)) {
-            const float *src = p.qrot + ((size_t)st * p.nh + h0 + (g < 4 ? g : g - 4)) * 2 * kHd + (g < 4 ? 0 : kHd) + 32 * t;
-#pragma unroll
-            for (int j = 0; j < 8; j++) {
-                const float4 v = *reinterpret_cast<const float4 *>(src + 4 * j);
-                bx[2 * j] = pack_h2(v.x, v.y);
-                bx[2 * j + 1] = pack_h2(v.z, v.w);
-            }
-        }
-
-        float m_run[2] = {-INFINITY, -INFINITY}, l_run[2] = {0.0f, 0.0f};  // lanes t < 2: heads 2t, 2t + 1
-        float o[8][4];                                                       // o[mb]: dims 16g + 2mb, +1 (rows) x heads 2t, 2t+1
-#pragma unroll
-        for (int i = 0; i < 8; i++) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.0f;
-
-        // K rows g, g+8, g+16, g+24 of a tile: dims 32t .. 32t+31 each (32 bytes, or 16 bytes of nibbles), and the rows' factors
-        uint4 kq[4][kKV];
-        float ksv[4], rwv[4], vsv[4];
-        auto request = [&](int ts) {
-#pragma unroll
-            for (int r = 0; r < 4; r++) {
-                const int pos = ts + g + 8 * r;
-                ksv[r] = rwv[r] = vsv[r] = 0.0f;
-#pragma unroll
-                for (int v = 0; v < kKV; v++) kq[r][v] = make_uint4(0, 0, 0, 0);
-                if (pos < c1) {
-                    const uint4 *src = reinterpret_cast<const uint4 *>(krow + (size_t)pos * kRowB + (kRowB / 4) * t);
-#pragma unroll
-                    for (int v = 0; v < kKV; v++) kq[r][v] = __ldcs(src + v);
-                    ksv[r] = p.ks[head_base + pos];
-                    rwv[r] = p.krn[head_base + pos];
-                    vsv[r] = p.vs[head_base + pos];
-                }
-            }
-        };
-        request(c0 + warp * kTile);
-        for (int tile = warp; tile < tiles; tile += kTcWarps) {
-            const int ts = c0 + tile * kTile, nt = min(kTile, c1 - ts);
-            // ---- V rows 2t, 2t+1, 2t+8, 2t+9 (+16): dims 16g .. 16g+15 each (16 bytes, or 8 bytes of nibbles in .x/.y), in flight during the scores ----
-            uint4 vq[8];
-#pragma unroll
-            for (int r = 0; r < 8; r++) {
-                const int pos = 2 * t + (r & 1) + 8 * ((r >> 1) & 1) + 16 * (r >> 2);
-                vq[r] = make_uint4(0, 0, 0, 0);
-                if (pos < nt) {
-                    if (BITS == 8) {
-                        vq[r] = __ldcs(reinterpret_cast<const uint4 *>(vrow + (size_t)(ts + pos) * kRowB + 16 * g));
-                    } else {
-                        const uint2 v2 = __ldcs(reinterpret_cast<const uint2 *>(vrow + (size_t)(ts + pos) * kRowB + 8 * g));
-                        vq[r].x = v2.x;
-                        vq[r].y = v2.y;
-                    }
-                }
-            }
-            // ---- scores: a product of 16 positions x (centroid, sign) of eight dimensions per step, two row blocks ----
-            float sc[2][4];  // [row block][c0..c3]
-#pragma unroll
-            for (int rb = 0; rb < 2; rb++) sc[rb][0] = sc[rb][1] = sc[rb][2] = sc[rb][3] = 0.0f;
-#pragma unroll
-            for (int i = 0; i < 16; i++) {  // dims 32 t + 2 i, + 1
-                const unsigned b0 = __byte_perm(bx[i], 0, sel0), b1 = __byte_perm(bx[i], 0, sel1);
-                const int w = BITS == 8 ? i >> 1 : i >> 2, e = BITS == 8 ? 2 * (i & 1) : 2 * (i & 3);
-#pragma unroll
-                for (int rb = 0; rb < 2; rb++) {
-                    const unsigned a = reinterpret_cast<const unsigned *>(&kq[2 * rb][0])[w], b = reinterpret_cast<const unsigned *>(&kq[2 * rb + 1][0])[w];  // rows g, g + 8 (+ 16 rb)
-                    mma_f16(sc[rb], lut_at<BITS>(lut, lane_k, a, e), lut_at<BITS>(lut, lane_k, b, e), lut_at<BITS>(lut, lane_k, a, e + 1), lut_at<BITS>(lut, lane_k, b, e + 1),
-                            b0, b1);
-                }
-            }
-            // lanes t < 2 hold the centroid sums of heads 2t, 2t+1; lanes t + 2 the sign sums of the same heads
-            float s[4][2], vw[4];  // [position g + 8 r][head 2t + i]
-#pragma unroll
-            for (int rb = 0; rb < 2; rb++)
-#pragma unroll
-                for (int q = 0; q < 4; q++) {
-                    const float other = __shfl_xor_sync(0xffffffffu, sc[rb][q], 2);
-                    const int r = 2 * rb + (q >> 1), i = q & 1;  // c0,c1: row g ; c2,c3: row g + 8
-                    const bool live = t < 2 && g + 8 * r < nt;  // lanes t >= 2 only feed the shuffle above
-                    s[r][i] = live ? p.attn_scale * (ksv[r] * (sc[rb][q] + rwv[r] * p.qjl_factor * other)) : -INFINITY;
-                }
-#pragma unroll
-            for (int r = 0; r < 4; r++) vw[r] = vsv[r];
-            request(tile + kTcWarps < tiles ? ts + kTcWarps * kTile : c1);  // the next tile's K rows travel during the rest of this one
-            // ---- online softmax over the tile (meaningful on lanes t < 2; the others carry copies of no use) ----
-            float wgt[4][2];
+    } else {
+        __shared__ TcPlan plan;
+        if (warp == 0) {
+            int tiles[2], parts[2], most = 0, shortest = 0x7fffffff, longest = 0;
 #pragma unroll
             for (int i = 0; i < 2; i++) {
-                float mx = fmaxf(fmaxf(s[0][i], s[1][i]), fmaxf(s[2][i], s[3][i]));
-                mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 4));
-                mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 8));
-                mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 16));
-                const float m_new = fmaxf(m_run[i], mx);
-                const float corr = m_new == -INFINITY ? 1.0f : __expf(m_run[i] - m_new);
-                float sum = 0.0f;
-#pragma unroll
-                for (int r = 0; r < 4; r++) {
-                    wgt[r][i] = s[r][i] == -INFINITY ? 0.0f : __expf(s[r][i] - m_new);
-                    sum += wgt[r][i];
-                }
-                l_run[i] = l_run[i] * corr + sum;  // this lane's own positions; added up over the lanes at the end
-                m_run[i] = m_new;
-                if (__any_sync(0xffffffffu, corr != 1.0f)) {
-#pragma unroll
-                    for (int mb = 0; mb < 8; mb++) {  // heads 2t + i live in accumulator columns i (rows d0) and i + 2 (rows d1)
-                        o[mb][i] *= corr;
-                        o[mb][i + 2] *= corr;
-                    }
-                }
+                const int st = 2 * lane + i;
+                TqSpan span{0, kTile};
+                if (st < p.shares) span = tq_span(p, st, cache_slot(p.slot_map, st / p.T));
+                plan.len[st] = span.len;
+                plan.chunk[st] = span.chunk;
+                const int n = (span.len + kTile - 1) / kTile;
+                most = max(most, n);
+                longest = max(longest, min(span.chunk / kTile, n));
+                if (n > 0) shortest = min(shortest, n);
+                tiles[i] = n * p.nkv;
+                parts[i] = (span.len + span.chunk - 1) / span.chunk * p.nkv;
             }
-            // weights x V scale, as fp16, to this warp's P[head][position] for the output products
-            __syncwarp();
-            if (t < 2) {
+            int a = tiles[0] + tiles[1], b = parts[0] + parts[1];
 #pragma unroll
-                for (int r = 0; r < 4; r++)
-#pragma unroll
-                    for (int i = 0; i < 2; i++)
-                        if (2 * t + i < 4) pwarp[(2 * t + i) * 32 + g + 8 * r] = __float2half_rn(wgt[r][i] * vw[r]);
+            for (int d = 1; d < 32; d <<= 1) {
+                const int x = __shfl_up_sync(0xffffffffu, a, d), y = __shfl_up_sync(0xffffffffu, b, d);
+                if (lane >= d) a += x, b += y;
             }
-            __syncwarp();
-            // ---- outputs: O^T[dims][heads] += V^T[dims][positions] P^T[positions][heads] ----
-#pragma unroll
-            for (int kb = 0; kb < 2; kb++) {
-                unsigned b0 = 0u, b1 = 0u;  // lane (n = g): P[head g][16 kb + 2t, +1] and [.. + 8, + 9]
-                if (g < GQ) {
-                    b0 = *reinterpret_cast<const unsigned *>(pwarp + g * 32 + 16 * kb + 2 * t);
-                    b1 = *reinterpret_cast<const unsigned *>(pwarp + g * 32 + 16 * kb + 2 * t + 8);
-                }
-                const unsigned *v0 = reinterpret_cast<const unsigned *>(&vq[4 * kb + 0]);  // position 16 kb + 2t
-                const unsigned *v1 = reinterpret_cast<const unsigned *>(&vq[4 * kb + 1]);  // + 1
-                const unsigned *v2 = reinterpret_cast<const unsigned *>(&vq[4 * kb + 2]);  // + 8
-                const unsigned *v3 = reinterpret_cast<const unsigned *>(&vq[4 * kb + 3]);  // + 9
-#pragma unroll
-                for (int mb = 0; mb < 8; mb++) {  // rows g, g + 8 of the block: dims 16 g + 2 mb, + 1
-                    const int w = BITS == 8 ? mb >> 1 : mb >> 2, by = BITS == 8 ? 2 * (mb & 1) : 2 * (mb & 3);
-                    auto pair = [&](unsigned x, unsigned y, int e) {
-                        return __byte_perm(lut_at<BITS>(lut, lane_v, x, e), lut_at<BITS>(lut, lane_v, y, e), 0x5410);
-                    };
-                    mma_f16(o[mb], pair(v0[w], v1[w], by), pair(v0[w], v1[w], by + 1), pair(v2[w], v3[w], by), pair(v2[w], v3[w], by + 1), b0, b1);
-                }
-            }
-        }
-#pragma unroll
-        for (int i = 0; i < 2; i++)
-#pragma unroll
-            for (int d = 4; d < 32; d <<= 1) l_run[i] += __shfl_xor_sync(0xffffffffu, l_run[i], d);
-
-        // ---- merge the warps: comb[warp][head][130] = o (dims 0..127), m, l ----
-        __syncthreads();  // the previous item's sums have been read
-        if (t < 2) {
-#pragma unroll
-            for (int i = 0; i < 2; i++) {
-                const int h = 2 * t + i;
-                if (h < 4) {
-                    float *dst = comb + (warp * 4 + h) * 130;
-#pragma unroll
-                    for (int mb = 0; mb < 8; mb++) {
-                        dst[16 * g + 2 * mb] = o[mb][i];
-                        dst[16 * g + 2 * mb + 1] = o[mb][i + 2];
-                    }
-                    if (g == 0) {
-                        dst[128] = m_run[i];
-                        dst[129] = l_run[i];
-                    }
-                }
+            plan.tiles[2 * lane + 1] = a - tiles[1];
+            plan.parts[2 * lane + 1] = b - parts[1];
+            plan.tiles[2 * lane + 2] = a;
+            plan.parts[2 * lane + 2] = b;
+            const int total = __shfl_sync(0xffffffffu, a, 31), all = __shfl_sync(0xffffffffu, b, 31);
+            most = __reduce_max_sync(0xffffffffu, most);
+            shortest = __reduce_min_sync(0xffffffffu, shortest);
+            longest = __reduce_max_sync(0xffffffffu, longest);
+            if (lane == 0) {
+                plan.tiles[0] = plan.parts[0] = 0;
+                // tiles of a share: a context of L tiles touches at most (L - 1) / least + 2 shares
+                const int least = max((most + p.splits - 2) / (p.splits - 1), 1), ctas = max(min((int)gridDim.x, total / least), 1), share = total / ctas,
+                          mean = total / (int)gridDim.x;
+                plan.ctas = ctas;
+                plan.equal = mean >= kTcShareTiles && 4 * share <= 5 * max(longest, mean) && share <= kTcShareContexts * shortest &&
+                             (all > (int)gridDim.x || 4 * longest > 5 * share);
+                const bool mine = (int)blockIdx.x < ctas && plan.equal;
+                plan.next = mine ? (int)((long long)total * blockIdx.x / ctas) : 0;
+                plan.end = mine ? (int)((long long)total * (blockIdx.x + 1) / ctas) : 0;
             }
         }
         __syncthreads();
-        for (int idx = tid; idx < GQ * kHd; idx += kTcWarps * 32) {
-            const int h = idx >> 7, d = idx & 127;
-            float gm = -INFINITY;
-#pragma unroll
-            for (int w = 0; w < kTcWarps; w++) gm = fmaxf(gm, comb[(w * 4 + h) * 130 + 128]);
-            float acc = 0.0f, lsum = 0.0f;
-#pragma unroll
-            for (int w = 0; w < kTcWarps; w++) {
-                const float m = comb[(w * 4 + h) * 130 + 128];
-                const float corr = m == -INFINITY ? 0.0f : __expf(m - gm);
-                acc += comb[(w * 4 + h) * 130 + d] * corr;
-                lsum += comb[(w * 4 + h) * 130 + 129] * corr;
+        if (blockIdx.x == 0)  // tokens that see nothing
+            for (int st = warp; st < p.shares; st += kTcWarps)
+                if (plan.len[st] == 0)
+                    for (int i = lane; i < p.nh * p.splits; i += 32) p.pm[(size_t)st * p.nh * p.splits + i] = -INFINITY;
+        auto absent = [&](int st, int kvh, int n) {  // places of parts that a context does not have
+            for (int i = tid; i < GQ * (p.splits - n); i += kTcWarps * 32) p.pm[((size_t)st * p.nh + kvh * GQ + i % GQ) * p.splits + n + i / GQ] = -INFINITY;
+        };
+        if (plan.equal) {
+            for (;;) {
+                const int u = plan.next, u1 = plan.end, total = plan.tiles[kTcShareTokens], ctas = plan.ctas;
+                if (u >= u1) break;
+                __syncthreads();  // everyone has read where the run goes on
+                const int st = plan_token(plan.tiles, u), len = plan.len[st], tl = (len + kTile - 1) / kTile, at = u - plan.tiles[st], kvh = at / tl, t0 = at - kvh * tl,
+                          t1 = min(tl, t0 + u1 - u), b0 = u - t0;
+                if (tid == 0) plan.next = u + t1 - t0;  // (read after the part's barriers)
+                const int first = (int)((((long long)b0 + 1) * ctas + total - 1) / total) - 1, last = (int)(((long long)(b0 + tl) * ctas + total - 1) / total) - 1;
+                const int split = blockIdx.x - first;
+                if (split == 0) absent(st, kvh, last - first + 1);
+                tc_part<GQ, BITS>(p, lut, pw, comb, st, kvh, split, cache_slot(p.slot_map, st / p.T), t0 * kTile, min(t1 * kTile, len));
             }
-            const size_t pi = ((size_t)st * p.nh + h0 + h) * p.splits + split;
-            p.po[pi * kHd + d] = acc;
-            if (d == 0) {
-                p.pm[pi] = gm;
-                p.pl[pi] = lsum;
+        } else {
+            for (int item = blockIdx.x; item < plan.parts[kTcShareTokens]; item += gridDim.x) {
+                const int st = plan_token(plan.parts, item), at = item - plan.parts[st], split = at / p.nkv, kvh = at - split * p.nkv, c0 = split * plan.chunk[st];
+                if (split == 0) absent(st, kvh, (plan.parts[st + 1] - plan.parts[st]) / p.nkv);
+                tc_part<GQ, BITS>(p, lut, pw, comb, st, kvh, split, cache_slot(p.slot_map, st / p.T), c0, min(c0 + plan.chunk[st], plan.len[st]));
             }
         }
     }
@@ -737,12 +767,12 @@ int tq_prep_launch(const Tq *tq, const TqPrep &a, cudaStream_t st) {
     return IM_OK;
 }
 
-// Contexts that can fill shares of kTcShareTiles tiles for two CTAs per SM (the kernel looks again at what they are: the looking costs shorter ones 5 %, a
-// step of four sequences of 1024 positions 991 -> 1051 us)
+// Launches whose contexts may be dealt out as equal shares: no more of them than CTAs (64 of 256 .. 2020 positions, eight KV heads: 88 us in parts, 107 in
+// shares), and a cache that can fill the CTAs with 16 tiles each (the kernel looks again at what the contexts are; the looking costs shorter ones 5 %).
 static bool tq_shares(const Device *dev, int nseq, int T, int nh, int nkv, int seq_len) {
     const int gq = nkv > 0 ? nh / nkv : 0;
-    return (gq == 1 || gq == 2 || gq == 4) && (long long)nseq * T <= kTcShareTokens &&
-           (long long)nseq * T * nkv * ((seq_len + kTile - 1) / kTile) >= 2ll * dev->sm_count * kTcShareTiles;
+    const long long contexts = (long long)nseq * T * nkv, fill = 2ll * dev->sm_count;
+    return (gq == 1 || gq == 2 || gq == 4) && (long long)nseq * T <= kTcShareTokens && contexts <= fill && contexts * ((seq_len + kTile - 1) / kTile) >= 16 * fill;
 }
 // Parts that the positions of a (sequence, token, KV head) are cut into: enough for two CTAs per SM with one tile per warp of a part; and where parts
 // can hold three tiles per warp, up to four times as many as CTAs, so that sequences of different lengths share the GPU evenly.
@@ -770,6 +800,21 @@ static int tq_call_scratch(im_tq *tq, int num_splits, int nseq, int T, int nh, i
     return rc;
 }
 
+template <int GQ, int BITS, bool SHARES>
+static int tc_launch(const Tq *tq, const AttnParams &p, unsigned grid, int items, cudaStream_t st) {
+    auto kern = tq_attention_tc_kernel<GQ, BITS, SHARES>;
+    static DeviceOnce once;  // per instantiation
+    if (once.first(tq->dev->ordinal)) IM_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTcSmem));
+    IM_CUDA_CHECK(launch_k(kern, dim3(grid), dim3(kTcWarps * 32), kTcSmem, st, p, items));
+    return IM_OK;
+}
+template <bool SHARES>
+static int tc_heads(const Tq *tq, const AttnParams &p, int gq, unsigned grid, int items, cudaStream_t st) {
+    if (tq->n_bits == 4)
+        return gq == 1 ? tc_launch<1, 4, SHARES>(tq, p, grid, items, st) : gq == 2 ? tc_launch<2, 4, SHARES>(tq, p, grid, items, st) : tc_launch<4, 4, SHARES>(tq, p, grid, items, st);
+    return gq == 1 ? tc_launch<1, 8, SHARES>(tq, p, grid, items, st) : gq == 2 ? tc_launch<2, 8, SHARES>(tq, p, grid, items, st) : tc_launch<4, 8, SHARES>(tq, p, grid, items, st);
+}
+
 int tq_attention_launch(const Tq *tq, float *scratch, const __half *q, const uint8_t *kc, const uint8_t *vc, const float *ks,
                         const float *vs, const float *krn, float attn_scale, __half *out, int nseq, int nh, int nkv, int max_seq,
                         int base_pos, const int *pos_dev, int T, int splits, bool own_parts, cudaStream_t st, const float *qrot, const int *slot_map) {
@@ -791,21 +836,11 @@ int tq_attention_launch(const Tq *tq, float *scratch, const __half *q, const uin
     dim3 grid(nkv, nseq * T, splits);
     const int gq = nh / nkv;
     if (qrot && (gq == 1 || gq == 2 || gq == 4) && nh % nkv == 0) {  // tensor-core kernel (needs the rotated queries)
-        static DeviceOnce once;
-        if (once.first(tq->dev->ordinal)) {  // the instantiations share one function-pointer type: set them all once
-            IM_CUDA_CHECK(cudaFuncSetAttribute(tq_attention_tc_kernel<1, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTcSmem));
-            IM_CUDA_CHECK(cudaFuncSetAttribute(tq_attention_tc_kernel<2, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTcSmem));
-            IM_CUDA_CHECK(cudaFuncSetAttribute(tq_attention_tc_kernel<4, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTcSmem));
-            IM_CUDA_CHECK(cudaFuncSetAttribute(tq_attention_tc_kernel<1, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTcSmem));
-            IM_CUDA_CHECK(cudaFuncSetAttribute(tq_attention_tc_kernel<2, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTcSmem));
-            IM_CUDA_CHECK(cudaFuncSetAttribute(tq_attention_tc_kernel<4, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTcSmem));
-        }
-        auto kern = tq->n_bits == 4 ? (gq == 1 ? tq_attention_tc_kernel<1, 4> : (gq == 2 ? tq_attention_tc_kernel<2, 4> : tq_attention_tc_kernel<4, 4>))
-                                    : (gq == 1 ? tq_attention_tc_kernel<1, 8> : (gq == 2 ? tq_attention_tc_kernel<2, 8> : tq_attention_tc_kernel<4, 8>));
-        const long long items = (long long)nkv * nseq * T * splits;
-        if (own_parts && splits > 1 && tq_shares(tq->dev, nseq, T, nh, nkv, pos_dev ? max_seq : base_pos + T)) p.shares = nseq * T;
+        const long long items = (long long)nkv * nseq * T * splits, fill = 2ll * tq->dev->sm_count;
         if (items > 0x7fffffffll) return fail(IM_ERR_BOUNDS, "attention over %lld parts", items);
-        IM_CUDA_CHECK(launch_k(kern, dim3((unsigned)(p.shares ? 2ll * tq->dev->sm_count : std::min(items, 2ll * tq->dev->sm_count))), dim3(kTcWarps * 32), kTcSmem, st, p, (int)items));
+        if (own_parts && splits > 1 && tq_shares(tq->dev, nseq, T, nh, nkv, pos_dev ? max_seq : base_pos + T)) p.shares = nseq * T;
+        const int rc = p.shares ? tc_heads<true>(tq, p, gq, (unsigned)fill, (int)items, st) : tc_heads<false>(tq, p, gq, (unsigned)std::min(items, fill), (int)items, st);
+        if (rc != IM_OK) return rc;
     } else
     {
         const bool b4 = tq->n_bits == 4;
