@@ -28,8 +28,9 @@ __device__ __forceinline__ float load_weight(const __half *w, const __half *awq,
 // Codes without a division per element: t = x * (1 / scale) + zp differs from the defining fl(fl(x / scale) + zp) by less
 // than 2^-20 (|x / scale| + |zp| + 1), so the two round to the same integer unless t lies that close to a half; an octet
 // with such a value (or a magnitude past 2^21) is recomputed by the definition.  An octet without one needs no clamp: x lies between the group's
-// extrema, so t is at most a half outside 0 .. qmax, give or take that error.  Groups with a value that is not finite, or whose minimum is a zero
-// (of equal extrema the first counts, and the sign of a zero shows in the zero point), take quantize_row_any.
+// extrema, so t is at most a half outside 0 .. qmax, give or take that error.  Groups with a value that is not finite take quantize_row_any.  Of a minimum
+// of zero the first place counts (its sign shows in the zero point): looked for only in warps that have one.  Nothing but zeros, 14336 x 4096, 4-bit with AWQ:
+// 176 us by quantize_row_any, 68 so.
 
 __device__ __forceinline__ unsigned quantize_one(float x, float scale, float zp, float qmax);
 
@@ -84,7 +85,7 @@ __device__ __forceinline__ void store_codes(uint8_t *packed, size_t octet, const
     }
 }
 
-// A row's share of a lane by the definition, whatever its values: all lanes of the warp.  octets: where the lane's octets lie, dead ones negative.
+// A lane's octets of a group by the definition, whatever its values: all lanes of the warp.  live: how many of them lie in the row (the others repeat the last one).
 template <int BITS, int C, bool AWQ>
 __device__ __noinline__ void quantize_row_any(const uint4 (&w)[C], const uint4 (&a)[C], int lane_of_group, int P, int live, size_t octet0, bool store, float *scale_out,
                                               float *zp_out, uint8_t *packed) {
@@ -125,8 +126,24 @@ __device__ __noinline__ void quantize_row_any(const uint4 (&w)[C], const uint4 (
     }
 }
 
+// Place of a group's first zero, its sign in the lowest bit: all lanes of the warp.  (Inlined, it takes ordinary groups 2 % of their time.)
+template <int C, bool AWQ>
+__device__ __noinline__ unsigned quantize_first_zero(const uint4 (&w)[C], const uint4 (&a)[C], unsigned lane_of_group, int P) {
+    unsigned first = 0xffffffffu;
+#pragma unroll
+    for (int i = 0; i < C; i++) {
+        float x[8];
+        quantize_values<AWQ>(w[i], a[i], x);
+#pragma unroll
+        for (int j = 0; j < 8; j++)
+            if (x[j] == 0.0f) first = min(first, ((lane_of_group + (unsigned)(i * P)) * 8 + j) * 2 + (__float_as_uint(x[j]) >> 31));
+    }
+    for (int o = P >> 1; o > 0; o >>= 1) first = min(first, __shfl_xor_sync(0xffffffffu, first, o));
+    return first;
+}
+
 template <int BITS, int C, bool AWQ>
-__global__ void __launch_bounds__(256, C == 8 ? 2 : 4) quantize_groups_kernel(const __half *__restrict__ w, const __half *__restrict__ awq, size_t rows, unsigned K, int P,
+__global__ void __launch_bounds__(256, 4) quantize_groups_kernel(const __half *__restrict__ w, const __half *__restrict__ awq, size_t rows, unsigned K, int P,
                                                                               unsigned G, float *__restrict__ scales, float *__restrict__ zps, uint8_t *__restrict__ packed) {
     constexpr float qmax = BITS == 4 ? 15.0f : 255.0f;
     constexpr float kMagic = 12582912.0f;  // 1.5 * 2^23: adding it rounds to an integer in the low mantissa bits
@@ -161,8 +178,12 @@ __global__ void __launch_bounds__(256, C == 8 ? 2 : 4) quantize_groups_kernel(co
         mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
     }
     if (__any_sync(0xffffffffu, !isfinite(mn) || !isfinite(mx) || mn == 0.0f)) {
-        quantize_row_any<BITS, C, AWQ>(raw, a, (int)p, P, live, octet0, store, scales + at, zps + at, packed);
-        return;
+        if (__any_sync(0xffffffffu, !isfinite(mn) || !isfinite(mx))) {
+            quantize_row_any<BITS, C, AWQ>(raw, a, (int)p, P, live, octet0, store, scales + at, zps + at, packed);
+            return;
+        }
+        const unsigned first = quantize_first_zero<C, AWQ>(raw, a, p, P);
+        if (mn == 0.0f) mn = __uint_as_float(first << 31);
     }
     float scale, zp;
     quantize_scale(mn, mx, true, qmax, scale, zp);
