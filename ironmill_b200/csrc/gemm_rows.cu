@@ -692,7 +692,8 @@ int rows_start(void (*kern)(RowsParams), int grid, int cluster, int threads, siz
     return IM_OK;
 }
 
-// Clusters of a size that the GPU holds at once, one CTA on an SM (asked for once per device: a cluster lies within a GPC, whose SMs need not divide evenly)
+// Clusters of a size that the GPU holds at once (a cluster lies within a GPC, whose SMs need not divide evenly); asked for once per form and device
+template <int NT, int BITS, bool INT>
 int rows_clusters(void (*kern)(RowsParams), int size, int threads, size_t smem, const Device *dev) {
     static std::atomic<int> held[64][kRMaxCluster + 1];
     const int at = dev->ordinal >= 0 && dev->ordinal < 64 ? dev->ordinal : -1;
@@ -710,7 +711,7 @@ int rows_clusters(void (*kern)(RowsParams), int size, int threads, size_t smem, 
     int n = 0;
     if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess) {
         cudaGetLastError();
-        n = 0;
+        return 0;  // (asked again next time)
     }
     if (at >= 0) held[at][size].store(n + 1);
     return n;
@@ -731,7 +732,7 @@ int rows_launch(RowsParams p, const Device *dev, cudaStream_t st) {
     // as long as they are not that much longer.
     const int tiles = p.total / p.G;
     p.slices = std::min(std::min(dev->sm_count / tiles, kRMaxCluster), std::max(1, p.G / KQ));
-    while (p.slices > 1 && rows_clusters(kern, p.slices, NW * 32, smem, dev) < tiles) p.slices--;
+    while (p.slices > 1 && rows_clusters<NT, BITS, INT>(kern, p.slices, NW * 32, smem, dev) < tiles) p.slices--;
     const int grid = (int)std::min<size_t>(std::min(dev->sm_count, std::max(1, p.total / KQ)), kGemmPartialBytes / ((size_t)2 * MP * kRRows * sizeof(float)));
     const int stages_sliced = p.slices > 0 ? ((p.G + p.slices - 1) / p.slices + KQ - 1) / KQ : 0, stages_shared = ((p.total + grid - 1) / grid + KQ - 1) / KQ;
     if (p.slices < 1 || stages_sliced > stages_shared + 3) p.slices = 1;
