@@ -17,9 +17,9 @@
 //   * tokens: packed for these fragments by the kernel that writes them (token_chunk below): the lane's four fragment registers
 //     of a token and eight columns are 16 contiguous bytes.  One thread brings the slabs of a few groups by cp.async.bulk;
 //   * a CTA works on 128 rows (four row-block pairs) with its warps on different groups of K.  Few row tiles: each belongs to a cluster
-//     of up to eight CTAs on slices of K, which add their sums through distributed shared memory.  Many: a CTA takes an equal
-//     share of the flattened [row tile][group] list, and row tiles cut by a CTA boundary are completed by whichever of their
-//     CTAs arrives last (a counter, nobody waits), adding the parts in CTA order.
+//     of up to eight CTAs on slices of K, which add their sums through distributed shared memory.  Many: a CTA each or,
+//     where the last wave would leave too many SMs idle, an equal share of the flattened [row tile][group] list; row tiles cut by a CTA boundary are
+//     completed by whichever of their CTAs arrives last (a counter, nobody waits), adding the parts in CTA order.
 // The joint form multiplies gate rows and up rows as the pair of row blocks and leaves f16(silu(f16 gate) f16(up)), if asked
 // divided by the next projection's activation scales and packed for it.
 //
@@ -55,6 +55,11 @@ template <int NT, bool INT>
 constexpr int rows_slab_max() { return INT ? planes_slab(NT * 2) : NT * 8 * 256; }
 template <int BITS>
 constexpr int rows_unit_bytes() { return 2 * TileGeom<BITS>::kTileBytes; }
+template <int NT, int BITS, bool INT>
+constexpr size_t rows_smem_bytes() {  // rings of tiles, token slabs, sums, barriers and the flag
+    return (size_t)rows_warps<NT, BITS, INT>() * rows_depth<NT, BITS, INT>() * rows_unit_bytes<BITS>() + (size_t)kRBStages * rows_klanes<NT, BITS, INT>() * rows_slab_max<NT, INT>() + 512 +
+           (size_t)(rows_klanes<NT, BITS, INT>() / 2) * rows_tokens<NT, INT>() * kRPad * 4 + 2 * kRBStages * 8 + 16;
+}
 
 struct RowsParams {
     const uint8_t *tiles[2];  // joint: gate, up; else both the matrix
@@ -694,14 +699,14 @@ int rows_start(void (*kern)(RowsParams), int grid, int cluster, int threads, siz
 
 // Clusters of a size that the GPU holds at once (a cluster lies within a GPC, whose SMs need not divide evenly); asked for once per form and device
 template <int NT, int BITS, bool INT>
-int rows_clusters(void (*kern)(RowsParams), int size, int threads, size_t smem, const Device *dev) {
+int rows_clusters(int size, const Device *dev) {
     static std::atomic<int> held[64][kRMaxCluster + 1];
     const int at = dev->ordinal >= 0 && dev->ordinal < 64 ? dev->ordinal : -1;
     if (at >= 0 && held[at][size].load() > 0) return held[at][size].load() - 1;
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(size);
-    cfg.blockDim = dim3(threads);
-    cfg.dynamicSmemBytes = smem;
+    cfg.blockDim = dim3(rows_warps<NT, BITS, INT>() * 32);
+    cfg.dynamicSmemBytes = rows_smem_bytes<NT, BITS, INT>();
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = size;
@@ -709,7 +714,7 @@ int rows_clusters(void (*kern)(RowsParams), int size, int threads, size_t smem, 
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess) {
+    if (cudaOccupancyMaxActiveClusters(&n, gemm_rows_kernel<NT, BITS, INT>, &cfg) != cudaSuccess) {
         cudaGetLastError();
         return 0;  // (asked again next time)
     }
@@ -717,27 +722,38 @@ int rows_clusters(void (*kern)(RowsParams), int size, int threads, size_t smem, 
     return n;
 }
 
+// How the row tiles are dealt out: a cluster of CTAs on slices of K for each, where there are few; a CTA for each; or equal shares of the list of all groups.
+struct RowsPlan {
+    int grid, slices;
+};
+// Counted in groups of K that the longest CTA takes.  The two ends of a share (sums and parts of two tiles through memory, a counter, the last CTA's
+// sum) cost as much as 11 to 18 of a launch by itself (24 tokens, 28672 x 2048 in two waves of whole tiles 24.2 us, in shares 26.8; 12288 x 4096 19.7 and 22.9;
+// 10240 x 8192 34.0 and 29.9), and 12 are the best line in whole steps (four 8B layers, 12 rows, gate and up: 64 groups or 49 in shares 662 and 649 us).
+constexpr int kRShareEnds = 12;
 template <int NT, int BITS, bool INT>
-int rows_launch(RowsParams p, const Device *dev, cudaStream_t st) {
-    constexpr int NW = rows_warps<NT, BITS, INT>(), KQ = rows_klanes<NT, BITS, INT>(), MP = rows_tokens<NT, INT>();
-    constexpr size_t smem = (size_t)NW * rows_depth<NT, BITS, INT>() * rows_unit_bytes<BITS>() + (size_t)kRBStages * KQ * rows_slab_max<NT, INT>() + 512 +
-                            (size_t)(KQ / 2) * MP * kRPad * 4 + 2 * kRBStages * 8 + 16;
+int rows_plan(int tiles, int G, const Device *dev, RowsPlan *out) {
+    constexpr int KQ = rows_klanes<NT, BITS, INT>(), MP = rows_tokens<NT, INT>();
+    constexpr size_t smem = rows_smem_bytes<NT, BITS, INT>();
     static_assert(smem <= 227 * 1024, "the rings of this form do not fit");
     if (smem > dev->smem_optin) return IM_ERR_BOUNDS;
-    auto kern = gemm_rows_kernel<NT, BITS, INT>;
     static DeviceOnce once;  // per instantiation
-    if (once.first(dev->ordinal)) IM_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    // Few row tiles: a cluster of CTAs per tile, as many as the GPU holds (at least one stage of groups each).  Otherwise equal shares of the
-    // list (two partial tiles of each CTA fit the scratch).  The two ends of a share cost about three stages, so slices that leave SMs idle win
-    // as long as they are not that much longer.
-    const int tiles = p.total / p.G;
-    p.slices = std::min(std::min(dev->sm_count / tiles, kRMaxCluster), std::max(1, p.G / KQ));
-    while (p.slices > 1 && rows_clusters<NT, BITS, INT>(kern, p.slices, NW * 32, smem, dev) < tiles) p.slices--;
-    const int grid = (int)std::min<size_t>(std::min(dev->sm_count, std::max(1, p.total / KQ)), kGemmPartialBytes / ((size_t)2 * MP * kRRows * sizeof(float)));
-    const int stages_sliced = p.slices > 0 ? ((p.G + p.slices - 1) / p.slices + KQ - 1) / KQ : 0, stages_shared = ((p.total + grid - 1) / grid + KQ - 1) / KQ;
-    if (p.slices < 1 || stages_sliced > stages_shared + 3) p.slices = 1;
-    else if (p.slices == 1) return rows_start(kern, tiles, 1, NW * 32, smem, st, p);  // a tile per CTA
-    return rows_start(kern, p.slices > 1 ? tiles * p.slices : grid, p.slices, NW * 32, smem, st, p);
+    if (once.first(dev->ordinal)) IM_CUDA_CHECK(cudaFuncSetAttribute(gemm_rows_kernel<NT, BITS, INT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const int sms = dev->sm_count, total = tiles * G;
+    int slices = std::max(1, std::min(std::min(sms / tiles, kRMaxCluster), G / KQ));
+    while (slices > 1 && rows_clusters<NT, BITS, INT>(slices, dev) < tiles) slices--;
+    const int own = slices > 1 ? (G + slices - 1) / slices : (tiles + sms - 1) / sms * G;
+    // two partial tiles of each CTA fit the scratch
+    const int grid = (int)std::min<size_t>(std::min(sms, std::max(1, total / KQ)), kGemmPartialBytes / ((size_t)2 * MP * kRRows * sizeof(float)));
+    *out = own <= (total + grid - 1) / grid + kRShareEnds ? RowsPlan{tiles * slices, slices} : RowsPlan{grid, 1};
+    return IM_OK;
+}
+
+template <int NT, int BITS, bool INT>
+int rows_launch(RowsParams p, const Device *dev, cudaStream_t st) {
+    RowsPlan plan;
+    if (const int rc = rows_plan<NT, BITS, INT>(p.total / p.G, p.G, dev, &plan); rc != IM_OK) return rc;
+    p.slices = plan.slices;
+    return rows_start(gemm_rows_kernel<NT, BITS, INT>, plan.grid, plan.slices, rows_warps<NT, BITS, INT>() * 32, rows_smem_bytes<NT, BITS, INT>(), st, p);
 }
 
 template <int BITS>
@@ -759,11 +775,21 @@ int planes_run(const RowsParams &p, const Device *dev, cudaStream_t st) {
 
 }  // namespace
 
-// At least eight groups of K: with fewer there is nothing to stream, and the tcgen05 kernels, which do not split so short a sum, give a token the same bits
-// whatever portion of a prompt it comes in.
-bool gemm_rows_takes(const AffineWeight *w, int M) {
-    return M >= 1 && w->G >= 8 && M <= (w->bits == 4 ? kRowsMaxTokens : kRowsMaxTokens8) && w->tiles && w->group_size == 128 && w->K % 128 == 0 && (w->bits == 4 || w->bits == 8) && w->nblk <= kSkMaxBlocks &&
-           (long long)w->nblk * w->G < (1 << 30) && w->dev->gemm_partial && w->dev->sk_counters;
+// At least eight groups of K: the slices and warps of shorter sums have nothing to stream.
+// The upper half of the token range (two groups to a stage, half the warps) only where the slices of K are not much longer than those of the tcgen05 kernel,
+// whose number no cluster limits (gemm_tc.cu): a group is 0.5 us, the other's adding up 2 us, a packing pass 1.3.  40 tokens, tcgen05 / here, 4-bit:
+// 4096 x 4096 (4 and 4 slices) 14.0 / 12.2 us, 2048 x 8192 (9 and 6) 13.7 / 14.4 with packing, 6144 x 4096 (3 and 2) 15.7 / 18.0; a wave of short whole tiles that need
+// packing, 17920 x 1536, 48 tokens: 15.3 / 15.6.
+bool gemm_rows_takes(const AffineWeight *w, int M, bool packs) {
+    if (M < 1 || w->G < 8 || M > (w->bits == 4 ? kRowsMaxTokens : kRowsMaxTokens8) || !w->tiles || w->group_size != 128 || w->K % 128 != 0 || (w->bits != 4 && w->bits != 8) ||
+        w->nblk > kSkMaxBlocks || (long long)w->nblk * w->G >= (1 << 30) || !w->dev->gemm_partial || !w->dev->sk_counters)
+        return false;
+    if (M <= (w->bits == 4 ? 32 : 16)) return true;
+    const int tiles = (w->nblk + 7) / 8, sms = w->dev->sm_count, other = std::max(1, std::min(sms / tiles, w->G / 4));
+    RowsPlan plan;
+    if ((w->bits == 4 ? rows_plan<6, 4, false>(tiles, w->G, w->dev, &plan) : M <= 24 ? rows_plan<3, 8, false>(tiles, w->G, w->dev, &plan) : rows_plan<4, 8, false>(tiles, w->G, w->dev, &plan)) != IM_OK) return false;
+    if (other == 1) return !packs || tiles > sms || w->G >= 16;
+    return (w->G + plan.slices - 1) / plan.slices - (w->G + other - 1) / other <= (packs ? 0 : 4);
 }
 
 int token_pack(const __half *x, const __half *awq, __half *out, int M, int K, cudaStream_t st) {

@@ -23,7 +23,8 @@ __device__ __forceinline__ uint4 pack_chunk(const __half (&h)[8]) {
 __host__ __device__ constexpr int planes_slab(int M) { return M * 384 + (M + 1) / 2 * 16; }
 constexpr int kPlanesMaxRows = 15;  // from 16 rows on a decode step's projections are the reference's matmul form (gemm_rows, gemm_affine_tc)
 
-bool gemm_rows_takes(const AffineWeight *w, int M);
+// packs: the tokens need a packing pass that the other kernel (gemm_tc.cu) would do without
+bool gemm_rows_takes(const AffineWeight *w, int M, bool packs = false);
 // f16(x / awq) (awq may be null) of M rows of K = a multiple of 128, packed; x anywhere, out 16-byte aligned and apart from it
 int token_pack(const __half *x, const __half *awq, __half *out, int M, int K, cudaStream_t st);
 // y[M, N] = packed tokens times w; with `up` (of w's form) the gated activation of both, divided by `div` if given; pack_out: packed for the next projection

@@ -426,7 +426,7 @@ int gemm_affine_gate_up(const AffineWeight *gate, const AffineWeight *up, const 
 int gemm_affine_tc(const AffineWeight *w, const __half *x, __half *y, int M, __half *xs_scratch, cudaStream_t st, TokenForm form, bool pack) {
     if (!gemm_takes(w) || M < 1) return IM_ERR_BOUNDS;
     // Few tokens over tiled weights: gemm_rows.cu (the tokens are packed in the scratch unless they come packed).
-    if (gemm_rows_takes(w, M) && (form == kTokensPacked || pack)) {
+    if (form == kTokensPacked || (pack && gemm_rows_takes(w, M, form == kTokensScaled || !w->awq))) {
         if (form != kTokensPacked) {
             if (const int rc = token_pack(x, form == kTokensRaw ? w->awq : nullptr, xs_scratch, M, w->K, st); rc != IM_OK) return rc;
             x = xs_scratch;

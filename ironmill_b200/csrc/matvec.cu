@@ -887,7 +887,7 @@ IM_EXPORT int im_cuda_matmul_affine(const im_affine_weight *w, const void *x_dev
     const size_t nx = (size_t)M * w->K * sizeof(__half), ny = (size_t)M * w->N * sizeof(__half);
     const uintptr_t x0 = reinterpret_cast<uintptr_t>(x_dev), y0 = reinterpret_cast<uintptr_t>(y_dev), s0 = reinterpret_cast<uintptr_t>(scratch_dev);
     const bool pack = s0 % 16 == 0 && (s0 >= x0 + nx || x0 >= s0 + nx) && (s0 >= y0 + ny || y0 >= s0 + nx);
-    const bool move = !(pack && gemm_rows_takes(w, M)) && (x0 % 16 != 0 || (!w->awq && x0 < y0 + ny && y0 < x0 + nx));
+    const bool move = !(pack && gemm_rows_takes(w, M, !w->awq)) && (x0 % 16 != 0 || (!w->awq && x0 < y0 + ny && y0 < x0 + nx));
     IM_REQUIRE((!move && !w->awq) || reinterpret_cast<uintptr_t>(scratch_dev) % 16 == 0, "the scratch must be 16-byte aligned");
     if (move) {
         IM_CUDA_CHECK(cudaMemcpyAsync(scratch_dev, x_dev, nx, cudaMemcpyDeviceToDevice, as_stream(stream)));

@@ -533,14 +533,15 @@ int Model::forward(int nseq, int T, cudaStream_t st, Prof *prof, bool all_logits
         // what a projection with activation scales reads, f16(x / awq), is written by the norm and by the activation's own kernel; in the epilogues of
         // attention and of the joint projection the divisions took more time than the pass that they would save
         // (few tokens: packed, as is the activation; gemm_rows.cu)
-        const bool rows = L.ffn_joint && gemm_rows_takes(L.gate, MT) && gemm_rows_takes(L.up, MT) && gemm_rows_takes(L.down, MT);
+        const bool rows = L.ffn_joint && gemm_rows_takes(L.gate, MT) && gemm_rows_takes(L.up, MT);
         int rc = L.ffn_joint ? residual_norm_scaled(m->hidden, m->ffn_down, L.post_ln, L.gate->awq, m->norm_out, m->residual, H, MT, eps, st, rows) : IM_ERR_BOUNDS;
         TokenForm form = rc == IM_OK ? (rows ? kTokensPacked : kTokensScaled) : kTokensRaw;
         if (rc == IM_ERR_BOUNDS) rc = im_cuda_fused_residual_rms_norm(m->hidden, m->ffn_down, L.post_ln, m->norm_out, m->residual, H, MT, eps, st);
         IM_TRY(rc);
         IM_MARK(kCatResNorm);
         if (form == kTokensPacked) {
-            IM_TRY(gemm_rows(L.gate, L.up, m->norm_out, m->ffn_gate, MT, L.down->awq, true, st));
+            form = gemm_rows_takes(L.down, MT) ? kTokensPacked : kTokensScaled;
+            IM_TRY(gemm_rows(L.gate, L.up, m->norm_out, m->ffn_gate, MT, L.down->awq, form == kTokensPacked, st));
         } else if (L.ffn_joint && gemm_affine_joins(L.gate, MT)) {
             IM_TRY(gemm_affine_gate_up(L.gate, L.up, m->norm_out, m->ffn_gate, MT, m->xs_scratch, st, form));
             form = kTokensRaw;

@@ -68,6 +68,24 @@ def test_prompt_in_short_portions(chunk):
     assert np.linalg.norm(out[1] - out[0]) / np.linalg.norm(out[0]) <= 3.6e-3
 
 
+@pytest.mark.parametrize("bits,chunk", [(4, 40), (8, 20)])
+def test_prompt_whose_down_projection_is_another_kernel(bits, chunk):
+    """Gate and up joint over packed tokens, the activation left unpacked for a down projection whose slices of K would be too long for clusters (8 row tiles
+    of 14336 columns); against the prompt at once, the bound of the test above for one layer."""
+    from ironmill_b200.engine import CudaConfig, CudaInference
+    cfg = _cfg("llama", 1, 1024, 14336, 8, 4, 200, 1e6, 1e-6)
+    tensors = synth_model(cfg, seed=33, awq=True, bits=bits)
+    tokens = H.rng_for("rows-down").integers(0, 200, 3 * chunk).astype(np.uint32)
+    out = []
+    for c in (3 * chunk, chunk):
+        conf = CudaConfig(max_seq_len=128, max_batch=1, prefill_chunk_size=c)
+        conf.without_turboquant()
+        eng = CudaInference(conf)
+        eng.load_weights(DictProvider(cfg, tensors))
+        out.append(eng.prefill(tokens).astype(np.float64))
+    assert np.linalg.norm(out[1] - out[0]) / np.linalg.norm(out[0]) <= 3.6e-3
+
+
 @pytest.mark.parametrize("bits,awq,batch", [(4, True, 1), (4, True, 2), (4, False, 3), (8, True, 5), (4, True, 9), (8, False, 15)])
 def test_decode_batches_over_planes(bits, awq, batch):
     """Steps of a few sequences (planes written by the norms, Q | K | V and gate | up joint) against the oracle model of the first ones, at the gate of decode
