@@ -56,7 +56,14 @@ struct Device {
     // device handle at a time.
     float *gemm_partial = nullptr;
 };
-constexpr size_t kGemmPartialBytes = (size_t)10 << 20;
+constexpr size_t kGemmPartialBytes = (size_t)10 << 20;  // ten slices of 128 tokens x 2048 rows (dense.cu)
+// A model's own: partial sums of its projections of few tokens (K slices, gemm_tc.cu; row tiles cut by CTA boundaries, gemm_rows.cu) and the counters of cut
+// tiles, zero between launches.  One of a model's projections in flight at a time.
+struct GemmScratch {
+    float *partial = nullptr;
+    int *counters = nullptr;
+};
+constexpr size_t kGemmScratchBytes = (size_t)10 << 20;  // three slices of 128 tokens x 6144 rows; two tiles of 48 tokens x 128 rows for each SM
 constexpr int kSkMaxBlocks = 1 << 17;  // row blocks the counters cover (2M rows)
 
 // cudaFuncSetAttribute applies to the current device: remember per device ordinal (not per thread) whether a
@@ -115,9 +122,10 @@ struct V2Params {
 
 // INT4 g128 GEMM on tcgen05 / TMEM (gemm_tc.cu): y[M, N] = f16(x / awq) * dequant(w)^T; xs_scratch holds M * K halves.
 // IM_ERR_BOUNDS when the weight is not INT4 or INT8 group-128.  pack: the scratch is 16-byte aligned and shares no memory with x and y.
+// own: where partial sums may go; without it (the stand-alone call, on any stream) only up to 64 tokens over few rows are cut along K, in the device handle's scratch.
 enum TokenForm { kTokensRaw, kTokensScaled, kTokensPacked };  // x as it is; f16(x / awq); that, packed for gemm_rows.cu (where gemm_rows_takes says so)
 int gemm_affine_tc(const AffineWeight *w, const __half *x, __half *y, int M, __half *xs_scratch, cudaStream_t st, TokenForm form = kTokensRaw,
-                   bool pack = true);
+                   bool pack = true, const GemmScratch *own = nullptr);
 // The gated activation y[M, N] = f16(silu(f16(gate x)) f16(up x)) in one launch, for two weights of the same form and activation scales;
 // only where gemm_affine_joins() says so.
 bool gemm_affine_joins(const AffineWeight *gate, int M);

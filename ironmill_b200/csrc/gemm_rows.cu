@@ -67,7 +67,7 @@ struct RowsParams {
     int slab, split_row;
     __half *y;
     const __half *div;        // joint: activation scales of the next projection, or none
-    float *partial;           // [grid][2][tokens][128]
+    float *partial;           // [grid][2][tokens][128], or none: every tile has its CTAs to itself
     int *counters;            // [row tiles], zero between launches
     int *err;
     int N, G, M, nblk, total;
@@ -739,7 +739,7 @@ struct RowsPlan {
 // 10240 x 8192 34.0 and 29.9), and 12 are the best line in whole steps (four 8B layers, 12 rows, gate and up: 64 groups or 49 in shares 662 and 649 us).
 constexpr int kRShareEnds = 12;
 template <int NT, int BITS, bool INT>
-int rows_plan(int tiles, int G, const Device *dev, RowsPlan *out) {
+int rows_plan(int tiles, int G, bool shares, const Device *dev, RowsPlan *out) {
     constexpr int KQ = rows_klanes<NT, BITS, INT>(), MP = rows_tokens<NT, INT>();
     constexpr size_t smem = rows_smem_bytes<NT, BITS, INT>();
     static_assert(smem <= 227 * 1024, "the rings of this form do not fit");
@@ -751,15 +751,15 @@ int rows_plan(int tiles, int G, const Device *dev, RowsPlan *out) {
     while (slices > 1 && rows_clusters<NT, BITS, INT>(slices, dev) < tiles) slices--;
     const int own = slices > 1 ? (G + slices - 1) / slices : (tiles + sms - 1) / sms * G;
     // two partial tiles of each CTA fit the scratch
-    const int grid = (int)std::min<size_t>(std::min(sms, std::max(1, total / KQ)), kGemmPartialBytes / ((size_t)2 * MP * kRRows * sizeof(float)));
-    *out = own <= (total + grid - 1) / grid + kRShareEnds ? RowsPlan{tiles * slices, slices} : RowsPlan{grid, 1};
+    const int grid = (int)std::min<size_t>(std::min(sms, std::max(1, total / KQ)), kGemmScratchBytes / ((size_t)2 * MP * kRRows * sizeof(float)));
+    *out = !shares || own <= (total + grid - 1) / grid + kRShareEnds ? RowsPlan{tiles * slices, slices} : RowsPlan{grid, 1};
     return IM_OK;
 }
 
 template <int NT, int BITS, bool INT>
 int rows_launch(RowsParams p, const Device *dev, cudaStream_t st) {
     RowsPlan plan;
-    if (const int rc = rows_plan<NT, BITS, INT>(p.total / p.G, p.G, dev, &plan); rc != IM_OK) return rc;
+    if (const int rc = rows_plan<NT, BITS, INT>(p.total / p.G, p.G, p.partial != nullptr, dev, &plan); rc != IM_OK) return rc;
     p.slices = plan.slices;
     return rows_start(gemm_rows_kernel<NT, BITS, INT>, plan.grid, plan.slices, rows_warps<NT, BITS, INT>() * 32, rows_smem_bytes<NT, BITS, INT>(), st, p);
 }
@@ -790,12 +790,12 @@ int planes_run(const RowsParams &p, const Device *dev, cudaStream_t st) {
 // packing, 17920 x 1536, 48 tokens: 15.3 / 15.6.
 bool gemm_rows_takes(const AffineWeight *w, int M, bool packs) {
     if (M < 1 || w->G < 8 || M > (w->bits == 4 ? kRowsMaxTokens : kRowsMaxTokens8) || !w->tiles || w->group_size != 128 || w->K % 128 != 0 || (w->bits != 4 && w->bits != 8) ||
-        w->nblk > kSkMaxBlocks || (long long)w->nblk * w->G >= (1 << 30) || !w->dev->gemm_partial || !w->dev->sk_counters)
+        w->nblk > kSkMaxBlocks || (long long)w->nblk * w->G >= (1 << 30))
         return false;
     if (M <= (w->bits == 4 ? 32 : 16)) return true;
     const int tiles = (w->nblk + 7) / 8, sms = w->dev->sm_count, other = std::max(1, std::min(sms / tiles, w->G / 4));
     RowsPlan plan;
-    if ((w->bits == 4 ? rows_plan<6, 4, false>(tiles, w->G, w->dev, &plan) : M <= 24 ? rows_plan<3, 8, false>(tiles, w->G, w->dev, &plan) : rows_plan<4, 8, false>(tiles, w->G, w->dev, &plan)) != IM_OK) return false;
+    if ((w->bits == 4 ? rows_plan<6, 4, false>(tiles, w->G, false, w->dev, &plan) : M <= 24 ? rows_plan<3, 8, false>(tiles, w->G, false, w->dev, &plan) : rows_plan<4, 8, false>(tiles, w->G, false, w->dev, &plan)) != IM_OK) return false;
     if (other == 1) return !packs || tiles > sms || w->G >= 16;
     return (w->G + plan.slices - 1) / plan.slices - (w->G + other - 1) / other <= (packs ? 0 : 4);
 }
@@ -806,19 +806,19 @@ int token_pack(const __half *x, const __half *awq, __half *out, int M, int K, cu
     return IM_OK;
 }
 
-static RowsParams rows_params(const AffineWeight *w, const AffineWeight *up, __half *y, int M, int joint) {
+static RowsParams rows_params(const AffineWeight *w, const AffineWeight *up, __half *y, int M, int joint, const GemmScratch *own) {
     RowsParams p{};
     p.tiles[0] = w->tiles;
     p.tiles[1] = up ? up->tiles : w->tiles;
-    p.y = y; p.partial = w->dev->gemm_partial; p.counters = w->dev->sk_counters; p.err = w->dev->err_flag;
+    p.y = y; p.partial = own ? own->partial : nullptr; p.counters = own ? own->counters : nullptr; p.err = w->dev->err_flag;
     p.N = w->N; p.G = w->G; p.M = M; p.nblk = w->nblk; p.joint = up ? joint : 0;
     p.wide = w->N % 4 == 0 && reinterpret_cast<uintptr_t>(y) % 8 == 0;
     p.total = (up ? (w->nblk + 3) / 4 : (w->nblk + 7) / 8) * w->G;
     return p;
 }
 
-int gemm_rows(const AffineWeight *w, const AffineWeight *up, const __half *packed, __half *y, int M, const __half *div, bool pack_out, cudaStream_t st) {
-    RowsParams p = rows_params(w, up, y, M, 1);
+int gemm_rows(const AffineWeight *w, const AffineWeight *up, const __half *packed, __half *y, int M, const __half *div, bool pack_out, const GemmScratch *own, cudaStream_t st) {
+    RowsParams p = rows_params(w, up, y, M, 1, own);
     p.xs[0] = p.xs[1] = reinterpret_cast<const uint8_t *>(packed);
     p.slab = M * 256; p.split_row = 1 << 30; p.div = div; p.packed = pack_out ? 1 : 0;
     return w->bits == 8 ? rows_run<8>(p, w->dev, st) : rows_run<4>(p, w->dev, st);
@@ -840,8 +840,8 @@ int norm_planes(const __half *a, const __half *b, const __half *gamma, const __h
 }
 
 int matvec_planes(const AffineWeight *w, const AffineWeight *up, const uint8_t *planes, const uint8_t *planes_from, int split_row, __half *y, int M, bool round_gate_up,
-                  cudaStream_t st) {
-    RowsParams p = rows_params(w, up, y, M, round_gate_up ? 1 : 2);
+                  const GemmScratch *own, cudaStream_t st) {
+    RowsParams p = rows_params(w, up, y, M, round_gate_up ? 1 : 2, own);
     p.xs[0] = planes;
     p.xs[1] = planes_from ? planes_from : planes;
     p.slab = planes_slab(M); p.split_row = planes_from ? split_row : 1 << 30;

@@ -28,7 +28,8 @@ bool gemm_rows_takes(const AffineWeight *w, int M, bool packs = false);
 // f16(x / awq) (awq may be null) of M rows of K = a multiple of 128, packed; x anywhere, out 16-byte aligned and apart from it
 int token_pack(const __half *x, const __half *awq, __half *out, int M, int K, cudaStream_t st);
 // y[M, N] = packed tokens times w; with `up` (of w's form) the gated activation of both, divided by `div` if given; pack_out: packed for the next projection
-int gemm_rows(const AffineWeight *w, const AffineWeight *up, const __half *packed, __half *y, int M, const __half *div, bool pack_out, cudaStream_t st);
+// own: for parts of row tiles that CTAs share (null: none are)
+int gemm_rows(const AffineWeight *w, const AffineWeight *up, const __half *packed, __half *y, int M, const __half *div, bool pack_out, const GemmScratch *own, cudaStream_t st);
 
 // The same for rows as 24-bit integers.
 bool planes_take(const AffineWeight *w, int M);
@@ -38,6 +39,6 @@ int rows_planes(const __half *x, const __half *awq, uint8_t *planes, int M, int 
 int norm_planes(const __half *a, const __half *b, const __half *gamma, const __half *awq, __half *residual, uint8_t *u, uint8_t *n, int H, int M, float eps, cudaStream_t st);
 // y[M, N]; rows from split_row on read planes_from (null: all read planes); with `up` the gated activation, of rounded or of f32 products
 int matvec_planes(const AffineWeight *w, const AffineWeight *up, const uint8_t *planes, const uint8_t *planes_from, int split_row, __half *y, int M, bool round_gate_up,
-                  cudaStream_t st);
+                  const GemmScratch *own, cudaStream_t st);
 
 }  // namespace im

@@ -423,7 +423,7 @@ int gemm_affine_gate_up(const AffineWeight *gate, const AffineWeight *up, const 
 
 // Y[M, N] = f16(X / awq) * dequant(W)^T for M tokens.  xs_scratch: M * K halves.  IM_ERR_BOUNDS when the weight is not
 // INT4 group-128 with K a multiple of 128 (the caller falls back to the matvec kernels).
-int gemm_affine_tc(const AffineWeight *w, const __half *x, __half *y, int M, __half *xs_scratch, cudaStream_t st, TokenForm form, bool pack) {
+int gemm_affine_tc(const AffineWeight *w, const __half *x, __half *y, int M, __half *xs_scratch, cudaStream_t st, TokenForm form, bool pack, const GemmScratch *own) {
     if (!gemm_takes(w) || M < 1) return IM_ERR_BOUNDS;
     // Few tokens over tiled weights: gemm_rows.cu (the tokens are packed in the scratch unless they come packed).
     if (form == kTokensPacked || (pack && gemm_rows_takes(w, M, form == kTokensScaled || !w->awq))) {
@@ -431,7 +431,7 @@ int gemm_affine_tc(const AffineWeight *w, const __half *x, __half *y, int M, __h
             if (const int rc = token_pack(x, form == kTokensRaw ? w->awq : nullptr, xs_scratch, M, w->K, st); rc != IM_OK) return rc;
             x = xs_scratch;
         }
-        return gemm_rows(w, nullptr, x, y, M, nullptr, false, st);
+        return gemm_rows(w, nullptr, x, y, M, nullptr, false, own, st);
     }
     const __half *xs;
     if (const int rc = scaled_tokens(w, x, M, xs_scratch, form != kTokensRaw, st, &xs); rc != IM_OK) return rc;
@@ -439,14 +439,16 @@ int gemm_affine_tc(const AffineWeight *w, const __half *x, __half *y, int M, __h
     GemmParams p{w->codes, w->sz, xs, y, w->N, w->K, w->G, M, w->dev->err_flag, nullptr, w->G};
     // One token tile and few row tiles (4096-6144 rows: 32-48 CTAs of 32-112 sequential stages): split K so that the grid covers the GPU.  100 tokens over
     // 4096 x 14336: 97 -> 35 us, over 6144 x 4096 32 -> 19.  More tokens are more tiles, or CTA pairs.  At least four groups per slice; the slices' f32 sums go through
-    // the device handle's scratch (one GEMM in flight per handle, like the tiled matvec).
-    if (M <= 128 && w->N % 4 == 0 && reinterpret_cast<uintptr_t>(y) % 8 == 0 && w->dev->gemm_partial) {
+    // the model's scratch, or the device handle's (up to 64 tokens: one such call in flight per handle, like the tiled matvec).
+    float *const partial = own ? own->partial : w->dev->gemm_partial;
+    const size_t partial_bytes = own ? kGemmScratchBytes : kGemmPartialBytes;
+    if (M <= (own ? 128 : 64) && w->N % 4 == 0 && reinterpret_cast<uintptr_t>(y) % 8 == 0 && partial) {
         const int tiles = (w->N + kGM - 1) / kGM;
         int splits = std::min(w->dev->sm_count / tiles, w->G / 4);
-        while (splits > 1 && (size_t)splits * M * w->N * sizeof(float) > kGemmPartialBytes) splits--;
+        while (splits > 1 && (size_t)splits * M * w->N * sizeof(float) > partial_bytes) splits--;
         if (splits > 1) {
             p.gps = (w->G + splits - 1) / splits;
-            p.partial = w->dev->gemm_partial;
+            p.partial = partial;
         }
     }
     if (w->bits == 8) {  // superblock_matmul_int8 (affine_matmul.metal:155-290): the same kernel, byte codes

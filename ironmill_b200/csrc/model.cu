@@ -211,6 +211,7 @@ struct Model : im_model {
     __half *hidden = nullptr, *norm_out = nullptr, *residual = nullptr, *qkv = nullptr, *q_d = nullptr, *k_d = nullptr,
            *attn_out = nullptr, *ffn_down = nullptr, *ffn_gate = nullptr, *ffn_up = nullptr, *xs_scratch = nullptr, *logits = nullptr,
            *logits_all = nullptr;
+    GemmScratch gemm_scratch;
     bool gemm_ok = false;  // every projection is INT4 or INT8 group-128: forwards of 16 tokens and more run the tensor-core GEMM
     uint8_t *planes[2] = {nullptr, nullptr};  // activations of up to 15 rows as byte planes, unrounded and rounded norms (null: some weight is not tiled for it)
     float *qrot = nullptr;  // [MT, nh_l, 2, hd] rotated queries
@@ -512,7 +513,7 @@ int Model::forward(int nseq, int T, cudaStream_t st, Prof *prof, bool all_logits
         // and the residual adds are separate element-wise launches (their bytes are a rounding error next to the GEMMs).
         Layer &L = m->layers[l];
         if (l == 0) {
-            IM_TRY(gemm_affine_tc(L.qkv, m->norm_out, m->qkv, MT, m->xs_scratch, st));
+            IM_TRY(gemm_affine_tc(L.qkv, m->norm_out, m->qkv, MT, m->xs_scratch, st, kTokensRaw, true, &m->gemm_scratch));
             IM_MARK(kCatQkv);
         }
         TqPrep a{};
@@ -526,7 +527,7 @@ int Model::forward(int nseq, int T, cudaStream_t st, Prof *prof, bool all_logits
         IM_MARK(kCatKvWrite);
         IM_TRY(attention_block(m, 1, a, m->qkv, L, nseq, T, attn_scale, attn_splits, slots, st));
         IM_MARK(kCatAttn);
-        IM_TRY(gemm_affine_tc(L.o, m->attn_out, m->ffn_down, MT, m->xs_scratch, st));
+        IM_TRY(gemm_affine_tc(L.o, m->attn_out, m->ffn_down, MT, m->xs_scratch, st, kTokensRaw, true, &m->gemm_scratch));
         IM_MARK(kCatOProj);
         IM_TRY(tp_allreduce(m, m->ffn_down, (size_t)MT * H, st));  // tensor parallel: o is row-split
         if (m->world > 1) IM_MARK(kCatComm);
@@ -541,18 +542,18 @@ int Model::forward(int nseq, int T, cudaStream_t st, Prof *prof, bool all_logits
         IM_MARK(kCatResNorm);
         if (form == kTokensPacked) {
             form = gemm_rows_takes(L.down, MT) ? kTokensPacked : kTokensScaled;
-            IM_TRY(gemm_rows(L.gate, L.up, m->norm_out, m->ffn_gate, MT, L.down->awq, form == kTokensPacked, st));
+            IM_TRY(gemm_rows(L.gate, L.up, m->norm_out, m->ffn_gate, MT, L.down->awq, form == kTokensPacked, &m->gemm_scratch, st));
         } else if (L.ffn_joint && gemm_affine_joins(L.gate, MT)) {
             IM_TRY(gemm_affine_gate_up(L.gate, L.up, m->norm_out, m->ffn_gate, MT, m->xs_scratch, st, form));
             form = kTokensRaw;
         } else {
-            IM_TRY(gemm_affine_tc(L.gate, m->norm_out, m->ffn_gate, MT, m->xs_scratch, st, form));
-            IM_TRY(gemm_affine_tc(L.up, m->norm_out, m->ffn_up, MT, m->xs_scratch, st, form));
+            IM_TRY(gemm_affine_tc(L.gate, m->norm_out, m->ffn_gate, MT, m->xs_scratch, st, form, true, &m->gemm_scratch));
+            IM_TRY(gemm_affine_tc(L.up, m->norm_out, m->ffn_up, MT, m->xs_scratch, st, form, true, &m->gemm_scratch));
             IM_TRY(silu_mul_rows(m->ffn_gate, m->ffn_up, L.down->awq, m->ffn_gate, MT, m->I_l, st));
             form = kTokensScaled;
         }
         IM_MARK(kCatFfn);
-        IM_TRY(gemm_affine_tc(L.down, m->ffn_gate, m->ffn_down, MT, m->xs_scratch, st, form));
+        IM_TRY(gemm_affine_tc(L.down, m->ffn_gate, m->ffn_down, MT, m->xs_scratch, st, form, true, &m->gemm_scratch));
         IM_MARK(kCatDown);
         IM_TRY(tp_allreduce(m, m->ffn_down, (size_t)MT * H, st));  // tensor parallel: down is row-split
         if (m->world > 1) IM_MARK(kCatComm);
@@ -563,7 +564,7 @@ int Model::forward(int nseq, int T, cudaStream_t st, Prof *prof, bool all_logits
             form = rc == IM_OK ? (qkv_rows ? kTokensPacked : kTokensScaled) : kTokensRaw;
             if (rc == IM_ERR_BOUNDS) rc = im_cuda_fused_residual_rms_norm(m->residual, m->ffn_down, Nx.input_ln, m->norm_out, m->hidden, H, MT, eps, st);
             IM_TRY(rc);
-            IM_TRY(gemm_affine_tc(Nx.qkv, m->norm_out, m->qkv, MT, m->xs_scratch, st, form));
+            IM_TRY(gemm_affine_tc(Nx.qkv, m->norm_out, m->qkv, MT, m->xs_scratch, st, form, true, &m->gemm_scratch));
             IM_MARK(kCatQkv);
         } else {
             IM_TRY(im_cuda_residual_add(m->residual, m->ffn_down, m->hidden, (size_t)MT * H, st));
@@ -578,7 +579,7 @@ int Model::forward(int nseq, int T, cudaStream_t st, Prof *prof, bool all_logits
         const bool fused4 = L.qkv->bits == 4 && L.gate->bits == 4 && L.up->bits == 4;
         if (l == 0) {
             IM_TRY(rows_planes(m->norm_out, L.qkv->awq, m->planes[0], MT, H, st));
-            IM_TRY(matvec_planes(L.qkv, nullptr, m->planes[0], nullptr, 0, m->qkv, MT, false, st));
+            IM_TRY(matvec_planes(L.qkv, nullptr, m->planes[0], nullptr, 0, m->qkv, MT, false, &m->gemm_scratch, st));
             IM_MARK(kCatQkv);
         }
         TqPrep a{};
@@ -593,16 +594,16 @@ int Model::forward(int nseq, int T, cudaStream_t st, Prof *prof, bool all_logits
         IM_TRY(attention_block(m, 1, a, m->qkv, L, nseq, T, attn_scale, attn_splits, slots, st));
         IM_MARK(kCatAttn);
         IM_TRY(rows_planes(m->attn_out, L.o->awq, m->planes[0], MT, m->q_dim, st));
-        IM_TRY(matvec_planes(L.o, nullptr, m->planes[0], nullptr, 0, m->ffn_down, MT, false, st));
+        IM_TRY(matvec_planes(L.o, nullptr, m->planes[0], nullptr, 0, m->ffn_down, MT, false, &m->gemm_scratch, st));
         IM_MARK(kCatOProj);
         IM_TRY(tp_allreduce(m, m->ffn_down, (size_t)MT * H, st));
         if (m->world > 1) IM_MARK(kCatComm);
         IM_TRY(norm_planes(m->hidden, m->ffn_down, L.post_ln, L.gate->awq, m->residual, nullptr, m->planes[0], H, MT, eps, st));
         IM_MARK(kCatResNorm);
-        IM_TRY(matvec_planes(L.gate, L.up, m->planes[0], nullptr, 0, m->ffn_gate, MT, !fused4, st));
+        IM_TRY(matvec_planes(L.gate, L.up, m->planes[0], nullptr, 0, m->ffn_gate, MT, !fused4, &m->gemm_scratch, st));
         IM_MARK(kCatFfn);
         IM_TRY(rows_planes(m->ffn_gate, L.down->awq, m->planes[0], MT, m->I_l, st));
-        IM_TRY(matvec_planes(L.down, nullptr, m->planes[0], nullptr, 0, m->ffn_down, MT, false, st));
+        IM_TRY(matvec_planes(L.down, nullptr, m->planes[0], nullptr, 0, m->ffn_down, MT, false, &m->gemm_scratch, st));
         IM_MARK(kCatDown);
         IM_TRY(tp_allreduce(m, m->ffn_down, (size_t)MT * H, st));
         if (m->world > 1) IM_MARK(kCatComm);
@@ -610,7 +611,7 @@ int Model::forward(int nseq, int T, cudaStream_t st, Prof *prof, bool all_logits
             Layer &Nx = m->layers[l + 1];
             const bool unrounded = Nx.qkv->bits == 4;  // Q's form; K and V read the rounded one
             IM_TRY(norm_planes(m->residual, m->ffn_down, Nx.input_ln, Nx.qkv->awq, m->hidden, unrounded ? m->planes[0] : nullptr, m->planes[1], H, MT, eps, st));
-            IM_TRY(matvec_planes(Nx.qkv, nullptr, unrounded ? m->planes[0] : m->planes[1], m->planes[1], m->q_dim, m->qkv, MT, false, st));
+            IM_TRY(matvec_planes(Nx.qkv, nullptr, unrounded ? m->planes[0] : m->planes[1], m->planes[1], m->q_dim, m->qkv, MT, false, &m->gemm_scratch, st));
             IM_MARK(kCatQkv);
         } else {
             IM_TRY(im_cuda_residual_add(m->residual, m->ffn_down, m->hidden, (size_t)MT * H, st));
@@ -836,6 +837,7 @@ int Model::alloc_logits_rows() {
 
 void Model::clear_step_error() {
     if (mega.bar) cudaMemset(mega.bar, 0, (size_t)(7 * cfg.num_layers + 1) * sizeof(unsigned));
+    if (gemm_scratch.counters) cudaMemset(gemm_scratch.counters, 0, (size_t)kSkMaxBlocks / 4 * sizeof(int));
 }
 
 int Model::hidden_rows(int rows, float *out_host) {
@@ -1273,6 +1275,9 @@ int Model::finalize() {
         if ((size_t)m->q_dim > kmax) kmax = (size_t)m->q_dim;
         IM_TRY(m->alloc((void **)&m->xs_scratch, MT * kmax * 2));
     }
+    IM_TRY(m->alloc((void **)&m->gemm_scratch.partial, kGemmScratchBytes));
+    IM_TRY(m->alloc((void **)&m->gemm_scratch.counters, (size_t)kSkMaxBlocks / 4 * sizeof(int)));
+    IM_CUDA_CHECK(cudaMemset(m->gemm_scratch.counters, 0, (size_t)kSkMaxBlocks / 4 * sizeof(int)));
     m->gemm_ok = true;
     for (Layer &L : m->layers)
         for (AffineWeight *w : {L.qkv, L.o, L.gate, L.up, L.down})

@@ -137,6 +137,26 @@ def test_scratch_that_shares_memory(dev, K, M, bits):
         assert H.rel_err(out.cpu().numpy(), want) <= TOL, at
 
 
+@pytest.mark.parametrize("N,K,M", [(19200, 1024, 24), (9600, 1024, 40), (256, 4096, 100)])
+def test_two_streams(dev, N, K, M):
+    # calls that keep nothing in the device handle: one beside another and beside a matvec, many row tiles and K slices of more than 64 tokens
+    from ironmill_b200 import ops
+    weights = [H.QWeight(N, K, seed=N + i, name="g2").gpu(dev) for i in range(2)]
+    xs = [torch.from_numpy(H.rng_for("g2-x", i).standard_normal((M, K)).astype(np.float16)).cuda() for i in range(2)]
+    want = [ops.matmul_affine(w, x) for w, x in zip(weights, xs)]
+    vec = ops.matvec_affine(weights[0], xs[0][:2])
+    streams = [torch.cuda.Stream() for _ in range(3)]
+    torch.cuda.synchronize()
+    got = [[], [], []]
+    for _ in range(40):
+        for i, st in enumerate(streams):
+            with torch.cuda.stream(st):
+                got[i].append(ops.matmul_affine(weights[i], xs[i]) if i < 2 else ops.matvec_affine(weights[0], xs[0][:2]))
+    torch.cuda.synchronize()
+    for i, ref in enumerate(want + [vec]):
+        assert all(torch.equal(y, ref) for y in got[i]), i
+
+
 @pytest.mark.parametrize("awq", [False, True])
 @pytest.mark.parametrize("K,M", [(1024, 5), (2048, 24), (1024, 48)])
 def test_few_tokens_anywhere(dev, K, M, awq):
