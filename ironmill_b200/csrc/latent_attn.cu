@@ -630,8 +630,15 @@ __global__ void __launch_bounds__(256) latent_out_kernel(const LatentArgs a, con
 // two row tiles by four quarters of the latent's columns.  A sum o' enters as three bf16 terms, which hold its 24 bits, so that every product is as exact
 // as the f32 one.  The rows of W_uv are requested before the predecessor has finished: a lane's 16-byte vectors are its fragments of two
 // k-steps.  16 tokens, 16 heads, 512 columns: 19.6 -> 9.4 us of a step.
-constexpr int kLoTok = 16, kLoRows = 32, kLoSteps = 8;  // steps of 32 columns that a warp holds in registers: latents of up to 1024 columns
+constexpr int kLoTok = 16, kLoRows = 32;
 inline size_t out_tc_smem(const LatentShape &s) { return (size_t)3 * kLoTok * (s.latP + 32) * 2 + (size_t)4 * kLoTok * (kLoRows + 1) * 4; }
+// A result by the definition: where a value, a weight or a sum is infinite, the terms' differences and products with zeros are NaN and it need not be.
+__device__ __noinline__ float latent_out_any(const __nv_bfloat16 *w, const float *x, float scale, int n) {
+    float sum = 0.0f;
+    for (int i = 0; i < n; i++) sum = fmaf(__bfloat162float(w[i]), x[i] * scale, sum);
+    return sum;
+}
+// STEPS: of 32 columns, which a warp holds in registers for its quarter (latents of up to 1024 columns: 8).
 template <int STEPS>
 __global__ void __launch_bounds__(256) latent_out_tc_kernel(const LatentArgs a, const LatentPart p, const float *__restrict__ src, int normalised, int M) {
     typedef __nv_bfloat16 T;
@@ -697,6 +704,8 @@ __global__ void __launch_bounds__(256) latent_out_tc_kernel(const LatentArgs a, 
         float sum = 0.0f;
 #pragma unroll
         for (int k = 0; k < 4; k++) sum += red[(k * kLoTok + b) * (kLoRows + 1) + v];
+        if (!isfinite(sum))
+            sum = latent_out_any(static_cast<const T *>(a.ukv) + ((size_t)h * (s.dimP + s.vP) + s.dimP + v0 + v) * a.uk_ld, src + ((size_t)(m0 + b) * s.heads + h) * s.latP, scale[b], s.latP);
         static_cast<T *>(a.out)[(size_t)(m0 + b) * a.ldo + h * s.vP + v0 + v] = from_f<T>(sum);
     }
 }
