@@ -505,28 +505,39 @@ int Model::forward(int nseq, int T, cudaStream_t st, Prof *prof, bool all_logits
         IM_TRY(tp_allreduce(m, m->ffn_down, (size_t)H, st));  // tensor parallel: the last layer's down projection
         IM_TRY(im_cuda_residual_add(m->residual, m->ffn_down, m->hidden, (size_t)H, st));
     }
-    // More than one token per sequence is the reference's prefill form (its matmul kernels round x / awq and the
-    // dequantised weights to fp16: affine_matmul.metal:44-74), whatever the count; so are decode batches of 16 and more.
-    const bool gemm = !mega && m->gemm_ok && (T > 1 || MT >= kGemmMinTokens);
-    for (int l = 0; l < c.num_layers && gemm; l++) {
-        // Dense contraction (prefill chunks, large decode batches): every projection is one tcgen05 GEMM; norms, SiLU
-        // and the residual adds are separate element-wise launches (their bytes are a rounding error next to the GEMMs).
-        Layer &L = m->layers[l];
-        if (l == 0) {
-            IM_TRY(gemm_affine_tc(L.qkv, m->norm_out, m->qkv, MT, m->xs_scratch, st, kTokensRaw, true, &m->gemm_scratch));
-            IM_MARK(kCatQkv);
-        }
+    // (QK-norm +) RoPE, K/V cache write and query rotation of a layer in one launch, then its attention; joint: from rows of Q | K | V, else from Q and K | V
+    auto attention = [&](Layer &L, bool joint) -> int {
         TqPrep a{};
-        a.qkv = m->qkv; a.stride = m->qkv_dim; a.k_off = m->q_dim; a.v_off = m->q_dim + m->kv_dim;
+        if (joint) {
+            a.qkv = m->qkv; a.stride = m->qkv_dim; a.k_off = m->q_dim; a.v_off = m->q_dim + m->kv_dim;
+        } else {
+            a.qkv = m->q_d; a.stride = m->q_dim; a.kv = m->k_d; a.kv_stride = 2 * m->kv_dim; a.k_off = 0; a.v_off = m->kv_dim;
+        }
         a.qw = L.q_norm; a.kw = L.k_norm; a.cosc = m->cosc; a.sinc = m->sinc;
         a.nh = m->nh_l; a.nkv = m->nkv_l; a.rotary_dim = c.rotary_dim ? c.rotary_dim : hd; a.with_norm = c.qk_norm ? 1 : 0;
         a.T = T; a.nseq = nseq; a.max_seq = c.max_seq_len; a.base_pos = 0; a.eps = eps; a.pos_dev = m->pos_dev; a.slot_map = slots;
         a.qrot = m->qrot; a.q_out = nullptr;
         a.kc = L.kc; a.vc = L.vc; a.ks = L.ks; a.vs = L.vs; a.krn = L.krn;
-        IM_TRY(attention_block(m, 0, a, m->qkv, L, nseq, T, attn_scale, attn_splits, slots, st));
+        __half *const q = joint ? m->qkv : m->q_d;
+        IM_TRY(attention_block(m, 0, a, q, L, nseq, T, attn_scale, attn_splits, slots, st));
         IM_MARK(kCatKvWrite);
-        IM_TRY(attention_block(m, 1, a, m->qkv, L, nseq, T, attn_scale, attn_splits, slots, st));
+        IM_TRY(attention_block(m, 1, a, q, L, nseq, T, attn_scale, attn_splits, slots, st));
         IM_MARK(kCatAttn);
+        return IM_OK;
+    };
+    // More than one token per sequence is the reference's prefill form (its matmul kernels round x / awq and the
+    // dequantised weights to fp16: affine_matmul.metal:44-74), whatever the count; so are decode batches of 16 and more.
+    const bool gemm = !mega && m->gemm_ok && (T > 1 || MT >= kGemmMinTokens);
+    for (int l = 0; l < c.num_layers && gemm; l++) {
+        // Dense contraction (prefill chunks, large decode batches): every projection is one GEMM, for few tokens on mma.sync (gemm_rows.cu), else on
+        // tcgen05 (gemm_tc.cu, gemm_pair.cu); norms, SiLU and the residual adds are separate element-wise launches (their bytes are a rounding error next
+        // to the GEMMs).
+        Layer &L = m->layers[l];
+        if (l == 0) {
+            IM_TRY(gemm_affine_tc(L.qkv, m->norm_out, m->qkv, MT, m->xs_scratch, st, kTokensRaw, true, &m->gemm_scratch));
+            IM_MARK(kCatQkv);
+        }
+        IM_TRY(attention(L, true));
         IM_TRY(gemm_affine_tc(L.o, m->attn_out, m->ffn_down, MT, m->xs_scratch, st, kTokensRaw, true, &m->gemm_scratch));
         IM_MARK(kCatOProj);
         IM_TRY(tp_allreduce(m, m->ffn_down, (size_t)MT * H, st));  // tensor parallel: o is row-split
@@ -582,17 +593,7 @@ int Model::forward(int nseq, int T, cudaStream_t st, Prof *prof, bool all_logits
             IM_TRY(matvec_planes(L.qkv, nullptr, m->planes[0], nullptr, 0, m->qkv, MT, false, &m->gemm_scratch, st));
             IM_MARK(kCatQkv);
         }
-        TqPrep a{};
-        a.qkv = m->qkv; a.stride = m->qkv_dim; a.k_off = m->q_dim; a.v_off = m->q_dim + m->kv_dim;
-        a.qw = L.q_norm; a.kw = L.k_norm; a.cosc = m->cosc; a.sinc = m->sinc;
-        a.nh = m->nh_l; a.nkv = m->nkv_l; a.rotary_dim = c.rotary_dim ? c.rotary_dim : hd; a.with_norm = c.qk_norm ? 1 : 0;
-        a.T = T; a.nseq = nseq; a.max_seq = c.max_seq_len; a.base_pos = 0; a.eps = eps; a.pos_dev = m->pos_dev; a.slot_map = slots;
-        a.qrot = m->qrot; a.q_out = nullptr;
-        a.kc = L.kc; a.vc = L.vc; a.ks = L.ks; a.vs = L.vs; a.krn = L.krn;
-        IM_TRY(attention_block(m, 0, a, m->qkv, L, nseq, T, attn_scale, attn_splits, slots, st));
-        IM_MARK(kCatKvWrite);
-        IM_TRY(attention_block(m, 1, a, m->qkv, L, nseq, T, attn_scale, attn_splits, slots, st));
-        IM_MARK(kCatAttn);
+        IM_TRY(attention(L, true));
         IM_TRY(rows_planes(m->attn_out, L.o->awq, m->planes[0], MT, m->q_dim, st));
         IM_TRY(matvec_planes(L.o, nullptr, m->planes[0], nullptr, 0, m->ffn_down, MT, false, &m->gemm_scratch, st));
         IM_MARK(kCatOProj);
@@ -631,18 +632,7 @@ int Model::forward(int nseq, int T, cudaStream_t st, Prof *prof, bool all_logits
             IM_TRY(im_cuda_matvec_affine(static_cast<const im_affine_weight *>(&L.kv_rows), m->norm_out, m->k_d, MT, st));
             IM_MARK(kCatQkv);
         }
-        // (QK-norm +) RoPE, K/V cache write and query rotation in one launch, then split attention + reduce
-        TqPrep a{};
-        a.qkv = m->q_d; a.stride = m->q_dim; a.kv = m->k_d; a.kv_stride = 2 * m->kv_dim; a.k_off = 0; a.v_off = m->kv_dim;
-        a.qw = L.q_norm; a.kw = L.k_norm; a.cosc = m->cosc; a.sinc = m->sinc;
-        a.nh = m->nh_l; a.nkv = m->nkv_l; a.rotary_dim = c.rotary_dim ? c.rotary_dim : hd; a.with_norm = c.qk_norm ? 1 : 0;
-        a.T = T; a.nseq = nseq; a.max_seq = c.max_seq_len; a.base_pos = 0; a.eps = eps; a.pos_dev = m->pos_dev; a.slot_map = slots;
-        a.qrot = m->qrot; a.q_out = nullptr;
-        a.kc = L.kc; a.vc = L.vc; a.ks = L.ks; a.vs = L.vs; a.krn = L.krn;
-        IM_TRY(attention_block(m, 0, a, m->q_d, L, nseq, T, attn_scale, attn_splits, slots, st));
-        IM_MARK(kCatKvWrite);
-        IM_TRY(attention_block(m, 1, a, m->q_d, L, nseq, T, attn_scale, attn_splits, slots, st));
-        IM_MARK(kCatAttn);
+        IM_TRY(attention(L, false));
         IM_TRY(im_cuda_matvec_affine(static_cast<im_affine_weight *>(L.o), m->attn_out, m->ffn_down, MT, st));
         IM_MARK(kCatOProj);
         IM_TRY(tp_allreduce(m, m->ffn_down, (size_t)MT * H, st));
