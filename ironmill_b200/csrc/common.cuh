@@ -120,7 +120,7 @@ struct V2Params {
     int *err;
 };
 
-// INT4 g128 GEMM on tcgen05 / TMEM (gemm_tc.cu): y[M, N] = f16(x / awq) * dequant(w)^T; xs_scratch holds M * K halves.
+// INT4 or INT8 g128 GEMM on the tensor cores (gemm_tc.cu; few tokens gemm_rows.cu, many gemm_pair.cu): y[M, N] = f16(x / awq) * dequant(w)^T; xs_scratch holds M * K halves.
 // IM_ERR_BOUNDS when the weight is not INT4 or INT8 group-128.  pack: the scratch is 16-byte aligned and shares no memory with x and y.
 // own: where partial sums may go; without it (the stand-alone call, on any stream) only up to 64 tokens over few rows are cut along K, in the device handle's scratch.
 enum TokenForm { kTokensRaw, kTokensScaled, kTokensPacked };  // x as it is; f16(x / awq); that, packed for gemm_rows.cu (where gemm_rows_takes says so)

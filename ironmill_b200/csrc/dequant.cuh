@@ -15,7 +15,9 @@ __device__ __forceinline__ __half2 place_codes(uint32_t v, uint32_t m, uint32_t 
     asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(d) : "r"(v), "r"(m), "r"(e));
     return *reinterpret_cast<__half2 *>(&d);
 }
-// (scale, zero) of a row and group for the conversions below: c = 1024 + z, d = -(64 + z).  0x6400 | q is the fp16 number 1024 + q, 0x6400 | 16 q the number
+// The conversions below are the published ones of mixed-precision GEMMs: a code in the mantissa of an fp16 exponent (Kim et al., "Who Says Elephants Can't
+// Run", 2022), the upper nibble brought down by an fma (Frantar et al., MARLIN, 2024); here with zero points and the exactness that they leave.
+// (scale, zero) of a row and group for them: c = 1024 + z, d = -(64 + z).  0x6400 | q is the fp16 number 1024 + q, 0x6400 | 16 q the number
 // 1024 + 16 q; where z is a whole or half number of at most 512 (plain), q - z = (1024 + q) - c = (1024 + 16 q) / 16 + d is exact for every code,
 // and the product with s is rounded once.
 struct GroupScale {

@@ -254,7 +254,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PairShape<TN, BITS>:
         if constexpr (BITS != 0) ok = weight_warps<TN, BITS>(p, As, full, empty, rank, pair, npairs);
     } else if (warp == kCopyWarp) {
         if (lane == 0) {
-            const uint32_t full0 = leader_addr(full), e = half_exponent();
+            const uint32_t full0 = leader_addr(full);
             int s = 0, use = 0;
             for (int w = pair; w < tiles; w += npairs) {
                 const int m0 = w % p.mtiles * TN + rank * (TN / 2), n0 = w / p.mtiles * (2 * kPRows) + rank * kPRows;

@@ -872,7 +872,7 @@ IM_EXPORT int im_cuda_matvec_f16(const void *w_dev, const void *x_dev, void *y_d
 }
 
 // superblock_matmul_int4 (crates/ironmill-inference/src/metal/shaders/quantized/affine_matmul.metal:10-152) on the
-// tcgen05 tensor cores (gemm_tc.cu).  INT4 group-128 weights only.
+// tensor cores (gemm_tc.cu; few tokens gemm_rows.cu).  INT4 or INT8 group-128 weights only.
 IM_EXPORT int im_cuda_matmul_affine(const im_affine_weight *w, const void *x_dev, void *y_dev, int M, void *scratch_dev, void *stream) {
     IM_GUARD_BEGIN
     using namespace im;

@@ -179,7 +179,7 @@ def silu_mul(gate: torch.Tensor, up: torch.Tensor, out: torch.Tensor | None = No
 
 
 def matmul_affine(w: AffineWeight, x: torch.Tensor, out: torch.Tensor | None = None, scratch: torch.Tensor | None = None) -> torch.Tensor:
-    """Dense INT4 g128 GEMM on the tcgen05 tensor cores: y[M, N] = f16(x / awq) @ dequant(w)^T.  scratch: M * K halves."""
+    """Dense INT4 or INT8 g128 GEMM on the tensor cores (tcgen05; few tokens mma.sync): y[M, N] = f16(x / awq) @ dequant(w)^T.  scratch: M * K halves."""
     M = _rows(x, w.K)
     y = out if out is not None else torch.empty((M, w.N), dtype=torch.float16, device=x.device)
     if scratch is None:

@@ -33,9 +33,13 @@ def test_few_tokens(dev, N, K, M, bits):
     w = qw.gpu(dev)
     x = (H.rng_for("gr-x", M).standard_normal((M, K))).astype(np.float16)
     ref = orc.matmul_affine(qw.packed, qw.scales_f16, qw.zps_f16, x, N, K, 128, bits, awq=qw.awq, threads=8)
-    for _ in range(2):  # the counters of cut tiles are back at zero after a launch
+    far = np.zeros(N, dtype=bool)  # rows with a far zero point, whose results are a hundred times the others'
+    far[np.nonzero(np.abs(qw.zps.reshape(N, -1)) > 500)[0]] = True
+    assert far.any() and not far.all()
+    for _ in range(2):
         y = ops.matmul_affine(w, torch.from_numpy(x).cuda()).cpu().numpy()
-        assert H.rel_err(y, ref) <= TOL, (N, K, M)
+        for part in (far, ~far):
+            assert H.rel_err(y[:, part], ref[:, part]) <= TOL, (N, K, M)
 
 
 @pytest.mark.parametrize("N,K,M", [(512, 2048, 65), (384, 1792, 128), (260, 14336, 100), (6144, 1024, 97)])
@@ -84,6 +88,43 @@ def test_prompt_whose_down_projection_is_another_kernel(bits, chunk):
         eng.load_weights(DictProvider(cfg, tensors))
         out.append(eng.prefill(tokens).astype(np.float64))
     assert np.linalg.norm(out[1] - out[0]) / np.linalg.norm(out[0]) <= 3.6e-3
+
+
+@pytest.mark.parametrize("bits,batch,chunk", [(4, 3, 24), (8, 9, 13), (4, 15, 48)])
+def test_row_tiles_cut_by_shares(bits, batch, chunk):
+    """Gate and up of more row tiles than SMs over a sum long enough for equal shares: tiles cut by CTA boundaries, launch after launch (the counters are back
+    at zero).  A prompt in portions against the prompt at once, then steps over byte planes against the oracle model of the first sequences."""
+    from ironmill_b200.engine import CudaConfig, CudaInference
+    from tests.oracle_model import OracleModel
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    H_, tiles = 2048, sms + 4
+    ff = tiles * 64 // 128 * 128  # a joint tile: 64 rows of each
+    assert ff // 64 > sms and 2 * (H_ // 128) > (ff // 64) * (H_ // 128) / sms + 13
+    cfg = _cfg("llama", 1, H_, ff, 8, 4, 200, 1e6, 1e-6)
+    tensors = synth_model(cfg, seed=45, awq=True, bits=bits)
+    tqc = orc.TqConstants(128, 8, seed=4)
+    rng = H.rng_for("cut")
+    prompt = rng.integers(0, 200, 2 * chunk).astype(np.uint32)
+    prompts = [rng.integers(0, 200, 2 + i % 3).astype(np.uint32) for i in range(batch)]
+    out = []
+    for c in (2 * chunk, chunk):
+        conf = CudaConfig(max_seq_len=128, max_batch=1, prefill_chunk_size=c)
+        conf.without_turboquant()
+        eng = CudaInference(conf)
+        eng.load_weights(DictProvider(cfg, tensors))
+        out.append(eng.prefill(prompt).astype(np.float64))
+    assert np.linalg.norm(out[1] - out[0]) / np.linalg.norm(out[0]) <= 3.6e-3  # as test_prompt_in_short_portions
+    eng = CudaInference(CudaConfig(max_seq_len=128, max_batch=batch, n_bits=8))
+    eng.load_weights(DictProvider(cfg, tensors), tq_signs=tqc.signs, tq_qjl=tqc.qjl)
+    ids = [eng.add_sequence(p) for p in prompts]
+    refs = [OracleModel(cfg, tensors, tqc, 128) for _ in prompts[:2]]
+    for ref, p in zip(refs, prompts):
+        ref.forward(p)
+    for _ in range(3):
+        fed = rng.integers(0, 200, batch)
+        got = eng.batch_decode_step(dict(zip(ids, fed.tolist())))
+        for i, ref in enumerate(refs):
+            assert float(np.abs(got[i][1] - ref.forward([int(fed[i])])).max()) <= 5e-2, (bits, batch, i)
 
 
 @pytest.mark.parametrize("bits,awq,batch", [(4, True, 1), (4, True, 2), (4, False, 3), (8, True, 5), (4, True, 9), (8, False, 15)])
