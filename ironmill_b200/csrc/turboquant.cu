@@ -505,7 +505,7 @@ __global__ void __launch_bounds__(kTcWarps * 32, 2) tq_attention_tc_kernel(const
             longest = __reduce_max_sync(0xffffffffu, longest);
             if (lane == 0) {
                 plan.tiles[0] = plan.parts[0] = 0;
-                // tiles of a share: a context of L tiles touches at most (L - 1) / least + 2 shares
+                // least tiles of a share: a context of L tiles touches at most 1 + ceil((L - 1) / least) shares, a part in each
                 const int least = max((most + p.splits - 2) / (p.splits - 1), 1), ctas = max(min((int)gridDim.x, total / least), 1), share = total / ctas,
                           mean = total / (int)gridDim.x;
                 plan.ctas = ctas;
